@@ -35,7 +35,8 @@ void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_slot
                  cudaStream_t st);
 void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long long total,
                             const uint32_t* order, unsigned long long* counter, uint32_t* err,
-                            unsigned long long* stats, unsigned blocks, unsigned threads, cudaStream_t st);
+                            unsigned long long* stats, unsigned blocks, unsigned threads, cudaStream_t st,
+                            bool walk);
 void launch_photon_sort(const TileDesc* tiles_dev, int ntiles, unsigned long long total, unsigned long long ncells,
                         uint32_t* cnt, const uint32_t* off, uint32_t* cur, uint32_t* order, uint32_t* err,
                         cudaStream_t st);
@@ -101,24 +102,6 @@ __global__ void k_scan_tree_tiles(const BTile* bt, int ntiles, const uint32_t* d
   rt[t].order = devlist + first;
   rt[t].obase = bt[t].cbase;
   rt[t].n = last - first;
-}
-
-// Crystal records of every tile in its tree's element order (TileDesc): position p of tile t holds
-// the crystal ridx[p] of that tile, so a leaf's crystals lie next to each other.
-__global__ void k_element_records_b(const BTile* __restrict__ bt, int ntiles, unsigned long long ncap,
-                                    const uint32_t* __restrict__ ridx, const float4* __restrict__ A,
-                                    const float4* __restrict__ Q, const float4* __restrict__ D, float4* EA,
-                                    float4* EQ, float4* ED, uint32_t* err) {
-  const unsigned long long g = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-  if (g >= ncap) return;
-  const BTile& t = bt[btile_of(bt, ntiles, g)];
-  const unsigned long long p = g - t.cbase;
-  if (p >= t.n) return;
-  const uint32_t s = ridx[g];
-  if (!index_ok(s < t.n, err, SITE_LEAF, s, t.n)) return;
-  EA[g] = A[t.cbase + s];
-  EQ[g] = Q[t.cbase + s];
-  ED[g] = D[t.cbase + s];
 }
 
 // ---- development (development.rs:59-188), batched; see fg_develop.cu for the reasoning ----
@@ -342,7 +325,7 @@ struct fg_batch {
   bool wait_probe = false;
   unsigned long long maxcells = 0, maxslots = 0;  // the largest tile's cells and bricks
   DBuf<float4> A, Q, D;
-  DBuf<float4> EA, EQ, ED;  // A, Q, D in the transport tree's element order (TileDesc)
+  CellBufs tcells;          // the crystals in cells, with their rank in the tree's walk order
   DBuf<uint64_t> keys;
   RTreeBufs rt;             // the reference tree of every tile: over its crystals, then its developed ones
   DBuf<RTile> rt_scan;      // the tree tiles of the scan's build (developed crystals, their expansion)
@@ -382,6 +365,14 @@ struct fg_batch {
 };
 
 namespace fg {
+
+// Largest half-dimension the synthesis can give a crystal (emulsion.rs:162-184: the radius clamp,
+// and the thickness of tabular crystals).
+static double synth_max_half_dim(const fg_tile_params& p) {
+  const double r = 0.48 * p.r_min, ar = p.tabular_aspect_ratio;
+  if (p.morphology != FG_TABULAR) return r;
+  return std::max(r, ar >= 0.0 ? std::max(r / ar, 0.05) : 0.05);
+}
 
 static void derive_tile(const fg_tile_params& p, SynthTile& s, TileDesc& t, ScanTile& c, BTile& b) {
   FG_REQUIRE(p.film_w > 0 && p.film_h > 0 && p.film_d > 0, "film dimensions must be positive");
@@ -453,6 +444,9 @@ static void derive_tile(const fg_tile_params& p, SynthTile& s, TileDesc& t, Scan
   t.theta_max = static_cast<float>(p.illumination_angle_rad);
   t.alpha = static_cast<float>(p.crystal_absorption_coeff);
   t.max_bounces = p.max_bounces;
+  t.cells = CellGrid{};
+  FG_REQUIRE(cells_layout(W, H, Dd, bridson_density(W, H, Dd, r) * vol, t.cells), "film dimensions must be finite");
+  cells_reach(t.cells, synth_max_half_dim(p), p.morphology == FG_CUBIC);
   c = ScanTile{};
   const uint32_t spp = std::max<uint32_t>(p.samples_per_pixel, 1);
   const uint32_t g = static_cast<uint32_t>(std::lround(std::sqrt(static_cast<double>(spp))));
@@ -508,13 +502,10 @@ static void upload_descriptors(fg_batch* B, cudaStream_t st) {
   for (uint32_t i = 0; i < B->ntiles; ++i) {
     const unsigned long long cb = B->syn[i].cbase;
     TileDesc& t = B->td[i];
-    t.a = B->EA.p + cb;
-    t.q = B->EQ.p + cb;
-    t.d = B->ED.p + cb;
     const unsigned long long nb = B->bt[i].nbase;
-    t.rnode = B->rt.rnode.p + B->bt[i].rbase;
-    t.rleaf = B->rt.rleaf.p + nb;
-    t.ridx = B->rt.ridx.p + cb;
+    t.cbase = cb;
+    t.nbase = nb;
+    B->tcells.attach(t.cells, cb);
     t.s2id = nullptr;
     t.counts = B->counts.p + cb;
     t.tile = B->exposure.p + B->exp_off[i];
@@ -576,20 +567,21 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
   FG_CUDA(cudaGetLastError());
 }
 
-// The reference tree of every tile over its crystals (in slot order), for the transport and the
-// development's touch queries.
+// The reference tree of every tile over its crystals (in slot order), for the development's touch
+// queries and the walk order of the transport's hits, and the crystals in cells.
 static void stage_bvh(fg_batch* B, cudaStream_t st) {
   rtree_build(B->rt, B->e->d_err, st);
-  k_element_records_b<<<grid_for(B->ncap, 256), 256, 0, st>>>(B->d_bt.p, static_cast<int>(B->ntiles), B->ncap,
-                                                              B->rt.ridx.p, B->A.p, B->Q.p, B->D.p, B->EA.p,
-                                                              B->EQ.p, B->ED.p, B->e->d_err);
-  FG_CUDA(cudaGetLastError());
+  const int nt = static_cast<int>(B->ntiles);
+  FG_CUDA(cudaMemsetAsync(B->tcells.cnt.p, 0, (B->tcells.ncells + 1) * sizeof(uint32_t), st));
+  launch_cells_count(B->d_td.p, nt, B->ncap, B->A.p, B->tcells.cnt.p, B->tcells.place.p, st);
+  cub_scan(B, B->tcells.cnt.p, B->tcells.off.p, B->tcells.ncells + 1, st);
+  launch_cells_fill(B->d_td.p, nt, B->ncap, B->A.p, B->Q.p, B->D.p, B->rt, B->tcells, B->e->d_err, st);
 }
 
 static void stage_transport(fg_batch* B, cudaStream_t st) {
   FG_CUDA(cudaMemsetAsync(B->counts.p, 0, B->ncap * sizeof(uint32_t), st));
   launch_transport_shape(B->d_td.p, static_cast<int>(B->ntiles), B->photons, B->porder.p, B->counter.p,
-                         B->e->d_err, B->dstats.p, B->tr_blocks, B->tr_threads, st);
+                         B->e->d_err, B->dstats.p, B->tr_blocks, B->tr_threads, st, false);
 }
 
 // Orders photon ids by emission cell (independent of the crystals: runs with synthesis).
@@ -809,9 +801,6 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   B->A.alloc(std::max<unsigned long long>(cap, 1), st);
   B->Q.alloc(std::max<unsigned long long>(cap, 1), st);
   B->D.alloc(std::max<unsigned long long>(cap, 1), st);
-  B->EA.alloc(std::max<unsigned long long>(cap, 1), st);
-  B->EQ.alloc(std::max<unsigned long long>(cap, 1), st);
-  B->ED.alloc(std::max<unsigned long long>(cap, 1), st);
   B->keys.alloc(std::max<unsigned long long>(cap, 1), st);
   B->parent.alloc(std::max<unsigned long long>(cap, 1), st);
   B->counts.alloc(std::max<unsigned long long>(cap, 1), st);
@@ -831,7 +820,7 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       // The synthesis's radius clamp (emulsion.rs:162-170) for cubes; the other shapes lie in their boxes.
       t.reach = rt_reach(B->params[i].morphology == FG_CUBIC ? 0.48 * B->params[i].r_min : 0.0);
     }
-    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC);
+    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC, 0, true);
     for (uint32_t i = 0; i < n; ++i) {
       FG_REQUIRE(rt[i].ebase == B->syn[i].cbase, "tree layout differs from the crystal slots");
       B->bt[i].nbase = rt[i].nbase;
@@ -839,13 +828,20 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       B->bt[i].rbase = rt[i].rbase;
       B->bt[i].rcap = rt[i].rcap;
       B->td[i].nnodes = rt[i].ncap;
-      B->td[i].nrec = rt[i].rcap;
       B->td[i].reach = rt[i].reach;
       rs[i] = rt[i];
       rs[i].exp64 = B->exp64.p + B->syn[i].cbase;
     }
     B->rt_scan.alloc(n, st);
     FG_CUDA(cudaMemcpyAsync(B->rt_scan.p, rs.data(), n * sizeof(RTile), cudaMemcpyHostToDevice, st));
+  }
+  {
+    unsigned long long cells = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+      B->td[i].cells.cell_base = cells;
+      cells += cells_of(B->td[i].cells);
+    }
+    B->tcells.alloc(cap, cells, st);
   }
   B->prep.alloc(std::max<unsigned long long>(cap, 1), st);
   B->devflag.alloc(cap + 1, st);
@@ -873,7 +869,10 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   FG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b3, B->pcnt.p, B->poff.p, static_cast<int64_t>(B->npcells + 1), st));
   size_t b4 = 0;
   FG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b4, B->devflag.p, B->devscan.p, static_cast<int64_t>(cap + 1), st));
-  B->cub_bytes = std::max(std::max(b1, b2), std::max(b3, b4));
+  size_t b5 = 0;
+  FG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b5, B->tcells.cnt.p, B->tcells.off.p,
+                                        static_cast<int64_t>(B->tcells.ncells + 1), st));
+  B->cub_bytes = std::max(std::max(std::max(b1, b2), std::max(b3, b4)), b5);
   B->cub_tmp.alloc(std::max<size_t>(B->cub_bytes, 1), st);
   for (auto& x : B->ev) FG_CUDA(cudaEventCreate(&x));
   layout_bins(B, bin0);
@@ -907,11 +906,11 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   uint32_t bits = 0;
   while ((1u << bits) < static_cast<uint32_t>(std::ceil(side))) ++bits;
   const unsigned long long px = static_cast<unsigned long long>(p.width_px) * p.height_px;
-  // Per crystal slot: records 48 (and 48 in the tree's element order), key 8, links and flags 36, expansion 8, scan prep 160, bin
-  // entries 32, tree elements 88 (order, node of, two copies of three 8-byte keys, flags, prefix
-  // sums, ranks, final order, leaf of) and 0.8 nodes of 224 B (plus slack); cells 4 B; bricks
-  // 8 B; photon order; images.
-  return static_cast<unsigned long long>(s.ccap) * 628ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
+  // Per crystal slot: records 48 (and 96 in the transport's cells), key 8, links and flags 36,
+  // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
+  // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
+  // 224 B (plus slack); transport cells 8 B; synthesis cells 4 B; bricks 8 B; photon order; images.
+  return static_cast<unsigned long long>(s.ccap) * 680ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          (8ull << (2 * s.slot_bits)) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
@@ -984,7 +983,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     em->stream = st;
     em->has64 = false;
     em->extent = std::max(std::max(cfg->width, cfg->height), cfg->depth);
-    em->max_half_dim = 0.48 * cfg->r_min;  // the radius clamp of the synthesis (emulsion.rs:162-170)
+    em->max_half_dim = synth_max_half_dim(p);
     em->any_cubic = cfg->morphology == FG_CUBIC;
     em->a = std::move(A);
     em->q = std::move(Q);
@@ -992,6 +991,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     alloc_state(em.get(), st);
     DBuf<uint32_t> none;
     build_emulsion_tree(e, em.get(), false, em->rt, none);
+    build_emulsion_cells(e, em.get());
     FG_CUDA(cudaEventRecord(e->timer.ev[1], st));
     FG_CUDA(cudaStreamSynchronize(st));
     e->timings.synth_ms = elapsed(e->timer.ev[0], e->timer.ev[1]);
@@ -1165,10 +1165,10 @@ fg_status fg_batch_wait(fg_batch* b, fg_batch_stats* stats) {
     s.graph = b->exec ? 1u : 0u;
     // Own kernels per run: Bridson (all colour classes in one launch; it also counts the points), thin +
     // brick counts, emit, set_n, photon order x2, transport, maxdim + threshold + developed list + link +
-    // roots + finalize, scan-tree inputs, scan prep, two bin passes, scan, density, the crystal records in
-    // the transport tree's order, and the two tree builds (each level's launches included, also those that
+    // roots + finalize, scan-tree inputs, scan prep, two bin passes, scan, density, the two passes over the
+    // transport's cells, and the two tree builds (each level's launches included, also those that
     // find no work; CUB scans not counted).
-    s.kernel_launches = 1 + 2 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 1 + 2 * rtree_kernel_launches(b->rt);
+    s.kernel_launches = 1 + 2 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt);
     b->stats = s;
     if (stats) *stats = s;
   });

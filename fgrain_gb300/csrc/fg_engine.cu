@@ -246,6 +246,7 @@ fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_
       FG_CUDA(cudaStreamSynchronize(st));
       DBuf<uint32_t> none;
       build_emulsion_tree(e, em.get(), false, em->rt, none);
+      build_emulsion_cells(e, em.get());
     } else {
       alloc_state(em.get(), st);
     }

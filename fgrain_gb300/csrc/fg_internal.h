@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/fgrain_cuda.h"
+#include "fg_cells.cuh"
 #include "fg_device.cuh"
 #include "fg_rtree.cuh"
 
@@ -143,6 +144,18 @@ struct RTreeBufs {
   DBuf<Node4> rnode;              // four-wide walk records (tile-local refs)
   DBuf<uint2> rleaf;              // leaf: first element (tile-local position), count
   DBuf<uint32_t> leafof;          // optional: leaf id of each element slot
+  DBuf<uint32_t> rank;            // optional: place of each element slot in the reference walk's order
+};
+
+// fg_cells.cu: the crystals of a batch's tiles (or one emulsion) in cells (CellGrid).
+struct CellBufs {
+  unsigned long long ncells = 0;
+  DBuf<uint32_t> cnt, off, place;  // per cell: crystals, first position; per slot: number in its cell
+  DBuf<float4> pos, q, d, leaf;
+  DBuf<uint2> by_rank;
+  void alloc(unsigned long long ncap, unsigned long long cells, cudaStream_t st);
+  // Sets the pointers of one tile's grid (cell_base set, first crystal slot cbase).
+  void attach(CellGrid& g, unsigned long long cbase) const;
 };
 }  // namespace fg
 
@@ -171,6 +184,10 @@ struct fg_emulsion {
   // The reference tree over all crystals in id order (the transport walks, the development's
   // radius queries).
   fg::RTreeBufs rt;
+  // The crystals in cells for the transport and the touch queries; grid.x.n is 0 for sets that stay
+  // on the tree walk (cells_suit).
+  fg::CellBufs cells;
+  fg::CellGrid grid{};
   // Mutable per-crystal state (Morton order).
   fg::DBuf<uint32_t> counts;
   fg::DBuf<uint8_t> developed;
@@ -206,14 +223,18 @@ void gather_sorted(fg_emulsion* em, const uint32_t* order, const double* pos, co
                    const double* quat, const double* sens, const int32_t* morph, int32_t morph_all,
                    cudaStream_t st);
 
+// fg_cells.cu, fg_transport.cu: the emulsion's cells, when they suit its crystals (after its tree).
+void build_emulsion_cells(fg_engine* e, fg_emulsion* em);
+
 // Sets RTile::ebase / nbase / ncap from ecap, copies the tiles to the device and allocates.  The
 // caller fills the source pointers and ecap of each tile, and RTile::n (and order) on the device
 // before each build.
 // Each tile gets min(ecap + 2, node_frac * ecap + 64) nodes (the reference tree has about 0.67
 // nodes per element; running out fails the build with the list-overflow error bit).
 // leafof (when wanted) gets max(elements, leafof_slots) words: it is indexed by element slot.
+// rank (when wanted) gets as many.
 void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cudaStream_t st, double node_frac = 1.0,
-                 size_t leafof_slots = 0);
+                 size_t leafof_slots = 0, bool want_rank = false);
 // Enqueues a build (capturable: no host synchronisation).  tiles_dev (optional) replaces the tile
 // array of the allocation by one with the same layout (ebase, nbase, ecap, ncap) but other element
 // sources, so that one set of buffers serves several trees in turn.

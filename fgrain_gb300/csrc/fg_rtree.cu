@@ -879,12 +879,14 @@ __global__ void k_rt_refit(RtArgs A, uint32_t* arrive) {
   }
 }
 
-// Walk records (fg_rtree.cuh): one thread per node.  A leaf fills its element range and the
-// leaf-of map; the root and every internal node at odd depth write their four-wide record, the
+// Walk records (fg_rtree.cuh): one thread per node.  A leaf fills its element range, the leaf-of
+// map and its elements' ranks (the walk takes the right subtree first, so leaves in descending
+// element position, and a leaf's elements in index order); the root and every internal node at odd depth write their four-wide record, the
 // grandchildren in the reference's visiting order (right before left, a leaf child in one slot).
 // An internal slot's box is rounded outward, padded and extended by the reach; a leaf slot's box
 // is rounded to nearest.
-__global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafof, unsigned long long leafof_n) {
+__global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafof, unsigned long long leafof_n,
+                             uint32_t* rank) {
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   for (unsigned long long g = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; g < A.N;
        g += stride) {
@@ -933,7 +935,12 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
       if (leafof)
         for (uint32_t k = 0; k < cn; ++k) {
           const uint32_t slot = A.ridx[st + k];
-          if (T.ebase + slot < leafof_n) leafof[T.ebase + slot] = id; else atomicOr(A.err, ERR_BAD_INDEX);
+          if (T.ebase + slot < leafof_n) {
+            leafof[T.ebase + slot] = id;
+            if (rank) rank[T.ebase + slot] = T.n - static_cast<uint32_t>(st - T.ebase) - cn + k;
+          } else {
+            atomicOr(A.err, ERR_BAD_INDEX);
+          }
         }
     }
     if (id != 1 && (leaf || !(A.ndepth[g] & 1u))) continue;
@@ -1046,7 +1053,7 @@ RtArgs rt_args(RTreeBufs& B, uint32_t* err) {
 }
 
 void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cudaStream_t st, double node_frac,
-                 size_t leafof_slots) {
+                 size_t leafof_slots, bool want_rank) {
   B.ntiles = static_cast<int>(tiles.size());
   unsigned long long e = 0, nn = 0;
   uint32_t emax = 0;
@@ -1102,6 +1109,7 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.rnode.alloc(std::max<unsigned long long>(rr, 1), st);
   B.rleaf.alloc(N1, st);
   if (want_leafof) B.leafof.alloc(std::max(E1, leafof_slots), st);
+  if (want_rank) B.rank.alloc(std::max(E1, leafof_slots), st);
   FG_CUDA(cudaMemsetAsync(B.ridx.p, 0, E1 * sizeof(uint32_t), st));
 }
 
@@ -1214,7 +1222,7 @@ void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, RTile* tiles_dev)
   // The global worklist is spent: its words count the children that reached each node.
   FG_CUDA(cudaMemsetAsync(B.wl0.p, 0, static_cast<size_t>(B.N) * sizeof(uint32_t), st));
   k_rt_refit<<<GN, RT_BLOCK, 0, st>>>(A, B.wl0.p);
-  k_rt_records<<<GN, RT_BLOCK, 0, st>>>(A, B.rnode.p, B.rleaf.p, B.leafof.p, B.leafof.n);
+  k_rt_records<<<GN, RT_BLOCK, 0, st>>>(A, B.rnode.p, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
   k_rt_depth_check<<<grid_for(static_cast<size_t>(B.ntiles), 128), 128, 0, st>>>(A);
   FG_CUDA(cudaGetLastError());
 }
@@ -1265,7 +1273,7 @@ void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_onl
   t.ecap = developed_only ? std::max<uint32_t>(m, 1) : std::max<uint32_t>(n, 1);
   t.n = developed_only ? m : n;
   std::vector<RTile> v{t};
-  rtree_alloc(B, v, developed_only, st, 1.0, n);
+  rtree_alloc(B, v, true, st, 1.0, n, !developed_only);
   rtree_build(B, e->d_err, st);
   B.count = t.n;
 }

@@ -1,19 +1,180 @@
 // Monte-Carlo photon transport (transport.rs:48-188 and optics.rs:75-196) as a persistent,
 // warp-scheduled kernel over one or many tiles, plus the exact replay of recorded segments.
 //
-// Work: photon ids of all tiles form one index space; each warp takes 32 ids at a time from a
-// global counter.  Every draw is a Philox block named by (photon, bounce, slot, tag), so results
-// do not depend on which warp or SM traces a photon.  Each segment walks the tile's reference tree
-// (fg_rtree.cuh) and absorbs its hits in the reference's traversal order as they are found
-// (Beer-Lambert, Bernoulli rounding of 5 E p s latent photons, energy *= max(1 - 0.9 p, 0.05)).
-// Counts reach HBM as warp-aggregated atomics.
+// Work: photon ids of all tiles form one index space; a warp's lanes take ids from a global
+// counter.  Every draw is a Philox block named by (photon, bounce, slot, tag), so results do not
+// depend on which warp or SM traces a photon.  Each segment finds the crystals it hits through the
+// tile's cells (fg_cells.cuh) and absorbs them in the reference's traversal order (Beer-Lambert,
+// Bernoulli rounding of 5 E p s latent photons, energy *= max(1 - 0.9 p, 0.05)).
 #include "fg_internal.h"
 #include "fg_transport.cuh"
 
 namespace fg {
 
 // ---------------------------------------------------------------------------------------------
-// Production kernel.  Every lane carries one photon through its bounces; a lane is in one of five
+// Production kernel.  Every lane carries one photon through its bounces; a lane has no photon, a
+// photon between bounces, a segment that visits its cells, or is done (the photon queue is spent).
+// The warp alternates between two kinds of work:
+//   - visit: every lane with room goes from row to row and lists the crystals whose ball comes
+//     within its segment (positions, in shared memory), in short uniform steps;
+//   - resolve, once CELL_WAIT lanes wait (segment visited, or list full) or none visits: the waiting
+//     lanes test their listed crystals' geometry and keep the hits with their rank; lanes whose
+//     segment is visited absorb the hits in rank order (the reference's traversal order) and end
+//     their bounces; lanes between bounces begin the next one, and empty lanes take the next
+//     photons of the position-ordered queue.
+// So lanes do not wait for their warp's next hit or longest segment, and the long code (geometry,
+// absorption, ends and beginnings of bounces) runs with many lanes.  Which lane traces a photon,
+// and when, never changes its result: its draws are named by (photon, bounce, slot, tag), and its
+// hits are absorbed in rank order.
+__global__ void __launch_bounds__(256, 4) k_transport(const TileDesc* __restrict__ tiles, int ntiles,
+                                                     unsigned long long total, const uint32_t* __restrict__ order,
+                                                     unsigned long long* next, uint32_t* err,
+                                                     unsigned long long* stats) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr uint32_t NONE = 0xffffffffu;
+  enum : int { EMPTY_LANE = 0, READY = 1, VISITING = 2, DONE = 3 };
+  // Per lane: entries 0 .. nh - 1 are hits (rank, path), nh .. nq - 1 listed positions.  A visit
+  // keeps the hits of lowest rank from `from` on; a segment with more (`more`) is visited again
+  // for the next ones, `done` hits having been absorbed.
+  __shared__ uint32_t s_rank[CELL_LIST][256];
+  __shared__ float s_path[CELL_HITS][256];
+  __shared__ uint32_t s_draw[3][256];  // the bounce's draws that its end uses
+  static_assert(CELL_HITS % 4 == 0, "a visit's hits start a Philox block");
+  const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  Photon ph{};
+  CellVisit v{};
+  float inv_y = 0.0f, inv_z = 0.0f;
+  uint32_t nh = 0, nq = 0, from = 0, done = 0;
+  bool more = false;
+  int tile = 0;
+  int state = EMPTY_LANE;
+  unsigned long long my_hits = 0;
+  auto begin = [&](const TileDesc& t) {
+    P4 rb;
+    const float step = bounce_step(t, ph, rb);
+    s_draw[0][tid] = rb.y;
+    s_draw[1][tid] = rb.z;
+    s_draw[2][tid] = rb.w;
+    inv_y = slab_inv(ph.dir.y);
+    inv_z = slab_inv(ph.dir.z);
+    cells_begin(t.cells, ph.pos, ph.dir, step, v);
+    nh = nq = from = done = 0;
+    more = false;
+    state = VISITING;
+  };
+  for (;;) {
+    {
+      const CellGrid& g = tiles[tile].cells;
+      for (;;) {
+        const bool room = state == VISITING && nq < CELL_LIST;
+        const bool test = room && v.c < v.cend;
+        const bool move = room && !test && !(v.iy > v.iy1 && v.iz >= v.iz1);
+        const unsigned tm = __ballot_sync(FULL, test), mm = __ballot_sync(FULL, move);
+        if (!(tm | mm) || __popc(__ballot_sync(FULL, state != DONE) & ~(tm | mm)) >= CELL_WAIT) break;
+        if (__popc(mm) > __popc(tm)) {
+          if (move) cells_advance(g, ph.pos, ph.dir, inv_y, inv_z, v, err);
+        } else if (test) {
+          const uint32_t p = v.c;
+          const bool two = p + 1 < v.cend && nq + 1 < CELL_LIST;
+          const float4 a = __ldg(&g.pos[p]), b = __ldg(&g.pos[two ? p + 1 : p]);
+          if (cell_near(a, ph.pos, ph.dir, v.step)) s_rank[nq++][tid] = p;
+          if (two && cell_near(b, ph.pos, ph.dir, v.step)) s_rank[nq++][tid] = p + 1;
+          v.c = p + 1 + (two ? 1u : 0u);
+        }
+      }
+    }
+    if (state == VISITING && (nq == CELL_LIST || cells_done(v))) {
+      const TileDesc& t = tiles[tile];
+      const float3 inv = make_float3(slab_inv(ph.dir.x), inv_y, inv_z);
+      for (uint32_t k = nh; k < nq; ++k) {
+        float path;
+        uint32_t rank;
+        if (!cell_hit(t, ph.pos, ph.dir, inv, v.step, s_rank[k][tid], path, rank) || rank < from) continue;
+        uint32_t at = nh;
+        if (nh < CELL_HITS) {
+          ++nh;
+        } else {  // the hit of highest rank gives way
+          more = true;
+          uint32_t top = rank;
+          for (uint32_t j = 0; j < CELL_HITS; ++j)
+            if (s_rank[j][tid] > top) {
+              top = s_rank[j][tid];
+              at = j;
+            }
+          if (top == rank) continue;
+        }
+        s_rank[at][tid] = rank;
+        s_path[at][tid] = path;
+      }
+      nq = nh;
+      if (cells_done(v)) {
+        P4 r{};
+        for (uint32_t k = 0; k < nh; ++k) {
+          uint32_t best = NONE, at = 0;
+          for (uint32_t j = 0; j < nh; ++j) {
+            const uint32_t rk = s_rank[j][tid];
+            if (rk < best) {
+              best = rk;
+              at = j;
+            }
+          }
+          s_rank[at][tid] = NONE;
+          from = best + 1;
+          if (!index_ok(best < t.n, err, SITE_CELL, best, t.n)) continue;
+          const uint2 c = __ldg(&t.cells.by_rank[best]);
+          absorb_hit(t, ph, done + k, r, s_path[at][tid], __uint_as_float(c.y), c.x, err);
+        }
+        if (more) {
+          done += nh;
+          nh = nq = 0;
+          more = false;
+          cells_begin(t.cells, ph.pos, ph.dir, v.step, v);
+        } else {
+          my_hits += done + nh;
+          state = bounce_end(t, ph, v.step, s_draw[0][tid], s_draw[1][tid], s_draw[2][tid]) ? READY : EMPTY_LANE;
+        }
+      }
+    }
+    if (state == READY) {
+      if (ph.b < tiles[tile].max_bounces) begin(tiles[tile]); else state = EMPTY_LANE;
+    }
+    unsigned need = __ballot_sync(FULL, state == EMPTY_LANE);
+    while (need) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(next, static_cast<unsigned long long>(__popc(need)));
+      base = __shfl_sync(FULL, base, 0);
+      if (state == EMPTY_LANE) {
+        const unsigned long long g = base + __popc(need & lt);
+        if (g >= total) {
+          state = DONE;
+        } else {
+          unsigned long long gid = order ? order[g] : g;
+          if (!index_ok(gid < total, err, SITE_PHOTON_ID, static_cast<uint32_t>(gid), static_cast<uint32_t>(g)))
+            gid = g;
+          int lo = 0, hi = ntiles - 1;
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (tiles[mid].photon_base <= gid) lo = mid; else hi = mid - 1;
+          }
+          tile = lo;
+          if (emit_photon(tiles[lo], static_cast<uint32_t>(gid - tiles[lo].photon_base), ph) &&
+              ph.b < tiles[lo].max_bounces)
+            begin(tiles[lo]);
+        }
+      }
+      need = __ballot_sync(FULL, state == EMPTY_LANE);
+    }
+    if (!__any_sync(FULL, state != DONE)) break;
+  }
+  if (stats) {
+    for (int o = 16; o > 0; o >>= 1) my_hits += __shfl_down_sync(FULL, my_hits, o);
+    if (lane == 0 && my_hits) atomicAdd(&stats[0], my_hits);
+  }
+}
+
+// The same over the reference tree itself, for crystal sets that cells do not suit (below):
+// Every lane carries one photon through its bounces; a lane is in one of five
 // states: no photon, a photon between bounces, a bounce walking (fg_transport.cuh: Bounce), a
 // walked bounce whose end is pending, or done (the photon queue is spent).  Each loop turn the warp
 // does one of two kinds of work:
@@ -27,7 +188,7 @@ namespace fg {
 // and when, never changes its result: its draws are named by (photon, bounce, slot, tag), and its
 // leaves are tested in walk order.
 // Launch bounds of 4 blocks of 256 per SM (64 registers): the walk is latency-bound.
-__global__ void __launch_bounds__(256, 4) k_transport(const TileDesc* __restrict__ tiles, int ntiles,
+__global__ void __launch_bounds__(256, 4) k_transport_walk(const TileDesc* __restrict__ tiles, int ntiles,
                                                      unsigned long long total, const uint32_t* __restrict__ order,
                                                      unsigned long long* next, uint32_t* err,
                                                      unsigned long long* stats) {
@@ -52,7 +213,8 @@ __global__ void __launch_bounds__(256, 4) k_transport(const TileDesc* __restrict
     if (!walkm || __popc(idlem) >= WALK_RESTART) {
       if (state == WALKED) {
         my_hits += w.nh;
-        state = bounce_end(tiles[tile], ph, w) ? READY : EMPTY_LANE;
+        const P4 rb = philox(ph.id, ph.b - 1, 0, TAG_BOUNCE, tiles[tile].k0, tiles[tile].k1);
+        state = bounce_end(tiles[tile], ph, w.step, rb.y, rb.z, rb.w) ? READY : EMPTY_LANE;
       }
       if (state == READY) {
         if (ph.b < tiles[tile].max_bounces) {
@@ -265,23 +427,24 @@ __global__ void k_element_records(const uint32_t* __restrict__ ridx, uint32_t n,
   od[p] = d[s];
 }
 
-// The transport descriptor of an emulsion; a, q, d are its crystal records in the tree's element
-// order (records, 3 n float4 written here).
+// The transport descriptor of an emulsion.  For the tree walk, a, q, d are its crystal records in
+// the tree's element order (records, 3 n float4 written here).
 TileDesc make_tile_desc(const fg_emulsion* em, const float* tile_dev, uint32_t tw, uint32_t th,
                         const fg_exposure_cfg& cfg, uint64_t seed, uint32_t* counts, float4* records,
                         uint32_t* err, cudaStream_t st) {
   TileDesc t{};
-  float4* oa = records;
-  float4* oq = records + em->n;
-  float4* od = records + 2ull * em->n;
-  if (em->n) {
+  t.cells = em->grid;
+  if (records && em->n) {
+    float4* oa = records;
+    float4* oq = records + em->n;
+    float4* od = records + 2ull * em->n;
     k_element_records<<<grid_for(em->n, 256), 256, 0, st>>>(em->rt.ridx.p, em->n, em->a.p, em->q.p, em->d.p, oa, oq,
                                                              od, err);
     FG_CUDA(cudaGetLastError());
+    t.a = oa;
+    t.q = oq;
+    t.d = od;
   }
-  t.a = oa;
-  t.q = oq;
-  t.d = od;
   t.rnode = em->rt.rnode.p;
   t.rleaf = em->rt.rleaf.p;
   t.ridx = em->rt.ridx.p;
@@ -318,20 +481,69 @@ TileDesc make_tile_desc(const fg_emulsion* em, const float* tile_dev, uint32_t t
 
 void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long long total,
                             const uint32_t* order, unsigned long long* counter, uint32_t* err,
-                            unsigned long long* stats, unsigned blocks, unsigned threads, cudaStream_t st) {
+                            unsigned long long* stats, unsigned blocks, unsigned threads, cudaStream_t st,
+                            bool walk) {
   if (total == 0) return;
   FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
   const unsigned long long warps = (total + 31) / 32;
   const unsigned long long need = (warps * 32 + threads - 1) / threads;
   blocks = static_cast<unsigned>(std::max<unsigned long long>(std::min<unsigned long long>(blocks, need), 1));
-  k_transport<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err, stats);
+  if (walk) {
+    k_transport_walk<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err, stats);
+  } else {
+    k_transport<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err, stats);
+  }
   FG_CUDA(cudaGetLastError());
+}
+
+// Cells suit a crystal set whose crystals reach no further than the mean spacing and that fills the
+// box evenly: then a segment tests a handful of crystals per layer of cells.  One giant crystal
+// drags every segment's rows out to its reach, a set bunched in a corner puts many crystals into one
+// cell, and a centre outside the box has no cell; such sets keep the tree walk, whose cost follows
+// the boxes.  Measured with one giant among the crystals of a 140 um film (ms, cells / walk): none
+// (reach 0.4 spacings for t-max's, 0.7 for tri-x's) 0.49 / 0.92 and 0.47 / 0.72; reach 1 spacing
+// 0.92 / 0.93 and 0.63 / 0.82; 1.5 spacings 1.45 / 0.90 and 0.97 / 0.91.
+constexpr double CELLS_MAX_REACH = 1.0;   // mean spacings
+constexpr uint32_t CELLS_MAX_COUNT = 16;  // crystals in one cell (half a crystal on average)
+
+void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
+  cudaStream_t st = e->stream;
+  em->grid = CellGrid{};
+  const uint32_t n = em->n;
+  CellGrid g{};
+  if (!n || !cells_layout(em->cfg.width, em->cfg.height, em->cfg.depth, n, g)) return;
+  cells_reach(g, em->max_half_dim, em->any_cubic);
+  const double spacing = std::cbrt(em->cfg.width * em->cfg.height * em->cfg.depth / n);
+  if (!(g.reach <= CELLS_MAX_REACH * spacing)) return;
+  em->cells.alloc(n, cells_of(g), st);
+  em->cells.attach(g, 0);
+  TileDesc t{};
+  t.cells = g;
+  t.n = n;
+  t.nnodes = static_cast<uint32_t>(em->rt.N);
+  DBuf<TileDesc> td(1, st);
+  DBuf<uint32_t> unfit(1, st);
+  FG_CUDA(cudaMemcpyAsync(td.p, &t, sizeof(TileDesc), cudaMemcpyHostToDevice, st));
+  FG_CUDA(cudaMemsetAsync(unfit.p, 0, sizeof(uint32_t), st));
+  FG_CUDA(cudaMemsetAsync(em->cells.cnt.p, 0, (em->cells.ncells + 1) * sizeof(uint32_t), st));
+  launch_cells_count(td.p, 1, n, em->a.p, em->cells.cnt.p, em->cells.place.p, st, CELLS_MAX_COUNT, unfit.p);
+  exclusive_scan_u32(em->cells.cnt.p, em->cells.off.p, em->cells.ncells + 1, st);
+  launch_cells_fill(td.p, 1, n, em->a.p, em->q.p, em->d.p, em->rt, em->cells, e->d_err, st);
+  uint32_t c = 0;
+  FG_CUDA(cudaMemcpyAsync(&c, unfit.p, sizeof(c), cudaMemcpyDeviceToHost, st));
+  FG_CUDA(cudaStreamSynchronize(st));
+  em->cells.cnt.release();
+  em->cells.place.release();
+  if (!c) em->grid = g;
+  else em->cells = CellBufs{};
 }
 
 void expose(fg_engine* e, fg_emulsion* em, const float* tile_dev, uint32_t tw, uint32_t th,
             const fg_exposure_cfg& cfg, uint64_t seed, unsigned long long* photons_out) {
   cudaStream_t st = e->stream;
-  DBuf<float4> records(3ull * std::max<uint32_t>(em->n, 1), st);
+  const bool walk = em->grid.x.n == 0;
+  DBuf<float4> records;
+  if (walk) records.alloc(3ull * std::max<uint32_t>(em->n, 1), st);
   TileDesc t = make_tile_desc(em, tile_dev, tw, th, cfg, seed, em->counts.p, records.p, e->d_err, st);
   if (photons_out) *photons_out = t.P;
   if (t.P == 0 || em->n == 0) return;
@@ -339,7 +551,7 @@ void expose(fg_engine* e, fg_emulsion* em, const float* tile_dev, uint32_t tw, u
   DBuf<unsigned long long> ctr(1, st);
   FG_CUDA(cudaMemcpyAsync(td.p, &t, sizeof(TileDesc), cudaMemcpyHostToDevice, st));
   launch_transport_shape(td.p, 1, t.P, nullptr, ctr.p, e->d_err, e->d_stats,
-                         static_cast<unsigned>(e->sm_count) * 4, 256, st);
+                         static_cast<unsigned>(e->sm_count) * 4, 256, st, walk);
 }
 
 void replay_segments(fg_engine* e, fg_emulsion* em, const fg_exposure_cfg& cfg, uint64_t seed,

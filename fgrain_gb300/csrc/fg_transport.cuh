@@ -1,22 +1,29 @@
 // Device code of the photon transport: tile descriptors, the reference-tree walk and the
 // per-photon bounce loop (transport.rs:101-185, optics.rs:100-196).
 #pragma once
+#include "fg_cells.cuh"
 #include "fg_device.cuh"
 #include "fg_rtree.cuh"
 
 namespace fg {
 
+constexpr int CELL_HITS = 12;     // hits of a segment absorbed per visit (the rest: visited again)
+constexpr int CELL_LIST = 16;     // hits and listed crystals of a lane
+constexpr int CELL_WAIT = 26;     // waiting lanes of a warp that resolve together
 constexpr int WALK_LEAVES = 6;    // leaves a lane may hold while its warp still walks (speculative traversal)
 constexpr int WALK_RESTART = 24;  // idle lanes of a warp that end and start their bounces together
 constexpr int WALK_EMPTY = INT32_MIN;
 constexpr uint32_t WALK_NONE = 0xffffffffu;
 
-// Everything one tile's transport needs, 16-byte aligned for vector loads.  The walk runs over the
-// tile's reference tree (fg_rtree.cuh): rnode / rleaf indexed by tile-local node id, ridx by
-// tile-local element position (a leaf's crystals in the reference's order).  The crystal records
-// a, q, d are in that element order too (position p holds the crystal ridx[p]), so a leaf's
-// crystals lie next to each other and are read without their slots.
+// Everything one tile's transport needs, 16-byte aligned for vector loads.  Segments find their
+// crystals through the cells (fg_cells.cuh).  The tree walk, for crystal sets that cells do not
+// suit, runs over the reference tree (fg_rtree.cuh): rnode / rleaf indexed by tile-local node id,
+// ridx by tile-local element position (a leaf's crystals in the reference's order), and the crystal
+// records a, q, d in that element order too (position p holds the crystal ridx[p]).
 struct __align__(16) TileDesc {
+  CellGrid cells;
+  unsigned long long cbase;  // first crystal slot
+  unsigned long long nbase;  // first node of the tile's tree
   const float4* a;
   const float4* q;
   const float4* d;
@@ -63,19 +70,6 @@ __device__ __forceinline__ double absorb64(double E, double path, double alpha, 
   const double frac = __dsub_rn(expected, static_cast<double>(whole));
   *count = whole + ((u < fmin(fmax(frac, 0.0), 1.0)) ? 1u : 0u);
   return __dmul_rn(E, fmax(__dsub_rn(1.0, __dmul_rn(p, 0.9)), 0.05));
-}
-
-// Adds n latent photons to crystal s, one atomic per distinct counter among the active lanes.
-// Lanes are grouped by the counter's address, not by s: the lanes of a warp may trace photons of
-// different tiles, whose crystals share local indices.
-__device__ __forceinline__ void add_counts(uint32_t* counts, uint32_t s, uint32_t n) {
-  uint32_t* const ctr = counts + s;
-  const unsigned act = __activemask();
-  const unsigned grp = __match_any_sync(act, reinterpret_cast<unsigned long long>(ctr));
-  const int leader = __ffs(grp) - 1;
-  uint32_t sum = 0;
-  for (unsigned m = grp; m; m &= m - 1) sum += __shfl_sync(grp, n, __ffs(m) - 1);
-  if ((threadIdx.x & 31) == leader && sum) atomicAdd(ctr, sum);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -135,24 +129,28 @@ __device__ __forceinline__ bool emit_photon(const TileDesc& t, uint32_t id, Phot
 struct Bounce {
   float3 inv, oi;     // 1 / dir (slab_inv) and pos * inv, for the slab tests
   float step, tlim;   // the step and the walk's reach along the ray
-  float E;            // packet energy, as the hits absorb it
   uint32_t nh;        // absorbing hits so far
   P4 r;               // the Philox block of hits nh & ~3 .. (nh & ~3) + 3
   int cur, sp;        // current record (~leaf for a leaf child, WALK_EMPTY when done) and stack depth
   uint32_t lv[WALK_LEAVES];  // leaves reached and not yet tested, in walk order
 };
 
-// Starts bounce ph.b (transport.rs:101-107): the free path, the segment's step and the walk from
-// the root record.
-__device__ __forceinline__ void bounce_begin(const TileDesc& t, Photon& ph, Bounce& w) {
+// Bounce ph.b's segment length (transport.rs:101-107): the free path, at most 1.5 depths.  rb
+// receives the bounce's draws (its end uses y, z, w).
+__device__ __forceinline__ float bounce_step(const TileDesc& t, Photon& ph, P4& rb) {
   const uint32_t b = ph.b++;
-  const P4 rb = philox(ph.id, b, 0, TAG_BOUNCE, t.k0, t.k1);
+  rb = philox(ph.id, b, 0, TAG_BOUNCE, t.k0, t.k1);
   const float fp = t.mu_t > 0.0f ? -__logf(fmaxf(1.0f - uf(rb.x), 1.17549435e-38f)) / t.mu_t : 1e6f;
-  w.step = fminf(fp, t.D * 1.5f);
+  return fminf(fp, t.D * 1.5f);
+}
+
+// Starts bounce ph.b: its segment and the walk from the root record.
+__device__ __forceinline__ void bounce_begin(const TileDesc& t, Photon& ph, Bounce& w) {
+  P4 rb;
+  w.step = bounce_step(t, ph, rb);
   w.inv = make_float3(slab_inv(ph.dir.x), slab_inv(ph.dir.y), slab_inv(ph.dir.z));
   w.oi = make_float3(ph.pos.x * w.inv.x, ph.pos.y * w.inv.y, ph.pos.z * w.inv.z);
   w.tlim = w.step * 1.00001f + 1e-3f;
-  w.E = ph.E;
   w.nh = 0;
   w.r = P4{};
   w.cur = 0;  // record 0: the root's
@@ -226,11 +224,63 @@ __device__ __forceinline__ void walk_step(const TileDesc& t, Bounce& w, int* sta
   w.cur = next != WALK_EMPTY ? next : (w.sp > 0 ? stack[--w.sp] : WALK_EMPTY);
 }
 
+// One absorbing hit inside the step (transport.rs:108-138): Beer-Lambert, Bernoulli rounding of
+// 5 E p s latent photons for crystal slot s, E *= max(1 - 0.9 p, 0.05); the n-th absorbing hit of
+// the bounce draws word n % 4 of Philox block n / 4.
+__device__ __forceinline__ void absorb_hit(const TileDesc& t, Photon& ph, uint32_t nh, P4& r, float path,
+                                           float sens, uint32_t s, uint32_t* err) {
+  if ((nh & 3) == 0) r = philox(ph.id, ph.b - 1, nh >> 2, TAG_HIT, t.k0, t.k1);
+  // 1 - exp(-alpha L) without the cancellation of a short chord (corner hits are common).
+  const float p = -expm1f(-t.alpha * path);
+  const float expected = ph.E * p * sens * 5.0f;
+  const float fl = floorf(expected);
+  const uint32_t cnt = static_cast<uint32_t>(fl) + (uf(word(r, nh & 3)) < expected - fl ? 1u : 0u);
+  if (cnt && index_ok(s < t.n, err, SITE_LEAF, s, t.n)) atomicAdd(t.counts + s, cnt);
+  ph.E *= fmaxf(1.0f - p * 0.9f, 0.05f);
+}
+
+// Slab test of a leaf box lo (x, y, z) to hi as lo * inv - o * inv (one FMA per plane), the box
+// grown by g, clipped to [0, tm] of the ray.
+__device__ __forceinline__ bool leaf_slab(float3 lo, float3 hi, float3 inv, float3 oi, float g, float tm) {
+  const float t1x = fmaf(lo.x - g, inv.x, -oi.x), t2x = fmaf(hi.x + g, inv.x, -oi.x);
+  const float t1y = fmaf(lo.y - g, inv.y, -oi.y), t2y = fmaf(hi.y + g, inv.y, -oi.y);
+  const float t1z = fmaf(lo.z - g, inv.z, -oi.z), t2z = fmaf(hi.z + g, inv.z, -oi.z);
+  const float te = fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
+  const float tx = fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tm));
+  return te <= tx;
+}
+
+// The crystal at cell position p against the segment: its geometry (crystal.rs:140-217) inside the
+// step, and its leaf as the walk tests it (the leaf's box extended by the reach meets the step, the
+// box itself the whole ray, bvh.rs:96-124).
+__device__ __forceinline__ bool cell_hit(const TileDesc& t, float3 pos, float3 dir, float3 inv, float step, uint32_t p,
+                                         float& path, uint32_t& rank) {
+  const float4 a = __ldg(&t.cells.pos[p]), q = __ldg(&t.cells.q[p]), d = __ldg(&t.cells.d[p]);
+  float t0, t1;
+  if (!fintersect(a, q, d, 1.0f, pos, dir, t0, t1)) return false;
+  if (!(t0 < step)) return false;
+  path = fmaxf(fminf(t1, step) - t0, 0.0f);
+  if (!(path > 0.0f)) return false;
+  const float4 l0 = __ldg(&t.cells.leaf[2ull * p]), l1 = __ldg(&t.cells.leaf[2ull * p + 1]);
+  rank = __float_as_uint(l1.z);
+  const float3 lo = make_float3(l0.x, l0.y, l0.z), hi = make_float3(l0.w, l1.x, l1.y);
+  const float3 oi = make_float3(pos.x * inv.x, pos.y * inv.y, pos.z * inv.z);
+  const float tlim = step * 1.00001f + 1e-3f;
+  return leaf_slab(lo, hi, inv, oi, t.reach, tlim) && leaf_slab(lo, hi, inv, oi, 0.0f, INFINITY);
+}
+
+// Whether the crystal's ball (a: centre, squared radius) comes within the segment (conservative for
+// cell_hit).
+__device__ __forceinline__ bool cell_near(float4 a, float3 pos, float3 dir, float step) {
+  const float wx = a.x - pos.x, wy = a.y - pos.y, wz = a.z - pos.z;
+  const float tc = fminf(fmaxf(wx * dir.x + wy * dir.y + wz * dir.z, 0.0f), step);
+  const float ex = wx - tc * dir.x, ey = wy - tc * dir.y, ez = wz - tc * dir.z;
+  return ex * ex + ey * ey + ez * ez <= a.w;
+}
+
 // Tests the crystals of the lane's oldest queued leaf by their geometry (crystal.rs:140-217) in
-// the reference's order, and absorbs each hit inside the step at once (transport.rs:108-138):
-// Beer-Lambert, Bernoulli rounding of 5 E p s latent photons, E *= max(1 - 0.9 p, 0.05); the
-// n-th absorbing hit of the bounce draws word n % 4 of Philox block n / 4.
-__device__ __forceinline__ void leaf_step(const TileDesc& t, const Photon& ph, Bounce& w, uint32_t* err) {
+// the reference's order, and absorbs each hit inside the step at once.
+__device__ __forceinline__ void leaf_step(const TileDesc& t, Photon& ph, Bounce& w, uint32_t* err) {
   const uint32_t id = w.lv[0];
 #pragma unroll
   for (int j = 0; j + 1 < WALK_LEAVES; ++j) w.lv[j] = w.lv[j + 1];
@@ -240,7 +290,6 @@ __device__ __forceinline__ void leaf_step(const TileDesc& t, const Photon& ph, B
   if (!index_ok(L.x + L.y <= t.n, err, SITE_LEAF, L.x, L.y)) return;
   const float3 pos = ph.pos, dir = ph.dir;
   const float step = w.step;
-  const uint32_t b = ph.b - 1;
   for (uint32_t k = 0; k < L.y; ++k) {
     const uint32_t e = L.x + k;  // element position: the crystal ridx[e]
     const float4 a = __ldg(&t.a[e]), d = __ldg(&t.d[e]);
@@ -262,48 +311,45 @@ __device__ __forceinline__ void leaf_step(const TileDesc& t, const Photon& ph, B
     if (!(t0 < step)) continue;
     const float path = fmaxf(fminf(t1, step) - t0, 0.0f);
     if (!(path > 0.0f)) continue;
-    if ((w.nh & 3) == 0) w.r = philox(ph.id, b, w.nh >> 2, TAG_HIT, t.k0, t.k1);
-    // 1 - exp(-alpha L) without the cancellation of a short chord (corner hits are common).
-    const float p = -expm1f(-t.alpha * path);
-    const float expected = w.E * p * a.w * 5.0f;
-    const float fl = floorf(expected);
-    const uint32_t cnt = static_cast<uint32_t>(fl) + (uf(word(w.r, w.nh & 3)) < expected - fl ? 1u : 0u);
-    if (cnt) {
-      const uint32_t s = __ldg(&t.ridx[e]);
-      if (index_ok(s < t.n, err, SITE_LEAF, s, t.n)) add_counts(t.counts, s, cnt);
-    }
-    w.E *= fmaxf(1.0f - p * 0.9f, 0.05f);
+    absorb_hit(t, ph, w.nh, w.r, path, a.w, __ldg(&t.ridx[e]), err);
     ++w.nh;
   }
 }
 
-// Ends the bounce whose walk is done (transport.rs:140-185): the move, the film's faces (escape,
-// or the anti-halation layer's reflection, optics.rs:150-196), Henyey-Greenstein scattering with
-// albedo and Russian roulette.  Returns whether the packet is still alive.
-__device__ __forceinline__ bool bounce_end(const TileDesc& t, Photon& ph, const Bounce& w) {
+// Ends a bounce of length `step` whose hits are absorbed (transport.rs:140-185): the move, the
+// film's faces (escape, or the anti-halation layer's reflection, optics.rs:150-196),
+// Henyey-Greenstein scattering with albedo and Russian roulette.  ry, rz, rw: the bounce's draws.
+// Returns whether the packet is still alive.
+__device__ __forceinline__ bool bounce_end(const TileDesc& t, Photon& ph, float step, uint32_t ry, uint32_t rz,
+                                           uint32_t rw) {
   const float PI2 = 6.283185307179586f;
   const uint32_t b = ph.b - 1;
-  const P4 rb = philox(ph.id, b, 0, TAG_BOUNCE, t.k0, t.k1);
   const float3 pos = ph.pos, dir = ph.dir;
-  const float step = w.step;
-  float E = w.E;
+  float E = ph.E;
   const float3 np = make_float3(pos.x + dir.x * step, pos.y + dir.y * step, pos.z + dir.z * step);
   if (np.x < 0.0f || np.x >= t.W || np.y < 0.0f || np.y >= t.H) return false;
   if (np.z <= 0.0f) return false;
-  if (np.z >= t.D) {
-    ph.pos = make_float3(np.x, np.y, t.D - 0.001f);
-    const P4 ra = philox(ph.id, b, 0, TAG_AH, t.k0, t.k1);
+  // One sine and cosine serve both the diffuse reflection and the scattering (lanes of a warp take
+  // either way together).
+  const bool bottom = np.z >= t.D;
+  P4 ra{};
+  if (bottom) {
+    ra = philox(ph.id, b, 0, TAG_AH, t.k0, t.k1);
     E *= t.eff_r;
     if (E < 1e-4f) {
       if (uf(ra.x) < 0.1f) E /= 0.1f; else return false;
     }
+  }
+  const bool diffuse = bottom && uf(ra.y) < 0.4f;
+  float sph = 0.0f, cph = 0.0f;
+  if (diffuse || !bottom) sincosf(PI2 * uf(diffuse ? ra.w : rz), &sph, &cph);
+  if (bottom) {
+    ph.pos = make_float3(np.x, np.y, t.D - 0.001f);
     float3 d2;
-    if (uf(ra.y) < 0.4f) {
-      const float u1 = uf(ra.z), u2 = uf(ra.w);
+    if (diffuse) {
+      const float u1 = uf(ra.z);
       const float rr = sqrtf(u1);
-      float s2, c2;
-      sincosf(PI2 * u2, &s2, &c2);
-      d2 = make_float3(rr * c2, rr * s2, -sqrtf(fmaxf(1.0f - u1, 0.0f)));
+      d2 = make_float3(rr * cph, rr * sph, -sqrtf(fmaxf(1.0f - u1, 0.0f)));
     } else {
       d2 = make_float3(dir.x, dir.y, -fabsf(dir.z));
     }
@@ -315,15 +361,13 @@ __device__ __forceinline__ bool bounce_end(const TileDesc& t, Photon& ph, const 
   ph.pos = np;
   float cth;
   if (fabsf(t.g) < 1e-4f) {
-    cth = 2.0f * uf(rb.y) - 1.0f;
+    cth = 2.0f * uf(ry) - 1.0f;
   } else {
-    const float term = (1.0f - t.g * t.g) / (1.0f - t.g + 2.0f * t.g * uf(rb.y));
+    const float term = (1.0f - t.g * t.g) / (1.0f - t.g + 2.0f * t.g * uf(ry));
     cth = (1.0f + t.g * t.g - term * term) / (2.0f * t.g);
   }
   cth = fminf(fmaxf(cth, -1.0f), 1.0f);
   const float sth = sqrtf(fmaxf(1.0f - cth * cth, 0.0f));
-  float sph, cph;
-  sincosf(PI2 * uf(rb.z), &sph, &cph);
   float3 u = fabsf(dir.x) > 0.1f ? make_float3(dir.z, 0.0f, -dir.x) : make_float3(0.0f, -dir.z, dir.y);
   {
     const float n = rsqrtf(u.x * u.x + u.y * u.y + u.z * u.z);
@@ -337,10 +381,19 @@ __device__ __forceinline__ bool bounce_end(const TileDesc& t, Photon& ph, const 
   ph.dir = make_float3(nd.x * n, nd.y * n, nd.z * n);
   E *= t.albedo;
   if (E < 1e-3f) {
-    if (uf(rb.w) < 0.1f) E /= 0.1f; else return false;
+    if (uf(rw) < 0.1f) E /= 0.1f; else return false;
   }
   ph.E = E;
   return true;
 }
+
+// Host launchers (fg_cells.cu).  The fill needs the prefix sum of the counts in c.off and the tree
+// with its ranks; slots 0 .. ncap - 1 cover the tiles' crystal slots.
+struct RTreeBufs;
+struct CellBufs;
+void launch_cells_count(const TileDesc* tiles, int ntiles, unsigned long long ncap, const float4* A, uint32_t* cnt,
+                        uint32_t* place, cudaStream_t st, uint32_t limit = 0, uint32_t* unfit = nullptr);
+void launch_cells_fill(const TileDesc* tiles, int ntiles, unsigned long long ncap, const float4* A, const float4* Q,
+                       const float4* D, const RTreeBufs& tree, const CellBufs& c, uint32_t* err, cudaStream_t st);
 
 }  // namespace fg
