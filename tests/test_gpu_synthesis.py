@@ -1,0 +1,41 @@
+"""The sampler's points at the edges of its columns: films of a fraction of a column, of one column
+and a cell, of one cell of depth, and of the deepest that eight columns per SM still take.  Points
+are exactly hard-core (the grid test is exact integer arithmetic) and as dense as Bridson leaves
+them (poisson.rs:14-132)."""
+import numpy as np
+import pytest
+
+import fgrain_gb300 as fg
+
+pytestmark = pytest.mark.gpu
+
+CELL = 3 ** -0.5  # cells per r_min
+
+
+# Film size in cells of r_min / sqrt(3) (columns are 8 x 8 cells over the full depth).
+@pytest.mark.parametrize("cells", [(3.0, 2.5, 4.0), (8.0, 8.0, 5.2), (9.0, 8.5, 1.0), (17.3, 31.9, 2.4),
+                                   (40.0, 25.1, 23.0), (33.0, 64.0, 30.5)])
+@pytest.mark.parametrize("r_min", [0.9, 1.2])
+def test_points_are_hard_core_and_dense(engine, cells, r_min):
+    from scipy.spatial import cKDTree
+
+    size = tuple(c * CELL * r_min for c in cells)
+    cfg = fg.EmulsionConfig(size, r_min, 0.4, 0.2)
+    em = fg.VirtualEmulsionLayer.synthesize(cfg, 5, engine)
+    pos = em.crystals()["pos"]
+    em.close()
+    n = len(pos)
+    assert n >= 1
+    # Positions are rounded to float: half an ulp of the largest coordinate on either side.
+    ulp = 2.0 ** -23 * max(size)
+    assert (pos >= 0).all() and (pos <= np.array(size) + ulp).all()
+    if n > 1:
+        d, _ = cKDTree(pos).query(pos, k=2)
+        assert d[:, 1].min() >= r_min * (1 - 1e-6) - ulp
+    # Bridson's density in the bulk plus its surface term (the model the thinning targets); the
+    # points left are at most the target plus what thinning's draws spare.
+    vol = np.prod(size)
+    target = (0.57793168 + 0.11306788 * r_min * sum(2 / s for s in size)) / r_min ** 3 * vol
+    assert n <= target + 4 * np.sqrt(target) + 2
+    if min(size) > 5 * r_min:
+        assert abs(n - target) <= 0.02 * target + 4
