@@ -65,8 +65,6 @@ struct __align__(16) BTile {
   uint32_t nbx, nby;
   float binw_x, binw_y;
   float pad;                  // leaf box padding
-  uint32_t ncap;              // node capacity of the tile's trees
-  uint32_t rbase, rcap;       // first walk record of the tile's tree, and their count
 };
 
 __device__ __forceinline__ int btile_of(const BTile* tiles, int ntiles, unsigned long long g) {
@@ -169,24 +167,23 @@ __device__ __forceinline__ void uf_unite_b(int* parent, int a, int b, uint32_t* 
   atomicOr(err, ERR_SPIN_LIMIT);
 }
 
-// Links each developed crystal to the developed crystals it touches (union-find), walking the
-// tile's reference tree with the query box: a leaf is reached iff its box and its ancestors' boxes
-// overlap the query (ancestor boxes contain their descendants'), and a crystal within the touch
-// distance lies inside its own leaf box, so the query finds it whatever the tree (bvh.rs:350-402);
-// the union-find roots do not depend on the order of the unions.
-__global__ void k_link_b(const BTile* __restrict__ bt, int ntiles, unsigned long long ncap,
-                         const float4* __restrict__ A, const float4* __restrict__ D, const Node4* __restrict__ rnode_all,
-                         const uint2* __restrict__ rleaf_all, const uint32_t* __restrict__ ridx_all,
-                         const uint8_t* __restrict__ developed, int* parent, const uint32_t* __restrict__ list,
-                         const uint32_t* __restrict__ ndev, uint32_t* err) {
+// Links each developed crystal to the developed crystals it touches (union-find), through the cells:
+// each pair is tested from its first position (the test is symmetric, and the union-find roots do
+// not depend on the order of the unions).  Divergent box queries of the reference tree took 5.8 ms
+// for the 2.1 M developed crystals of a 2048 x 2048 px tri-x image and 0.27 ms for one 64 x 64 px
+// tile's 1,142 (a chain of dependent record loads); the development's whole stage went from 6.1 to
+// 1.2 ms and from 0.30 to 0.08 ms with the cells.
+__global__ void k_link_b(const BTile* __restrict__ bt, const TileDesc* __restrict__ td, int ntiles,
+                         unsigned long long ncap, const float4* __restrict__ A, const float4* __restrict__ D,
+                         const uint32_t* __restrict__ place, const uint8_t* __restrict__ developed, int* parent,
+                         const uint32_t* __restrict__ list, const uint32_t* __restrict__ ndev, uint32_t* err) {
   const unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
   if (i >= ncap || i >= *ndev) return;
   const unsigned long long g = list[i];
-  const BTile& t = bt[btile_of(bt, ntiles, g)];
+  const int ti = btile_of(bt, ntiles, g);
+  const BTile& t = bt[ti];
+  const CellGrid& grid = td[ti].cells;
   const uint32_t s = static_cast<uint32_t>(g - t.cbase);
-  const Node4* nodes = rnode_all + t.rbase;
-  const uint2* leaves = rleaf_all + t.nbase;
-  const uint32_t* ridx = ridx_all + t.cbase;
   const float4* Ab = A + t.cbase;
   const float4* Db = D + t.cbase;
   const uint8_t* dev = developed + t.cbase;
@@ -196,13 +193,10 @@ __global__ void k_link_b(const BTile* __restrict__ bt, int ntiles, unsigned long
   const double rc = __dmul_rn(static_cast<double>(fmaxf(fmaxf(d.x, d.y), d.z)), t.fe);
   const double search = __dmul_rn(__dadd_rn(rc, __dmul_rn(t.max_base, t.fe)), t.prox);
   const float R = static_cast<float>(search) * 1.0001f + 1e-3f;
-  const float3 lo = make_float3(a.x - R, a.y - R, a.z - R), hi = make_float3(a.x + R, a.y + R, a.z + R);
   const float fef = static_cast<float>(t.fe), proxf = static_cast<float>(t.prox);
   const float rcf = fmaxf(fmaxf(d.x, d.y), d.z) * fef;
-  if (t.n < 2) return;
-  const uint32_t nmax = t.ncap;
   auto test = [&](uint32_t j) {
-    if (j <= s || j >= t.n || !dev[j]) return;
+    if (j >= t.n || !dev[j]) return;
     const float4 aj = Ab[j], dj = Db[j];
     const float dx = aj.x - a.x, dy = aj.y - a.y, dz = aj.z - a.z;
     const float d2 = dx * dx + dy * dy + dz * dz;
@@ -224,13 +218,10 @@ __global__ void k_link_b(const BTile* __restrict__ bt, int ntiles, unsigned long
     }
     if (hit) uf_unite_b(parent, static_cast<int>(g), static_cast<int>(t.cbase + j), err);
   };
-  auto leaf = [&](uint32_t id) {
-    if (!index_ok(id < nmax, err, SITE_LEAF, id, nmax)) return;
-    const uint2 L = leaves[id];
-    if (!index_ok(L.x + L.y <= t.n, err, SITE_LEAF, L.x, L.y)) return;
-    for (uint32_t k = 0; k < L.y; ++k) test(ridx[L.x + k]);
-  };
-  rt_walk4_box(nodes, lo, hi, t.rcap, err, leaf);
+  const float R2 = R * R;
+  cells_around(grid, make_float3(a.x, a.y, a.z), R, place[g], err, [&](uint32_t p, float d2) {
+    if (d2 <= R2) test(cell_slot(grid, p));
+  });
 }
 
 __global__ void k_roots_b(unsigned long long ncap, const uint8_t* developed, int* parent, uint32_t* size,
@@ -567,10 +558,10 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
   FG_CUDA(cudaGetLastError());
 }
 
-// The reference tree of every tile over its crystals (in slot order), for the development's touch
-// queries and the walk order of the transport's hits, and the crystals in cells.
+// The reference tree of every tile over its crystals (in slot order), for its leaf boxes and walk
+// order, and the crystals in cells.
 static void stage_bvh(fg_batch* B, cudaStream_t st) {
-  rtree_build(B->rt, B->e->d_err, st);
+  rtree_build(B->rt, B->e->d_err, st, false);
   const int nt = static_cast<int>(B->ntiles);
   FG_CUDA(cudaMemsetAsync(B->tcells.cnt.p, 0, (B->tcells.ncells + 1) * sizeof(uint32_t), st));
   launch_cells_count(B->d_td.p, nt, B->ncap, B->A.p, B->tcells.cnt.p, B->tcells.place.p, st);
@@ -610,8 +601,8 @@ static void stage_develop(fg_batch* B, cudaStream_t st) {
   FG_CUDA(cudaMemsetAsync(B->devflag.p + B->ncap, 0, sizeof(uint32_t), st));
   cub_scan(B, B->devflag.p, B->devscan.p, B->ncap + 1, st);
   k_devlist_b<<<G, 256, 0, st>>>(B->ncap, B->devflag.p, B->devscan.p, B->devlist.p);
-  k_link_b<<<G, 256, 0, st>>>(B->d_bt.p, nt, B->ncap, B->A.p, B->D.p, B->rt.rnode.p, B->rt.rleaf.p, B->rt.ridx.p,
-                              B->developed.p, B->parent.p, B->devlist.p, B->devscan.p + B->ncap, e->d_err);
+  k_link_b<<<G, 256, 0, st>>>(B->d_bt.p, B->d_td.p, nt, B->ncap, B->A.p, B->D.p, B->tcells.place.p, B->developed.p,
+                              B->parent.p, B->devlist.p, B->devscan.p + B->ncap, e->d_err);
   FG_CUDA(cudaMemsetAsync(B->size.p, 0, B->ncap * sizeof(uint32_t), st));
   k_roots_b<<<G, 256, 0, st>>>(B->ncap, B->developed.p, B->parent.p, B->size.p, e->d_err);
   k_finalize_b<<<G, 256, 0, st>>>(B->d_bt.p, nt, B->ncap, B->developed.p, B->parent.p, B->size.p, B->exp64.p,
@@ -626,7 +617,7 @@ static void stage_scan(fg_batch* B, cudaStream_t st) {
   // The scan's tree: the same buffers, rebuilt over each tile's developed crystals (the transport
   // and the touch queries are done with the first tree by now).
   k_scan_tree_tiles<<<grid_for(B->ntiles, 128), 128, 0, st>>>(B->d_bt.p, nt, B->devscan.p, B->devlist.p, B->rt_scan.p);
-  rtree_build(B->rt, e->d_err, st, B->rt_scan.p);
+  rtree_build(B->rt, e->d_err, st, false, B->rt_scan.p);
   launch_scan_prep_list(B->d_sc.p, nt, B->devlist.p, B->devscan.p + B->ncap, B->ncap, B->prep.p, st);
   FG_CUDA(cudaMemsetAsync(B->bin_cnt.p, 0, (B->nbins + 1) * sizeof(uint32_t), st));
   FG_CUDA(cudaMemsetAsync(B->bin_cur.p, 0, (B->nbins + 1) * sizeof(uint32_t), st));
@@ -820,13 +811,10 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       // The synthesis's radius clamp (emulsion.rs:162-170) for cubes; the other shapes lie in their boxes.
       t.reach = rt_reach(B->params[i].morphology == FG_CUBIC ? 0.48 * B->params[i].r_min : 0.0);
     }
-    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC, 0, true);
+    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC, 0, true, false);
     for (uint32_t i = 0; i < n; ++i) {
       FG_REQUIRE(rt[i].ebase == B->syn[i].cbase, "tree layout differs from the crystal slots");
       B->bt[i].nbase = rt[i].nbase;
-      B->bt[i].ncap = rt[i].ncap;
-      B->bt[i].rbase = rt[i].rbase;
-      B->bt[i].rcap = rt[i].rcap;
       B->td[i].nnodes = rt[i].ncap;
       B->td[i].reach = rt[i].reach;
       rs[i] = rt[i];
@@ -909,8 +897,8 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   // Per crystal slot: records 48 (and 96 in the transport's cells), key 8, links and flags 36,
   // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
-  // 224 B (plus slack); transport cells 8 B; synthesis cells 4 B; bricks 8 B; photon order; images.
-  return static_cast<unsigned long long>(s.ccap) * 680ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
+  // 152 B (plus slack); transport cells 8 B; synthesis cells 4 B; bricks 8 B; photon order; images.
+  return static_cast<unsigned long long>(s.ccap) * 620ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          (8ull << (2 * s.slot_bits)) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
@@ -1168,7 +1156,7 @@ fg_status fg_batch_wait(fg_batch* b, fg_batch_stats* stats) {
     // roots + finalize, scan-tree inputs, scan prep, two bin passes, scan, density, the two passes over the
     // transport's cells, and the two tree builds (each level's launches included, also those that
     // find no work; CUB scans not counted).
-    s.kernel_launches = 1 + 2 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt);
+    s.kernel_launches = 1 + 2 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt, false);
     b->stats = s;
     if (stats) *stats = s;
   });

@@ -1,5 +1,6 @@
 // Builds the cells of fg_cells.cuh: count the crystals of every cell, prefix sum, then write each
-// crystal's record at its position with its leaf box and walk rank from the reference tree.
+// crystal's record at its position with its leaf box and walk rank from the reference tree; place
+// then holds the position of each slot.
 //
 // Both passes stream the crystals in slot order (compact blocks of the film), so the counters and
 // the scattered records of a warp fall into few cache lines.
@@ -43,7 +44,7 @@ __global__ void k_cells_count(const TileDesc* __restrict__ tiles, int ntiles, un
 
 __global__ void k_cells_fill(const TileDesc* __restrict__ tiles, int ntiles, unsigned long long ncap,
                              const float4* __restrict__ A, const float4* __restrict__ Q, const float4* __restrict__ D,
-                             const uint32_t* __restrict__ off, const uint32_t* __restrict__ place,
+                             const uint32_t* __restrict__ off, uint32_t* __restrict__ place,
                              const uint32_t* __restrict__ rank, const uint32_t* __restrict__ leafof,
                              const double* __restrict__ box64, float4* __restrict__ pos, float4* __restrict__ q,
                              float4* __restrict__ d, float4* __restrict__ leaf, uint2* __restrict__ by_rank,
@@ -57,6 +58,7 @@ __global__ void k_cells_fill(const TileDesc* __restrict__ tiles, int ntiles, uns
   const uint32_t p = off[cell_index(t.cells, a)] + place[g];
   const uint32_t r = rank[g], lf = leafof[g];
   if (!index_ok(p < t.cells.npos && r < t.n && lf < t.nnodes, err, SITE_CELL, p, r)) return;
+  place[g] = p;
   pos[p] = make_float4(a.x, a.y, a.z, cell_ball2(dd));
   q[p] = Q[g];
   d[p] = dd;
@@ -64,7 +66,8 @@ __global__ void k_cells_fill(const TileDesc* __restrict__ tiles, int ntiles, uns
   const double* b = box64 + 6ull * (t.nbase + lf);
   leaf[2ull * p] = make_float4(__double2float_rn(b[0]), __double2float_rn(b[1]), __double2float_rn(b[2]),
                                __double2float_rn(b[3]));
-  leaf[2ull * p + 1] = make_float4(__double2float_rn(b[4]), __double2float_rn(b[5]), __uint_as_float(r), 0.0f);
+  leaf[2ull * p + 1] = make_float4(__double2float_rn(b[4]), __double2float_rn(b[5]), __uint_as_float(r),
+                                   __uint_as_float(static_cast<uint32_t>(s)));
   by_rank[t.cbase + r] = make_uint2(static_cast<uint32_t>(s), __float_as_uint(a.w));
 }
 

@@ -34,7 +34,7 @@ struct __align__(16) CellGrid {
   float _pad;
   const float4* q;
   const float4* d;
-  const float4* leaf;     // two per position: leaf box lo xyz, hi x; hi y, hi z, rank (bits), unused
+  const float4* leaf;     // two per position: leaf box lo xyz, hi x; hi y, hi z, rank, slot (bits)
   const uint2* by_rank;   // per rank: crystal slot, sensitivity (bits)
   unsigned long long cell_base;  // first cell of this tile in the allocation
   float hx, hy, hz;       // the box
@@ -107,6 +107,7 @@ struct CellVisit {
   uint32_t c, cend;       // positions of the row still to test
 };
 
+// The grid must lie in device memory (the read goes through the read-only path).
 __device__ __forceinline__ CellAxis cell_axis(const CellAxis& a) {
   const float4 v = __ldg(reinterpret_cast<const float4*>(&a));
   return CellAxis{v.x, v.y, v.z, __float_as_uint(v.w)};
@@ -164,6 +165,34 @@ __device__ __forceinline__ void cells_advance(const CellGrid& g, float3 o, float
   if (!index_ok(c0 <= c1 && c1 <= g.npos, err, SITE_CELL, c0, c1)) return;
   v.c = c0;
   v.cend = c1;
+}
+
+// Every crystal after position p whose centre lies within R of p's centre a in each axis (fn(position,
+// squared distance)): the rows from p's own on, so each pair is seen once, from its first crystal.
+template <class F>
+__device__ __forceinline__ void cells_around(const CellGrid& g, float3 a, float R, uint32_t p, uint32_t* err, F&& fn) {
+  const CellAxis ax = cell_axis(g.x), ay = cell_axis(g.y), az = cell_axis(g.z);
+  const float Rs = R + g.slack;
+  const int x0 = cell_coord(a.x - Rs, ax.inv, ax.last), x1 = cell_coord(a.x + Rs, ax.inv, ax.last);
+  const int z0 = cell_coord(a.z - Rs, az.inv, az.last), z1 = cell_coord(a.z + Rs, az.inv, az.last);
+  const int yc = cell_coord(a.y, ay.inv, ay.last), y1 = cell_coord(a.y + Rs, ay.inv, ay.last);
+  const int zc = cell_coord(a.z, az.inv, az.last);
+  for (int y = yc; y <= y1; ++y)
+    for (int z = y == yc ? zc : z0; z <= z1; ++z) {
+      const uint32_t* row = g.off + (static_cast<uint32_t>(y) * az.n + static_cast<uint32_t>(z)) * ax.n;
+      const uint32_t c0 = y == yc && z == zc ? p + 1 : __ldg(row + x0), c1 = __ldg(row + x1 + 1);
+      if (!index_ok(c1 <= g.npos, err, SITE_CELL, c0, c1)) continue;
+      for (uint32_t c = c0; c < c1; ++c) {
+        const float4 b = __ldg(&g.pos[c]);
+        const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+        fn(c, dx * dx + dy * dy + dz * dz);
+      }
+    }
+}
+
+// Crystal slot at a position.
+__device__ __forceinline__ uint32_t cell_slot(const CellGrid& g, uint32_t p) {
+  return __float_as_uint(__ldg(&g.leaf[2ull * p + 1].w));
 }
 
 }  // namespace fg

@@ -5,9 +5,8 @@
 // index order.  Its clumps are exactly the connected components of the symmetric "touch" graph
 // |p_i - p_j|^2 <= ((r_i fe + r_j fe) prox)^2 over developed crystals (every touch test uses the
 // base expansion fe; the boost is applied after a component is complete).  Here each developed
-// crystal finds its touching neighbours through a box query on the emulsion's reference tree
-// (the four-wide walk records, fg_rtree.cuh) and links them with a
-// lock-free union-find.  Clump ids follow the reference's numbering: components ranked by their
+// crystal finds its touching neighbours through the emulsion's cells (fg_cells.cuh), or a box query
+// on its reference tree where the set has none, and links them with a lock-free union-find.  Clump ids follow the reference's numbering: components ranked by their
 // smallest crystal index.  Touch decisions are exact: an FP32 test with an error margin, and the
 // reference's FP64 expression when the margin is too thin to decide.
 #include <cstring>
@@ -62,7 +61,10 @@ __device__ __forceinline__ void uf_unite(int* parent, int a, int b, uint32_t* er
   atomicOr(err, ERR_SPIN_LIMIT);
 }
 
-__global__ void k_link(CrystalsView cv, const Node4* __restrict__ rec, uint32_t nrec, const uint2* __restrict__ rleaf,
+// The cells see each pair from its first position, the tree query from its lower slot; the roots do
+// not depend on it (the touch test is symmetric).
+__global__ void k_link(CrystalsView cv, const CellGrid* __restrict__ grid, const uint32_t* __restrict__ place,
+                       const Node4* __restrict__ rec, uint32_t nrec, const uint2* __restrict__ rleaf,
                        uint32_t nleaf, const uint32_t* __restrict__ ridx, uint32_t n,
                        const uint8_t* __restrict__ developed, double fe, double prox,
                        double max_base, int* parent, DevCounters* dc, uint32_t* err) {
@@ -79,7 +81,7 @@ __global__ void k_link(CrystalsView cv, const Node4* __restrict__ rec, uint32_t 
   const float rcf = fmaxf(fmaxf(d.x, d.y), d.z) * fef;
   unsigned long long fb = 0;
   auto test = [&](uint32_t j) {
-    if (j <= s || j >= n || !developed[j]) return;
+    if (j >= n || !developed[j]) return;
     const float4 aj = cv.a[j], dj = cv.d[j];
     const float dx = aj.x - a.x, dy = aj.y - a.y, dz = aj.z - a.z;
     const float d2 = dx * dx + dy * dy + dz * dz;
@@ -104,12 +106,22 @@ __global__ void k_link(CrystalsView cv, const Node4* __restrict__ rec, uint32_t 
     }
     if (touch_hit) uf_unite(parent, static_cast<int>(s), static_cast<int>(j), err);
   };
-  rt_walk4_box(rec, lo, hi, nrec, err, [&](uint32_t leaf) {
-    if (!index_ok(leaf < nleaf, err, SITE_LEAF, leaf, nleaf)) return;
-    const uint2 L = rleaf[leaf];
-    if (!index_ok(L.x + L.y <= n, err, SITE_LEAF, L.x, L.y)) return;
-    for (uint32_t k = 0; k < L.y; ++k) test(ridx[L.x + k]);
-  });
+  if (grid) {
+    const float R2 = R * R;
+    cells_around(*grid, make_float3(a.x, a.y, a.z), R, place[s], err, [&](uint32_t p, float d2) {
+      if (d2 <= R2) test(cell_slot(*grid, p));
+    });
+  } else {
+    rt_walk4_box(rec, lo, hi, nrec, err, [&](uint32_t leaf) {
+      if (!index_ok(leaf < nleaf, err, SITE_LEAF, leaf, nleaf)) return;
+      const uint2 L = rleaf[leaf];
+      if (!index_ok(L.x + L.y <= n, err, SITE_LEAF, L.x, L.y)) return;
+      for (uint32_t k = 0; k < L.y; ++k) {
+        const uint32_t j = ridx[L.x + k];
+        if (j > s) test(j);
+      }
+    });
+  }
   if (fb) atomicAdd(&dc->fallbacks, fb);
 }
 
@@ -210,7 +222,7 @@ void develop(fg_engine* e, fg_emulsion* em, const fg_dev_cfg& cfg, fg_dev_report
   FG_CUDA(cudaStreamSynchronize(st));
   double max_base;
   std::memcpy(&max_base, &mbits, sizeof(double));
-  k_link<<<G, 256, 0, st>>>(em->view(), em->rt.rnode.p, static_cast<uint32_t>(em->rt.R), em->rt.rleaf.p,
+  k_link<<<G, 256, 0, st>>>(em->view(), em->grid_dev.p, em->cells.place.p, em->rt.rnode.p, static_cast<uint32_t>(em->rt.R), em->rt.rleaf.p,
                             static_cast<uint32_t>(em->rt.N), em->rt.ridx.p, n, em->developed.p, cfg.filament_expansion,
                             cfg.clumping_proximity_factor, max_base, parent.p, dc.p, e->d_err);
   k_roots<<<G, 256, 0, st>>>(n, em->developed.p, parent.p, s2id, size.p, minid.p, e->d_err);

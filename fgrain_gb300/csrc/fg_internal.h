@@ -150,7 +150,7 @@ struct RTreeBufs {
 // fg_cells.cu: the crystals of a batch's tiles (or one emulsion) in cells (CellGrid).
 struct CellBufs {
   unsigned long long ncells = 0;
-  DBuf<uint32_t> cnt, off, place;  // per cell: crystals, first position; per slot: number in its cell
+  DBuf<uint32_t> cnt, off, place;  // per cell: crystals, first position; per slot: its position
   DBuf<float4> pos, q, d, leaf;
   DBuf<uint2> by_rank;
   void alloc(unsigned long long ncap, unsigned long long cells, cudaStream_t st);
@@ -188,6 +188,7 @@ struct fg_emulsion {
   // on the tree walk (cells_suit).
   fg::CellBufs cells;
   fg::CellGrid grid{};
+  fg::DBuf<fg::CellGrid> grid_dev;  // grid, in device memory (device code reads its axes as vectors)
   // Mutable per-crystal state (Morton order).
   fg::DBuf<uint32_t> counts;
   fg::DBuf<uint8_t> developed;
@@ -234,12 +235,14 @@ void build_emulsion_cells(fg_engine* e, fg_emulsion* em);
 // leafof (when wanted) gets max(elements, leafof_slots) words: it is indexed by element slot.
 // rank (when wanted) gets as many.
 void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cudaStream_t st, double node_frac = 1.0,
-                 size_t leafof_slots = 0, bool want_rank = false);
+                 size_t leafof_slots = 0, bool want_rank = false, bool walks = true);
 // Enqueues a build (capturable: no host synchronisation).  tiles_dev (optional) replaces the tile
 // array of the allocation by one with the same layout (ebase, nbase, ecap, ncap) but other element
 // sources, so that one set of buffers serves several trees in turn.
-void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, RTile* tiles_dev = nullptr);
-unsigned rtree_kernel_launches(const RTreeBufs& B);
+// walks: also the boxes above the leaves and the walk records (a build that only gives leaves, ranks
+// and leaf boxes does without).
+void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, RTile* tiles_dev = nullptr);
+unsigned rtree_kernel_launches(const RTreeBufs& B, bool walks);
 // One tile's build in memory the caller holds (nothing allocated): bytes needed for a tile of ecap
 // elements, and the attach that carves every buffer (the tile descriptor too) from `base`
 // (256-byte aligned).  The tile's source pointers are set by the caller; tile.n may be written on
@@ -251,7 +254,7 @@ void rtree_attach(RTreeBufs& B, RTile tile, bool want_leafof, uint32_t leafof_sl
 // expansion (the scan's tree, transmittance.rs:86-89), elements in crystal-id order.  list keeps
 // the developed element list alive for the build.
 void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_only, RTreeBufs& B,
-                         DBuf<uint32_t>& list);
+                         DBuf<uint32_t>& list, bool walks = true);
 
 // fg_develop.cu
 void develop(fg_engine* e, fg_emulsion* em, const fg_dev_cfg& cfg, fg_dev_report* rep);

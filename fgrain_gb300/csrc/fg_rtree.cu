@@ -539,7 +539,7 @@ __device__ __forceinline__ void rt_store_box(const RtArgs& A, uint32_t id, const
 }
 
 // Four blocks per SM (64 registers; the block's shared memory is about 53 KB): 9 % faster than two.
-__global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
+__global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
   extern __shared__ __align__(32) unsigned char rt_cta_raw[];
   RtCtaSmem& S = *reinterpret_cast<RtCtaSmem*>(rt_cta_raw);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
           for (int j = 0; j < cn; ++j) rt_fold_box(A.tiles[t], S.idx[S.off[cur][i] + j], k);
           rt_store_box(A, id, k);
         } else {
-          A.P[s + static_cast<uint32_t>(atomicAdd(&S.nint, 1))] = id;  // its box after the last level
+          if (walks) A.P[s + static_cast<uint32_t>(atomicAdd(&S.nint, 1))] = id;  // its box after the last level
           const double ca = axis == 0 ? clo[0] : (axis == 1 ? clo[1] : clo[2]);
           const double cb = axis == 0 ? chi[0] : (axis == 1 ? chi[1] : chi[2]);
           const double mid = __dmul_rn(0.5, __dadd_rn(ca, cb));
@@ -678,10 +678,11 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
           S.mid[i] = mid;
           S.child[i] = static_cast<uint32_t>(nb + l);
           A.nsplit[id] = axis;
-          A.nmid[id] = mid;
-          A.nchild[id] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
-          A.parent[nb + l] = id;
-          A.parent[nb + l + 1] = id;
+          if (walks) {
+            A.nchild[id] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
+            A.parent[nb + l] = id;
+            A.parent[nb + l + 1] = id;
+          }
         }
       }
       __syncthreads();
@@ -813,7 +814,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
     }
     // The internal nodes' boxes, deepest level first: each the union of its children's, written
     // by this block before the barrier (leaves at their creation, internal nodes a level below).
-    for (int L = S.nlvl - 1; L >= 0; --L) {
+    for (int L = walks ? S.nlvl - 1 : -1; L >= 0; --L) {
       const int b0 = L ? S.lvend[L - 1] : 0, b1 = S.lvend[L];
       for (int k = b0 + tid; k < b1; k += RT_CTA_T) {
         const uint32_t id = A.P[s + static_cast<uint32_t>(k)];
@@ -879,12 +880,14 @@ __global__ void k_rt_refit(RtArgs A, uint32_t* arrive) {
   }
 }
 
-// Walk records (fg_rtree.cuh): one thread per node.  A leaf fills its element range, the leaf-of
-// map and its elements' ranks (the walk takes the right subtree first, so leaves in descending
-// element position, and a leaf's elements in index order); the root and every internal node at odd depth write their four-wide record, the
+// One thread per node.  A leaf fills the leaf-of map and its elements' ranks (the walk takes the
+// right subtree first, so leaves in descending element position, and a leaf's elements in index
+// order).  With WALKS it also fills its element range, and the root and every internal node at odd
+// depth write their four-wide record (fg_rtree.cuh), the
 // grandchildren in the reference's visiting order (right before left, a leaf child in one slot).
 // An internal slot's box is rounded outward, padded and extended by the reach; a leaf slot's box
 // is rounded to nearest.
+template <bool WALKS>
 __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafof, unsigned long long leafof_n,
                              uint32_t* rank) {
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
@@ -920,7 +923,7 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
       *out = nd;
     };
     if (id == 0) {  // the super-root slot: an empty tree's record 0
-      if (T.n == 0 && T.rcap > 0) put(0, R);
+      if (WALKS && T.n == 0 && T.rcap > 0) put(0, R);
       continue;
     }
     if (id == 1 && T.n == 0) continue;
@@ -931,7 +934,7 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
         atomicOr(A.err, ERR_BAD_INDEX);
         continue;
       }
-      rleaf[g] = make_uint2(static_cast<uint32_t>(st - T.ebase), cn);
+      if (WALKS) rleaf[g] = make_uint2(static_cast<uint32_t>(st - T.ebase), cn);
       if (leafof)
         for (uint32_t k = 0; k < cn; ++k) {
           const uint32_t slot = A.ridx[st + k];
@@ -943,7 +946,7 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
           }
         }
     }
-    if (id != 1 && (leaf || !(A.ndepth[g] & 1u))) continue;
+    if (!WALKS || (id != 1 && (leaf || !(A.ndepth[g] & 1u)))) continue;
     // Slot k takes node c (a global id inside the tile): its box and reference.
     int k = 0;
     bool bad = false;
@@ -1053,7 +1056,7 @@ RtArgs rt_args(RTreeBufs& B, uint32_t* err) {
 }
 
 void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cudaStream_t st, double node_frac,
-                 size_t leafof_slots, bool want_rank) {
+                 size_t leafof_slots, bool want_rank, bool walks) {
   B.ntiles = static_cast<int>(tiles.size());
   unsigned long long e = 0, nn = 0;
   uint32_t emax = 0;
@@ -1106,8 +1109,10 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.bq.alloc(N1, st);
   B.bqpar.alloc(N1, st);
   B.cnt.alloc(4, st);
-  B.rnode.alloc(std::max<unsigned long long>(rr, 1), st);
-  B.rleaf.alloc(N1, st);
+  if (walks) {
+    B.rnode.alloc(std::max<unsigned long long>(rr, 1), st);
+    B.rleaf.alloc(N1, st);
+  }
   if (want_leafof) B.leafof.alloc(std::max(E1, leafof_slots), st);
   if (want_rank) B.rank.alloc(std::max(E1, leafof_slots), st);
   FG_CUDA(cudaMemsetAsync(B.ridx.p, 0, E1 * sizeof(uint32_t), st));
@@ -1192,7 +1197,7 @@ void rtree_attach(RTreeBufs& B, RTile tile, bool want_leafof, uint32_t leafof_sl
   FG_CUDA(cudaMemcpyAsync(B.tiles.p, &tile, sizeof(RTile), cudaMemcpyHostToDevice, st));
 }
 
-void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, RTile* tiles_dev) {
+void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, RTile* tiles_dev) {
   if (B.ntiles == 0) return;
   RtArgs A = rt_args(B, err);
   if (tiles_dev) A.tiles = tiles_dev;
@@ -1218,11 +1223,15 @@ void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, RTile* tiles_dev)
   static_assert(sizeof(RtCtaSmem) <= 56 * 1024, "four blocks of the block phase must fit an SM");
   FG_CUDA(cudaFuncSetAttribute(k_rt_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(sizeof(RtCtaSmem))));
-  k_rt_cta<<<GC, RT_CTA_T, sizeof(RtCtaSmem), st>>>(A);
-  // The global worklist is spent: its words count the children that reached each node.
-  FG_CUDA(cudaMemsetAsync(B.wl0.p, 0, static_cast<size_t>(B.N) * sizeof(uint32_t), st));
-  k_rt_refit<<<GN, RT_BLOCK, 0, st>>>(A, B.wl0.p);
-  k_rt_records<<<GN, RT_BLOCK, 0, st>>>(A, B.rnode.p, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
+  k_rt_cta<<<GC, RT_CTA_T, sizeof(RtCtaSmem), st>>>(A, walks);
+  if (walks) {
+    // The global worklist is spent: its words count the children that reached each node.
+    FG_CUDA(cudaMemsetAsync(B.wl0.p, 0, static_cast<size_t>(B.N) * sizeof(uint32_t), st));
+    k_rt_refit<<<GN, RT_BLOCK, 0, st>>>(A, B.wl0.p);
+    k_rt_records<true><<<GN, RT_BLOCK, 0, st>>>(A, B.rnode.p, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
+  } else {
+    k_rt_records<false><<<GN, RT_BLOCK, 0, st>>>(A, nullptr, nullptr, B.leafof.p, B.leafof.n, B.rank.p);
+  }
   k_rt_depth_check<<<grid_for(static_cast<size_t>(B.ntiles), 128), 128, 0, st>>>(A);
   FG_CUDA(cudaGetLastError());
 }
@@ -1243,7 +1252,7 @@ __global__ void k_rt_id_scatter(const uint32_t* id2s, uint32_t n, const uint32_t
 }
 
 void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_only, RTreeBufs& B,
-                         DBuf<uint32_t>& list) {
+                         DBuf<uint32_t>& list, bool walks) {
   cudaStream_t st = e->stream;
   const uint32_t n = em->n;
   RTile t{};
@@ -1273,13 +1282,13 @@ void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_onl
   t.ecap = developed_only ? std::max<uint32_t>(m, 1) : std::max<uint32_t>(n, 1);
   t.n = developed_only ? m : n;
   std::vector<RTile> v{t};
-  rtree_alloc(B, v, true, st, 1.0, n, !developed_only);
-  rtree_build(B, e->d_err, st);
+  rtree_alloc(B, v, true, st, 1.0, n, !developed_only, walks);
+  rtree_build(B, e->d_err, st, walks);
   B.count = t.n;
 }
 
-unsigned rtree_kernel_launches(const RTreeBufs& B) {
-  return B.ntiles ? 1u + 8u * static_cast<unsigned>(B.levels) + 5u : 0u;
+unsigned rtree_kernel_launches(const RTreeBufs& B, bool walks) {
+  return B.ntiles ? 1u + 8u * static_cast<unsigned>(B.levels) + (walks ? 5u : 4u) : 0u;
 }
 
 }  // namespace fg

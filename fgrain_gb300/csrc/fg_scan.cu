@@ -674,7 +674,7 @@ static void plan_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cf
   const uint32_t a = std::max<uint32_t>(g * g, 1);
   FG_REQUIRE(a <= SCAN_THREADS, "samples_per_pixel too large (at most 256 strata)");
   FG_REQUIRE(cfg.width_px > 0 && cfg.height_px > 0, "scan size must be positive");
-  build_emulsion_tree(e, em, true, P.tree, P.tree_list);
+  build_emulsion_tree(e, em, true, P.tree, P.tree_list, false);
   ScanTile& t = P.t;
   t = ScanTile{};
   t.lbox64 = P.tree.box64.p;

@@ -533,9 +533,13 @@ void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   FG_CUDA(cudaMemcpyAsync(&c, unfit.p, sizeof(c), cudaMemcpyDeviceToHost, st));
   FG_CUDA(cudaStreamSynchronize(st));
   em->cells.cnt.release();
-  em->cells.place.release();
-  if (!c) em->grid = g;
-  else em->cells = CellBufs{};
+  if (c) {
+    em->cells = CellBufs{};
+    return;
+  }
+  em->grid = g;
+  em->grid_dev.alloc(1, st);
+  FG_CUDA(cudaMemcpyAsync(em->grid_dev.p, &em->grid, sizeof(CellGrid), cudaMemcpyHostToDevice, st));
 }
 
 void expose(fg_engine* e, fg_emulsion* em, const float* tile_dev, uint32_t tw, uint32_t th,

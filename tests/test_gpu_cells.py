@@ -69,3 +69,27 @@ def test_counts_match_the_oracle(engine, name):
     np.testing.assert_array_less(np.abs(got - ref), 2.0 + 1e-3 * ref + 1e-9)
     assert abs(engine.timings()["hits"] - hits) <= 2 + 1e-3 * hits
     em.close()
+
+
+@pytest.mark.parametrize("name", ["even", "many hits", "one crystal", "one long row", "one giant", "outside the box"])
+def test_clumps_match_the_oracle(engine, name):
+    """Development (development.rs:59-188) over the cells, or over the tree where the set has none:
+    mask, clump ids and expansions exactly."""
+    (w, h, d), pos, dims, quat, morph, _ = case(name)
+    quat = quat / np.linalg.norm(quat, axis=1, keepdims=True)
+    n = len(pos)
+    cfg = fg.EmulsionConfig((w, h, d), 1.0, 0.5, 0.2, fg.Morphology(morph))
+    counts = np.random.default_rng(14).integers(0, 8, n).astype(np.uint32)
+    em = fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(n), engine=engine)
+    em.set_latent_counts(counts)
+    dcfg = fg.DevelopmentConfig(4, 1.2, 1.25, 0.85)
+    rep = fg.develop_emulsion(em, dcfg)
+    cr = orc.Crystals(pos, dims, quat, np.ones(n), np.full(n, morph))
+    cr.latent[:] = counts
+    ref = orc.develop(cr, dcfg)
+    dv, cl, ex = em.development()
+    np.testing.assert_array_equal(dv, cr.developed)
+    np.testing.assert_array_equal(cl, cr.clump)
+    np.testing.assert_array_equal(ex, np.where(cr.developed, cr.expansion, 0.0))
+    assert rep.total_clumps == ref["total_clumps"]
+    em.close()
