@@ -1,4 +1,6 @@
 // Transmittance scan kernels: binning of developed crystals and the binned scan itself.
+#include <type_traits>
+
 #include "fg_internal.h"
 #include "fg_scan.cuh"
 
@@ -105,19 +107,26 @@ enum : int { K_CUBE = 0, K_CUBE_DF = 1, K_ELLIPSOID = 2, K_FP64 = 3 };
 
 // Shared-memory image of a staged crystal (index c of the current chunk).  Coordinates are
 // relative to the bin corner and carried as float pairs (hi + lo) so that ray-minus-crystal
-// offsets are accurate to ~1e-8 um.
+// offsets are accurate to ~1e-8 um.  176 bytes, read as float4: 11 is odd, so the lanes of a warp,
+// which test different crystals, spread over the banks.
+struct __align__(16) Staged {
+  float4 rect;        // x0, x1, y0, y1 (high words, with slack) outside of which no ray hits
+  float4 c;           // centre: x hi, x lo, y hi, y lo
+  float4 lbh, lbl;    // leaf box x0, x1, y0, y1: high words, low words
+  float4 misc;        // delta, err, sig, kind (bits)
+  float4 g[6];        // ScanPrep::g
+};
 struct ScanSmem {
-  float cxh[SCAN_CH], cxl[SCAN_CH], cyh[SCAN_CH], cyl[SCAN_CH];
-  // Leaf box x / y extent relative to the corner, float pairs: x0, x1, y0, y1.
-  float lbh[4][SCAN_CH], lbl[4][SCAN_CH];
-  float m[SCAN_CH], delta[SCAN_CH], err[SCAN_CH], sig[SCAN_CH];
-  float g[21][SCAN_CH];
+  Staged k[SCAN_CH];
   int s[SCAN_CH];
-  int kind[SCAN_CH];
   double T[SCAN_THREADS];
 };
 
 constexpr float EPS32 = 5.9604645e-8f;  // 2^-24
+
+// Slack of a comparison on the high words of two coordinates of magnitude up to v (um): they differ
+// from their float pairs by half an ulp each, and the difference rounds once more.
+__device__ __forceinline__ float hi_slack(float v) { return 1e-4f + 5e-7f * v; }
 
 // Stages crystal s for vertical rays relative to the bin corner (bx0, by0).  Everything is
 // derived in FP64 once per crystal and CTA, then rounded:
@@ -138,7 +147,6 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
   split64(lb[3], P.ch[3], P.cl[3]);
   split64(lb[1], P.ch[4], P.cl[4]);
   split64(lb[4], P.ch[5], P.cl[5]);
-  P.m = m;
   P.delta = static_cast<float>(t.z0 - k.pos.z);
   P.sig = t.sigma_c ? t.sigma_c[s] : t.sigma;
   const double x = k.q[0], y = k.q[1], z = k.q[2], w = k.q[3];
@@ -147,19 +155,22 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
   const double R1[3] = {2.0 * (x * y + z * w), 1.0 - 2.0 * (x * x + z * z), 2.0 * (y * z - x * w)};
   const double R2[3] = {2.0 * (x * z - y * w), 2.0 * (y * z + x * w), 1.0 - 2.0 * (x * x + y * y)};
   const double D[3] = {k.dims.x * e64, k.dims.y * e64, k.dims.z * e64};
-#pragma unroll
-  for (int i = 0; i < 21; ++i) P.g[i] = 0.0f;
+  float hx = 0.0f, hy = 0.0f;
   if (k.morph == 0) {
     float invmax = 0.0f;
     const float Dmax = static_cast<float>(fmax(fmax(D[0], D[1]), D[2]));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      split64(R0[i], P.g[i], P.g[3 + i]);
-      split64(R1[i], P.g[6 + i], P.g[9 + i]);
       const float inv = static_cast<float>(1.0 / (-R2[i]));
-      P.g[12 + i] = inv;
-      split64(D[i], P.g[15 + i], P.g[18 + i]);
+      float r0, r0l, r1, r1l, d, dl;
+      split64(R0[i], r0, r0l);
+      split64(R1[i], r1, r1l);
+      split64(D[i], d, dl);
+      P.g[i] = make_float4(r0, r1, inv, d);
+      P.g[3 + i] = make_float4(r0l, r1l, dl, 0.0f);
       invmax = fmaxf(invmax, fabsf(inv));
+      hx += fabsf(r0) * d;
+      hy += fabsf(r1) * d;
     }
     if (!(invmax < 1e30f)) {
       P.kind = K_FP64;
@@ -182,46 +193,69 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
     const double Dmin = fmin(fmin(D[0], D[1]), D[2]);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      P.g[i] = static_cast<float>(R0[i] / D[i]);
-      P.g[3 + i] = static_cast<float>(R1[i] / D[i]);
       const double ei = -R2[i] / D[i];
-      P.g[6 + i] = static_cast<float>(ei);
+      P.g[i] = make_float4(static_cast<float>(R0[i] / D[i]), static_cast<float>(R1[i] / D[i]), static_cast<float>(ei), 0.0f);
+      P.g[3 + i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       A += ei * ei;
+      const float Df = static_cast<float>(D[i]), u = static_cast<float>(R0[i]) * Df, v = static_cast<float>(R1[i]) * Df;
+      hx += u * u;
+      hy += v * v;
     }
-    P.g[9] = static_cast<float>(A);
-    P.g[10] = static_cast<float>(1.0 / A);
+    hx = sqrtf(hx);
+    hy = sqrtf(hy);
+    P.g[0].w = static_cast<float>(1.0 / A);
     // h = 1 - |P_perp|^2; P (|P| <= sqrt(2) m / Dmin) and P_perp = P + tc e carry ~8 eps |P|
     // each, so |d h| <= 2 |P_perp| 8 eps sqrt(3) Pmax + 4 eps; four times that as the bound.
     const float Pmax = static_cast<float>(1.4142135623730951 * m64 / Dmin);
     P.err = 4.0f * (2.0f * 1.05f * 8.0f * EPS32 * 1.7320508f * Pmax + 4.0f * EPS32) + 1e-9f;
   }
+  P.g[4].w = hx * 1.0001f;
+  P.g[5].w = hy * 1.0001f;
 }
 
-// Stages crystal s for the bin whose 16-px-square corner is (bxh + bxl, byh + byl): the
-// bin-independent terms (from t.prep, or derived here), and the centre and leaf box relative to
-// the corner as float pairs (float arithmetic only).
+// Stages crystal s, whose bin-independent terms are P, for the bin whose 16-px-square corner is (bxh +
+// bxl, byh + byl): those terms, and the centre and leaf box relative to the corner as float pairs
+// (float arithmetic only).
+__device__ __forceinline__ void stage_prepared(const ScanPrep& P, ScanSmem& sm, int c, uint32_t s, float bxh, float bxl,
+                                               float byh, float byl) {
+  Staged& S = sm.k[c];
+  float4 ctr, lbh, lbl;
+  pair_sub(P.ch[0], P.cl[0], bxh, bxl, ctr.x, ctr.y);
+  pair_sub(P.ch[1], P.cl[1], byh, byl, ctr.z, ctr.w);
+  pair_sub(P.ch[2], P.cl[2], bxh, bxl, lbh.x, lbl.x);
+  pair_sub(P.ch[3], P.cl[3], bxh, bxl, lbh.y, lbl.y);
+  pair_sub(P.ch[4], P.cl[4], byh, byl, lbh.z, lbl.z);
+  pair_sub(P.ch[5], P.cl[5], byh, byl, lbh.w, lbl.w);
+  // A hit lies within the geometry's extent and inside the leaf box.
+  const float rx = P.g[4].w + hi_slack(fabsf(ctr.x)), ry = P.g[5].w + hi_slack(fabsf(ctr.z));
+  S.rect = make_float4(fmaxf(ctr.x - rx, lbh.x - hi_slack(fabsf(lbh.x))), fminf(ctr.x + rx, lbh.y + hi_slack(fabsf(lbh.y))),
+                       fmaxf(ctr.z - ry, lbh.z - hi_slack(fabsf(lbh.z))), fminf(ctr.z + ry, lbh.w + hi_slack(fabsf(lbh.w))));
+  S.c = ctr;
+  S.lbh = lbh;
+  S.lbl = lbl;
+  S.misc = make_float4(P.delta, P.err, P.sig, __int_as_float(P.kind));
+#pragma unroll
+  for (int i = 0; i < 6; ++i) S.g[i] = P.g[i];
+  sm.s[c] = static_cast<int>(s);
+}
+
+// Out of line, for scans without prepared terms: inlined, the FP64 derivation would cost the scan's
+// loops their registers.
+static __device__ __noinline__ void stage_derived(const ScanTile& t, ScanSmem& sm, int c, uint32_t s, float bxh,
+                                                  float bxl, float byh, float byl) {
+  ScanPrep P;
+  prep_crystal(t, s, P);
+  stage_prepared(P, sm, c, s, bxh, bxl, byh, byl);
+}
+
+// stage_prepared with the terms from t.prep, or derived here.
 __device__ __forceinline__ void stage_crystal(const ScanTile& t, ScanSmem& sm, int c, uint32_t s, float bxh,
                                               float bxl, float byh, float byl) {
-  ScanPrep P;
   if (t.prep) {
-    P = t.prep[s];
+    stage_prepared(t.prep[s], sm, c, s, bxh, bxl, byh, byl);
   } else {
-    prep_crystal(t, s, P);
+    stage_derived(t, sm, c, s, bxh, bxl, byh, byl);
   }
-  pair_sub(P.ch[0], P.cl[0], bxh, bxl, sm.cxh[c], sm.cxl[c]);
-  pair_sub(P.ch[1], P.cl[1], byh, byl, sm.cyh[c], sm.cyl[c]);
-  pair_sub(P.ch[2], P.cl[2], bxh, bxl, sm.lbh[0][c], sm.lbl[0][c]);
-  pair_sub(P.ch[3], P.cl[3], bxh, bxl, sm.lbh[1][c], sm.lbl[1][c]);
-  pair_sub(P.ch[4], P.cl[4], byh, byl, sm.lbh[2][c], sm.lbl[2][c]);
-  pair_sub(P.ch[5], P.cl[5], byh, byl, sm.lbh[3][c], sm.lbl[3][c]);
-  sm.m[c] = P.m;
-  sm.delta[c] = P.delta;
-  sm.err[c] = P.err;
-  sm.sig[c] = P.sig;
-  sm.kind[c] = P.kind;
-  sm.s[c] = static_cast<int>(s);
-#pragma unroll
-  for (int i = 0; i < 21; ++i) sm.g[i][c] = P.g[i];
 }
 
 // Staging terms of every developed crystal of every tile, once per crystal (k_scan reads them).
@@ -277,43 +311,79 @@ void launch_scan_prep(const ScanTile* tiles, int ntiles, unsigned long long nslo
   FG_CUDA(cudaGetLastError());
 }
 
-// Decision and chord of one scanner ray against staged crystal c.  The ray's origin is a float pair
-// relative to the bin's 16-px corner; a pair whose decision falls inside its error bound is
-// decided with the reference's FP64 expressions (counted in nfb).
-__device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm, uint32_t c, float oxh, float oxl,
-                                          float oyh, float oyl, uint32_t px, uint32_t py, uint32_t sx, uint32_t sy,
-                                          float& chord, uint32_t& nfb) {
-  const float m = sm.m[c], delta = sm.delta[c];
-  const int kind = sm.kind[c];
-  // Geometry reach: a cube lies within sqrt(3) m of its centre, an ellipsoid within its own box.
-  const float reach = (kind == K_ELLIPSOID ? m : 1.7320509f * m) * 1.00001f + 1e-9f;
-  {
-    // Quick rejection on the high words alone: they differ from the float pairs by a few units in
-    // the last place, far inside the slack, so a pair rejected here fails the exact test below.
-    const float cxh = sm.cxh[c], cyh = sm.cyh[c];
-    const float slack = 1e-4f + 4.8e-7f * (fabsf(oxh) + fabsf(cxh) + fabsf(oyh) + fabsf(cyh));
-    if (fabsf(oxh - cxh) > reach + slack || fabsf(oyh - cyh) > reach + slack) return false;
-  }
+// One thread's scanner ray in a bin: pixel, stratum and the ray origin relative to the corner of
+// the 16-pixel square holding the bin (float pairs), shared by the forward scan and its adjoint.
+struct ScanRay {
+  uint32_t bin;
+  bool active;
+  float bxh, bxl, byh, byl;  // corner of the 16-pixel square holding the bin (um, float pairs)
+  float oxh, oxl, oyh, oyl;
+  float4 warp;     // x0, x1, y0, y1 of the warp's rays (high words)
+};
+
+// Pixel in the bin and stratum of thread tid.  A warp's pixels form a compact block (Morton order in
+// bins of 2^k pixels: 4 x 2 pixels of 4 strata), so that it meets few crystals.
+__device__ __forceinline__ void scan_place(const ScanTile& t, uint32_t tid, uint32_t& pix, uint32_t& lx, uint32_t& ly,
+                                           uint32_t& st) {
+  pix = tid / t.spp;
+  st = tid % t.spp;
+  const bool morton = (t.bin_px & (t.bin_px - 1)) == 0;
+  lx = morton ? morton2_compact(pix) : pix % t.bin_px;
+  ly = morton ? morton2_compact(pix >> 1) : pix / t.bin_px;
+}
+
+// The ray's place among the bin's: pixel-major in rows, strata in order.
+__device__ __forceinline__ uint32_t scan_slot(const ScanTile& t, uint32_t tid) {
+  uint32_t pix, lx, ly, st;
+  scan_place(t, tid, pix, lx, ly, st);
+  return pix < t.bin_px * t.bin_px ? (ly * t.bin_px + lx) * t.spp + st : SCAN_THREADS;
+}
+
+// The FP64 decision and chord of the calling thread's ray against crystal s (rare: the ray is formed
+// anew here, so that the scan does not keep its pixel and stratum in registers).
+static __device__ __noinline__ bool scan_chord_fp64(const ScanTile& t, uint32_t s, uint32_t bin, float& chord) {
+  uint32_t pix, lx, ly, st;
+  scan_place(t, threadIdx.x, pix, lx, ly, st);
+  double ox, oy;
+  scan_origin64(t, (bin % t.nbx) * t.bin_px + lx, (bin / t.nbx) * t.bin_px + ly, st % t.g, st / t.g, ox, oy);
+  bool hit;
+  chord = static_cast<float>(scan_chord64(t, s, ox, oy, hit));
+  return hit;
+}
+
+// Decision and chord of one scanner ray against staged crystal c, whose rectangle holds the ray.  The
+// ray's origin is a float pair relative to the bin's 16-px corner; a pair whose decision falls inside
+// its error bound is decided with the reference's FP64 expressions (counted in nfb).
+// DF: the crystal is a K_CUBE_DF (it is none otherwise).
+template <bool DF>
+__device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm, uint32_t c, const ScanRay& R, float& chord,
+                                          uint32_t& nfb) {
+  const float oxh = R.oxh, oxl = R.oxl, oyh = R.oyh, oyl = R.oyl;
+  const Staged& S = sm.k[c];
+  const float4 misc = S.misc, ctr = S.c, lb = S.lbh;
+  const float delta = misc.x;
+  const int kind = __float_as_int(misc.w);
   // Ray minus crystal centre, x and y, as float pairs.
   float dh, dl, dx, dxl, dy, dyl;
-  two_sum(oxh, -sm.cxh[c], dh, dl);
-  fast_two_sum(dh, dl + (oxl - sm.cxl[c]), dx, dxl);
-  two_sum(oyh, -sm.cyh[c], dh, dl);
-  fast_two_sum(dh, dl + (oyl - sm.cyl[c]), dy, dyl);
-  if (fabsf(dx) > reach || fabsf(dy) > reach) return false;
-  // The leaf box (strict containment in x and y; the origin lies above every box in z): margins
-  // of float-pair differences, exact to ~1e-12 um.
-  float lm = INFINITY;
-  {
+  two_sum(oxh, -ctr.x, dh, dl);
+  fast_two_sum(dh, dl + (oxl - ctr.y), dx, dxl);
+  two_sum(oyh, -ctr.z, dh, dl);
+  fast_two_sum(dh, dl + (oyl - ctr.w), dy, dyl);
+  // The leaf box (strict containment in x and y; the origin lies above every box in z): its margins
+  // on the high words, and where those are too close to call, of float-pair differences, exact to
+  // about 1e-12 um.
+  float lm = fminf(fminf(oxh - lb.x, lb.y - oxh), fminf(oyh - lb.z, lb.w - oyh));
+  if (fabsf(lm) <= hi_slack(fabsf(oxh) + fabsf(oyh))) {
+    const float4 ll = S.lbl;
     float h, l;
-    two_sum(oxh, -sm.lbh[0][c], h, l);
-    lm = fminf(lm, h + (l + (oxl - sm.lbl[0][c])));
-    two_sum(sm.lbh[1][c], -oxh, h, l);
-    lm = fminf(lm, h + (l + (sm.lbl[1][c] - oxl)));
-    two_sum(oyh, -sm.lbh[2][c], h, l);
-    lm = fminf(lm, h + (l + (oyl - sm.lbl[2][c])));
-    two_sum(sm.lbh[3][c], -oyh, h, l);
-    lm = fminf(lm, h + (l + (sm.lbl[3][c] - oyl)));
+    two_sum(oxh, -lb.x, h, l);
+    lm = h + (l + (oxl - ll.x));
+    two_sum(lb.y, -oxh, h, l);
+    lm = fminf(lm, h + (l + (ll.y - oxl)));
+    two_sum(oyh, -lb.z, h, l);
+    lm = fminf(lm, h + (l + (oyl - ll.z)));
+    two_sum(lb.w, -oyh, h, l);
+    lm = fminf(lm, h + (l + (ll.w - oyl)));
   }
   const float EBL = 1e-9f;
   if (lm < -EBL) return false;
@@ -321,20 +391,21 @@ __device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm,
   bool hit = false;
   chord = 0.0f;
   if (!amb) {
-    if (kind != K_ELLIPSOID) {
+    if (DF || kind != K_ELLIPSOID) {
       float tmin = -INFINITY, tmax = INFINITY;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        const float inv = sm.g[12 + i][c], Dh = sm.g[15 + i][c];
+        const float4 gi = S.g[i];
+        const float inv = gi.z, Dh = gi.w;
         float a1, a2;
-        if (kind == K_CUBE) {
-          const float lo_i = fmaf(sm.g[i][c], dx, sm.g[6 + i][c] * dy);
+        if (!DF) {
+          const float lo_i = fmaf(gi.x, dx, gi.y * dy);
           a1 = -Dh - lo_i;
           a2 = Dh - lo_i;
         } else {
           // Local origin as a float pair, then the two face offsets exactly rounded.
-          const float R0h = sm.g[i][c], R0l = sm.g[3 + i][c], R1h = sm.g[6 + i][c], R1l = sm.g[9 + i][c];
-          const float Dl = sm.g[18 + i][c];
+          const float4 gl = S.g[3 + i];
+          const float R0h = gi.x, R0l = gl.x, R1h = gi.y, R1l = gl.y, Dl = gl.z;
           float p0, e0, p1, e1, sh, sl;
           two_prod(R0h, dx, p0, e0);
           two_prod(R1h, dy, p1, e1);
@@ -350,7 +421,7 @@ __device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm,
         tmin = fmaxf(tmin, fminf(t1, t2));
         tmax = fminf(tmax, fmaxf(t1, t2));
       }
-      const float E = kind == K_CUBE ? sm.err[c] : 4.0f * 3.0f * EPS32 * (fabsf(tmin) + fabsf(tmax)) + 1e-9f;
+      const float E = !DF ? misc.y : 4.0f * 3.0f * EPS32 * (fabsf(tmin) + fabsf(tmax)) + 1e-9f;
       const float m1 = tmax - tmin, m2 = tmax + delta;
       const float E2 = E + 4.0f * 3.0f * EPS32 * fabsf(delta) + 2e-6f;
       if (m1 > 2.0f * E && m2 > E2) {
@@ -361,16 +432,18 @@ __device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm,
       }
     } else {
       float P[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) P[i] = fmaf(sm.g[i][c], dx, sm.g[3 + i][c] * dy);
-      const float e0 = sm.g[6][c], e1 = sm.g[7][c], e2 = sm.g[8][c];
-      const float iA = sm.g[10][c];
+      const float4 g0 = S.g[0], g1 = S.g[1], g2 = S.g[2];
+      P[0] = fmaf(g0.x, dx, g0.y * dy);
+      P[1] = fmaf(g1.x, dx, g1.y * dy);
+      P[2] = fmaf(g2.x, dx, g2.y * dy);
+      const float e0 = g0.z, e1 = g1.z, e2 = g2.z;
+      const float iA = g0.w;
       // Closest approach along the ray (t' = tc) and the offset there: h = 1 - |P_perp|^2
       // has the sign of the reference's discriminant.
       const float tc = -(P[0] * e0 + P[1] * e1 + P[2] * e2) * iA;
       const float q0 = fmaf(tc, e0, P[0]), q1 = fmaf(tc, e1, P[1]), q2 = fmaf(tc, e2, P[2]);
       const float hh = 1.0f - (q0 * q0 + q1 * q1 + q2 * q2);
-      const float E = sm.err[c];
+      const float E = misc.y;
       if (hh > E) {
         const float sq = sqrtf(hh * iA);
         const float t0 = tc - sq, t1 = tc + sq;
@@ -388,31 +461,17 @@ __device__ __forceinline__ bool scan_pair(const ScanTile& t, const ScanSmem& sm,
   }
   if (amb) {
     ++nfb;
-    double ox64, oy64;
-    scan_origin64(t, px, py, sx, sy, ox64, oy64);
-    bool h64;
-    const double c64 = scan_chord64(t, static_cast<uint32_t>(sm.s[c]), ox64, oy64, h64);
-    hit = h64;
-    chord = static_cast<float>(c64);
+    hit = scan_chord_fp64(t, static_cast<uint32_t>(sm.s[c]), R.bin, chord);
   }
   return hit;
 }
 
-// One thread's scanner ray in a bin: pixel, stratum and the ray origin relative to the corner of
-// the 16-pixel square holding the bin (float pairs), shared by the forward scan and its adjoint.
-struct ScanRay {
-  uint32_t px, py, sx, sy, st;
-  bool active;
-  float bxh, bxl, byh, byl;  // corner of the 16-pixel square holding the bin (um, float pairs)
-  float oxh, oxl, oyh, oyl;
-};
-
 __device__ __forceinline__ ScanRay scan_ray(const ScanTile& t, uint32_t bin, uint32_t tid) {
   ScanRay R;
+  R.bin = bin;
   const uint32_t bx = bin % t.nbx, by = bin / t.nbx;
-  const uint32_t a = t.spp;
-  const uint32_t pix = tid / a, st = tid % a;
-  const uint32_t lx = pix % t.bin_px, ly = pix / t.bin_px;
+  uint32_t pix, lx, ly, st;
+  scan_place(t, tid, pix, lx, ly, st);
   const uint32_t px = bx * t.bin_px + lx, py = by * t.bin_px + ly;
   const bool active = pix < t.bin_px * t.bin_px && px < t.w && py < t.h;
   const uint32_t sx = st % t.g, sy = st / t.g;
@@ -452,17 +511,73 @@ __device__ __forceinline__ ScanRay scan_ray(const ScanTile& t, uint32_t bin, uin
     two_prod(Yh, cyh, p, e);
     fast_two_sum(p, e + (Yh * cyl + Yl * cyh), oyh, oyl);
   }
-  R.px = px;
-  R.py = py;
-  R.sx = sx;
-  R.sy = sy;
-  R.st = st;
   R.active = active;
   R.oxh = oxh;
   R.oxl = oxl;
   R.oyh = oyh;
   R.oyl = oyl;
+  float x0 = active ? oxh : INFINITY, x1 = active ? oxh : -INFINITY;
+  float y0 = active ? oyh : INFINITY, y1 = active ? oyh : -INFINITY;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+    x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+    y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+    y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+  }
+  R.warp = make_float4(x0, x1, y0, y1);
   return R;
+}
+
+// fn<DF>(c) for every staged crystal whose rectangle holds the ray.  The warp picks, 32 crystals at
+// a time, those whose rectangle meets its rays, and each lane notes which of them hold its own ray;
+// then every lane goes through its own crystals, so that a turn does not wait for the warp's other
+// rays (they are hit by about a third of the same crystals).  The float-pair cubes (one in five of
+// random orientation) are decided at once, all lanes together: their code is long, and the lanes'
+// own turns would nearly always include one.  All 32 lanes call it.  (A NaN rejects nothing.)
+template <class F>
+__device__ __forceinline__ void scan_staged(const ScanSmem& sm, uint32_t cnt, const ScanRay& R, F&& fn) {
+  static_assert(SCAN_CH == 128, "four words of candidates");
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t mine[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (uint32_t w = 0; w < 4; ++w) {
+    const uint32_t b = 32 * w;
+    if (b >= cnt) break;
+    bool near = b + lane < cnt, pair = false;
+    if (near) {
+      const Staged& S = sm.k[b + lane];
+      const float4 r = S.rect;
+      near = !(r.x > R.warp.y || r.y < R.warp.x || r.z > R.warp.w || r.w < R.warp.z);
+      pair = __float_as_int(S.misc.w) == K_CUBE_DF;
+    }
+    const unsigned nm = __ballot_sync(0xffffffffu, near), pm = __ballot_sync(0xffffffffu, pair);
+    for (unsigned m = nm & ~pm; m; m &= m - 1) {
+      const float4 r = sm.k[b + __ffs(m) - 1].rect;
+      if (!(R.oxh < r.x || R.oxh > r.y || R.oyh < r.z || R.oyh > r.w)) mine[w] |= m & (0u - m);
+    }
+    for (unsigned m = nm & pm; m; m &= m - 1) {
+      const uint32_t c = b + __ffs(m) - 1;
+      const float4 r = sm.k[c].rect;
+      if (R.active && !(R.oxh < r.x || R.oxh > r.y || R.oyh < r.z || R.oyh > r.w)) fn(c, std::true_type{});
+    }
+  }
+  if (!R.active) return;
+  uint32_t b = 0;
+  for (;;) {
+    if (!mine[0]) {
+      if (!(mine[1] | mine[2] | mine[3])) break;
+      b += 32;
+      mine[0] = mine[1];
+      mine[1] = mine[2];
+      mine[2] = mine[3];
+      mine[3] = 0;
+      continue;
+    }
+    const uint32_t c = b + __ffs(mine[0]) - 1;
+    mine[0] &= mine[0] - 1;
+    fn(c, std::false_type{});
+  }
 }
 
 // Tile of global bin gb (last tile whose first bin <= gb).
@@ -475,8 +590,15 @@ __device__ __forceinline__ int scan_tile_of(const ScanTile* tiles, int ntiles, u
   return lo;
 }
 
-// Launch bounds of 4 x 256 threads per SM (64 registers): bins of 4 x 4 pixels run 64-thread CTAs,
-// and more of them in flight cover the staging and the FP64 fallbacks (measured 18 % faster).
+// What bounds it: issue slots (75 % issue activity at 21 of 32 lanes; DRAM 1 %).  A bin of 8 x 8
+// tri-x pixels at full development stages 130 crystals; 30 of each 84 staged meet a warp's rays, and
+// a ray is decided against 17 of them (scan_staged).  Testing every staged crystal for every ray,
+// all lanes of a row of pixels in step, took 10.4 ms for a 2048 x 2048 px tri-x image (23.7 M rays,
+// 390 M hits); culling by warp 6.0; the lanes' own lists, with the float-pair cubes decided
+// together, 5.3.
+//
+// Launch bounds of 4 x 256 threads per SM (64 registers; 3: 9.5 against 8.9 ms for the scan stage):
+// more CTAs in flight cover the staging and the FP64 fallbacks.
 __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __restrict__ tiles,
                                                        int ntiles, uint32_t* err,
                                                        unsigned long long* stats) {
@@ -487,9 +609,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __rest
   const uint32_t a = t.spp;
   const uint32_t tid = threadIdx.x;
   const ScanRay R = scan_ray(t, bin, tid);
-  const uint32_t px = R.px, py = R.py, sx = R.sx, sy = R.sy, st = R.st;
   const bool active = R.active;
-  const float oxh = R.oxh, oxl = R.oxl, oyh = R.oyh, oyl = R.oyl;
   long long Lfix = 0;  // chord sum (sigma-weighted when per crystal), 2^-40 um units
   uint32_t nh = 0, nfb = 0;
   const uint32_t b0 = min(t.bin_off[bin], t.items_cap), b1 = min(t.bin_off[bin + 1], t.items_cap);
@@ -500,25 +620,28 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __rest
     for (uint32_t c = tid; c < cnt; c += blockDim.x)
       stage_crystal(t, sm, c, t.bin_items[base + c], R.bxh, R.bxl, R.byh, R.byl);
     __syncthreads();
-    if (!active) continue;
-    for (uint32_t c = 0; c < cnt; ++c) {
+    scan_staged(sm, cnt, R, [&](uint32_t c, auto df) {
       float chord;
-      const bool hit = scan_pair(t, sm, c, oxh, oxl, oyh, oyl, px, py, sx, sy, chord, nfb);
-      if (hit) {
-        ++nh;
-        const float v = per_crystal ? sm.sig[c] * fmaxf(chord, 0.0f) : fmaxf(chord, 0.0f);
-        Lfix += fix40(v);
-      }
-    }
+      if (!scan_pair<decltype(df)::value>(t, sm, c, R, chord, nfb)) return;
+      ++nh;
+      const float v = per_crystal ? sm.k[c].misc.z * fmaxf(chord, 0.0f) : fmaxf(chord, 0.0f);
+      Lfix += fix40(v);
+    });
   }
   float T = 1.0f;
   if (active) {
     // Lfix * 2^-40 rounded once to float (the conversion rounds, the power-of-two scale is exact).
     const float L = u64_to_float_rn(static_cast<unsigned long long>(Lfix)) * 0x1p-40f;
     T = per_crystal ? expf(-L) : expf(-t.sigma * L);
-    if (t.ray_hits) t.ray_hits[(static_cast<size_t>(py) * t.w + px) * a + st] = static_cast<uint16_t>(min(nh, 65535u));
+    if (t.ray_hits) {
+      uint32_t pix, lx, ly, st;
+      scan_place(t, tid, pix, lx, ly, st);
+      const uint32_t px = (bin % t.nbx) * t.bin_px + lx, py = (bin / t.nbx) * t.bin_px + ly;
+      t.ray_hits[(static_cast<size_t>(py) * t.w + px) * a + st] = static_cast<uint16_t>(min(nh, 65535u));
+    }
   }
-  sm.T[tid] = f2d_exact(T);
+  const uint32_t slot = scan_slot(t, tid);
+  if (slot < SCAN_THREADS) sm.T[slot] = f2d_exact(T);
   __syncthreads();
   // Per pixel: thread p finishes the bin's p-th pixel, so the FP64 work runs on consecutive lanes
   // (a pixel's strata are a consecutive threads; one thread in a per pixel would leave most lanes
@@ -585,20 +708,21 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* _
     for (uint32_t c = tid; c < cnt; c += blockDim.x)
       stage_crystal(t, sm, c, t.bin_items[base + c], R.bxh, R.bxl, R.byh, R.byl);
     __syncthreads();
-    if (!R.active) continue;
-    for (uint32_t c = 0; c < cnt; ++c) {
+    scan_staged(sm, cnt, R, [&](uint32_t c, auto df) {
       float chord;
-      if (scan_pair(t, sm, c, R.oxh, R.oxl, R.oyh, R.oyl, R.px, R.py, R.sx, R.sy, chord, nfb)) {
-        const float v = per_crystal ? sm.sig[c] * fmaxf(chord, 0.0f) : fmaxf(chord, 0.0f);
-        Lfix += fix40(v);
-      }
-    }
+      if (!scan_pair<decltype(df)::value>(t, sm, c, R, chord, nfb)) return;
+      const float v = per_crystal ? sm.k[c].misc.z * fmaxf(chord, 0.0f) : fmaxf(chord, 0.0f);
+      Lfix += fix40(v);
+    });
   }
   float coef = 0.0f;
   if (R.active) {
     const float L = u64_to_float_rn(static_cast<unsigned long long>(Lfix)) * 0x1p-40f;  // as in k_scan
     const float T = per_crystal ? expf(-L) : expf(-t.sigma * L);
-    coef = wpx[static_cast<size_t>(R.py) * t.w + R.px] / static_cast<float>(a) * T;
+    uint32_t pix, lx, ly, st;
+    scan_place(t, tid, pix, lx, ly, st);
+    const uint32_t px = (bin % t.nbx) * t.bin_px + lx, py = (bin / t.nbx) * t.bin_px + ly;
+    coef = wpx[static_cast<size_t>(py) * t.w + px] / static_cast<float>(a) * T;
   }
   for (uint32_t base = b0; base < b1; base += SCAN_CH) {
     const uint32_t cnt = min(static_cast<uint32_t>(SCAN_CH), b1 - base);
@@ -608,13 +732,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* _
       gsum[c] = 0.0;
     }
     __syncthreads();
-    if (R.active && coef != 0.0f) {
-      for (uint32_t c = 0; c < cnt; ++c) {
-        float chord;
-        if (scan_pair(t, sm, c, R.oxh, R.oxl, R.oyh, R.oyl, R.px, R.py, R.sx, R.sy, chord, nfb))
-          atomicAdd(&gsum[c], static_cast<double>(coef) * static_cast<double>(fmaxf(chord, 0.0f)));
-      }
-    }
+    scan_staged(sm, cnt, R, [&](uint32_t c, auto df) {
+      if (coef == 0.0f) return;
+      float chord;
+      if (scan_pair<decltype(df)::value>(t, sm, c, R, chord, nfb))
+        atomicAdd(&gsum[c], static_cast<double>(coef) * static_cast<double>(fmaxf(chord, 0.0f)));
+    });
     __syncthreads();
     for (uint32_t c = tid; c < cnt; c += blockDim.x)
       if (gsum[c] != 0.0) atomicAdd(&g[sm.s[c]], gsum[c]);

@@ -32,10 +32,13 @@ struct __align__(16) ScanPrep {
   // Centre x, y (um) as the scan sees it, and the x and y extent of the crystal's leaf box in the
   // scan's tree, as float pairs (hi + lo): x, y, leaf x0, x1, y0, y1.
   float ch[6], cl[6];
-  float g[21];     // per-kind terms (see stage_crystal)
-  float m, delta, err, sig;
+  // Per-kind terms.  Cubes: axis i's R_0i, R_1i (high words), 1 / (-R_2i), half-size (high word) in
+  // g[i]; the low words of R_0i, R_1i and the half-size in g[3 + i].xyz.  Ellipsoids: R_0i / D_i,
+  // R_1i / D_i, -R_2i / D_i in g[i].xyz, 1 / A in g[0].w.  The geometry lies within hx = g[4].w,
+  // hy = g[5].w of its centre in x and y (rounded up).
+  float4 g[6];
+  float delta, err, sig;
   int kind;
-  int pad_[2];
 };
 static_assert(sizeof(ScanPrep) == 160, "ScanPrep layout");
 
