@@ -89,15 +89,21 @@ __global__ void __launch_bounds__(RED_THREADS) k_otf_grads(const float* __restri
   }
 }
 
-__global__ void k_sum_partials(const double* partial, int n, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double a = 0.0, b = 0.0;
-  for (int i = 0; i < n; ++i) {
-    a += partial[2 * i];
-    b += partial[2 * i + 1];
+// The partials' sums in index order (one chain of additions each, so the result does not depend on the
+// launch): the block stages them in shared memory, thread 0 adds one sum and thread 1 the other.
+// (One thread reading them from global memory took 107 us for 1,024.)
+__global__ void __launch_bounds__(RED_THREADS) k_sum_partials(const double* __restrict__ partial, int n, double* out) {
+  __shared__ double sh[2 * RED_THREADS];
+  double a = 0.0;
+  for (int base = 0; base < n; base += RED_THREADS) {
+    const int m = min(RED_THREADS, n - base);
+    for (int i = threadIdx.x; i < 2 * m; i += RED_THREADS) sh[i] = partial[2 * base + i];
+    __syncthreads();
+    if (threadIdx.x < 2)
+      for (int i = 0; i < m; ++i) a += sh[2 * i + threadIdx.x];
+    __syncthreads();
   }
-  out[0] = a;
-  out[1] = b;
+  if (threadIdx.x < 2) out[threadIdx.x] = a;
 }
 
 // Weight of output position o on input position i for one clamp-to-edge 3-tap pass.
@@ -132,6 +138,11 @@ __global__ void k_otf_adjoint(const float* __restrict__ G, uint32_t w, uint32_t 
   wpx[i] = static_cast<float>(-e * acc);
 }
 
+__global__ void k_to_float(const double* __restrict__ in, uint32_t n, float* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = static_cast<float>(in[i]);
+}
+
 // T per pixel (device) for the differentiable scan: the forward scan in Negative mode with the
 // given per-crystal opacities (Morton order on the device, or null for the config's opacity).
 void scan_T(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed, const float* sigma_sorted,
@@ -162,9 +173,8 @@ fg_status fg_scan_signal(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg*
     const size_t np = static_cast<size_t>(cfg->width_px) * cfg->height_px;
     DBuf<float> sig, T(std::max<size_t>(np, 1), st), H(std::max<size_t>(np, 1), st), S(std::max<size_t>(np, 1), st);
     if (sigma_per_crystal) {
-      const std::vector<float> sv = to_sorted(em, sigma_per_crystal);
-      sig.alloc(std::max<size_t>(sv.size(), 1), st);
-      if (!sv.empty()) FG_CUDA(cudaMemcpyAsync(sig.p, sv.data(), sv.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+      sig.alloc(std::max<uint32_t>(em->n, 1), st);
+      by_id_to_device(em, sigma_per_crystal, sig.p, st);
     }
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
     scan_T(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, T.p);
@@ -193,44 +203,44 @@ fg_status fg_scan_backward(fg_engine* e, const fg_emulsion* em, const fg_scan_cf
     const size_t np = static_cast<size_t>(w) * h;
     DBuf<float> sig, T(std::max<size_t>(np, 1), st), Gd(std::max<size_t>(np, 1), st), W(std::max<size_t>(np, 1), st);
     if (sigma_per_crystal) {
-      const std::vector<float> sv = to_sorted(em, sigma_per_crystal);
-      sig.alloc(std::max<size_t>(sv.size(), 1), st);
-      if (!sv.empty()) FG_CUDA(cudaMemcpyAsync(sig.p, sv.data(), sv.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+      sig.alloc(std::max<uint32_t>(em->n, 1), st);
+      by_id_to_device(em, sigma_per_crystal, sig.p, st);
     }
     if (np) FG_CUDA(cudaMemcpyAsync(Gd.p, dL_dsignal, np * sizeof(float), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
-    // Forward transmittance, recomputed from the developed mask.
-    scan_T(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, T.p);
+    // Forward transmittance, recomputed from the developed mask: by the per-crystal adjoint on its
+    // way, or alone.
+    DBuf<double> g;
+    DBuf<float> gf;
+    const bool crystals = dL_dsigma && em->n;
+    if (crystals) {
+      k_otf_adjoint<<<grid_for(np, 256), 256, 0, st>>>(Gd.p, w, h, tp, exposure, W.p);
+      FG_CUDA(cudaGetLastError());
+      g.alloc(em->n, st);
+      gf.alloc(em->n, st);
+      FG_CUDA(cudaMemsetAsync(g.p, 0, em->n * sizeof(double), st));
+      scan_adjoint(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, W.p, g.p, T.p);
+      k_to_float<<<grid_for(em->n, 256), 256, 0, st>>>(g.p, em->n, gf.p);
+      FG_CUDA(cudaGetLastError());
+    } else {
+      scan_T(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, T.p);
+    }
     // Exposure multiplier and OTF width.
     const int nblk = static_cast<int>(std::min<size_t>((np + RED_THREADS - 1) / RED_THREADS, 1024));
     DBuf<double> part(2 * static_cast<size_t>(std::max(nblk, 1)), st), sums(2, st);
     FG_CUDA(cudaMemsetAsync(sums.p, 0, 2 * sizeof(double), st));
     if (np) {
       k_otf_grads<<<nblk, RED_THREADS, 0, st>>>(T.p, Gd.p, w, h, tp, part.p);
-      k_sum_partials<<<1, 32, 0, st>>>(part.p, nblk, sums.p);
+      k_sum_partials<<<1, RED_THREADS, 0, st>>>(part.p, nblk, sums.p);
       FG_CUDA(cudaGetLastError());
     }
     double hs[2] = {0.0, 0.0};
     FG_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    // Per-crystal opacities.
-    DBuf<double> g;
-    if (dL_dsigma && em->n) {
-      k_otf_adjoint<<<grid_for(np, 256), 256, 0, st>>>(Gd.p, w, h, tp, exposure, W.p);
-      FG_CUDA(cudaGetLastError());
-      g.alloc(em->n, st);
-      FG_CUDA(cudaMemsetAsync(g.p, 0, em->n * sizeof(double), st));
-      scan_adjoint(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, W.p, g.p);
-    }
     FG_CUDA(cudaEventRecord(e->timer.ev[1], st));
-    std::vector<double> gs(dL_dsigma ? em->n : 0);
-    if (dL_dsigma && em->n) FG_CUDA(cudaMemcpyAsync(gs.data(), g.p, em->n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (crystals) device_to_by_id(em, gf.p, dL_dsigma, st);
     FG_CUDA(cudaStreamSynchronize(st));
     if (dL_dexposure) *dL_dexposure = hs[0];
     if (dL_dotf_sigma) *dL_dotf_sigma = exposure * hs[1];
-    if (dL_dsigma) {
-      std::vector<float> gf(gs.begin(), gs.end());
-      from_sorted(em, gf, dL_dsigma);
-    }
     e->timings.scan_ms = elapsed(e->timer.ev[0], e->timer.ev[1]);
     e->timings.total_ms = e->timings.scan_ms;
     end_call(e);

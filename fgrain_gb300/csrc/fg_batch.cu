@@ -43,8 +43,6 @@ void launch_photon_sort(const TileDesc* tiles_dev, int ntiles, unsigned long lon
 void launch_density(float* d, unsigned long long n, cudaStream_t st);
 void launch_scan(const ScanTile* tiles, int ntiles, unsigned long long nbins, unsigned threads, uint32_t* err,
                  unsigned long long* stats, cudaStream_t st);
-void launch_scan_prep(const ScanTile* tiles, int ntiles, unsigned long long nslots, ScanPrep* prep,
-                      cudaStream_t st);
 void launch_scan_prep_list(const ScanTile* tiles, int ntiles, const uint32_t* list, const uint32_t* nlist,
                            unsigned long long cap, ScanPrep* prep, cudaStream_t st);
 uint32_t scan_bin_px(uint32_t spp);

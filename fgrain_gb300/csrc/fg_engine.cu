@@ -315,18 +315,15 @@ fg_status fg_emulsion_download(fg_engine* e, const fg_emulsion* em, fg_crystals_
 fg_status fg_emulsion_get_counts(fg_engine* e, const fg_emulsion* em, uint32_t* counts) {
   return guard(e, [&] {
     FG_REQUIRE(em && counts, "null argument");
-    std::vector<uint32_t> v(em->n);
-    if (em->n) FG_CUDA(cudaMemcpyAsync(v.data(), em->counts.p, em->n * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
+    device_to_by_id(em, em->counts.p, counts, e->stream);
     FG_CUDA(cudaStreamSynchronize(e->stream));
-    from_sorted(em, v, counts);
   });
 }
 
 fg_status fg_emulsion_set_counts(fg_engine* e, fg_emulsion* em, const uint32_t* counts) {
   return guard(e, [&] {
     FG_REQUIRE(em && counts, "null argument");
-    const std::vector<uint32_t> v = to_sorted(em, counts);
-    if (em->n) FG_CUDA(cudaMemcpyAsync(em->counts.p, v.data(), em->n * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream));
+    by_id_to_device(em, counts, em->counts.p, e->stream);
     FG_CUDA(cudaStreamSynchronize(e->stream));
   });
 }
@@ -336,17 +333,16 @@ fg_status fg_emulsion_get_development(fg_engine* e, const fg_emulsion* em, uint8
   return guard(e, [&] {
     FG_REQUIRE(em, "null emulsion");
     const uint32_t n = em->n;
-    std::vector<uint8_t> dv(n);
-    std::vector<double> ex(n);
-    if (n) {
-      FG_CUDA(cudaMemcpyAsync(dv.data(), em->developed.p, n, cudaMemcpyDeviceToHost, e->stream));
-      FG_CUDA(cudaMemcpyAsync(ex.data(), em->exp64.p, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-      if (clump) FG_CUDA(cudaMemcpyAsync(clump, em->clump.p, n * sizeof(int64_t), cudaMemcpyDeviceToHost, e->stream));
-    }
+    if (developed) device_to_by_id(em, em->developed.p, developed, e->stream);
+    if (expansion) device_to_by_id(em, em->exp64.p, expansion, e->stream);
+    if (clump && n) FG_CUDA(cudaMemcpyAsync(clump, em->clump.p, n * sizeof(int64_t), cudaMemcpyDeviceToHost, e->stream));
     FG_CUDA(cudaStreamSynchronize(e->stream));
-    if (developed) from_sorted(em, dv, developed);
-    if (expansion) from_sorted(em, ex, expansion);
   });
+}
+
+__global__ void k_to_float(const double* __restrict__ in, uint32_t n, float* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = static_cast<float>(in[i]);
 }
 
 fg_status fg_emulsion_set_development(fg_engine* e, fg_emulsion* em, const uint8_t* developed,
@@ -354,14 +350,11 @@ fg_status fg_emulsion_set_development(fg_engine* e, fg_emulsion* em, const uint8
   return guard(e, [&] {
     FG_REQUIRE(em && developed && expansion, "null argument");
     const uint32_t n = em->n;
-    const std::vector<uint8_t> dv = to_sorted(em, developed);
-    const std::vector<double> ex = to_sorted(em, expansion);
-    std::vector<float> ex32(n);
-    for (uint32_t s = 0; s < n; ++s) ex32[s] = static_cast<float>(ex[s]);
     if (n) {
-      FG_CUDA(cudaMemcpyAsync(em->developed.p, dv.data(), n, cudaMemcpyHostToDevice, e->stream));
-      FG_CUDA(cudaMemcpyAsync(em->exp64.p, ex.data(), n * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-      FG_CUDA(cudaMemcpyAsync(em->exp32.p, ex32.data(), n * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+      by_id_to_device(em, developed, em->developed.p, e->stream);
+      by_id_to_device(em, expansion, em->exp64.p, e->stream);
+      k_to_float<<<grid_for(n, 256), 256, 0, e->stream>>>(em->exp64.p, n, em->exp32.p);
+      FG_CUDA(cudaGetLastError());
       FG_CUDA(cudaMemsetAsync(em->clump.p, 0xff, n * sizeof(int64_t), e->stream));
     }
     FG_CUDA(cudaStreamSynchronize(e->stream));
@@ -424,8 +417,8 @@ static void run_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg* cfg
   if (image8) { d_img.alloc(npx, st); so.image8 = d_img.p; }
   if (ray_hits) { d_hits.alloc(npx * a, st); so.ray_hits = d_hits.p; }
   if (sigma) {
-    const std::vector<float> sv = to_sorted(em, sigma);
-    to_device(d_sig, sv.data(), sv.size(), st);
+    d_sig.alloc(std::max<uint32_t>(em->n, 1), st);
+    by_id_to_device(em, sigma, d_sig.p, st);
   }
   FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
   scan(e, em, *cfg, seed, sigma ? d_sig.p : nullptr, so);

@@ -266,16 +266,61 @@ struct ScanOut {
   float* d_neg = nullptr;    // -log10(clamp(T)) + 0.05
   uint16_t* ray_hits = nullptr;
 };
-// Host permutation helpers between crystal id order and Morton order.
+// Host arrays in crystal-id order to and from device arrays in slot order.  The permutation runs on
+// the device (a random gather of millions of values costs the host milliseconds); where its scratch
+// cannot be allocated it runs on the host.
 template <class T>
-std::vector<T> to_sorted(const fg_emulsion* em, const T* by_id) {
-  std::vector<T> v(em->n);
-  for (uint32_t s = 0; s < em->n; ++s) v[s] = by_id[em->h_s2id.empty() ? s : em->h_s2id[s]];
-  return v;
+__global__ void k_permute(const T* __restrict__ in, const uint32_t* __restrict__ idx, uint32_t n, T* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = in[idx[i]];
 }
 template <class T>
-void from_sorted(const fg_emulsion* em, const std::vector<T>& sorted, T* by_id) {
-  for (uint32_t s = 0; s < em->n; ++s) by_id[em->h_s2id.empty() ? s : em->h_s2id[s]] = sorted[s];
+bool permute_scratch(DBuf<T>& b, size_t n, cudaStream_t st) {
+  try {
+    b.alloc(n, st);
+  } catch (const Error& x) {
+    if (x.st != FG_ERR_OOM) throw;
+    (void)cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+template <class T>
+void by_id_to_device(const fg_emulsion* em, const T* by_id, T* slots, cudaStream_t st) {
+  const uint32_t n = em->n;
+  if (!n) return;
+  DBuf<T> tmp;
+  if (em->h_s2id.empty()) {
+    FG_CUDA(cudaMemcpyAsync(slots, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
+  } else if (permute_scratch(tmp, n, st)) {
+    FG_CUDA(cudaMemcpyAsync(tmp.p, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
+    k_permute<<<(n + 255) / 256, 256, 0, st>>>(tmp.p, em->sorted_to_id.p, n, slots);
+    FG_CUDA(cudaGetLastError());
+  } else {
+    std::vector<T> v(n);
+    for (uint32_t s = 0; s < n; ++s) v[s] = by_id[em->h_s2id[s]];
+    FG_CUDA(cudaMemcpyAsync(slots, v.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
+    FG_CUDA(cudaStreamSynchronize(st));
+  }
+}
+// Enqueues the copy; the caller synchronises before it reads by_id.
+template <class T>
+void device_to_by_id(const fg_emulsion* em, const T* slots, T* by_id, cudaStream_t st) {
+  const uint32_t n = em->n;
+  if (!n) return;
+  DBuf<T> tmp;
+  if (em->h_s2id.empty()) {
+    FG_CUDA(cudaMemcpyAsync(by_id, slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+  } else if (permute_scratch(tmp, n, st)) {
+    k_permute<<<(n + 255) / 256, 256, 0, st>>>(slots, em->id_to_sorted.p, n, tmp.p);
+    FG_CUDA(cudaGetLastError());
+    FG_CUDA(cudaMemcpyAsync(by_id, tmp.p, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+  } else {
+    std::vector<T> v(n);
+    FG_CUDA(cudaMemcpyAsync(v.data(), slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+    FG_CUDA(cudaStreamSynchronize(st));
+    for (uint32_t s = 0; s < n; ++s) by_id[em->h_s2id[s]] = v[s];
+  }
 }
 
 // fg_image.cu: the separable 3-tap clamp-to-edge filter (two passes through tmp), in the
@@ -299,9 +344,10 @@ float elapsed(cudaEvent_t a, cudaEvent_t b);
 void scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed,
           const float* sigma_sorted, const ScanOut& out);
 // g_sorted[s] += sum over the rays of each pixel p of wpx[p] / spp * T_ray * chord_s (device
-// arrays; wpx has one weight per pixel, g_sorted one FP64 sum per crystal in Morton order).
+// arrays; wpx has one weight per pixel, g_sorted one FP64 sum per crystal in Morton order).  T
+// receives the transmittance that the forward scan in Negative mode gives.
 void scan_adjoint(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed,
-                  const float* sigma_sorted, const float* wpx, double* g_sorted);
+                  const float* sigma_sorted, const float* wpx, double* g_sorted, float* T);
 
 // fg_transport.cu
 void expose(fg_engine* e, fg_emulsion* em, const float* tile_dev, uint32_t tw, uint32_t th,

@@ -258,31 +258,14 @@ __device__ __forceinline__ void stage_crystal(const ScanTile& t, ScanSmem& sm, i
   }
 }
 
-// Staging terms of every developed crystal of every tile, once per crystal (k_scan reads them).
-__global__ void k_scan_prep(const ScanTile* __restrict__ tiles, int ntiles, unsigned long long nslots,
-                            ScanPrep* __restrict__ prep) {
-  const unsigned long long g = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-  if (g >= nslots) return;
-  int lo = 0, hi = ntiles - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tiles[mid].slot_base <= g) lo = mid; else hi = mid - 1;
-  }
-  const ScanTile& t = tiles[lo];
-  const unsigned long long s = g - t.slot_base;
-  if (s >= t.n || !t.developed[s]) return;
-  ScanPrep P;
-  prep_crystal(t, static_cast<uint32_t>(s), P);
-  prep[g] = P;
-}
-
-// k_scan_prep over a list of the developed crystals' slots (*nlist of them, at most cap): one
-// thread per listed crystal, so the FP64 derivation runs with every lane busy.
+// Staging terms of the listed developed crystals (their slots; *nlist of them, at most cap, or cap
+// when nlist is null), once per crystal (k_scan reads them): one thread per listed crystal, so the
+// FP64 derivation runs with every lane busy.
 __global__ void k_scan_prep_list(const ScanTile* __restrict__ tiles, int ntiles, const uint32_t* __restrict__ list,
                                  const uint32_t* __restrict__ nlist, unsigned long long cap,
                                  ScanPrep* __restrict__ prep) {
   const unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-  if (i >= cap || i >= *nlist) return;
+  if (i >= cap || (nlist && i >= *nlist)) return;
   const unsigned long long g = list[i];
   int lo = 0, hi = ntiles - 1;
   while (lo < hi) {
@@ -301,13 +284,6 @@ void launch_scan_prep_list(const ScanTile* tiles, int ntiles, const uint32_t* li
                            unsigned long long cap, ScanPrep* prep, cudaStream_t st) {
   if (cap == 0) return;
   k_scan_prep_list<<<grid_for(cap, 128), 128, 0, st>>>(tiles, ntiles, list, nlist, cap, prep);
-  FG_CUDA(cudaGetLastError());
-}
-
-void launch_scan_prep(const ScanTile* tiles, int ntiles, unsigned long long nslots, ScanPrep* prep,
-                      cudaStream_t st) {
-  if (nslots == 0) return;
-  k_scan_prep<<<grid_for(nslots, 128), 128, 0, st>>>(tiles, ntiles, nslots, prep);
   FG_CUDA(cudaGetLastError());
 }
 
@@ -590,6 +566,41 @@ __device__ __forceinline__ int scan_tile_of(const ScanTile* tiles, int ntiles, u
   return lo;
 }
 
+// fn(pixel index, mean transmittance) for the bin's pixels, from the strata in sm.T.  Thread p
+// finishes the bin's p-th pixel, so the FP64 work runs on consecutive lanes (a pixel's strata are spp
+// consecutive entries; one thread in spp per pixel would leave most lanes of each FP64 instruction
+// idle on GB300's narrow FP64 pipe).
+template <class F>
+__device__ __forceinline__ void scan_means(const ScanTile& t, const ScanSmem& sm, uint32_t bin, uint32_t tid, F&& fn) {
+  const uint32_t a = t.spp;
+  for (uint32_t p = tid; p * a < blockDim.x; p += blockDim.x) {
+    const uint32_t bx = bin % t.nbx, by = bin / t.nbx;
+    const uint32_t qx = bx * t.bin_px + p % t.bin_px, qy = by * t.bin_px + p / t.bin_px;
+    if (p >= t.bin_px * t.bin_px || qx >= t.w || qy >= t.h) continue;
+    // FP64 mean over strata in the reference's order (sy, sx), then f32 (transmittance.rs:142).
+    double acc = 0.0;
+    for (uint32_t k = 0; k < a; ++k) acc = __dadd_rn(acc, sm.T[p * a + k]);
+    // Division by a power of two is the multiplication by its exact reciprocal.
+    const float mean = (float)((a & (a - 1)) == 0 ? __dmul_rn(acc, 1.0 / static_cast<double>(a))
+                                                   : __ddiv_rn(acc, static_cast<double>(a)));
+    fn(static_cast<size_t>(qy) * t.w + qx, mean);
+  }
+}
+
+// Adds a warp's FP64 decisions and hits to the counters (may be null).
+__device__ __forceinline__ void scan_count(unsigned long long* stats, uint32_t nfb, uint32_t nh) {
+  if (!stats) return;
+  unsigned long long f = nfb, hsum = nh;
+  for (int o = 16; o > 0; o >>= 1) {
+    f += __shfl_down_sync(0xffffffffu, f, o);
+    hsum += __shfl_down_sync(0xffffffffu, hsum, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (f) atomicAdd(&stats[1], f);
+    if (hsum) atomicAdd(&stats[2], hsum);
+  }
+}
+
 // What bounds it: issue slots (75 % issue activity at 21 of 32 lanes; DRAM 1 %).  A bin of 8 x 8
 // tri-x pixels at full development stages 130 crystals; 30 of each 84 staged meet a warp's rays, and
 // a ray is decided against 17 of them (scan_staged).  Testing every staged crystal for every ray,
@@ -643,20 +654,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __rest
   const uint32_t slot = scan_slot(t, tid);
   if (slot < SCAN_THREADS) sm.T[slot] = f2d_exact(T);
   __syncthreads();
-  // Per pixel: thread p finishes the bin's p-th pixel, so the FP64 work runs on consecutive lanes
-  // (a pixel's strata are a consecutive threads; one thread in a per pixel would leave most lanes
-  // of each FP64 instruction idle on GB300's narrow FP64 pipe).
-  for (uint32_t p = tid; p * a < blockDim.x; p += blockDim.x) {
-    const uint32_t bx = bin % t.nbx, by = bin / t.nbx;
-    const uint32_t qx = bx * t.bin_px + p % t.bin_px, qy = by * t.bin_px + p / t.bin_px;
-    if (p >= t.bin_px * t.bin_px || qx >= t.w || qy >= t.h) continue;
-    // FP64 mean over strata in the reference's order (sy, sx), then f32 (transmittance.rs:142).
-    double acc = 0.0;
-    for (uint32_t k = 0; k < a; ++k) acc = __dadd_rn(acc, sm.T[p * a + k]);
-    // Division by a power of two is the multiplication by its exact reciprocal.
-    const float mean = (float)((a & (a - 1)) == 0 ? __dmul_rn(acc, 1.0 / static_cast<double>(a))
-                                                   : __ddiv_rn(acc, static_cast<double>(a)));
-    const size_t idx = static_cast<size_t>(qy) * t.w + qx;
+  scan_means(t, sm, bin, tid, [&](size_t idx, float mean) {
     float v;
     if (t.mode == 0) {
       v = mean;
@@ -670,27 +668,19 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __rest
     if (t.image8) t.image8[idx] = static_cast<uint8_t>(rintf(fminf(fmaxf(v, 0.0f), 1.0f) * 255.0f));
     // The mean transmittance; launch_density turns it into the density in a pass of its own.
     if (t.d_neg) t.d_neg[idx] = mean;
-  }
-  if (stats) {
-    unsigned long long f = nfb, hsum = nh;
-    for (int o = 16; o > 0; o >>= 1) {
-      f += __shfl_down_sync(0xffffffffu, f, o);
-      hsum += __shfl_down_sync(0xffffffffu, hsum, o);
-    }
-    if ((tid & 31) == 0) {
-      if (f) atomicAdd(&stats[1], f);
-      if (hsum) atomicAdd(&stats[2], hsum);
-    }
-  }
+  });
+  scan_count(stats, nfb, nh);
 }
 
 // Adjoint of k_scan with respect to the per-crystal opacities (single tile).  The forward is
 // recomputed from the developed mask: pass 1 forms each ray's optical depth exactly as k_scan
-// does, pass 2 re-stages the bin's crystals and adds w[p] / spp * T_ray * chord_s for every hit to
-// a per-crystal FP64 sum in shared memory, flushed with one global atomic per staged crystal.
+// does and writes the pixels' transmittance; pass 2 stages the bin's crystals again (unless all of
+// them are still there) and adds w[p] / spp * T_ray * chord_s for every hit to a per-crystal FP64 sum
+// in shared memory, flushed with one global atomic per staged crystal.
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* __restrict__ tiles,
                                                                const float* __restrict__ wpx,
-                                                               double* __restrict__ g) {
+                                                               double* __restrict__ g, float* __restrict__ Tpx,
+                                                               unsigned long long* stats) {
   __shared__ ScanSmem sm;
   __shared__ double gsum[SCAN_CH];
   const ScanTile& t = tiles[0];
@@ -700,7 +690,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* _
   const ScanRay R = scan_ray(t, bin, tid);
   const uint32_t b0 = min(t.bin_off[bin], t.items_cap), b1 = min(t.bin_off[bin + 1], t.items_cap);
   const bool per_crystal = t.sigma_c != nullptr;
-  uint32_t nfb = 0;
+  uint32_t nfb = 0, nh = 0;
   long long Lfix = 0;
   for (uint32_t base = b0; base < b1; base += SCAN_CH) {
     const uint32_t cnt = min(static_cast<uint32_t>(SCAN_CH), b1 - base);
@@ -711,24 +701,30 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* _
     scan_staged(sm, cnt, R, [&](uint32_t c, auto df) {
       float chord;
       if (!scan_pair<decltype(df)::value>(t, sm, c, R, chord, nfb)) return;
+      ++nh;
       const float v = per_crystal ? sm.k[c].misc.z * fmaxf(chord, 0.0f) : fmaxf(chord, 0.0f);
       Lfix += fix40(v);
     });
   }
-  float coef = 0.0f;
+  scan_count(stats, nfb, nh);  // the forward's
+  float coef = 0.0f, T = 1.0f;
   if (R.active) {
     const float L = u64_to_float_rn(static_cast<unsigned long long>(Lfix)) * 0x1p-40f;  // as in k_scan
-    const float T = per_crystal ? expf(-L) : expf(-t.sigma * L);
+    T = per_crystal ? expf(-L) : expf(-t.sigma * L);
     uint32_t pix, lx, ly, st;
     scan_place(t, tid, pix, lx, ly, st);
     const uint32_t px = (bin % t.nbx) * t.bin_px + lx, py = (bin / t.nbx) * t.bin_px + ly;
     coef = wpx[static_cast<size_t>(py) * t.w + px] / static_cast<float>(a) * T;
   }
+  const uint32_t slot = scan_slot(t, tid);
+  if (slot < SCAN_THREADS) sm.T[slot] = f2d_exact(T);
+  __syncthreads();
+  scan_means(t, sm, bin, tid, [&](size_t idx, float mean) { Tpx[idx] = mean; });
   for (uint32_t base = b0; base < b1; base += SCAN_CH) {
     const uint32_t cnt = min(static_cast<uint32_t>(SCAN_CH), b1 - base);
     __syncthreads();
     for (uint32_t c = tid; c < cnt; c += blockDim.x) {
-      stage_crystal(t, sm, c, t.bin_items[base + c], R.bxh, R.bxl, R.byh, R.byl);
+      if (b1 - b0 > SCAN_CH) stage_crystal(t, sm, c, t.bin_items[base + c], R.bxh, R.bxl, R.byh, R.byl);
       gsum[c] = 0.0;
     }
     __syncthreads();
@@ -854,7 +850,7 @@ static void plan_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cf
   t.prep = P.prep.p;
   P.td.alloc(1, st);
   FG_CUDA(cudaMemcpyAsync(P.td.p, &t, sizeof(ScanTile), cudaMemcpyHostToDevice, st));
-  launch_scan_prep(P.td.p, 1, em->n, P.prep.p, st);
+  launch_scan_prep_list(P.td.p, 1, P.tree_list.p, nullptr, P.tree.count, P.prep.p, st);
   // Whole warps only: the closing reductions shuffle across all 32 lanes.
   P.threads = ((t.bin_px * t.bin_px * a + 31) / 32) * 32;
 }
@@ -872,10 +868,10 @@ void scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t 
 // Adjoint of the scan with respect to the per-crystal opacities: g[s] += sum over the rays of
 // pixel p of w[p] / spp * T_ray * chord_s (w = dL/dT of the pixel, T_ray the ray's transmittance).
 void scan_adjoint(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed,
-                  const float* sigma_sorted, const float* wpx, double* g_sorted) {
+                  const float* sigma_sorted, const float* wpx, double* g_sorted, float* T) {
   ScanPlan P;
   plan_scan(e, em, cfg, seed, sigma_sorted, ScanOut{}, P);
-  k_scan_adjoint<<<P.nbins, P.threads, 0, e->stream>>>(P.td.p, wpx, g_sorted);
+  k_scan_adjoint<<<P.nbins, P.threads, 0, e->stream>>>(P.td.p, wpx, g_sorted, T, e->d_stats);
   FG_CUDA(cudaGetLastError());
   FG_CUDA(cudaStreamSynchronize(e->stream));
 }
