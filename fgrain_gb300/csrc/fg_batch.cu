@@ -312,6 +312,7 @@ struct fg_batch {
   DBuf<uint32_t> probe;    // the failure drill's flag (zero, never set)
   uint32_t wait_limit = 0;
   bool wait_probe = false;
+  bool key32 = true;       // every crystal is finite: the tree's centroids are the positions
   unsigned long long maxcells = 0, maxslots = 0;  // the largest tile's cells and bricks
   DBuf<float4> A, Q, D;
   CellBufs tcells;          // the crystals in cells, with their rank in the tree's walk order
@@ -559,7 +560,7 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
 // The reference tree of every tile over its crystals (in slot order), for its leaf boxes and walk
 // order, and the crystals in cells.
 static void stage_bvh(fg_batch* B, cudaStream_t st) {
-  rtree_build(B->rt, B->e->d_err, st, false);
+  rtree_build(B->rt, B->e->d_err, st, false, B->key32);
   const int nt = static_cast<int>(B->ntiles);
   FG_CUDA(cudaMemsetAsync(B->tcells.cnt.p, 0, (B->tcells.ncells + 1) * sizeof(uint32_t), st));
   launch_cells_count(B->d_td.p, nt, B->ncap, B->A.p, B->tcells.cnt.p, B->tcells.place.p, st);
@@ -615,7 +616,7 @@ static void stage_scan(fg_batch* B, cudaStream_t st) {
   // The scan's tree: the same buffers, rebuilt over each tile's developed crystals (the transport
   // and the touch queries are done with the first tree by now).
   k_scan_tree_tiles<<<grid_for(B->ntiles, 128), 128, 0, st>>>(B->d_bt.p, nt, B->devscan.p, B->devlist.p, B->rt_scan.p);
-  rtree_build(B->rt, e->d_err, st, false, B->rt_scan.p);
+  rtree_build(B->rt, e->d_err, st, false, false, B->rt_scan.p);
   launch_scan_prep_list(B->d_sc.p, nt, B->devlist.p, B->devscan.p + B->ncap, B->ncap, B->prep.p, st);
   FG_CUDA(cudaMemsetAsync(B->bin_cnt.p, 0, (B->nbins + 1) * sizeof(uint32_t), st));
   FG_CUDA(cudaMemsetAsync(B->bin_cur.p, 0, (B->nbins + 1) * sizeof(uint32_t), st));
@@ -805,6 +806,7 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       t.a = B->A.p + B->syn[i].cbase;
       t.d = B->D.p + B->syn[i].cbase;
       t.ecap = B->syn[i].ccap;
+      B->key32 = B->key32 && std::isfinite(synth_max_half_dim(B->params[i]));
       t.pad = B->bt[i].pad;
       // The synthesis's radius clamp (emulsion.rs:162-170) for cubes; the other shapes lie in their boxes.
       t.reach = rt_reach(B->params[i].morphology == FG_CUBIC ? 0.48 * B->params[i].r_min : 0.0);

@@ -325,6 +325,7 @@ enum : uint32_t {
   SITE_PHOTON_ID = 6,    // transport: ordered photon id past the photon count
   SITE_NODE = 7,         // tree walk: record index out of range
   SITE_LEAF = 8,         // tree walk: leaf id or its element range out of range
+  SITE_TREE = 10,        // tree build: an element's new place outside its node
   SITE_CELL = 9,         // cells: position range, position or rank out of range
 };
 

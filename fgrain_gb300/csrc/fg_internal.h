@@ -124,11 +124,13 @@ struct StageTimer {
 // emulsion).  Element positions and nodes are laid out tile after tile (RTile::ebase, nbase).
 struct RTreeBufs {
   int ntiles = 0;
-  int levels = 0;                 // global split levels before the per-warp finish
+  int levels = 0;                 // most global split levels before the per-block finish
+  int wpw = 8;                    // words per warp of the levels' chunks
   unsigned long long E = 0, N = 0, nblk = 0;
   uint32_t count = 0;             // elements of a one-tile tree built on the host's request
   DBuf<RTile> tiles;
-  DBuf<uint32_t> idx0, idx1, nof0, nof1, flag, bb, blk, P, Q;
+  DBuf<uint32_t> idx0, idx1, nof0, nof1, bits, wp, P, Q;
+  DBuf<unsigned long long> blk;         // running sum of the big flags, per chunk of positions
   DBuf<unsigned long long> key0, key1;  // three ordered centroid keys per element (SoA), travelling with the order
   DBuf<uint32_t> ridx;            // final element order (slots): a leaf's crystals in reference order
   DBuf<unsigned long long> acc;   // per node: ordered centroid minima, maxima (3 each)
@@ -136,10 +138,10 @@ struct RTreeBufs {
   DBuf<uint32_t> parent;          // per node: parent id (0xffffffff for a root)
   DBuf<uint32_t> nstart, ncount, ntile, ndepth;
   DBuf<int> nsplit;               // split axis, -1 for a leaf
-  DBuf<double> nmid;
   DBuf<int2> nchild;              // global ids of the children
-  DBuf<uint32_t> wl0, wl1, bq, bqpar, cnt;  // global worklists (wl0 then the refit's arrival counts),
-                                            // block queue (node, buffer parity), counts
+  DBuf<unsigned long long> nthr;  // split threshold (a key)
+  DBuf<uint32_t> wl0, wl1, bq, bqpar, cnt;  // worklists (wl0 then the refit's arrival counts), block
+                                            // queue (node, buffer parity), counts and chunk starts
   unsigned long long R = 0;       // walk records (all tiles)
   DBuf<Node4> rnode;              // four-wide walk records (tile-local refs)
   DBuf<uint2> rleaf;              // leaf: first element (tile-local position), count
@@ -240,8 +242,9 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
 // array of the allocation by one with the same layout (ebase, nbase, ecap, ncap) but other element
 // sources, so that one set of buffers serves several trees in turn.
 // walks: also the boxes above the leaves and the walk records (a build that only gives leaves, ranks
-// and leaf boxes does without).
-void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, RTile* tiles_dev = nullptr);
+// and leaf boxes does without).  key32: every tile's crystals are finite FP32 records without FP64
+// copies and without expansion (then their centroids are their positions).
+void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, bool key32, RTile* tiles_dev = nullptr);
 unsigned rtree_kernel_launches(const RTreeBufs& B, bool walks);
 // One tile's build in memory the caller holds (nothing allocated): bytes needed for a tile of ecap
 // elements, and the attach that carves every buffer (the tile descriptor too) from `base`

@@ -1,22 +1,22 @@
 // Device builder of the reference tree (BVH::build / subdivide, bvh.rs:157-295); see fg_rtree.cuh.
 //
-// The tree's topology is built top-down, one level at a time over all tiles of a batch:
-//   reduce  each pending node's centroid box (min / max on order-preserving 64-bit keys of the
-//           FP64 values: exact whatever the order, and on the integer pipes);
+// The tree's topology is built top-down, one level at a time over all tiles of a batch, by one
+// cooperative kernel (k_rt_levels) whose blocks pass the phases of a level together:
 //   decide  leaf or split (largest centroid extent, midpoint 0.5 (lo + hi)), children ids;
-//   flag    every element of a splitting node: centroid >= mid ("big"), with the prefix sum of the
-//           flags (ranks of bigs inside each node's contiguous range) in the same passes;
-//   pq      P_m = position of the m-th big from the left, Q_m = of the m-th small from the right;
-//   place   every element moves to where the reference's swap partition puts it (below).
+//   flag    every element of a splitting node: centroid >= mid ("big"), with the running number of
+//           bigs (a prefix sum along each tile, chunk by chunk); P and Q list the positions of the
+//           bigs and of the smalls by that number;
+//   place   every element moves to where the reference's swap partition puts it (below), and its
+//           centroid joins its child's centroid box (min / max on order-preserving keys: exact
+//           whatever the order, and on the integer pipes).
 // The splits read only the centroids (bvh.rs:196-258), so each element's three order-preserving
-// 64-bit centroid keys (of its FP64 max_dim box, computed once) travel with it, and every pass
-// reads them in order and does no FP64 work.  Nodes of at most RT_CTA_MAX elements leave the
-// global levels: one thread block each builds their subtree with the elements in shared memory,
-// the same passes per level, all levels down to the leaves.  Centroid boxes are reduced
-// segment-wise (a node is a contiguous range of positions).  The node boxes (the union of the
-// elements' boxes, which the reference stores but never splits on) are formed bottom up: a block
-// forms those of its subtree after its last level, k_rt_refit those above the blocks' subtrees;
-// min and max are exact, so the order does not matter.
+// centroid keys travel with it, and every pass reads them in order.  A centroid is the midpoint of
+// the FP64 max_dim box, which for FP32 crystals without expansion is the FP32 position itself: such
+// trees carry 32-bit keys, the others 64-bit ones.  Nodes of at most RT_CTA_MAX elements leave the
+// global levels: one thread block each builds their subtree with the elements in shared memory, the
+// same passes per level, all levels down to the leaves.  The leaf boxes (the union of the elements'
+// boxes) are formed by a pass over the leaves; the boxes above them, which only the walks need,
+// bottom up (min and max are exact, so the order does not matter).
 //
 // The swap partition (bvh.rs:244-258: i from the left, j from the right; a small at i stays and i
 // advances, a big at i is swapped with j and j retreats) examines the range as two streams: the
@@ -28,8 +28,9 @@
 //   r < li, the m-th big:     Q_{m-1} - 1            (bigs fill the right end in examination order)
 //   r >= li, the m-th small from the right:  P_m     (takes the place of the m-th big)
 //   r >= li, big:             r - 1                  (shifts one place towards the middle)
-// S is the left child's size.  A simulation of the reference loop confirms the rule and the closed
-// forms of K and li on random ranges.
+// where P_m is the m-th big from the left and Q_m the m-th small from the right; S is the left
+// child's size.  A simulation of the reference loop confirms the rule and the closed forms of K and
+// li on random ranges.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -44,8 +45,8 @@ namespace {
 
 constexpr unsigned RT_BLOCK = 256;
 
-// Global split levels for trees of up to emax elements: halving down to the per-block size, plus a
-// wide margin for uneven splits (unused levels cost only launches that find no work).
+// Most global split levels for trees of up to emax elements: halving down to the per-block size,
+// plus a wide margin for uneven splits (the kernel ends with the last level that has work).
 int levels_for(uint32_t emax) {
   if (emax <= static_cast<uint32_t>(RT_CTA_MAX)) return 0;
   int lv = 0;
@@ -53,7 +54,16 @@ int levels_for(uint32_t emax) {
   return std::min(lv + 8, 44);
 }
 
-constexpr unsigned SCAN_ITEMS = 2048;  // entries per block of the prefix sum (256 threads x 8)
+// Work goes by chunks of consecutive positions (a tile's chunks start at its first): wpw words of 32
+// positions for each of a block's eight warps.  A warp's words follow one another, so small builds
+// take short chunks: enough blocks, and less latency in a row (309 k elements:
+// 330 us with eight words, 242 with two; 705 k with 64-bit keys: 454 and 542).
+constexpr int RT_WARPS = RT_BLOCK / 32;
+constexpr int RT_WPW_LARGE = 8, RT_WPW_SMALL = 2;
+constexpr unsigned long long RT_LARGE = 600ull * 1000ull;  // elements from which chunks are long
+constexpr unsigned rt_chunk(int wpw) { return 32u * RT_WARPS * static_cast<unsigned>(wpw); }
+constexpr unsigned RT_CNT_BAR = 4;               // RtArgs::cnt: the grid barrier's arrivals
+constexpr unsigned RT_CNT_TILES = 16;            // first of ntiles + 1 words: chunks before each tile
 
 __device__ __forceinline__ unsigned long long ord64(double v) {
   const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
@@ -63,28 +73,66 @@ __device__ __forceinline__ double unord64(unsigned long long u) {
   const unsigned long long b = (u & 0x8000000000000000ull) ? (u & 0x7fffffffffffffffull) : ~u;
   return __longlong_as_double(static_cast<long long>(b));
 }
-
-__device__ __forceinline__ int rt_tile_of(const RTile* tiles, int ntiles, unsigned long long x) {
-  int lo = 0, hi = ntiles - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tiles[mid].ebase <= x) lo = mid; else hi = mid - 1;
-  }
-  return lo;
+__device__ __forceinline__ uint32_t ord32(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
+__device__ __forceinline__ float unord32(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+__device__ __forceinline__ unsigned long long umin64(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
+__device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+
+// Centroid keys of either width: made so that -0 orders as +0, as the FP64 comparisons see them.
+// key >= threshold(mid) iff the centroid >= mid.
+struct Key32 {
+  using T = uint32_t;
+  __device__ static double value(T k) { return static_cast<double>(unord32(k)); }
+  __device__ static T threshold(double mid) { return ord32(__double2float_ru(mid) + 0.0f); }
+  __device__ static T warp_min(T k) { return __reduce_min_sync(0xffffffffu, k); }
+  __device__ static T warp_max(T k) { return __reduce_max_sync(0xffffffffu, k); }
+  __device__ static void make(const RTile& t, uint32_t s, T k[3]) {
+    const float4 a = t.a[s];
+    k[0] = ord32(a.x + 0.0f);
+    k[1] = ord32(a.y + 0.0f);
+    k[2] = ord32(a.z + 0.0f);
+  }
+};
+struct Key64 {
+  using T = unsigned long long;
+  __device__ static double value(T k) { return unord64(k); }
+  __device__ static T threshold(double mid) { return ord64(mid); }
+  // As two 32-bit reductions: the high words, then the low words of the lanes holding that high word.
+  __device__ static T warp_min(T k) {
+    const uint32_t hi = static_cast<uint32_t>(k >> 32), h = __reduce_min_sync(0xffffffffu, hi);
+    const uint32_t l = __reduce_min_sync(0xffffffffu, hi == h ? static_cast<uint32_t>(k) : 0xffffffffu);
+    return (static_cast<T>(h) << 32) | l;
+  }
+  __device__ static T warp_max(T k) {
+    const uint32_t hi = static_cast<uint32_t>(k >> 32), h = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t l = __reduce_max_sync(0xffffffffu, hi == h ? static_cast<uint32_t>(k) : 0u);
+    return (static_cast<T>(h) << 32) | l;
+  }
+  __device__ static void make(const RTile& t, uint32_t s, T k[3]) {
+    double lo[3], hi[3], cc[3];
+    rt_box_pm(rt_pm(t, s), lo, hi, cc);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) k[i] = ord64(__dadd_rn(cc[i], 0.0));
+  }
+};
 
 struct RtArgs {
   RTile* tiles;
   int ntiles;
   unsigned long long E, N;
   uint32_t* idx[2];
-  // Keys of the element at position x, field f at key[c][f * E + x]: ord64 of the centroid xyz.
-  unsigned long long* key[2];
+  // Keys of the element at position x, field f at key[c][f * E + x]: centroid xyz (Key32 or Key64).
+  void* key[2];
   uint32_t* nof[2];
-  uint32_t* flag;
-  uint32_t* bb;
-  uint32_t* blk;
-  uint32_t* P;
+  uint32_t* bits;   // big flags, 32 positions a word (chunk by chunk)
+  uint32_t* wp;     // bigs of the tile before each word
+  unsigned long long* blk;  // per chunk: level tag, state and count of the running sum
+  uint32_t* P;      // positions of the tile's bigs and smalls by number (tile-relative, at ebase)
   uint32_t* Q;
   uint32_t* ridx;
   unsigned long long* acc;
@@ -92,12 +140,12 @@ struct RtArgs {
   uint32_t* parent;  // parent id of each node (RT_NONE for a root)
   uint32_t *nstart, *ncount, *ntile, *ndepth;
   int* nsplit;
-  double* nmid;
+  unsigned long long* nthr;  // split threshold (a key)
   int2* nchild;
-  uint32_t* wl[2];
+  uint32_t* wl[2];  // nodes pending for the levels of either parity
   uint32_t* bq;     // block queue: nodes of at most RT_CTA_MAX elements
   uint32_t* bqpar;  // and the buffer parity holding their elements
-  uint32_t* cnt;    // [0], [1] worklist counts, [2] block queue count
+  uint32_t* cnt;    // [0], [1] worklist counts, [2] block queue count, RT_CNT_BAR, RT_CNT_TILES
   uint32_t* err;
 };
 
@@ -112,18 +160,12 @@ __device__ __forceinline__ bool alloc_pair(const RtArgs& A, int t, uint32_t& l) 
 }
 
 constexpr uint32_t RT_NONE = 0xffffffffu;
-constexpr uint32_t RT_BOX_ONLY = 2;  // block-queue entry of a finished leaf: only its box is formed
 
 // Hands a new node of n elements (held in buffer `par`) to the phase that builds it: the global
-// levels (more than RT_CTA_MAX elements; its centroid accumulators start empty) or one block.
+// levels (more than RT_CTA_MAX elements) or one block.
 __device__ __forceinline__ void rt_enqueue(const RtArgs& A, uint32_t id, uint32_t n, int par) {
   A.nsplit[id] = -1;
   if (n > static_cast<uint32_t>(RT_CTA_MAX)) {
-    unsigned long long* a = A.acc + 6ull * id;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) a[k] = ~0ull;  // minima
-#pragma unroll
-    for (int k = 3; k < 6; ++k) a[k] = 0ull;  // maxima
     A.wl[par][atomicAdd(&A.cnt[par], 1u)] = id;
   } else if (n > 0) {
     const uint32_t q = atomicAdd(&A.cnt[2], 1u);
@@ -132,85 +174,476 @@ __device__ __forceinline__ void rt_enqueue(const RtArgs& A, uint32_t id, uint32_
   }
 }
 
-// The 6 reduction keys of the element at position x of a key array (field f at key[f * stride +
-// x]): centroid xyz as minima, then as maxima.  Min and max are exact in any order, and on the
-// ordered 64-bit keys they run on the integer pipes (GB300's FP64 pipe is narrow).
-__device__ __forceinline__ void rt_keys(const unsigned long long* key, unsigned long long stride, unsigned long long x,
-                                        unsigned long long k[6]) {
+// Empties a node's centroid accumulators (minima, then maxima).
+__device__ __forceinline__ void rt_acc_clear(const RtArgs& A, uint32_t id) {
+  unsigned long long* a = A.acc + 6ull * id;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    k[i] = key[i * stride + x];
-    k[3 + i] = k[i];
+  for (int k = 0; k < 3; ++k) {
+    a[k] = ~0ull;
+    a[3 + k] = 0ull;
   }
 }
 
-// The three centroid keys of element slot s of tile T, written to position x of key[f * stride +
-// x] (normalised so that -0 orders as +0, as the FP64 comparisons see them).
-__device__ __forceinline__ void rt_key3(const RTile& T, uint32_t s, unsigned long long* key, unsigned long long stride,
-                                        unsigned long long x) {
-  double lo[3], hi[3], cc[3];
-  rt_box_pm(rt_pm(T, s), lo, hi, cc);
+// One warp's running centroid box of one node, per lane; flush adds it to the node's accumulators.
+template <class K>
+struct RtRun {
+  typename K::T lo[3], hi[3];
+  __device__ void clear() {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) key[i * stride + x] = ord64(__dadd_rn(cc[i], 0.0));
-}
-
-// Element order and roots.  Thread x < E fills position x; one thread per tile sets up its root.
-__global__ void k_rt_init(RtArgs A) {
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  const unsigned long long g0 = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-  for (unsigned long long x = g0; x < A.E; x += stride) {
-    const int t = rt_tile_of(A.tiles, A.ntiles, x);
-    const RTile& T = A.tiles[t];
-    const unsigned long long k = x - T.ebase;
-    uint32_t v = RT_DONE;
-    if (k < T.n) {
-      const uint32_t slot = T.order ? static_cast<uint32_t>(T.order[k] - T.obase) : static_cast<uint32_t>(k);
-      A.idx[0][x] = slot;
-      rt_key3(T, slot, A.key[0], A.E, x);
-      v = T.n > static_cast<uint32_t>(RT_CTA_MAX) ? static_cast<uint32_t>(T.nbase + 1) : RT_DONE;
+    for (int i = 0; i < 3; ++i) {
+      lo[i] = ~static_cast<typename K::T>(0);
+      hi[i] = 0;
     }
-    A.nof[0][x] = v;
   }
-  for (unsigned long long t = g0; t < static_cast<unsigned long long>(A.ntiles); t += stride) {
-    RTile& T = A.tiles[t];
-    T.nodes = 2;
-    T.depth = T.n ? 1 : 0;
-    const unsigned long long root = T.nbase + 1;
-    A.nstart[root] = static_cast<uint32_t>(T.ebase);
-    A.ncount[root] = T.n;
+  __device__ void add(const typename K::T k[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      lo[i] = min(lo[i], k[i]);
+      hi[i] = max(hi[i], k[i]);
+    }
+  }
+  // All 32 lanes; lanes 0-5 do one atomic each.
+  __device__ void flush(const RtArgs& A, uint32_t id) {
+    unsigned long long v = 0;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const typename K::T l = K::warp_min(lo[i]), h = K::warp_max(hi[i]);
+      if (lane == i) v = l;
+      if (lane == 3 + i) v = h;
+    }
+    unsigned long long* a = A.acc + 6ull * id;
+    if (lane < 3) atomicMin(a + lane, v);
+    else if (lane < 6) atomicMax(a + lane, v);
+    clear();
+  }
+};
+
+// All blocks of the (cooperative) grid arrive before any leaves; what they wrote is visible then.
+// The wait is bounded: false (error set) when it gives up, and the kernel then ends.
+__device__ bool rt_grid_sync(const RtArgs& A) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    if (gridDim.x > 1) {
+      __threadfence();
+      volatile uint32_t* bar = A.cnt + RT_CNT_BAR;
+      const uint32_t ticket = atomicAdd(A.cnt + RT_CNT_BAR, 1u);
+      const uint32_t target = (ticket / gridDim.x + 1u) * gridDim.x;
+      uint32_t spins = 0;
+      while (static_cast<int32_t>(*bar - target) < 0) {
+        if (++spins > (1u << 24)) {
+          atomicOr(A.err, ERR_SPIN_LIMIT);
+          ok = 0;
+          break;
+        }
+        __nanosleep(32);
+      }
+      __threadfence();
+    }
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Running sum of the chunk counts along a tile: chunk ch (first: the tile's first) adds `total` and
+// gets the sum of the tile's earlier chunks.  One warp calls it.  A chunk publishes its own count,
+// then looks back over the counts or sums of the chunks before it until it meets a sum; chunks are
+// taken in increasing order by blocks that all run, so every count arrives.  The wait is bounded.
+// Words are tagged with the level, so they need no clearing between levels.
+__device__ __forceinline__ uint32_t rt_chunk_sum(const RtArgs& A, uint32_t ch, uint32_t first, uint32_t level,
+                                                 uint32_t total) {
+  const unsigned long long tag = static_cast<unsigned long long>(level + 1u) << 40;
+  const unsigned long long COUNT = 1ull << 32, SUM = 2ull << 32;
+  const uint32_t lane = threadIdx.x & 31;
+  if (ch == first) {
+    if (lane == 0) atomicExch(A.blk + ch, tag | SUM | total);
+    return 0;
+  }
+  if (lane == 0) atomicExch(A.blk + ch, tag | COUNT | total);
+  uint32_t sum = 0, spins = 0;
+  for (uint32_t back = ch;;) {  // chunks back - 1 - lane
+    const bool in = lane < back - first;
+    const unsigned long long w = in ? *(volatile unsigned long long*)(A.blk + (back - 1 - lane)) : tag | SUM;
+    const bool ready = (w >> 40) == (tag >> 40);
+    if (!__all_sync(0xffffffffu, ready)) {
+      if (++spins > (1u << 22)) {
+        if (lane == 0) atomicOr(A.err, ERR_SPIN_LIMIT);
+        break;
+      }
+      continue;
+    }
+    const unsigned sums = __ballot_sync(0xffffffffu, (w & SUM) != 0);
+    const int last = sums ? __ffs(sums) - 1 : 31;
+    sum += __reduce_add_sync(0xffffffffu, static_cast<int>(lane) <= last ? static_cast<uint32_t>(w) : 0u);
+    if (sums) break;
+    back -= 32;
+  }
+  if (lane == 0) atomicExch(A.blk + ch, tag | SUM | (sum + total));
+  return sum;
+}
+
+// Bigs of the tile before tile-relative position r (word base wb of the tile).
+__device__ __forceinline__ uint32_t rt_rank(const RtArgs& A, uint32_t wb, uint32_t r) {
+  const uint32_t w = wb + (r >> 5);
+  return A.wp[w] + __popc(A.bits[w] & ((1u << (r & 31u)) - 1u));
+}
+__device__ __forceinline__ uint32_t rt_big(const RtArgs& A, uint32_t wb, uint32_t r) {
+  return (A.bits[wb + (r >> 5)] >> (r & 31u)) & 1u;
+}
+
+// The chunk's tile (the last whose first chunk is <= ch), by one thread.
+__device__ __forceinline__ int rt_chunk_tile(const uint32_t* start, int ntiles, uint32_t ch) {
+  int lo = 0, hi = ntiles - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= ch) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Element order, keys and the global levels, all of them.  Work goes by chunks of the tiles' elements
+// (tiles with few elements in a large range cost only what they hold); a warp takes WPW words of 32
+// consecutive positions.  One launch instead of eight per level, levels without work
+// included: a level of few elements costs three grid barriers.
+//
+// Bound by latency more than by the streams (Key32: about 56 B per element and level, a third of the
+// copy bandwidth): each word's node, element and keys are read while the word before is placed.
+// Against eight launches per level with 64-bit keys, 18.9 M elements in 25 tiles: 11.5 -> 4.9 ms; the
+// whole build of one tile's 3,556: 0.19 -> 0.10 ms, of 309 k: 0.60 -> 0.35 ms.
+template <class K, int WPW>
+__global__ void __launch_bounds__(RT_BLOCK, 4) k_rt_levels(RtArgs A, int levels) {
+  using T = typename K::T;
+  constexpr unsigned RT_CHUNK = rt_chunk(WPW), RT_WORDS = RT_CHUNK / 32;
+  __shared__ int s_tile;
+  __shared__ uint32_t s_wsum[RT_BLOCK / 32], s_base;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t* cst = A.cnt + RT_CNT_TILES;
+  const unsigned g0 = blockIdx.x * RT_BLOCK + tid, gs = gridDim.x * RT_BLOCK;
+  // Roots, and the first chunk of every tile (block 0).
+  for (int t = static_cast<int>(g0); t < A.ntiles; t += static_cast<int>(gs)) {
+    RTile& R = A.tiles[t];
+    R.nodes = 2;
+    R.depth = R.n ? 1 : 0;
+    const uint32_t root = static_cast<uint32_t>(R.nbase + 1);
+    A.nstart[root] = static_cast<uint32_t>(R.ebase);
+    A.ncount[root] = R.n;
     A.ntile[root] = static_cast<uint32_t>(t);
     A.ndepth[root] = 1;
     A.parent[root] = RT_NONE;
-    rt_enqueue(A, static_cast<uint32_t>(root), T.n, 0);
+    rt_acc_clear(A, root);
+    rt_enqueue(A, root, R.n, 0);
   }
+  if (blockIdx.x == 0) {
+    uint32_t carry = 0;
+    for (int base = 0; base < A.ntiles; base += RT_BLOCK) {
+      const int t = base + tid;
+      const uint32_t v = t < A.ntiles ? (A.tiles[t].n + RT_CHUNK - 1) / RT_CHUNK : 0u;
+      uint32_t incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) s_wsum[warp] = incl;
+      __syncthreads();
+      uint32_t off = carry, tot = 0;
+      for (int w = 0; w < static_cast<int>(RT_BLOCK / 32); ++w) {
+        if (w < warp) off += s_wsum[w];
+        tot += s_wsum[w];
+      }
+      if (t < A.ntiles) cst[t] = off + incl - v;
+      carry += tot;
+      __syncthreads();
+    }
+    if (tid == 0) cst[A.ntiles] = carry;
+  }
+  if (!rt_grid_sync(A)) return;
+  const uint32_t nch = *(volatile uint32_t*)(cst + A.ntiles);
+  // Order, keys and the roots' centroid boxes.
+  {
+    T* key = static_cast<T*>(A.key[0]);
+    for (uint32_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+      if (tid == 0) s_tile = rt_chunk_tile(cst, A.ntiles, ch);
+      __syncthreads();
+      const RTile& R = A.tiles[s_tile];
+      const uint32_t r0 = (ch - cst[s_tile]) * RT_CHUNK + warp * (32 * WPW);
+      const bool big = R.n > static_cast<uint32_t>(RT_CTA_MAX);
+      RtRun<K> run;
+      run.clear();
+#pragma unroll
+      for (int j = 0; j < WPW; ++j) {
+        const uint32_t r = r0 + j * 32 + lane;
+        if (r >= R.n) continue;
+        const unsigned long long x = R.ebase + r;
+        const uint32_t slot = R.order ? static_cast<uint32_t>(R.order[r] - R.obase) : r;
+        T k[3];
+        K::make(R, slot, k);
+        A.idx[0][x] = slot;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) key[f * A.E + x] = k[f];
+        if (big) run.add(k);
+        A.nof[0][x] = big ? static_cast<uint32_t>(R.nbase + 1) : RT_DONE;
+      }
+      __syncwarp();
+      if (big) run.flush(A, static_cast<uint32_t>(R.nbase + 1));
+      __syncthreads();
+    }
+  }
+  if (!rt_grid_sync(A)) return;
+  int L = 0;
+  for (; L < levels; ++L) {
+    const int c = L & 1, o = c ^ 1;
+    const T* key = static_cast<const T*>(A.key[c]);
+    T* keyo = static_cast<T*>(A.key[o]);
+    const uint32_t nw = *(volatile uint32_t*)(A.cnt + c);
+    if (nw == 0) break;
+    // Leaf or split for every pending node of this level (subdivide, bvh.rs:200-270).  (Each warp
+    // deciding for the nodes it meets saves a barrier but repeats the FP64 chain: 5.4 ms against 4.9
+    // on 18.9 M elements, 261 us against 242 on 309 k.)
+    if (g0 == 0) A.cnt[o] = 0;  // read by all before the last barrier; filled by the place phase
+    for (uint32_t i = g0; i < nw; i += gs) {
+      const uint32_t node = A.wl[c][i];
+      const int t = static_cast<int>(A.ntile[node]);
+      const unsigned long long* a = A.acc + 6ull * node;
+      double clo[3], chi[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        clo[k] = K::value(static_cast<T>(__ldcg(a + k)));
+        chi[k] = K::value(static_cast<T>(__ldcg(a + 3 + k)));
+      }
+      const double ex = __dsub_rn(chi[0], clo[0]), ey = __dsub_rn(chi[1], clo[1]), ez = __dsub_rn(chi[2], clo[2]);
+      const int axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
+      const double ext = axis == 0 ? ex : (axis == 1 ? ey : ez);
+      uint32_t l = 0;
+      if (ext <= 1e-7 || !alloc_pair(A, t, l)) {
+        A.nsplit[node] = -1;  // leaf (degenerate centroids, or no node capacity left)
+        continue;
+      }
+      A.nsplit[node] = axis;
+      A.nthr[node] = K::threshold(__dmul_rn(0.5, __dadd_rn(clo[axis], chi[axis])));
+      const uint32_t id = static_cast<uint32_t>(A.tiles[t].nbase + l);
+      A.nchild[node] = make_int2(static_cast<int>(id), static_cast<int>(id + 1));
+      A.parent[id] = node;
+      A.parent[id + 1] = node;
+      rt_acc_clear(A, id);
+      rt_acc_clear(A, id + 1);
+    }
+    if (!rt_grid_sync(A)) return;
+    // Flags, their running number, and the positions of bigs and smalls by number.
+    for (uint32_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+      if (tid == 0) s_tile = rt_chunk_tile(cst, A.ntiles, ch);
+      __syncthreads();
+      const RTile& R = A.tiles[s_tile];
+      const uint32_t first = cst[s_tile];
+      const uint32_t r0 = (ch - first) * RT_CHUNK + warp * (32 * WPW);
+      uint32_t mybits = 0, myact = 0;  // lane j: word j's flags and its positions of splitting nodes
+      uint32_t cur = RT_NONE;
+      int axis = -1;
+      T thr = 0;
+      uint32_t nodes[WPW];
+#pragma unroll
+      for (int j = 0; j < WPW; ++j) {
+        const uint32_t r = r0 + j * 32 + lane;
+        nodes[j] = r < R.n ? A.nof[c][R.ebase + r] : RT_DONE;
+      }
+#pragma unroll
+      for (int j = 0; j < WPW; ++j) {
+        const uint32_t r = r0 + j * 32 + lane;
+        const uint32_t node = nodes[j];
+        bool act = false, flag = false;
+        for (unsigned todo = __ballot_sync(0xffffffffu, !(node & RT_DONE)); todo;) {
+          const uint32_t nd = __shfl_sync(0xffffffffu, node, __ffs(todo) - 1);
+          if (nd != cur) {
+            cur = nd;
+            axis = A.nsplit[nd];
+            thr = static_cast<T>(A.nthr[nd]);
+          }
+          if (node == nd && axis >= 0) {
+            act = true;
+            flag = key[axis * A.E + R.ebase + r] >= thr;
+          }
+          todo &= ~__ballot_sync(0xffffffffu, node == nd);
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, flag), a = __ballot_sync(0xffffffffu, act);
+        if (lane == j) {
+          mybits = b;
+          myact = a;
+        }
+      }
+      uint32_t incl = __popc(mybits);
+#pragma unroll
+      for (int d = 1; d < WPW; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+      }
+      if (lane == WPW - 1) s_wsum[warp] = incl;
+      __syncthreads();
+      uint32_t off = 0, tot = 0;
+      for (int w = 0; w < static_cast<int>(RT_BLOCK / 32); ++w) {
+        if (w < warp) off += s_wsum[w];
+        tot += s_wsum[w];
+      }
+      if (warp == 0) {
+        const uint32_t b = rt_chunk_sum(A, ch, first, static_cast<uint32_t>(L), tot);
+        if (lane == 0) s_base = b;
+      }
+      __syncthreads();
+      const uint32_t mywp = s_base + off + incl - __popc(mybits);
+      if (lane < WPW) {
+        const uint32_t w = ch * RT_WORDS + warp * WPW + lane;
+        A.bits[w] = mybits;
+        A.wp[w] = mywp;
+      }
+      for (int j = 0; j < WPW; ++j) {
+        const uint32_t b = __shfl_sync(0xffffffffu, mybits, j), a = __shfl_sync(0xffffffffu, myact, j);
+        const uint32_t p = __shfl_sync(0xffffffffu, mywp, j) + __popc(b & lt);
+        const uint32_t r = r0 + j * 32 + lane;
+        if (!((a >> lane) & 1u) || p > r) continue;
+        if ((b >> lane) & 1u) A.P[R.ebase + p] = r; else A.Q[R.ebase + (r - p)] = r;
+      }
+      __syncthreads();
+    }
+    if (!rt_grid_sync(A)) return;
+    // Every element of a splitting node moves to its place after the reference's swap partition and
+    // joins its child's centroid box; elements of new leaves are done; the children are set up.
+    for (uint32_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+      if (tid == 0) s_tile = rt_chunk_tile(cst, A.ntiles, ch);
+      __syncthreads();
+      const RTile& R = A.tiles[s_tile];
+      const uint32_t first = cst[s_tile], wb = first * RT_WORDS;
+      const uint32_t r0 = (ch - first) * RT_CHUNK + warp * (32 * WPW);
+      // The node at hand: split axis, start and size, bigs before it, smalls, end of the left stream,
+      // left child's size, children.
+      uint32_t cur = RT_NONE, s = 0, n = 0, bs = 0, St = 0, li = 0, Sp = 0;
+      int axis = -1;
+      int2 kid = make_int2(0, 0);
+      RtRun<K> run[2];
+      run[0].clear();
+      run[1].clear();
+      auto flush = [&]() {
+        if (axis < 0) return;
+        if (Sp > static_cast<uint32_t>(RT_CTA_MAX)) run[0].flush(A, static_cast<uint32_t>(kid.x));
+        if (n - Sp > static_cast<uint32_t>(RT_CTA_MAX)) run[1].flush(A, static_cast<uint32_t>(kid.y));
+      };
+      // A word's node, element and keys are read while the word before is placed.
+      uint32_t pnode = RT_DONE, pel = 0;
+      T pk[3] = {0, 0, 0};
+      auto fetch = [&](uint32_t q) {
+        pnode = RT_DONE;
+        if (q >= R.n) return;
+        pnode = A.nof[c][R.ebase + q];
+        if (pnode & RT_DONE) return;
+        pel = A.idx[c][R.ebase + q];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) pk[f] = key[f * A.E + R.ebase + q];
+      };
+      fetch(r0 + lane);
+#pragma unroll 1
+      for (int j = 0; j < WPW; ++j) {
+        const uint32_t q = r0 + j * 32 + lane;  // tile-relative position
+        const unsigned long long x = R.ebase + q;
+        const bool in = q < R.n;
+        const uint32_t node = pnode, el = pel;
+        const T k[3] = {pk[0], pk[1], pk[2]};
+        if (j + 1 < WPW) fetch(q + 32);
+        if (in && (node & RT_DONE)) A.nof[o][x] = RT_DONE;
+        for (unsigned todo = __ballot_sync(0xffffffffu, !(node & RT_DONE)); todo;) {
+          const uint32_t nd = __shfl_sync(0xffffffffu, node, __ffs(todo) - 1);
+          if (nd != cur) {
+            flush();
+            run[0].clear();
+            run[1].clear();
+            cur = nd;
+            axis = A.nsplit[nd];
+            s = A.nstart[nd] - static_cast<uint32_t>(R.ebase);
+            n = A.ncount[nd];
+            if (axis >= 0) {
+              bs = rt_rank(A, wb, s);
+              uint32_t Bt = rt_rank(A, wb, s + n - 1) + rt_big(A, wb, s + n - 1) - bs;
+              if (Bt > n) {  // only after a wait that gave up
+                atomicOr(A.err, ERR_BAD_INDEX);
+                Bt = n;
+              }
+              St = n - Bt;
+              li = St + (St < n ? rt_big(A, wb, s + St) : 0u);
+              // The reference splits at count / 2 when every centroid fell on one side (bvh.rs:260-265).
+              Sp = (St == 0 || St == n) ? n / 2 : St;
+              kid = A.nchild[nd];
+            }
+          }
+          if (node == nd) {
+            if (axis < 0) {  // a leaf of this level: its order is final
+              A.ridx[x] = el;
+              A.nof[o][x] = RT_DONE;
+            } else {
+              const uint32_t r = q - s;
+              const uint32_t w = A.bits[wb + (q >> 5)];
+              const uint32_t Bb = A.wp[wb + (q >> 5)] + __popc(w & lt) - bs;
+              const bool big = (w >> lane) & 1u;
+              // Where P or Q gives the place: the big's partner Q_{m-1} (m - 1 = Bb), the small's P_m.
+              uint32_t dest = r;
+              const bool look = (r < li) == big && !(big && Bb == 0);
+              if (look) {
+                const uint32_t at = big ? s - bs + (St - Bb) : bs + (St - (r - Bb)) - 1;
+                dest = at < R.n ? (big ? A.Q[R.ebase + at] : A.P[R.ebase + at]) - s : n;
+                if (big) --dest;
+              } else if (big) {
+                dest = r < li ? n - 1 : r - 1;
+              }
+              if (index_ok(dest < n, A.err, SITE_TREE, dest, n)) {
+                const bool left = dest < Sp;
+                const uint32_t csize = left ? Sp : n - Sp;
+                const unsigned long long y = R.ebase + s + dest;
+                const bool deep = csize > static_cast<uint32_t>(RT_CTA_MAX);
+#pragma unroll
+                for (int f = 0; f < 3; ++f) keyo[f * A.E + y] = k[f];
+                A.idx[o][y] = el;
+                A.nof[o][y] = deep ? static_cast<uint32_t>(left ? kid.x : kid.y) : RT_DONE;
+                if (deep) {
+                  if (left) run[0].add(k); else run[1].add(k);
+                }
+              }
+              if (r == 0) {
+                const uint32_t dep = A.ndepth[nd] + 1;
+#pragma unroll
+                for (int side = 0; side < 2; ++side) {
+                  const uint32_t id = static_cast<uint32_t>(side ? kid.y : kid.x), cs = side ? n - Sp : Sp;
+                  A.nstart[id] = static_cast<uint32_t>(R.ebase) + s + (side ? Sp : 0u);
+                  A.ncount[id] = cs;
+                  A.ntile[id] = static_cast<uint32_t>(s_tile);
+                  A.ndepth[id] = dep;
+                  rt_enqueue(A, id, cs, o);
+                }
+                atomicMax(&A.tiles[s_tile].depth, dep);
+              }
+            }
+          }
+          todo &= ~__ballot_sync(0xffffffffu, node == nd);
+        }
+      }
+      flush();
+      __syncthreads();
+    }
+    if (!rt_grid_sync(A)) return;
+  }
+  if (g0 == 0 && *(volatile uint32_t*)(A.cnt + (L & 1)) != 0) atomicOr(A.err, ERR_LIST_OVERFLOW);  // levels spent
 }
-
-__device__ __forceinline__ unsigned long long umin64(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
-__device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
 // Segment-wise reduction over a warp's 32 consecutive positions: lanes with equal `seg` form
 // contiguous runs (a node is a contiguous range of positions, so equal values at two lanes mean
 // the same node in between).  On return the first lane of each run holds the run's minima
 // (k[0..2]) and maxima (k[3..5]); the return value says whether this lane is a run's first.
 // Lanes without a node pass a seg value no other lane has.  All 32 lanes call it.
-__device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, unsigned long long k[6]) {
+template <class K>
+__device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, typename K::T k[6]) {
   const int lane = threadIdx.x & 31;
-  if (__all_sync(0xffffffffu, __shfl_sync(0xffffffffu, seg, 0) == seg)) {
-    // One node across the warp (the common case): each 64-bit minimum or maximum as two 32-bit
-    // warp reductions, the high words, then the low words of the lanes holding that high word.
+  if (__all_sync(0xffffffffu, __shfl_sync(0xffffffffu, seg, 0) == seg)) {  // one node across the warp
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const uint32_t hi = static_cast<uint32_t>(k[i] >> 32), lo = static_cast<uint32_t>(k[i]);
-      uint32_t h, l;
-      if (i < 3) {
-        h = __reduce_min_sync(0xffffffffu, hi);
-        l = __reduce_min_sync(0xffffffffu, hi == h ? lo : 0xffffffffu);
-      } else {
-        h = __reduce_max_sync(0xffffffffu, hi);
-        l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
-      }
-      k[i] = (static_cast<unsigned long long>(h) << 32) | l;
-    }
+    for (int i = 0; i < 6; ++i) k[i] = i < 3 ? K::warp_min(k[i]) : K::warp_max(k[i]);
     return lane == 0;
   }
 #pragma unroll
@@ -219,260 +652,12 @@ __device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, unsigned long long k
     const bool take = lane + o < 32 && ns == seg;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      const unsigned long long y = __shfl_down_sync(0xffffffffu, k[i], o);
-      if (take) k[i] = i < 3 ? umin64(k[i], y) : umax64(k[i], y);
+      const typename K::T y = __shfl_down_sync(0xffffffffu, k[i], o);
+      if (take) k[i] = i < 3 ? min(k[i], y) : max(k[i], y);
     }
   }
   const uint32_t up = __shfl_up_sync(0xffffffffu, seg, 1);
   return lane == 0 || up != seg;
-}
-
-__device__ __forceinline__ void rt_keys_empty(unsigned long long k[6]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    k[i] = ~0ull;
-    k[3 + i] = 0ull;
-  }
-}
-
-// Centroid box of every pending node: segment-wise per warp, then one set of 6 atomics per warp
-// and node.
-__global__ void k_rt_reduce(RtArgs A, int c) {
-  if (A.cnt[c] == 0) return;
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  for (unsigned long long base = blockIdx.x * static_cast<unsigned long long>(blockDim.x); base < A.E; base += stride) {
-    const unsigned long long x = base + threadIdx.x;
-    const uint32_t node = x < A.E ? A.nof[c][x] : RT_DONE;
-    const bool act = !(node & RT_DONE);
-    if (!__any_sync(0xffffffffu, act)) continue;
-    unsigned long long k[6];
-    if (act) rt_keys(A.key[c], A.E, x, k); else rt_keys_empty(k);
-    const bool head = rt_seg_reduce(act ? node : (RT_DONE | (threadIdx.x & 31)), k);
-    if (act && head) {
-      unsigned long long* a = A.acc + 6ull * node;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) atomicMin(a + i, k[i]);
-#pragma unroll
-      for (int i = 3; i < 6; ++i) atomicMax(a + i, k[i]);
-    }
-  }
-}
-
-// Leaf or split for every pending node of this level (subdivide, bvh.rs:200-270).
-__global__ void k_rt_decide(RtArgs A, int c) {
-  const uint32_t nw = A.cnt[c];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += gridDim.x * blockDim.x) {
-    const uint32_t node = A.wl[c][i];
-    const int t = static_cast<int>(A.ntile[node]);
-    const unsigned long long* a = A.acc + 6ull * node;
-    double clo[3], chi[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      clo[k] = unord64(a[k]);
-      chi[k] = unord64(a[3 + k]);
-    }
-    const double ex = __dsub_rn(chi[0], clo[0]), ey = __dsub_rn(chi[1], clo[1]), ez = __dsub_rn(chi[2], clo[2]);
-    const int axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
-    const double ext = axis == 0 ? ex : (axis == 1 ? ey : ez);
-    uint32_t l = 0;
-    if (A.ncount[node] <= 4 || ext <= 1e-7 || !alloc_pair(A, t, l)) {
-      A.nsplit[node] = -1;  // leaf (degenerate centroids, or no node capacity left)
-      const uint32_t q = atomicAdd(&A.cnt[2], 1u);  // a block forms its box
-      A.bq[q] = node;
-      A.bqpar[q] = RT_BOX_ONLY;
-      continue;
-    }
-    A.nsplit[node] = axis;
-    A.nmid[node] = __dmul_rn(0.5, __dadd_rn(clo[axis], chi[axis]));
-    const unsigned long long nb = A.tiles[t].nbase;
-    A.nchild[node] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
-    A.parent[nb + l] = node;
-    A.parent[nb + l + 1] = node;
-  }
-}
-
-// Exclusive prefix sum of flag[0..E] into bb, in blocks of SCAN_ITEMS: block sums, one block
-// scanning the block sums, then each block's own scan.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, uint32_t& total) {
-  const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= static_cast<unsigned>(o)) incl += y;
-  }
-  if (lane == 31) sh[w] = incl;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t s = lane < blockDim.x / 32 ? sh[lane] : 0u;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= static_cast<unsigned>(o)) s += y;
-    }
-    sh[lane] = s;
-  }
-  __syncthreads();
-  total = sh[blockDim.x / 32 - 1];
-  const uint32_t r = incl - v + (w ? sh[w - 1] : 0u);
-  __syncthreads();
-  return r;
-}
-
-// The flag of position x: its element's centroid >= the split of its node ("big"), 0 when the
-// node does not split (or x is done or past the end).
-__device__ __forceinline__ uint32_t rt_flag(const RtArgs& A, int c, unsigned long long x) {
-  if (x >= A.E) return 0u;
-  const uint32_t node = A.nof[c][x];
-  if (node & RT_DONE) return 0u;
-  const int axis = A.nsplit[node];
-  if (axis < 0) return 0u;
-  return A.key[c][axis * A.E + x] < ord64(A.nmid[node]) ? 0u : 1u;
-}
-
-// Flags and their block sums.
-__global__ void __launch_bounds__(RT_BLOCK) k_rt_scan_blocks(RtArgs A, int c, unsigned long long nb) {
-  if (A.cnt[c] == 0) return;
-  __shared__ uint32_t sh[32];
-  for (unsigned long long b = blockIdx.x; b < nb; b += gridDim.x) {
-    const unsigned long long x0 = b * SCAN_ITEMS + threadIdx.x * 8ull;
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (x0 + k <= A.E) {
-        const uint32_t f = rt_flag(A, c, x0 + k);
-        A.flag[x0 + k] = f;
-        s += f;
-      }
-    uint32_t tot;
-    block_excl_scan(s, sh, tot);
-    if (threadIdx.x == 0) A.blk[b] = tot;
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_rt_scan_top(RtArgs A, int c, unsigned long long nb) {
-  if (A.cnt[c] == 0) return;
-  __shared__ uint32_t sh[32];
-  uint32_t carry = 0;
-  for (unsigned long long base = 0; base < nb; base += 1024) {
-    const unsigned long long i = base + threadIdx.x;
-    const uint32_t v = i < nb ? A.blk[i] : 0u;
-    uint32_t tot;
-    const uint32_t e = block_excl_scan(v, sh, tot);
-    if (i < nb) A.blk[i] = carry + e;
-    carry += tot;
-  }
-}
-
-__global__ void __launch_bounds__(RT_BLOCK) k_rt_scan_final(RtArgs A, int c, unsigned long long nb) {
-  if (A.cnt[c] == 0) return;
-  __shared__ uint32_t sh[32];
-  for (unsigned long long b = blockIdx.x; b < nb; b += gridDim.x) {
-    const unsigned long long x0 = b * SCAN_ITEMS + threadIdx.x * 8ull;
-    uint32_t f[8], s = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      f[k] = x0 + k <= A.E ? A.flag[x0 + k] : 0u;
-      s += f[k];
-    }
-    uint32_t tot;
-    uint32_t acc = A.blk[b] + block_excl_scan(s, sh, tot);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (x0 + k <= A.E) {
-        A.bb[x0 + k] = acc;
-        acc += f[k];
-      }
-  }
-}
-
-// Ranks: P_m (m-th big from the left) and Q_m (m-th small from the right), relative positions.
-__global__ void k_rt_pq(RtArgs A, int c) {
-  if (A.cnt[c] == 0) return;
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  for (unsigned long long x = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; x < A.E;
-       x += stride) {
-    const uint32_t node = A.nof[c][x];
-    if ((node & RT_DONE) || A.nsplit[node] < 0) continue;
-    const uint32_t s = A.nstart[node], n = A.ncount[node];
-    const uint32_t r = static_cast<uint32_t>(x - s);
-    const uint32_t bs = A.bb[s];
-    const uint32_t Bb = A.bb[x] - bs, Bt = A.bb[s + n] - bs, St = n - Bt;
-    if (A.flag[x]) {
-      A.P[s + Bb] = r;  // m = Bb + 1
-    } else {
-      const uint32_t mr = St - (r - Bb);  // right rank, 1-based
-      A.Q[s + mr - 1] = r;
-    }
-  }
-}
-
-// Moves every element of a splitting node to its place after the reference's swap partition;
-// finishes the elements of new leaves; sets up the children.
-__global__ void k_rt_place(RtArgs A, int c) {
-  if (A.cnt[c] == 0) return;
-  const int o = c ^ 1;
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  for (unsigned long long x = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; x < A.E;
-       x += stride) {
-    const uint32_t node = A.nof[c][x];
-    if (node & RT_DONE) {
-      A.nof[o][x] = RT_DONE;
-      continue;
-    }
-    const uint32_t el = A.idx[c][x];
-    if (A.nsplit[node] < 0) {  // a leaf of this level: its order is final
-      A.ridx[x] = el;
-      A.nof[o][x] = RT_DONE;
-      continue;
-    }
-    const uint32_t s = A.nstart[node], n = A.ncount[node];
-    const uint32_t r = static_cast<uint32_t>(x - s);
-    const uint32_t bs = A.bb[s];
-    const uint32_t Bb = A.bb[x] - bs, Bt = A.bb[s + n] - bs, St = n - Bt;
-    const uint32_t li = St + (St < n ? A.flag[s + St] : 0u);
-    const bool big = A.flag[x] != 0;
-    uint32_t dest;
-    if (r < li) {
-      dest = big ? ((Bb == 0 ? n : A.Q[s + Bb - 1]) - 1) : r;
-    } else {
-      dest = big ? r - 1 : A.P[s + (St - (r - Bb)) - 1];
-    }
-    // The reference splits at count / 2 when every centroid fell on one side (bvh.rs:260-265).
-    const uint32_t Sp = (St == 0 || St == n) ? n / 2 : St;
-    const int2 ch = A.nchild[node];
-    const bool left = dest < Sp;
-    const uint32_t child = static_cast<uint32_t>(left ? ch.x : ch.y);
-    const uint32_t csize = left ? Sp : n - Sp;
-    A.idx[o][s + dest] = el;
-#pragma unroll
-    for (int f = 0; f < 3; ++f) A.key[o][f * A.E + s + dest] = A.key[c][f * A.E + x];
-    A.nof[o][s + dest] = csize > static_cast<uint32_t>(RT_CTA_MAX) ? child : RT_DONE;
-    if (r == 0) {
-      const uint32_t t = A.ntile[node], dep = A.ndepth[node] + 1;
-      const uint32_t cs[2] = {Sp, n - Sp};
-      const uint32_t cid[2] = {static_cast<uint32_t>(ch.x), static_cast<uint32_t>(ch.y)};
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const uint32_t id = cid[k];
-        A.nstart[id] = s + (k ? Sp : 0u);
-        A.ncount[id] = cs[k];
-        A.ntile[id] = t;
-        A.ndepth[id] = dep;
-        rt_enqueue(A, id, cs[k], o);
-      }
-      atomicMax(&A.tiles[t].depth, dep);
-    }
-  }
-}
-
-__global__ void k_rt_level_end(RtArgs A, int c) {
-  // The worklist of this level has been consumed; the next level's count was filled by place.
-  A.cnt[c] = 0;
-}
-
-__global__ void k_rt_check(RtArgs A, int c) {
-  if (A.cnt[c] != 0) atomicOr(A.err, ERR_LIST_OVERFLOW);  // nodes left after the last level
 }
 
 // The block queue: one block builds the whole subtree of a node of at most RT_CTA_MAX elements
@@ -486,22 +671,22 @@ constexpr int RT_LEAF_MAX = 4;                               // subdivide's leaf
 constexpr int RT_CTA_LV = RT_CTA_MAX / (RT_LEAF_MAX + 1);    // nodes of more than 4 per level (204)
 constexpr int RT_CTA_SL = 2 * RT_CTA_LV;                     // leaves of at most 4 made by one level
 constexpr uint8_t RT_CTA_FREE = 0xff;                        // position of a finished range
-constexpr int RT_CTA_LVMAX = RT_MAX_DEPTH + 1;               // levels of a job (deeper trees are rejected)
 static_assert(RT_CTA_LV < RT_CTA_FREE, "level slots must fit a byte");
 static_assert(RT_CTA_MAX <= 2048, "positions are packed in 11 bits");
 
+template <class K>
 struct RtCtaSmem {
-  unsigned long long key[3][RT_CTA_MAX];  // the job's centroid keys, at their load position (home)
+  typename K::T key[3][RT_CTA_MAX];  // the job's centroid keys, at their load position (home)
   // Per level: the nodes' centroid accumulators (reduce to decide), then the flags' prefix sum and
   // the ranks (flags to place); the two uses do not overlap.
   union {
-    unsigned long long acc[RT_CTA_LV][6];   // per level node: ordered minima, maxima
+    typename K::T acc[RT_CTA_LV][6];        // per level node: minima, maxima
     struct {
       uint16_t bb[RT_CTA_MAX + 1];          // exclusive prefix sum of the flags
       uint16_t P[RT_CTA_MAX], Q[RT_CTA_MAX];
     } r;
   } u;
-  double mid[RT_CTA_LV];
+  typename K::T thr[RT_CTA_LV];           // split threshold
   uint32_t idx[RT_CTA_MAX];               // element slot
   uint16_t home[RT_CTA_MAX];              // element's load position (its keys)
   uint32_t id[2][RT_CTA_LV];              // this level's nodes and the next's
@@ -518,53 +703,20 @@ struct RtCtaSmem {
   int8_t axis[RT_CTA_LV];
   int nl, nsl, nnext, nslnew;
   uint32_t maxdep;
-  int nint, nlvl;                         // internal nodes of the job so far, and levels
-  uint16_t lvend[RT_CTA_LVMAX];           // internal nodes listed after each level
 };
 
-// Folds the max_dim box of element slot `slot` into k (minima 0-2, maxima 3-5, ordered keys).
-__device__ __forceinline__ void rt_fold_box(const RTile& T, uint32_t slot, unsigned long long k[6]) {
-  double lo[3], hi[3], cc[3];
-  rt_box_pm(rt_pm(T, slot), lo, hi, cc);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    k[m] = umin64(k[m], ord64(lo[m]));
-    k[3 + m] = umax64(k[3 + m], ord64(hi[m]));
-  }
-}
-
-__device__ __forceinline__ void rt_store_box(const RtArgs& A, uint32_t id, const unsigned long long k[6]) {
-#pragma unroll
-  for (int m = 0; m < 6; ++m) A.box64[6ull * id + m] = unord64(k[m]);
-}
-
-// Four blocks per SM (64 registers; the block's shared memory is about 53 KB): 9 % faster than two.
-__global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
+// Four blocks per SM (64 registers; the block's shared memory is about 53 KB with 64-bit keys): 9 %
+// faster than two.
+template <class K>
+__global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
+  using T = typename K::T;
   extern __shared__ __align__(32) unsigned char rt_cta_raw[];
-  RtCtaSmem& S = *reinterpret_cast<RtCtaSmem*>(rt_cta_raw);
+  RtCtaSmem<K>& S = *reinterpret_cast<RtCtaSmem<K>*>(rt_cta_raw);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const uint32_t nq = A.cnt[2];
   for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
     const uint32_t root = A.bq[q], par = A.bqpar[q];
     const uint32_t s = A.nstart[root];
-    if (par == RT_BOX_ONLY) {  // a leaf of the global levels: its box, from all its elements
-      const RTile& T = A.tiles[A.ntile[root]];
-      const uint32_t cn = A.ncount[root];
-      if (tid < 6) S.u.acc[0][tid] = tid < 3 ? ~0ull : 0ull;
-      __syncthreads();
-      unsigned long long k[6];
-      rt_keys_empty(k);
-      for (uint32_t j = tid; j < cn; j += RT_CTA_T) rt_fold_box(T, A.ridx[s + j], k);
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        atomicMin(&S.u.acc[0][m], k[m]);
-        atomicMax(&S.u.acc[0][3 + m], k[3 + m]);
-      }
-      __syncthreads();
-      if (tid == 0) rt_store_box(A, root, S.u.acc[0]);
-      __syncthreads();
-      continue;
-    }
     const int n = static_cast<int>(min(A.ncount[root], static_cast<uint32_t>(RT_CTA_MAX)));
     const uint32_t t = A.ntile[root];
     const unsigned long long nb = A.tiles[t].nbase;
@@ -572,7 +724,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
     for (int x = tid; x < RT_CTA_MAX; x += RT_CTA_T) {
       if (x < n) {
 #pragma unroll
-        for (int f = 0; f < 3; ++f) S.key[f][x] = A.key[par][f * A.E + s + x];
+        for (int f = 0; f < 3; ++f) S.key[f][x] = static_cast<const T*>(A.key[par])[f * A.E + s + x];
         S.home[x] = static_cast<uint16_t>(x);
         S.idx[x] = A.idx[par][s + x];
         S.nd[x] = n > RT_LEAF_MAX ? 0 : RT_CTA_FREE;
@@ -582,8 +734,6 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
     }
     if (tid == 0) {
       S.maxdep = 0;
-      S.nint = 0;
-      S.nlvl = 0;
       if (n > RT_LEAF_MAX) {
         S.nl = 1;
         S.nsl = 0;
@@ -607,10 +757,6 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
         const uint32_t e = S.sl[i], id = S.slid[i];
         const int o0 = static_cast<int>(e & 2047u), cn = static_cast<int>((e >> 11) & 7u);
         const uint32_t dp = e >> 14;
-        unsigned long long k[6];
-        rt_keys_empty(k);
-        for (int j = 0; j < cn; ++j) rt_fold_box(A.tiles[t], S.idx[o0 + j], k);
-        rt_store_box(A, id, k);
         A.nstart[id] = s + static_cast<uint32_t>(o0);
         A.ncount[id] = static_cast<uint32_t>(cn);
         A.ntile[id] = t;
@@ -618,7 +764,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
         A.nsplit[id] = -1;
         atomicMax(&S.maxdep, dp);
       }
-      for (int i = tid; i < nl * 6; i += RT_CTA_T) S.u.acc[i / 6][i % 6] = (i % 6) < 3 ? ~0ull : 0ull;
+      for (int i = tid; i < nl * 6; i += RT_CTA_T) S.u.acc[i / 6][i % 6] = (i % 6) < 3 ? ~static_cast<T>(0) : static_cast<T>(0);
       __syncthreads();
       if (nl == 0) break;
       if (tid == 0) {
@@ -632,9 +778,14 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
         const uint32_t node = S.nd[x];
         const bool act = node != RT_CTA_FREE;
         if (!__any_sync(0xffffffffu, act)) continue;
-        unsigned long long kk[6];
-        if (act) rt_keys(&S.key[0][0], RT_CTA_MAX, S.home[x], kk); else rt_keys_empty(kk);
-        const bool head = rt_seg_reduce(act ? node : (0x100u | static_cast<uint32_t>(lane)), kk);
+        T kk[6];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const T v = S.key[i][act ? S.home[x] : 0];
+          kk[i] = act ? v : ~static_cast<T>(0);
+          kk[3 + i] = act ? v : static_cast<T>(0);
+        }
+        const bool head = rt_seg_reduce<K>(act ? node : (0x100u | static_cast<uint32_t>(lane)), kk);
         if (act && head) {
 #pragma unroll
           for (int i = 0; i < 3; ++i) atomicMin(&S.u.acc[node][i], kk[i]);
@@ -650,8 +801,8 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
         double clo[3], chi[3];
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-          clo[m] = unord64(S.u.acc[i][m]);
-          chi[m] = unord64(S.u.acc[i][3 + m]);
+          clo[m] = K::value(S.u.acc[i][m]);
+          chi[m] = K::value(S.u.acc[i][3 + m]);
         }
         A.nstart[id] = s + S.off[cur][i];
         A.ncount[id] = static_cast<uint32_t>(cn);
@@ -665,31 +816,20 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
         if (cn <= RT_LEAF_MAX || ext <= 1e-7 || !alloc_pair(A, static_cast<int>(t), l)) {
           S.axis[i] = -1;  // leaf (degenerate centroids, or no node capacity left)
           A.nsplit[id] = -1;
-          unsigned long long k[6];
-          rt_keys_empty(k);
-          for (int j = 0; j < cn; ++j) rt_fold_box(A.tiles[t], S.idx[S.off[cur][i] + j], k);
-          rt_store_box(A, id, k);
         } else {
-          if (walks) A.P[s + static_cast<uint32_t>(atomicAdd(&S.nint, 1))] = id;  // its box after the last level
           const double ca = axis == 0 ? clo[0] : (axis == 1 ? clo[1] : clo[2]);
           const double cb = axis == 0 ? chi[0] : (axis == 1 ? chi[1] : chi[2]);
           const double mid = __dmul_rn(0.5, __dadd_rn(ca, cb));
           S.axis[i] = static_cast<int8_t>(axis);
-          S.mid[i] = mid;
+          S.thr[i] = K::threshold(mid);
           S.child[i] = static_cast<uint32_t>(nb + l);
           A.nsplit[id] = axis;
-          if (walks) {
-            A.nchild[id] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
-            A.parent[nb + l] = id;
-            A.parent[nb + l + 1] = id;
-          }
+          A.nchild[id] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
+          A.parent[nb + l] = id;
+          A.parent[nb + l + 1] = id;
         }
       }
       __syncthreads();
-      if (tid == 0) {
-        if (S.nlvl < RT_CTA_LVMAX) S.lvend[S.nlvl++] = static_cast<uint16_t>(S.nint);
-        else atomicOr(A.err, ERR_STACK_OVERFLOW);  // deeper than the depth check allows
-      }
       // Flags and their exclusive prefix sum: thread tid owns positions RT_CTA_PER * tid + k.
       {
         uint32_t f[RT_CTA_PER], sum = 0;
@@ -699,7 +839,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
           const uint32_t node = S.nd[x];
           f[k] = 0;
           if (node != RT_CTA_FREE && S.axis[node] >= 0)
-            f[k] = S.key[S.axis[node]][S.home[x]] < ord64(S.mid[node]) ? 0u : 1u;
+            f[k] = S.key[S.axis[node]][S.home[x]] < S.thr[node] ? 0u : 1u;
           sum += f[k];
         }
         uint32_t incl = sum;
@@ -812,45 +952,96 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A, bool walks) {
       cur ^= 1;
       __syncthreads();
     }
-    // The internal nodes' boxes, deepest level first: each the union of its children's, written
-    // by this block before the barrier (leaves at their creation, internal nodes a level below).
-    for (int L = walks ? S.nlvl - 1 : -1; L >= 0; --L) {
-      const int b0 = L ? S.lvend[L - 1] : 0, b1 = S.lvend[L];
-      for (int k = b0 + tid; k < b1; k += RT_CTA_T) {
-        const uint32_t id = A.P[s + static_cast<uint32_t>(k)];
-        const int2 ch = A.nchild[id];
-        const double* a = A.box64 + 6ull * static_cast<unsigned long long>(ch.x);
-        const double* b = A.box64 + 6ull * static_cast<unsigned long long>(ch.y);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          A.box64[6ull * id + m] = unord64(umin64(ord64(a[m]), ord64(b[m])));
-          A.box64[6ull * id + 3 + m] = unord64(umax64(ord64(a[3 + m]), ord64(b[3 + m])));
-        }
-      }
-      __syncthreads();
-    }
     for (int x = tid; x < n; x += RT_CTA_T) A.ridx[s + x] = S.idx[x];
     if (tid == 0) atomicMax(&A.tiles[t].depth, S.maxdep);
     __syncthreads();
   }
 }
 
-// Node boxes above the blocks' subtrees (the BVHNode aabb: the union of the node's elements'
-// max_dim boxes, bvh.rs:196-204).  Every block-queue entry (a subtree's root, or a leaf of the
-// global levels) has its box; one thread per entry climbs: at each parent the first child to
+// Leaves, by tile (blockIdx.y): the leaf box (the union of its elements' max_dim boxes, bvh.rs:196-204),
+// the leaf-of map and the elements' ranks (the walk takes the right subtree first, so leaves in
+// descending element position, and a leaf's elements in index order); rleaf (may be null) gets the
+// element range.  Boxes fold as order-preserving integers, or, for FP32 crystals without expansion
+// (FP32), as the exact float pairs p -+ m, rounded to FP64 once per leaf: GB300's FP64 pipe is narrow.
+template <bool FP32>
+__global__ void k_rt_leaves(RtArgs A, uint2* rleaf, uint32_t* leafof, unsigned long long leafof_n, uint32_t* rank) {
+  const RTile& T = A.tiles[blockIdx.y];
+  if (blockIdx.x == 0 && threadIdx.x == 0 && T.depth > static_cast<uint32_t>(RT_MAX_DEPTH))
+    atomicOr(A.err, ERR_STACK_OVERFLOW);
+  if (T.n == 0) return;
+  const uint32_t nodes = min(T.nodes, T.ncap);
+  // (After a failed node allocation, ids below the capacity may never have been set up; the build
+  // has flagged the error, and the checks below keep this pass inside its buffers.)
+  for (uint32_t id = 1 + blockIdx.x * blockDim.x + threadIdx.x; id < nodes; id += gridDim.x * blockDim.x) {
+    const unsigned long long g = T.nbase + id;
+    if (A.nsplit[g] >= 0) continue;
+    const uint32_t st = A.nstart[g], cn = A.ncount[g];
+    if (st < T.ebase || st - T.ebase + static_cast<unsigned long long>(cn) > T.n) {
+      atomicOr(A.err, ERR_BAD_INDEX);
+      continue;
+    }
+    const uint32_t r0 = static_cast<uint32_t>(st - T.ebase);
+    if (rleaf) rleaf[g] = make_uint2(r0, cn);
+    unsigned long long k[6];
+    float h[6], l[6];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      k[m] = ~0ull;
+      k[3 + m] = 0ull;
+      h[m] = INFINITY;
+      h[3 + m] = -INFINITY;
+      l[m] = l[3 + m] = 0.0f;
+    }
+    for (uint32_t j = 0; j < cn; ++j) {
+      const uint32_t slot = A.ridx[st + j];
+      if (T.ebase + slot >= leafof_n) {
+        atomicOr(A.err, ERR_BAD_INDEX);
+        continue;
+      }
+      leafof[T.ebase + slot] = id;
+      if (rank) rank[T.ebase + slot] = T.n - r0 - cn + j;
+      if (FP32) {
+        const float4 a = T.a[slot], d = T.d[slot];
+        const float p[3] = {a.x, a.y, a.z}, dm = fmaxf(fmaxf(d.x, d.y), d.z);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          // p -+ dm as an exact pair (Knuth's two-sum).
+          const float q = p[m % 3], w = m < 3 ? -dm : dm;
+          const float s = q + w, z = s - q, e = (q - (s - z)) + (w - z);
+          const bool take = m < 3 ? (s < h[m] || (s == h[m] && e < l[m])) : (s > h[m] || (s == h[m] && e > l[m]));
+          if (take) {
+            h[m] = s;
+            l[m] = e;
+          }
+        }
+        continue;
+      }
+      const double4_32a v = rt_pm(T, slot);
+      const double p[3] = {v.x, v.y, v.z};
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        k[m] = umin64(k[m], ord64(__dsub_rn(p[m], v.w)));
+        k[3 + m] = umax64(k[3 + m], ord64(__dadd_rn(p[m], v.w)));
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+      A.box64[6ull * g + m] = FP32 ? __dadd_rn(static_cast<double>(h[m]), static_cast<double>(l[m])) : unord64(k[m]);
+  }
+}
+
+// Node boxes above the leaves (the BVHNode aabb: the union of the node's elements' max_dim boxes,
+// bvh.rs:196-204), for the walks.  One thread per leaf climbs: at each parent the first child to
 // arrive stops and the second forms the parent's box as the union of both children's.  Boxes are
 // published with a fence before the arrival count and read through L2.  `arrive` holds one zeroed
 // counter per node.
 __global__ void k_rt_refit(RtArgs A, uint32_t* arrive) {
-  const uint32_t nq = A.cnt[2];
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-    unsigned long long node = A.bq[q];
-    if (node >= A.N) {
-      atomicOr(A.err, ERR_BAD_INDEX);
-      continue;
-    }
-    const RTile& T = A.tiles[A.ntile[node]];
-    const unsigned long long nlo = T.nbase, nhi = T.nbase + T.ncap;
+  const RTile& T = A.tiles[blockIdx.y];
+  const unsigned long long nlo = T.nbase, nhi = T.nbase + T.ncap;
+  const uint32_t nodes = T.n ? min(T.nodes, T.ncap) : 0;
+  for (uint32_t id = 1 + blockIdx.x * blockDim.x + threadIdx.x; id < nodes; id += gridDim.x * blockDim.x) {
+    unsigned long long node = T.nbase + id;
+    if (A.nsplit[node] >= 0) continue;
     for (int up = 0; up <= RT_MAX_DEPTH; ++up) {
       const uint32_t p = A.parent[node];
       if (p == RT_NONE) break;
@@ -880,16 +1071,12 @@ __global__ void k_rt_refit(RtArgs A, uint32_t* arrive) {
   }
 }
 
-// One thread per node.  A leaf fills the leaf-of map and its elements' ranks (the walk takes the
-// right subtree first, so leaves in descending element position, and a leaf's elements in index
-// order).  With WALKS it also fills its element range, and the root and every internal node at odd
-// depth write their four-wide record (fg_rtree.cuh), the
+// Walk records, one thread per node: the root and every internal node at odd depth write their
+// four-wide record (fg_rtree.cuh), the
 // grandchildren in the reference's visiting order (right before left, a leaf child in one slot).
 // An internal slot's box is rounded outward, padded and extended by the reach; a leaf slot's box
 // is rounded to nearest.
-template <bool WALKS>
-__global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafof, unsigned long long leafof_n,
-                             uint32_t* rank) {
+__global__ void k_rt_records(RtArgs A, Node4* rec) {
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   for (unsigned long long g = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; g < A.N;
        g += stride) {
@@ -923,30 +1110,12 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
       *out = nd;
     };
     if (id == 0) {  // the super-root slot: an empty tree's record 0
-      if (WALKS && T.n == 0 && T.rcap > 0) put(0, R);
+      if (T.n == 0 && T.rcap > 0) put(0, R);
       continue;
     }
     if (id == 1 && T.n == 0) continue;
     const bool leaf = A.nsplit[g] < 0;
-    if (leaf) {
-      const uint32_t st = A.nstart[g], cn = A.ncount[g];
-      if (st < T.ebase || st - T.ebase + static_cast<unsigned long long>(cn) > T.n) {
-        atomicOr(A.err, ERR_BAD_INDEX);
-        continue;
-      }
-      if (WALKS) rleaf[g] = make_uint2(static_cast<uint32_t>(st - T.ebase), cn);
-      if (leafof)
-        for (uint32_t k = 0; k < cn; ++k) {
-          const uint32_t slot = A.ridx[st + k];
-          if (T.ebase + slot < leafof_n) {
-            leafof[T.ebase + slot] = id;
-            if (rank) rank[T.ebase + slot] = T.n - static_cast<uint32_t>(st - T.ebase) - cn + k;
-          } else {
-            atomicOr(A.err, ERR_BAD_INDEX);
-          }
-        }
-    }
-    if (!WALKS || (id != 1 && (leaf || !(A.ndepth[g] & 1u)))) continue;
+    if (id != 1 && (leaf || !(A.ndepth[g] & 1u))) continue;
     // Slot k takes node c (a global id inside the tile): its box and reference.
     int k = 0;
     bool bad = false;
@@ -1011,11 +1180,6 @@ __global__ void k_rt_records(RtArgs A, Node4* rec, uint2* rleaf, uint32_t* leafo
   }
 }
 
-__global__ void k_rt_depth_check(RtArgs A) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < A.ntiles && A.tiles[t].depth > static_cast<uint32_t>(RT_MAX_DEPTH)) atomicOr(A.err, ERR_STACK_OVERFLOW);
-}
-
 }  // namespace
 
 RtArgs rt_args(RTreeBufs& B, uint32_t* err) {
@@ -1030,8 +1194,8 @@ RtArgs rt_args(RTreeBufs& B, uint32_t* err) {
   A.key[1] = B.key1.p;
   A.nof[0] = B.nof0.p;
   A.nof[1] = B.nof1.p;
-  A.flag = B.flag.p;
-  A.bb = B.bb.p;
+  A.bits = B.bits.p;
+  A.wp = B.wp.p;
   A.blk = B.blk.p;
   A.P = B.P.p;
   A.Q = B.Q.p;
@@ -1044,7 +1208,7 @@ RtArgs rt_args(RTreeBufs& B, uint32_t* err) {
   A.ntile = B.ntile.p;
   A.ndepth = B.ndepth.p;
   A.nsplit = B.nsplit.p;
-  A.nmid = B.nmid.p;
+  A.nthr = B.nthr.p;
   A.nchild = B.nchild.p;
   A.wl[0] = B.wl0.p;
   A.wl[1] = B.wl1.p;
@@ -1060,6 +1224,7 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.ntiles = static_cast<int>(tiles.size());
   unsigned long long e = 0, nn = 0;
   uint32_t emax = 0;
+  unsigned long long nch = 0;  // chunks
   unsigned long long rr = 0;
   for (auto& t : tiles) {
     t.ebase = e;
@@ -1072,6 +1237,9 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
     rr += t.rcap;
     emax = std::max(emax, t.ecap);
   }
+  B.wpw = e < RT_LARGE ? RT_WPW_SMALL : RT_WPW_LARGE;
+  const unsigned chunk = rt_chunk(B.wpw);
+  for (auto& t : tiles) nch += (std::max(t.ecap, 1u) + chunk - 1) / chunk;
   FG_REQUIRE(e < 0x7fffffffull && nn < 0x7fffffffull, "too many elements for one reference-tree build");
   B.E = e;
   B.N = nn;
@@ -1079,6 +1247,8 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.levels = levels_for(emax);
   const size_t E1 = static_cast<size_t>(std::max<unsigned long long>(e, 1));
   const size_t N1 = static_cast<size_t>(std::max<unsigned long long>(nn, 1));
+  // Pending nodes have more than RT_CTA_MAX elements; the walks' refit counts every node's arrivals.
+  const size_t wl = walks ? N1 : static_cast<size_t>(e / RT_CTA_MAX + tiles.size() + 1);
   B.tiles.alloc(tiles.size(), st);
   FG_CUDA(cudaMemcpyAsync(B.tiles.p, tiles.data(), tiles.size() * sizeof(RTile), cudaMemcpyHostToDevice, st));
   B.idx0.alloc(E1, st);
@@ -1087,10 +1257,10 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.key1.alloc(3 * E1, st);
   B.nof0.alloc(E1, st);
   B.nof1.alloc(E1, st);
-  B.flag.alloc(E1 + 1, st);
-  B.bb.alloc(E1 + 1, st);
-  B.nblk = (E1 + 1 + SCAN_ITEMS - 1) / SCAN_ITEMS;
-  B.blk.alloc(B.nblk, st);
+  B.nblk = nch;
+  B.bits.alloc(nch * (chunk / 32), st);
+  B.wp.alloc(nch * (chunk / 32), st);
+  B.blk.alloc(nch, st);
   B.P.alloc(E1, st);
   B.Q.alloc(E1, st);
   B.ridx.alloc(E1, st);
@@ -1102,13 +1272,13 @@ void rtree_alloc(RTreeBufs& B, std::vector<RTile>& tiles, bool want_leafof, cuda
   B.ntile.alloc(N1, st);
   B.ndepth.alloc(N1, st);
   B.nsplit.alloc(N1, st);
-  B.nmid.alloc(N1, st);
+  B.nthr.alloc(N1, st);
   B.nchild.alloc(N1, st);
-  B.wl0.alloc(N1, st);
-  B.wl1.alloc(N1, st);
+  B.wl0.alloc(wl, st);
+  B.wl1.alloc(wl, st);
   B.bq.alloc(N1, st);
   B.bqpar.alloc(N1, st);
-  B.cnt.alloc(4, st);
+  B.cnt.alloc(RT_CNT_TILES + tiles.size() + 1, st);
   if (walks) {
     B.rnode.alloc(std::max<unsigned long long>(rr, 1), st);
     B.rleaf.alloc(N1, st);
@@ -1125,7 +1295,7 @@ size_t carve(RTreeBufs* B, uint32_t ecap, bool want_leafof, uint32_t leafof_slot
   const size_t E1 = std::max<uint32_t>(ecap, 1);
   const size_t N1 = rt_attach_nodes(E1);
   const size_t nblk = rt_attach_blocks(E1);
-  static_assert(SCAN_ITEMS == 2048, "rt_attach_blocks assumes 2048 entries per prefix-sum block");
+  static_assert(rt_chunk(RT_WPW_LARGE) == 2048, "rt_attach_blocks assumes chunks of 2048 positions");
   size_t off = 0;
   auto take = [&](auto& buf, size_t count) {
     using T = typename std::remove_reference<decltype(*buf.p)>::type;
@@ -1142,8 +1312,8 @@ size_t carve(RTreeBufs* B, uint32_t ecap, bool want_leafof, uint32_t leafof_slot
   take(b.key1, 3 * E1);
   take(b.nof0, E1);
   take(b.nof1, E1);
-  take(b.flag, E1 + 1);
-  take(b.bb, E1 + 1);
+  take(b.bits, E1 + 1);
+  take(b.wp, E1 + 1);
   take(b.blk, nblk);
   take(b.P, E1);
   take(b.Q, E1);
@@ -1156,13 +1326,13 @@ size_t carve(RTreeBufs* B, uint32_t ecap, bool want_leafof, uint32_t leafof_slot
   take(b.ntile, N1);
   take(b.ndepth, N1);
   take(b.nsplit, N1);
-  take(b.nmid, N1);
+  take(b.nthr, N1);
   take(b.nchild, N1);
   take(b.wl0, N1);
   take(b.wl1, N1);
   take(b.bq, N1);
   take(b.bqpar, N1);
-  take(b.cnt, 4);
+  take(b.cnt, RT_CNT_TILES + 2);
   take(b.rnode, N1 / 2 + 1);
   take(b.rleaf, N1);
   if (want_leafof) take(b.leafof, std::max<uint32_t>(leafof_slots, 1));
@@ -1172,6 +1342,7 @@ size_t carve(RTreeBufs* B, uint32_t ecap, bool want_leafof, uint32_t leafof_slot
     B->N = N1;
     B->R = N1 / 2 + 1;
     B->nblk = nblk;
+    B->wpw = RT_WPW_LARGE;
     B->levels = levels_for(ecap);
   }
   return (off + 255) / 256 * 256;
@@ -1188,6 +1359,7 @@ void rtree_attach(RTreeBufs& B, RTile tile, bool want_leafof, uint32_t leafof_sl
   const size_t need = carve(nullptr, tile.ecap, want_leafof, leafof_slots, nullptr);
   FG_REQUIRE(need == rtree_attach_bytes(tile.ecap, want_leafof, leafof_slots), "tree scratch layout mismatch");
   FG_REQUIRE(need <= bytes, "tree scratch too small");
+  FG_REQUIRE(tile.ecap >= rt_chunk(RT_WPW_LARGE), "tree scratch: the flag words need a chunk's worth of elements");
   carve(&B, tile.ecap, want_leafof, leafof_slots, base);
   tile.ebase = 0;
   tile.nbase = 0;
@@ -1197,42 +1369,58 @@ void rtree_attach(RTreeBufs& B, RTile tile, bool want_leafof, uint32_t leafof_sl
   FG_CUDA(cudaMemcpyAsync(B.tiles.p, &tile, sizeof(RTile), cudaMemcpyHostToDevice, st));
 }
 
-void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, RTile* tiles_dev) {
-  if (B.ntiles == 0) return;
-  RtArgs A = rt_args(B, err);
-  if (tiles_dev) A.tiles = tiles_dev;
-  const unsigned G = static_cast<unsigned>(std::min<unsigned long long>((B.E + RT_BLOCK) / RT_BLOCK, 152ull * 16));
-  const unsigned GN = static_cast<unsigned>(std::min<unsigned long long>((B.N + RT_BLOCK - 1) / RT_BLOCK, 152ull * 16));
-  const unsigned GS = static_cast<unsigned>(std::min<unsigned long long>(B.nblk, 152ull * 16));
-  FG_CUDA(cudaMemsetAsync(B.cnt.p, 0, 4 * sizeof(uint32_t), st));
-  k_rt_init<<<G, RT_BLOCK, 0, st>>>(A);
-  for (int L = 0; L < B.levels; ++L) {
-    const int c = L & 1;
-    k_rt_reduce<<<G, RT_BLOCK, 0, st>>>(A, c);
-    k_rt_decide<<<GN, RT_BLOCK, 0, st>>>(A, c);
-    k_rt_scan_blocks<<<GS, RT_BLOCK, 0, st>>>(A, c, B.nblk);
-    k_rt_scan_top<<<1, 1024, 0, st>>>(A, c, B.nblk);
-    k_rt_scan_final<<<GS, RT_BLOCK, 0, st>>>(A, c, B.nblk);
-    k_rt_pq<<<G, RT_BLOCK, 0, st>>>(A, c);
-    k_rt_place<<<G, RT_BLOCK, 0, st>>>(A, c);
-    k_rt_level_end<<<1, 1, 0, st>>>(A, c);
-  }
-  k_rt_check<<<1, 1, 0, st>>>(A, B.levels & 1);
+namespace {
+
+template <class K>
+void build_topology(const RTreeBufs& B, const RtArgs& A, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  FG_CUDA(cudaGetDevice(&dev));
+  FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // The launch bounds let four blocks share an SM, so the whole grid runs at once.
+  const unsigned GL = static_cast<unsigned>(std::max<unsigned long long>(std::min<unsigned long long>(B.nblk, 4ull * sms), 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(GL);
+  cfg.blockDim = dim3(RT_BLOCK);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  FG_CUDA(B.wpw == RT_WPW_SMALL ? cudaLaunchKernelEx(&cfg, k_rt_levels<K, RT_WPW_SMALL>, A, B.levels)
+                                : cudaLaunchKernelEx(&cfg, k_rt_levels<K, RT_WPW_LARGE>, A, B.levels));
   const unsigned GC = static_cast<unsigned>(
       std::min<unsigned long long>(B.E / (RT_LEAF_MAX + 1) + static_cast<unsigned long long>(B.ntiles), 152ull * 8));
-  static_assert(sizeof(RtCtaSmem) <= 56 * 1024, "four blocks of the block phase must fit an SM");
-  FG_CUDA(cudaFuncSetAttribute(k_rt_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(sizeof(RtCtaSmem))));
-  k_rt_cta<<<GC, RT_CTA_T, sizeof(RtCtaSmem), st>>>(A, walks);
+  static_assert(sizeof(RtCtaSmem<K>) <= 56 * 1024, "four blocks of the block phase must fit an SM");
+  FG_CUDA(cudaFuncSetAttribute(k_rt_cta<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(sizeof(RtCtaSmem<K>))));
+  k_rt_cta<K><<<GC, RT_CTA_T, sizeof(RtCtaSmem<K>), st>>>(A);
+  FG_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void rtree_build(RTreeBufs& B, uint32_t* err, cudaStream_t st, bool walks, bool key32, RTile* tiles_dev) {
+  if (B.ntiles == 0) return;
+  FG_REQUIRE(B.ntiles <= 65535, "too many trees for one build");
+  RtArgs A = rt_args(B, err);
+  if (tiles_dev) A.tiles = tiles_dev;
+  FG_CUDA(cudaMemsetAsync(B.cnt.p, 0, RT_CNT_TILES * sizeof(uint32_t), st));
+  FG_CUDA(cudaMemsetAsync(B.blk.p, 0, static_cast<size_t>(B.nblk) * sizeof(unsigned long long), st));
+  if (key32) build_topology<Key32>(B, A, st); else build_topology<Key64>(B, A, st);
+  // Per-tile grids over the nodes (about 0.67 per element).
+  const unsigned long long per = (B.N / static_cast<unsigned long long>(B.ntiles) + RT_BLOCK) / RT_BLOCK;
+  const unsigned GX = static_cast<unsigned>(std::max<unsigned long long>(std::min<unsigned long long>(per, 152ull * 16), 1));
+  const dim3 GN(GX, static_cast<unsigned>(B.ntiles));
+  if (key32) k_rt_leaves<true><<<GN, RT_BLOCK, 0, st>>>(A, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
+  else k_rt_leaves<false><<<GN, RT_BLOCK, 0, st>>>(A, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
   if (walks) {
-    // The global worklist is spent: its words count the children that reached each node.
+    // The worklist is spent: its words count the children that reached each node.
     FG_CUDA(cudaMemsetAsync(B.wl0.p, 0, static_cast<size_t>(B.N) * sizeof(uint32_t), st));
     k_rt_refit<<<GN, RT_BLOCK, 0, st>>>(A, B.wl0.p);
-    k_rt_records<true><<<GN, RT_BLOCK, 0, st>>>(A, B.rnode.p, B.rleaf.p, B.leafof.p, B.leafof.n, B.rank.p);
-  } else {
-    k_rt_records<false><<<GN, RT_BLOCK, 0, st>>>(A, nullptr, nullptr, B.leafof.p, B.leafof.n, B.rank.p);
+    k_rt_records<<<static_cast<unsigned>(std::min<unsigned long long>((B.N + RT_BLOCK - 1) / RT_BLOCK, 152ull * 16)),
+                   RT_BLOCK, 0, st>>>(A, B.rnode.p);
   }
-  k_rt_depth_check<<<grid_for(static_cast<size_t>(B.ntiles), 128), 128, 0, st>>>(A);
   FG_CUDA(cudaGetLastError());
 }
 
@@ -1283,12 +1471,13 @@ void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_onl
   t.n = developed_only ? m : n;
   std::vector<RTile> v{t};
   rtree_alloc(B, v, true, st, 1.0, n, !developed_only, walks);
-  rtree_build(B, e->d_err, st, walks);
+  // FP32 crystals without expansion: the centroids are the positions themselves.
+  rtree_build(B, e->d_err, st, walks, !em->has64 && !developed_only && std::isfinite(em->max_half_dim));
   B.count = t.n;
 }
 
 unsigned rtree_kernel_launches(const RTreeBufs& B, bool walks) {
-  return B.ntiles ? 1u + 8u * static_cast<unsigned>(B.levels) + (walks ? 5u : 4u) : 0u;
+  return B.ntiles ? (walks ? 5u : 3u) : 0u;
 }
 
 }  // namespace fg

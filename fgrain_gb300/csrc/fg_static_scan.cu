@@ -265,7 +265,7 @@ void static_scan(const fg_device_crystals* c, const fg_emulsion_cfg* film, const
     rt.n = ndev;
     rt.pad = static_cast<float>(std::max(film->width, film->height) * 2e-6 + 1e-5);
     rtree_attach(tree, rt, true, FG_STATIC_SCAN_MAX_CRYSTALS, base + kTreeOff, kTreeBytes, st);
-    rtree_build(tree, err, st, false);
+    rtree_build(tree, err, st, false, false);
   }
   t.lbox64 = tree.box64.p;
   t.leafof = tree.leafof.p;
