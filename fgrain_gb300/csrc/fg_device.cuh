@@ -14,15 +14,17 @@ struct P4 {
   uint32_t x, y, z, w;
 };
 
+constexpr uint32_t PHILOX_M0 = 0xD2511F53u, PHILOX_M1 = 0xCD9E8D57u;  // round multipliers
+constexpr uint32_t PHILOX_W0 = 0x9E3779B9u, PHILOX_W1 = 0xBB67AE85u;  // key increments
 __host__ __device__ __forceinline__ P4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
                                               uint32_t k0, uint32_t k1) {
 #pragma unroll
   for (int r = 0; r < 10; ++r) {
 #ifdef __CUDA_ARCH__
-    const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+    const uint32_t hi0 = __umulhi(PHILOX_M0, c0), lo0 = PHILOX_M0 * c0;
+    const uint32_t hi1 = __umulhi(PHILOX_M1, c2), lo1 = PHILOX_M1 * c2;
 #else
-    const uint64_t m0 = (uint64_t)0xD2511F53u * c0, m1 = (uint64_t)0xCD9E8D57u * c2;
+    const uint64_t m0 = (uint64_t)PHILOX_M0 * c0, m1 = (uint64_t)PHILOX_M1 * c2;
     const uint32_t hi0 = (uint32_t)(m0 >> 32), lo0 = (uint32_t)m0;
     const uint32_t hi1 = (uint32_t)(m1 >> 32), lo1 = (uint32_t)m1;
 #endif
@@ -31,8 +33,8 @@ __host__ __device__ __forceinline__ P4 philox(uint32_t c0, uint32_t c1, uint32_t
     c1 = lo1;
     c2 = n2;
     c3 = lo0;
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
+    k0 += PHILOX_W0;
+    k1 += PHILOX_W1;
   }
   return P4{c0, c1, c2, c3};
 }

@@ -13,12 +13,14 @@ enum : uint32_t {
   TAG_THIN = 0x54480000u,
 };
 
-// True when the cell word w holds a point closer than r to the candidate, (ox, oy, oz) being the
-// cell's corner relative to the candidate (fixed point).
+// True when the point of an occupied cell (word w) is closer than r to the candidate, (ox, oy, oz)
+// being the cell's corner relative to the candidate (fixed point), oz less SYN_OCC_Z: the word's
+// occupancy bit comes down with its z.
+constexpr int SYN_OCC_Z = static_cast<int>(OCC >> 20);
 __device__ __forceinline__ bool syn_conflict(uint32_t w, int ox, int oy, int oz) {
   const int ex = ox + static_cast<int>(w & 1023u);
   const int ey = oy + static_cast<int>((w >> 10) & 1023u);
-  const int ez = oz + static_cast<int>((w >> 20) & 1023u);
+  const int ez = oz + static_cast<int>(w >> 20);
   return ex * ex + ey * ey + ez * ez < SYN_R2X;
 }
 
@@ -33,24 +35,19 @@ __device__ __forceinline__ void syn_mark(uint32_t* rows, int row, int rx) {
 // The 27 cells of the inner block in the order of syn_near_free's mask bits: the rows above and
 // below in y of the three layers (6 bits a layer), then the rows of the candidate's own y, its own
 // row last.  The last bits are visited first: they are the likeliest to hold a conflict.
-struct SynNear {
-  int off[27], ox[27], oy[27], oz[27];  // region index offset; cell corner offset (fixed point)
-};
-__device__ __forceinline__ void syn_near_entry(SynNear& t, int k) {
+// An entry: the cell's corner offset (fixed point, z less SYN_OCC_Z) and its region index offset.
+__device__ __forceinline__ int4 syn_near_entry(int k) {
   const int dx = k % 3 - 1;
   const int dy = k < 18 ? ((k / 3) % 2 ? 1 : -1) : 0;
   const int dz = k < 18 ? k / 6 - 1 : (k < 21 ? -1 : (k < 24 ? 1 : 0));
-  t.off[k] = (dz * SYN_R + dy) * SYN_R + dx;
-  t.ox[k] = dx * SYN_Q;
-  t.oy[k] = dy * SYN_Q;
-  t.oz[k] = dz * SYN_Q;
+  return make_int4(dx * SYN_Q, dy * SYN_Q, dz * SYN_Q - SYN_OCC_Z, (dz * SYN_R + dy) * SYN_R + dx);
 }
 
 // First half of the candidate test, one lane per candidate: the points in the 27 cells of the inner
 // 3x3x3 block.  They reject about 87 % of Bridson candidates, so the lanes that survive are few and
 // the rest of the test runs warp-cooperatively (syn_outer_free).  A point in the candidate's own
 // cell always conflicts (two points of a cell are less than r apart).
-__device__ __forceinline__ bool syn_near_free(const uint32_t* grid, const uint32_t* rows, const SynNear& t, int rx,
+__device__ __forceinline__ bool syn_near_free(const uint32_t* grid, const uint32_t* rows, const int4* cells27, int rx,
                                               int row, int rb, int lx, int ly, int lz) {
   const uint32_t* w = rows + row;
   const int sh = rx - 1;
@@ -63,7 +60,8 @@ __device__ __forceinline__ bool syn_near_free(const uint32_t* grid, const uint32
   while (m) {
     const int k = 31 - __clz(static_cast<int>(m));
     m ^= 1u << k;
-    if (syn_conflict(grid[rb + t.off[k]], t.ox[k] - lx, t.oy[k] - ly, t.oz[k] - lz)) return false;
+    const int4 c = cells27[k];
+    if (syn_conflict(grid[rb + c.w], c.x - lx, c.y - ly, c.z - lz)) return false;
   }
   return true;
 }
@@ -87,7 +85,7 @@ __device__ __forceinline__ bool syn_outer_hit(const uint32_t* grid, const uint32
     while (m) {
       const int k = 31 - __clz(static_cast<int>(m));
       m ^= 1u << k;
-      if (syn_conflict(g[k], (k - 2) * SYN_Q - cx, dy * SYN_Q - cy, dz * SYN_Q - cz)) {
+      if (syn_conflict(g[k], (k - 2) * SYN_Q - cx, dy * SYN_Q - cy, dz * SYN_Q - SYN_OCC_Z - cz)) {
         hit = true;
         break;
       }
@@ -158,11 +156,38 @@ __device__ __forceinline__ uint32_t syn_word(int X, int Y, int Z) {
          static_cast<uint32_t>(X & 1023);
 }
 
-// What bounds it: issue slots (76 % issue activity at 24 of 32 lanes; DRAM 1 %): about 660 warp
+// philox with its ten round keys from a table (the same in every step of a column): eighteen
+// additions a draw less.
+__device__ __forceinline__ P4 philox_keys(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const uint4* keys) {
+#pragma unroll
+  for (int r = 0; r < 5; ++r) {
+    const uint4 k = keys[r];  // the keys of two rounds
+    const uint32_t a0 = __umulhi(PHILOX_M1, c2) ^ c1 ^ k.x, a2 = __umulhi(PHILOX_M0, c0) ^ c3 ^ k.y;
+    const uint32_t a1 = PHILOX_M1 * c2, a3 = PHILOX_M0 * c0;
+    c0 = __umulhi(PHILOX_M1, a2) ^ a1 ^ k.z;
+    c1 = PHILOX_M1 * a2;
+    c2 = __umulhi(PHILOX_M0, a0) ^ a3 ^ k.w;
+    c3 = PHILOX_M0 * a0;
+  }
+  return P4{c0, c1, c2, c3};
+}
+
+// An entry of the active list: the cell's region coordinates (SYN_R < 16; a region that fits in
+// shared memory has fewer than 256 layers).
+static_assert(SYN_R <= 16 && 256 * SYN_R * (SYN_R + 1) * 4 + 252 * SYN_B * SYN_B * 2 > 220 * 1024,
+              "4 + 4 + 8 bits hold a position");
+__device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
+  return static_cast<uint16_t>(rx | ry << 4 | rz << 8);
+}
+
+// What bounds it: issue slots (76 % issue activity at 24 of 32 lanes; DRAM 1 %): about 620 warp
 // instructions a step, 31 rounds of 8 steps for the 115 points of a t-max column, which is within
 // 10 % of one step per point kept and one per point retired.  Visiting only the occupied cells (one
 // in nine, from the occupancy rows) instead of testing all 27 + 90 took the kernel from 38.8 to
-// 28.5 ms on a 1600 x 1600 px t-max image and from 10.4 to 7.7 ms on a 2048 x 2048 px tri-x one.
+// 28.5 ms on a 1600 x 1600 px t-max image; the instructions taken out since (one bounds check by
+// subtraction in each axis, round keys and neighbour cells from shared memory, positions packed by
+// coordinate, the resolution in region coordinates) took it to 26.7 ms, and from 7.7 to 7.2 ms on a
+// 2048 x 2048 px tri-x one.
 //
 // Launch bounds of 8 CTAs per SM (32 registers): more columns in flight hide the round's barriers.
 // A column with its one-cell spill and the halo stages 14 x 14 cells per layer, so eight CTAs fit
@@ -190,7 +215,8 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
   __shared__ unsigned s_rmask[SYN_WARPS];  // later candidates that passed the near cells, untested
   __shared__ uint32_t s_cxy[SYN_WARPS][32];  // valid candidates: x | y << 16 from the region's corner
   __shared__ int s_cz[SYN_WARPS][32];
-  __shared__ SynNear s_near;
+  __shared__ int4 s_near[27];
+  __shared__ uint4 s_key[5];  // Philox round keys
 
   // Column of this CTA: colour class, tile, then the j-th column of this class in that tile.
   const uint32_t cb[4] = {class_base.x, class_base.y, class_base.z, class_base.w};
@@ -261,7 +287,11 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       w = __ldcg(tc + (static_cast<size_t>(gz) * t.gh + gy) * t.gw + gx);
     grid[i] = w;
   }
-  if (tid < 27) syn_near_entry(s_near, tid);
+  if (tid < 5) {
+    const uint32_t a = t.k0 + 2 * tid * PHILOX_W0, b = t.k1 + 2 * tid * PHILOX_W1;
+    s_key[tid] = make_uint4(a, b, a + PHILOX_W0, b + PHILOX_W1);
+  }
+  if (tid < 27) s_near[tid] = syn_near_entry(tid);
   if (tid == 0) {
     s_nact = 0;
     s_ncom = 0;
@@ -281,19 +311,15 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
   const int bcells = bw * bh * gd;
   for (int base = 0; base < bcells; base += blockDim.x) {
     const int i = base + tid;
-    int ridx = 0;
-    bool o = false;
-    if (i < bcells) {
-      const int lx = i % bw, ly = (i / bw) % bh, lz = i / (bw * bh);
-      ridx = ((lz + 2) * SYN_R + (ly + SYN_HALO)) * SYN_R + (lx + SYN_HALO);
-      o = (grid[ridx] & OCC) != 0;
-    }
+    const int lx = i % bw, ly = (i / bw) % bh, lz = i / (bw * bh);
+    const bool o =
+        i < bcells && (grid[((lz + 2) * SYN_R + (ly + SYN_HALO)) * SYN_R + (lx + SYN_HALO)] & OCC) != 0;
     const unsigned m = __ballot_sync(0xffffffffu, o);
     if (lane == 0) s_wsum[warp] = __popc(m);
     __syncthreads();
     int off = s_nact;
     for (int w = 0; w < warp; ++w) off += s_wsum[w];
-    if (o) active[off + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(ridx);
+    if (o) active[off + __popc(m & ((1u << lane) - 1u))] = syn_pos(lx + SYN_HALO, ly + SYN_HALO, lz + 2);
     __syncthreads();
     if (tid == 0)
       for (int w = 0; w < SYN_WARPS; ++w) s_nact += s_wsum[w];
@@ -314,7 +340,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       grid[ridx] = syn_word(X, Y, Z);
       syn_mark(rows, rz * SYN_R + ry, rx);
       ++s_ncom;
-      if (index_ok(s_nact < acap, err, SITE_SYN_ACTIVE, s_nact, blockIdx.x)) active[s_nact++] = static_cast<uint16_t>(ridx);
+      if (index_ok(s_nact < acap, err, SITE_SYN_ACTIVE, s_nact, blockIdx.x)) active[s_nact++] = syn_pos(rx, ry, rz);
       break;
     }
   }
@@ -332,15 +358,15 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     // draws one Philox block of the warp's stream: lanes 0-29 place the candidates and lane 31's
     // draw picks the active point (shuffled to the warp); lane 0 records the pick for the
     // retirement.
+    static_assert(SYN_HALO - SYN_SPILL == 2, "a candidate's neighbourhood reaches two cells");
     static_assert(SYN_K < 32, "lane 31 draws the pick");
-    const P4 r = philox(static_cast<uint32_t>(iter), static_cast<uint32_t>(warp * 32 + lane), colkey, TAG_CAND,
-                        t.k0, t.k1);
+    const P4 r = philox_keys(static_cast<uint32_t>(iter), static_cast<uint32_t>(tid), colkey, TAG_CAND, s_key);
     const uint32_t rpick = __shfl_sync(0xffffffffu, r.x, 31);
     const int pick = static_cast<int>((static_cast<unsigned long long>(rpick) * static_cast<unsigned>(nact)) >> 32);
     if (lane == 0) s_pick[warp] = pick;
     const int pr = active[pick];
-    const uint32_t pw = grid[pr];
-    const int prx = pr % SYN_R, pry = (pr / SYN_R) % SYN_R, prz = pr / (SYN_R * SYN_R);
+    const int prx = pr & 15, pry = (pr >> 4) & 15, prz = pr >> 8;
+    const uint32_t pw = grid[(prz * SYN_R + pry) * SYN_R + prx];
     const int BX = (prx + ox) * SYN_Q + static_cast<int>(pw & 1023u);
     const int BY = (pry + oy) * SYN_Q + static_cast<int>((pw >> 10) & 1023u);
     const int BZ = (prz - 2) * SYN_Q + static_cast<int>((pw >> 20) & 1023u);
@@ -352,26 +378,21 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       const float st = sqrtf(fmaxf(1.0f - ct * ct, 0.0f));
       float sp, cp;
       sincospif(uf(r.z) * 2.0f, &sp, &cp);
-      const float rad = cbrtf(7.0f * u + 1.0f) * 1.7320508075688772f;  // r = sqrt(3) cells
-      const float fx = static_cast<float>(BX) * (1.0f / SYN_Q) + rad * st * cp;
-      const float fy = static_cast<float>(BY) * (1.0f / SYN_Q) + rad * st * sp;
-      const float fz = static_cast<float>(BZ) * (1.0f / SYN_Q) + rad * ct;
-      if (fx >= 0.0f && fy >= 0.0f && fz >= 0.0f) {
-        X = static_cast<int>(floorf(fx * SYN_Q));
-        Y = static_cast<int>(floorf(fy * SYN_Q));
-        Z = static_cast<int>(floorf(fz * SYN_Q));
-        if (X < static_cast<int>(t.XW) && Y < static_cast<int>(t.YW) && Z < static_cast<int>(t.ZW)) {
-          const int cx = X >> 10, cy = Y >> 10, cz = Z >> 10;
-          const int rx = cx - ox, ry = cy - oy, rz = cz + 2;
-          // The neighbourhood must lie inside the staged region (it does for candidates within 2r
-          // of a point of the column); a candidate that fails the check is rejected.
-          if (cx >= x0 - SYN_SPILL && cx < x1 + SYN_SPILL && cy >= y0 - SYN_SPILL && cy < y1 + SYN_SPILL &&
-              index_ok(rx >= 2 && rx <= SYN_R - 3 && ry >= 2 && ry <= SYN_R - 3 && rz >= 2 && rz <= nz - 3, err,
-                       SITE_SYN_REGION, static_cast<uint32_t>(rx | (ry << 8) | (rz << 16)), blockIdx.x)) {
-            rb = (rz * SYN_R + ry) * SYN_R + rx;
-            valid = syn_near_free(grid, rows, s_near, rx, rz * SYN_R + ry, rb, X & 1023, Y & 1023, Z & 1023);
-          }
-        }
+      const float rad = cbrtf(7.0f * u + 1.0f) * 1.7320508075688772f * SYN_Q;  // r = sqrt(3) cells
+      // Rounded down, so a negative coordinate fails the unsigned bound.
+      X = __float2int_rd(__fadd_rn(static_cast<float>(BX), __fmul_rn(rad * st, cp)));
+      Y = __float2int_rd(__fadd_rn(static_cast<float>(BY), __fmul_rn(rad * st, sp)));
+      Z = __float2int_rd(__fadd_rn(static_cast<float>(BZ), __fmul_rn(rad, ct)));
+      // Candidates lie in the column and its spill; those of the staged region's cells 2 .. SYN_R - 3
+      // in x and y (x1 <= x0 + SYN_B) and 2 .. nz - 3 in z (ZW <= gd * SYN_Q), so their
+      // neighbourhoods lie inside the region.
+      const int rx = (X >> 10) - ox, ry = (Y >> 10) - oy, rz = (Z >> 10) + 2;
+      if (static_cast<uint32_t>(X) < t.XW && static_cast<uint32_t>(Y) < t.YW && static_cast<uint32_t>(Z) < t.ZW &&
+          static_cast<uint32_t>(rx - (SYN_HALO - SYN_SPILL)) < static_cast<uint32_t>(x1 - x0 + 2 * SYN_SPILL) &&
+          static_cast<uint32_t>(ry - (SYN_HALO - SYN_SPILL)) < static_cast<uint32_t>(y1 - y0 + 2 * SYN_SPILL)) {
+        const int row = rz * SYN_R + ry;
+        rb = row * SYN_R + rx;
+        valid = syn_near_free(grid, rows, s_near, rx, row, rb, X & 1023, Y & 1023, Z & 1023);
       }
     }
     unsigned rest;
@@ -391,7 +412,8 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       // first candidate (lane order) that is free in the grid and at least r from the points
       // accepted for warps < w; with none left, its point retires.
       //
-      // Lane w speaks for warp w and holds its winner (first grid-free candidate).  That order keeps
+      // Lane w speaks for warp w and holds its winner (first grid-free candidate; x and y from the
+      // region's corner).  That order keeps
       // a winner unless it lies within r of a point accepted for an earlier warp, so the warps keep
       // their winners in runs up to the next warp whose winner conflicts; only that warp searches
       // its other candidates against the points accepted so far.  Conflicts between winners come
@@ -402,8 +424,8 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
         if (m) {
           fw = __ffs(m) - 1;
           const uint32_t xy = s_cxy[lane][fw];
-          PX = static_cast<int>(xy & 0xffffu) + ox * SYN_Q;
-          PY = static_cast<int>(xy >> 16) + oy * SYN_Q;
+          PX = static_cast<int>(xy & 0xffffu);
+          PY = static_cast<int>(xy >> 16);
           PZ = s_cz[lane][fw];
         }
       }
@@ -411,13 +433,12 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
 #pragma unroll
       for (int u = 0; u < SYN_WARPS - 1; ++u) {
         const int ux = __shfl_sync(0xffffffffu, PX, u), uy = __shfl_sync(0xffffffffu, PY, u);
-        const int uz = __shfl_sync(0xffffffffu, PZ, u), uf = __shfl_sync(0xffffffffu, fw, u);
-        if (u < lane && fw >= 0 && uf >= 0) {
-          const int ex = PX - ux, ey = PY - uy, ez = PZ - uz;
-          if (ex * ex + ey * ey + ez * ez < SYN_R2X) cm |= 1u << u;
-        }
+        const int uz = __shfl_sync(0xffffffffu, PZ, u);
+        const int ex = PX - ux, ey = PY - uy, ez = PZ - uz;
+        if (ex * ex + ey * ey + ez * ez < SYN_R2X) cm |= 1u << u;
       }
       const unsigned has = __ballot_sync(0xffffffffu, fw >= 0);  // warps with a winner
+      cm &= has & ((1u << lane) - 1u);
       unsigned accw = 0, acc = 0;  // warps that keep their winner; warps that keep a point
       bool near = false;           // this lane's winner lies within r of a point kept instead of a winner
       for (int cur = 0; cur < SYN_WARPS;) {
@@ -440,8 +461,8 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
         int X = 0, Y = 0, Z = 0;
         if (ok) {
           const uint32_t xy = s_cxy[wb][lane];
-          X = static_cast<int>(xy & 0xffffu) + ox * SYN_Q;
-          Y = static_cast<int>(xy >> 16) + oy * SYN_Q;
+          X = static_cast<int>(xy & 0xffffu);
+          Y = static_cast<int>(xy >> 16);
           Z = s_cz[wb][lane];
         }
 #pragma unroll
@@ -464,7 +485,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
           }
           const int lx_ = __shfl_sync(0xffffffffu, X, l), ly_ = __shfl_sync(0xffffffffu, Y, l);
           const int lz_ = __shfl_sync(0xffffffffu, Z, l);
-          const int cb = (((lz_ >> 10) + 2) * SYN_R + ((ly_ >> 10) - oy)) * SYN_R + ((lx_ >> 10) - ox);
+          const int cb = (((lz_ >> 10) + 2) * SYN_R + (ly_ >> 10)) * SYN_R + (lx_ >> 10);
           if (!syn_outer_hit(grid, rows, cb, lx_ & 1023, ly_ & 1023, lz_ & 1023, lane)) {
             c = l;
             break;
@@ -487,24 +508,23 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       }
       // Commit the kept points, appending to the active list in warp order.
       bool inside = false, committed = false;
-      int cridx = 0;
+      uint16_t cpos = 0;
       if (lane < SYN_WARPS && ((acc >> lane) & 1u)) {
-        const int ccx = PX >> 10, ccy = PY >> 10, ccz = PZ >> 10;
-        const int rx = ccx - ox, ry = ccy - oy, rz = ccz + 2;
+        const int rx = PX >> 10, ry = PY >> 10, rz = (PZ >> 10) + 2;
         if (index_ok(rx >= 1 && rx < SYN_R && ry >= 1 && ry < SYN_R && rz >= 0 && rz < nz, err, SITE_SYN_COMMIT,
                      static_cast<uint32_t>(rx | (ry << 8) | (rz << 16)), blockIdx.x)) {
-          cridx = (rz * SYN_R + ry) * SYN_R + rx;
-          grid[cridx] = syn_word(PX, PY, PZ);
+          cpos = syn_pos(rx, ry, rz);
+          grid[(rz * SYN_R + ry) * SYN_R + rx] = syn_word(PX, PY, PZ);
           syn_mark(rows, rz * SYN_R + ry, rx);
           committed = true;
-          inside = ccx >= x0 && ccx < x1 && ccy >= y0 && ccy < y1;
+          inside = rx >= SYN_HALO && rx < SYN_HALO + bw && ry >= SYN_HALO && ry < SYN_HALO + bh;
         }
       }
       const unsigned im = __ballot_sync(0xffffffffu, inside);
       const int nbase = s_nact;
       if (inside) {
         const int pos = nbase + __popc(im & ((1u << lane) - 1u));
-        if (index_ok(pos < acap, err, SITE_SYN_ACTIVE, pos, blockIdx.x)) active[pos] = static_cast<uint16_t>(cridx);
+        if (index_ok(pos < acap, err, SITE_SYN_ACTIVE, pos, blockIdx.x)) active[pos] = cpos;
       }
       const unsigned cmm = __ballot_sync(0xffffffffu, committed);
       const int n0 = min(nbase + __popc(im), acap);
