@@ -210,10 +210,10 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
   uint16_t* active = reinterpret_cast<uint16_t*>(rows + SYN_R * nz);  // SYN_B^2 * (nz - 4)
   __shared__ int s_nact, s_wsum[SYN_WARPS];
   __shared__ int s_ncom;  // points this column commits (each fills one empty cell of its tile)
-  __shared__ int s_pick[SYN_WARPS];
-  __shared__ unsigned s_vmask[SYN_WARPS];  // the step's first valid candidate (at most one lane)
+  __shared__ int4 s_pick[SYN_WARPS / 4];   // the steps' picks
+  __shared__ int4 s_win[SYN_WARPS];        // the step's winner from the region's corner; w: whether it has one
   __shared__ unsigned s_rmask[SYN_WARPS];  // later candidates that passed the near cells, untested
-  __shared__ uint32_t s_cxy[SYN_WARPS][32];  // valid candidates: x | y << 16 from the region's corner
+  __shared__ uint32_t s_cxy[SYN_WARPS][32];  // those: x | y << 16 from the region's corner
   __shared__ int s_cz[SYN_WARPS][32];
   __shared__ int4 s_near[27];
   __shared__ uint4 s_key[5];  // Philox round keys
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     const P4 r = philox_keys(static_cast<uint32_t>(iter), static_cast<uint32_t>(tid), colkey, TAG_CAND, s_key);
     const uint32_t rpick = __shfl_sync(0xffffffffu, r.x, 31);
     const int pick = static_cast<int>((static_cast<unsigned long long>(rpick) * static_cast<unsigned>(nact)) >> 32);
-    if (lane == 0) s_pick[warp] = pick;
+    if (lane == 0) reinterpret_cast<int*>(s_pick)[warp] = pick;
     const int pr = active[pick];
     const int prx = pr & 15, pry = (pr >> 4) & 15, prz = pr >> 8;
     const uint32_t pw = grid[(prz * SYN_R + pry) * SYN_R + prx];
@@ -397,111 +397,79 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     }
     unsigned rest;
     const bool first = syn_outer_free(grid, rows, valid, rb, X & 1023, Y & 1023, Z & 1023, lane, rest);
-    const unsigned vm = __ballot_sync(0xffffffffu, first);
-    if (first || ((rest >> lane) & 1u)) {
+    const bool none = __ballot_sync(0xffffffffu, first) == 0u;
+    if (first || (none && lane == 0)) s_win[warp] = make_int4(X - ox * SYN_Q, Y - oy * SYN_Q, Z, first);
+    if ((rest >> lane) & 1u) {
       s_cxy[warp][lane] = static_cast<uint32_t>(X - ox * SYN_Q) | static_cast<uint32_t>(Y - oy * SYN_Q) << 16;
       s_cz[warp][lane] = Z;
     }
-    if (lane == 0) {
-      s_vmask[warp] = vm;
-      s_rmask[warp] = rest;
-    }
+    if (lane == 0) s_rmask[warp] = rest;
     __syncthreads();
     if (warp == 0) {
       // The round's steps in warp order, exactly as if they ran one after another: warp w keeps its
       // first candidate (lane order) that is free in the grid and at least r from the points
-      // accepted for warps < w; with none left, its point retires.
+      // accepted for warps < w; with none left, its point retires.  The other warps wait meanwhile:
+      // this is the round's serial part, kept short.
       //
-      // Lane w speaks for warp w and holds its winner (first grid-free candidate; x and y from the
-      // region's corner).  That order keeps
+      // Lane w speaks for warp w and holds its winner (first grid-free candidate).  That order keeps
       // a winner unless it lies within r of a point accepted for an earlier warp, so the warps keep
       // their winners in runs up to the next warp whose winner conflicts; only that warp searches
-      // its other candidates against the points accepted so far.  Conflicts between winners come
-      // from shuffles; a point kept instead of a winner is tested against the later winners once.
-      int fw = -1, PX = 0, PY = 0, PZ = 0;
-      if (lane < SYN_WARPS) {
-        const unsigned m = s_vmask[lane];
-        if (m) {
-          fw = __ffs(m) - 1;
-          const uint32_t xy = s_cxy[lane][fw];
-          PX = static_cast<int>(xy & 0xffffu);
-          PY = static_cast<int>(xy >> 16);
-          PZ = s_cz[lane][fw];
-        }
-      }
-      unsigned cm = 0;  // bit u: this lane's winner conflicts with warp u's (u < lane)
-#pragma unroll
-      for (int u = 0; u < SYN_WARPS - 1; ++u) {
-        const int ux = __shfl_sync(0xffffffffu, PX, u), uy = __shfl_sync(0xffffffffu, PY, u);
-        const int uz = __shfl_sync(0xffffffffu, PZ, u);
-        const int ex = PX - ux, ey = PY - uy, ez = PZ - uz;
-        if (ex * ex + ey * ey + ez * ez < SYN_R2X) cm |= 1u << u;
-      }
-      const unsigned has = __ballot_sync(0xffffffffu, fw >= 0);  // warps with a winner
-      cm &= has & ((1u << lane) - 1u);
+      // its other candidates against the points accepted so far.  The 64 pairs of winners are tested
+      // two to a lane: lane 4 w + q holds warp w's against those of warps q and q + 4.
+      static_assert(SYN_WARPS == 8, "two pairs of winners to a lane");
+      auto close = [](const int4& p, const int4& q) {
+        const int ex = p.x - q.x, ey = p.y - q.y, ez = p.z - q.z;
+        return ex * ex + ey * ey + ez * ez < SYN_R2X;
+      };
+      int4 P = s_win[lane & 7];
+      const int4 pw4 = s_win[lane >> 2];
+      const unsigned b0 = __ballot_sync(0xffffffffu, close(pw4, s_win[lane & 3]));
+      const unsigned b1 = __ballot_sync(0xffffffffu, close(pw4, s_win[(lane & 3) + 4]));
+      const unsigned has = __ballot_sync(0xffffffffu, lane < SYN_WARPS && P.w != 0);  // warps with a winner
+      const int sh = 4 * (lane & 7);
+      // Bit u: this lane's winner conflicts with warp u's (u < lane).
+      const unsigned cm = (((b0 >> sh) & 15u) | ((b1 >> sh) & 15u) << 4) & has & ((1u << (lane & 7)) - 1u);
       unsigned accw = 0, acc = 0;  // warps that keep their winner; warps that keep a point
       bool near = false;           // this lane's winner lies within r of a point kept instead of a winner
       for (int cur = 0; cur < SYN_WARPS;) {
         // A warp from cur on keeps its winner unless it conflicts with a kept point; up to the first
         // such warp, every warp with a winner keeps it.
         const unsigned from = ~((1u << cur) - 1u);
-        const bool bad = lane >= cur && fw >= 0 &&
-                         (near || (cm & (accw | (has & from & ((1u << lane) - 1u)))) != 0u);
+        const bool bad = lane >= cur && ((has >> lane) & 1u) != 0u && (near || (cm & (accw | from)) != 0u);
         const unsigned bm = __ballot_sync(0xffffffffu, bad);
         const int wb = bm ? __ffs(bm) - 1 : SYN_WARPS;
         const unsigned run = has & from & ((1u << wb) - 1u);
         accw |= run;
         acc |= run;
         if (wb == SYN_WARPS) break;
-        // Warp wb: its first valid candidate at least r from every point kept for warps < wb.  Its
-        // untested candidates take the outer test here, in lane order, until one passes (the grid
-        // is as the candidate phase saw it: the round commits after it is resolved).
-        const unsigned m = s_vmask[wb], mr = s_rmask[wb];
-        bool ok = ((m | mr) >> lane) & 1u;
-        int X = 0, Y = 0, Z = 0;
+        // Warp wb: its first candidate after the winner that is at least r from every point kept
+        // for warps < wb and passes the outer test, in lane order (the grid is as the candidate
+        // phase saw it: the round commits after it is resolved).
+        bool ok = (s_rmask[wb] >> lane) & 1u;
+        int4 C = make_int4(0, 0, 0, 1);
         if (ok) {
           const uint32_t xy = s_cxy[wb][lane];
-          X = static_cast<int>(xy & 0xffffu);
-          Y = static_cast<int>(xy >> 16);
-          Z = s_cz[wb][lane];
+          C.x = static_cast<int>(xy & 0xffffu);
+          C.y = static_cast<int>(xy >> 16);
+          C.z = s_cz[wb][lane];
         }
-#pragma unroll
-        for (int u = 0; u < SYN_WARPS - 1; ++u) {
-          const int ux = __shfl_sync(0xffffffffu, PX, u), uy = __shfl_sync(0xffffffffu, PY, u);
-          const int uz = __shfl_sync(0xffffffffu, PZ, u);
-          if ((acc >> u) & 1u) {
-            const int ex = X - ux, ey = Y - uy, ez = Z - uz;
-            if (ex * ex + ey * ey + ez * ez < SYN_R2X) ok = false;
-          }
-        }
+        for (unsigned a = __any_sync(0xffffffffu, ok) ? acc : 0u; a; a &= a - 1u)
+          if (close(C, s_win[__ffs(a) - 1])) ok = false;
         unsigned okm = __ballot_sync(0xffffffffu, ok);
-        int c = -1;
         while (okm) {
           const int l = __ffs(okm) - 1;
           okm &= okm - 1;
-          if ((m >> l) & 1u) {
-            c = l;
-            break;
-          }
-          const int lx_ = __shfl_sync(0xffffffffu, X, l), ly_ = __shfl_sync(0xffffffffu, Y, l);
-          const int lz_ = __shfl_sync(0xffffffffu, Z, l);
+          const int lx_ = __shfl_sync(0xffffffffu, C.x, l), ly_ = __shfl_sync(0xffffffffu, C.y, l);
+          const int lz_ = __shfl_sync(0xffffffffu, C.z, l);
           const int cb = (((lz_ >> 10) + 2) * SYN_R + (ly_ >> 10)) * SYN_R + (lx_ >> 10);
           if (!syn_outer_hit(grid, rows, cb, lx_ & 1023, ly_ & 1023, lz_ & 1023, lane)) {
-            c = l;
+            if (lane == l) s_win[wb] = C;
+            __syncwarp();
+            const int4 N = s_win[wb];
+            acc |= 1u << wb;
+            if (lane == wb) P = N;
+            near = near || close(P, N);  // looked at for the warps after wb only
             break;
-          }
-        }
-        if (c >= 0) {
-          const int qx = __shfl_sync(0xffffffffu, X, c), qy = __shfl_sync(0xffffffffu, Y, c);
-          const int qz = __shfl_sync(0xffffffffu, Z, c);
-          acc |= 1u << wb;
-          if (lane == wb) {
-            PX = qx;
-            PY = qy;
-            PZ = qz;
-          } else if (lane > wb && fw >= 0) {
-            const int ex = PX - qx, ey = PY - qy, ez = PZ - qz;
-            if (ex * ex + ey * ey + ez * ez < SYN_R2X) near = true;
           }
         }
         cur = wb + 1;
@@ -510,57 +478,48 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       bool inside = false, committed = false;
       uint16_t cpos = 0;
       if (lane < SYN_WARPS && ((acc >> lane) & 1u)) {
-        const int rx = PX >> 10, ry = PY >> 10, rz = (PZ >> 10) + 2;
+        const int rx = P.x >> 10, ry = P.y >> 10, rz = (P.z >> 10) + 2;
         if (index_ok(rx >= 1 && rx < SYN_R && ry >= 1 && ry < SYN_R && rz >= 0 && rz < nz, err, SITE_SYN_COMMIT,
                      static_cast<uint32_t>(rx | (ry << 8) | (rz << 16)), blockIdx.x)) {
           cpos = syn_pos(rx, ry, rz);
-          grid[(rz * SYN_R + ry) * SYN_R + rx] = syn_word(PX, PY, PZ);
+          grid[(rz * SYN_R + ry) * SYN_R + rx] = syn_word(P.x, P.y, P.z);
           syn_mark(rows, rz * SYN_R + ry, rx);
           committed = true;
           inside = rx >= SYN_HALO && rx < SYN_HALO + bw && ry >= SYN_HALO && ry < SYN_HALO + bh;
         }
       }
       const unsigned im = __ballot_sync(0xffffffffu, inside);
-      const int nbase = s_nact;
       if (inside) {
-        const int pos = nbase + __popc(im & ((1u << lane) - 1u));
+        const int pos = nact + __popc(im & ((1u << lane) - 1u));
         if (index_ok(pos < acap, err, SITE_SYN_ACTIVE, pos, blockIdx.x)) active[pos] = cpos;
       }
       const unsigned cmm = __ballot_sync(0xffffffffu, committed);
-      const int n0 = min(nbase + __popc(im), acap);
+      const int n0 = min(nact + __popc(im), acap);
       __syncwarp();  // the appended entries are visible to the retirement below
       // Retire the points of failed steps, each once, as if removed one after another in descending
       // list order, each by moving the list's current last entry into its place (a swap-remove).
       // The removal of rank k takes the entry then at n0 - 1 - k; when that position was itself
-      // refilled by an earlier removal, its entry is the one that removal took, so each removal
-      // follows that chain (pointer jumping over the ranks) to an original position.
-      const bool mine = lane < SYN_WARPS && !((acc >> lane) & 1u);
-      const int mypick = lane < SYN_WARPS ? s_pick[lane] : -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, mine ? mypick : -1 - lane);
-      const bool first = mine && lane == __ffs(peers) - 1;
+      // refilled by the removal of a lower rank, its entry is the one that removal took, and so on
+      // down.  Nibble k of `tail` holds 1 + the rank of the pick at n0 - 1 - k, 0 for none.
+      const int mypick = reinterpret_cast<const int*>(s_pick)[lane & 7];
+      unsigned eq = 0, gt = 0;  // warps with this lane's pick; with a later one
+#pragma unroll
+      for (int h = 0; h < SYN_WARPS / 4; ++h) {
+        const int4 q = s_pick[h];
+        eq |= (q.x == mypick ? 1u : 0u) << (4 * h) | (q.y == mypick ? 2u : 0u) << (4 * h) |
+              (q.z == mypick ? 4u : 0u) << (4 * h) | (q.w == mypick ? 8u : 0u) << (4 * h);
+        gt |= (q.x > mypick ? 1u : 0u) << (4 * h) | (q.y > mypick ? 2u : 0u) << (4 * h) |
+              (q.z > mypick ? 4u : 0u) << (4 * h) | (q.w > mypick ? 8u : 0u) << (4 * h);
+      }
+      const bool first = lane < SYN_WARPS && ((acc >> lane) & 1u) == 0u && (eq & ~acc & ((1u << lane) - 1u)) == 0u;
       const unsigned dm = __ballot_sync(0xffffffffu, first);
-      int rank = 0;
-#pragma unroll
-      for (int w2 = 0; w2 < SYN_WARPS; ++w2) {
-        const int p2 = __shfl_sync(0xffffffffu, mypick, w2);
-        if (((dm >> w2) & 1u) && p2 > mypick) ++rank;
+      int k = __popc(gt & dm);  // rank
+      const unsigned at = static_cast<unsigned>(n0 - 1 - mypick);
+      const unsigned tail = __reduce_or_sync(0xffffffffu, first && at < 8u ? static_cast<unsigned>(k + 1) << (4 * at) : 0u);
+      if (tail && first) {
+        for (int e; (e = static_cast<int>(tail >> (4 * k) & 15u)) != 0 && e - 1 < k;) k = e - 1;
       }
-      int src = n0 - 1 - rank, ptr = -1;
-#pragma unroll
-      for (int w2 = 0; w2 < SYN_WARPS; ++w2) {
-        const int p2 = __shfl_sync(0xffffffffu, mypick, w2);
-        if (((dm >> w2) & 1u) && w2 != lane && p2 == src) ptr = w2;
-      }
-      if (!first) ptr = -1;
-#pragma unroll
-      for (int hop = 1; hop < SYN_WARPS; hop <<= 1) {  // chains are shorter than SYN_WARPS
-        const int at = ptr < 0 ? lane : ptr;
-        const int ps = __shfl_sync(0xffffffffu, src, at), pp = __shfl_sync(0xffffffffu, ptr, at);
-        if (ptr >= 0) {
-          src = ps;
-          ptr = pp;
-        }
-      }
+      const int src = n0 - 1 - k;
       uint16_t moved = 0;
       if (first && index_ok(src >= 0 && src < n0, err, SITE_SYN_ACTIVE, src, blockIdx.x)) moved = active[src];
       __syncwarp();
