@@ -25,7 +25,7 @@
 namespace fg {
 
 void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], int gdmax, uint32_t* cells,
-                    uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, uint32_t wait_limit = 0,
+                    uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, int sms, uint32_t wait_limit = 0,
                     const uint32_t* probe = nullptr);
 size_t bridson_smem(int gdmax);
 void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_cells, unsigned long long max_slots,
@@ -545,7 +545,7 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
   FG_CUDA(cudaMemsetAsync(B->npts.p, 0, B->ntiles * sizeof(uint32_t), st));
   mark(B->ev[8], st, capturing);
   launch_bridson(B->d_syn.p, nt, B->cols, B->gdmax, B->cells.p, B->npts.p, B->coldone.p, e->d_err, st,
-                 B->wait_limit, B->wait_probe ? B->probe.p : nullptr);
+                 e->sm_count, B->wait_limit, B->wait_probe ? B->probe.p : nullptr);
   mark(B->ev[7], st, capturing);
   FG_CUDA(cudaMemsetAsync(B->flags.p + B->nslots, 0, sizeof(uint32_t), st));
   launch_synth_post(B->d_syn.p, nt, B->maxcells, B->maxslots, B->cells.p, B->npts.p, B->flags.p, st);
@@ -955,7 +955,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     FG_CUDA(cudaMemsetAsync(cells.p, 0, ncells * sizeof(uint32_t), st));
     FG_CUDA(cudaMemsetAsync(npts.p, 0, sizeof(uint32_t), st));
     DBuf<uint32_t> coldone(std::max(cols[0] + cols[1] + cols[2] + cols[3], 1u), st);
-    launch_bridson(d_syn.p, 1, cols, gdmax, cells.p, npts.p, coldone.p, e->d_err, st);
+    launch_bridson(d_syn.p, 1, cols, gdmax, cells.p, npts.p, coldone.p, e->d_err, st, e->sm_count);
     FG_CUDA(cudaMemsetAsync(flags.p + nbr, 0, sizeof(uint32_t), st));
     launch_synth_post(d_syn.p, 1, ncells, nbr, cells.p, npts.p, flags.p, st);
     exclusive_scan_u32(flags.p, scan.p, nbr + 1ull, st);

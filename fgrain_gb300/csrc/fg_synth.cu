@@ -172,6 +172,21 @@ __device__ __forceinline__ P4 philox_keys(uint32_t c0, uint32_t c1, uint32_t c2,
   return P4{c0, c1, c2, c3};
 }
 
+// The draws of a step's lane (thread `slot` of the column): a lane that places a candidate gets its
+// offset from the active point in the shell [r, 2 r] (fixed point), the last lane the bits (.x) that
+// pick the active point.
+__device__ __forceinline__ float3 syn_draw(int iter, int slot, int lane, uint32_t colkey, const uint4* keys) {
+  const P4 r = philox_keys(static_cast<uint32_t>(iter), static_cast<uint32_t>(slot), colkey, TAG_CAND, keys);
+  const float u = uf(r.x);
+  const float ct = uf(r.y) * 2.0f - 1.0f;
+  const float st = sqrtf(fmaxf(1.0f - ct * ct, 0.0f));
+  float sp, cp;
+  sincospif(uf(r.z) * 2.0f, &sp, &cp);
+  const float rad = cbrtf(7.0f * u + 1.0f) * 1.7320508075688772f * SYN_Q;  // r = sqrt(3) cells
+  const float x = __fmul_rn(rad * st, cp);
+  return make_float3(lane < SYN_K ? x : __uint_as_float(r.x), __fmul_rn(rad * st, sp), __fmul_rn(rad, ct));
+}
+
 // An entry of the active list: the cell's region coordinates (SYN_R < 16; a region that fits in
 // shared memory has fewer than 256 layers).
 static_assert(SYN_R <= 16 && 256 * SYN_R * (SYN_R + 1) * 4 + 252 * SYN_B * SYN_B * 2 > 220 * 1024,
@@ -186,19 +201,28 @@ __device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
 // in nine, from the occupancy rows) instead of testing all 27 + 90 took the kernel from 38.8 to
 // 28.5 ms on a 1600 x 1600 px t-max image; the instructions taken out since (one bounds check by
 // subtraction in each axis, round keys and neighbour cells from shared memory, positions packed by
-// coordinate, the resolution in region coordinates) took it to 26.7 ms, and from 7.7 to 7.2 ms on a
+// coordinate) and the shorter resolution took it to 24.6 ms, and from 7.7 to 6.6 ms on a
 // 2048 x 2048 px tri-x one.
 //
 // Launch bounds of 8 CTAs per SM (32 registers): more columns in flight hide the round's barriers.
 // A column with its one-cell spill and the halo stages 14 x 14 cells per layer, so eight CTAs fit
 // in the SM's 228 KB of shared memory for depths up to 23 cells.
+//
+// FEW: with few columns in flight the latency of a round counts instead (5,600 cycles, of which 1,950
+// are the resolution by one warp).  4 CTAs per SM leave 64 registers, and the seven warps that wait
+// draw the next round's candidates meanwhile.  The classes run nearly one after another, so 20
+// columns an SM are about five in flight: on t-max films of 25 .. 1,936 columns it takes .34 - .45
+// against .40 - .51 ms, at 2,601 .521 against .581, at 3,249 (21 an SM) .617 against .621, at 4,356
+// .814 against .726.
+constexpr unsigned SYN_FEW = 20;  // columns an SM
 // All columns of all four colour classes in one launch, class after class in block order.  A column
 // starts once the columns of lower classes next to it have written their cells back (their done
 // flags), which gives every column the cell state it would see if the classes ran one launch
 // after another: only the eight neighbouring columns share cells with it, and a neighbour of a
 // higher class waits for it in turn.  The flags are waited on by lower block indices only, so
 // the wait ends as the earlier blocks finish; it is bounded all the same (ERR_SPIN_LIMIT).
-__global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* __restrict__ tiles,
+template <bool FEW>
+__global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const SynthTile* __restrict__ tiles,
                                                             int ntiles, uint4 class_base, int nz,
                                                             uint32_t* __restrict__ cells,
                                                             uint32_t* __restrict__ npts, uint32_t* done,
@@ -216,7 +240,8 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
   __shared__ uint32_t s_cxy[SYN_WARPS][32];  // those: x | y << 16 from the region's corner
   __shared__ int s_cz[SYN_WARPS][32];
   __shared__ int4 s_near[27];
-  __shared__ uint4 s_key[5];  // Philox round keys
+  __shared__ uint4 s_key[5];              // Philox round keys
+  __shared__ float3 s_off[FEW ? 32 : 1];  // the next round's draws of the resolving warp
 
   // Column of this CTA: colour class, tile, then the j-th column of this class in that tile.
   const uint32_t cb[4] = {class_base.x, class_base.y, class_base.z, class_base.w};
@@ -344,6 +369,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
       break;
     }
   }
+  float3 off = FEW ? syn_draw(0, tid, lane, colkey, s_key) : float3{};
   const int max_iter = 16 * SYN_B * SYN_B * gd + 64;
   for (int iter = 0;; ++iter) {
     __syncthreads();
@@ -360,8 +386,12 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     // retirement.
     static_assert(SYN_HALO - SYN_SPILL == 2, "a candidate's neighbourhood reaches two cells");
     static_assert(SYN_K < 32, "lane 31 draws the pick");
-    const P4 r = philox_keys(static_cast<uint32_t>(iter), static_cast<uint32_t>(tid), colkey, TAG_CAND, s_key);
-    const uint32_t rpick = __shfl_sync(0xffffffffu, r.x, 31);
+    if (!FEW) {
+      off = syn_draw(iter, tid, lane, colkey, s_key);
+    } else if (warp == 0 && iter > 0) {
+      off = s_off[lane];
+    }
+    const uint32_t rpick = __shfl_sync(0xffffffffu, __float_as_uint(off.x), 31);
     const int pick = static_cast<int>((static_cast<unsigned long long>(rpick) * static_cast<unsigned>(nact)) >> 32);
     if (lane == 0) reinterpret_cast<int*>(s_pick)[warp] = pick;
     const int pr = active[pick];
@@ -373,16 +403,10 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     bool valid = false;
     int X = 0, Y = 0, Z = 0, rb = 0;
     if (lane < SYN_K) {
-      const float u = uf(r.x);
-      const float ct = uf(r.y) * 2.0f - 1.0f;
-      const float st = sqrtf(fmaxf(1.0f - ct * ct, 0.0f));
-      float sp, cp;
-      sincospif(uf(r.z) * 2.0f, &sp, &cp);
-      const float rad = cbrtf(7.0f * u + 1.0f) * 1.7320508075688772f * SYN_Q;  // r = sqrt(3) cells
       // Rounded down, so a negative coordinate fails the unsigned bound.
-      X = __float2int_rd(__fadd_rn(static_cast<float>(BX), __fmul_rn(rad * st, cp)));
-      Y = __float2int_rd(__fadd_rn(static_cast<float>(BY), __fmul_rn(rad * st, sp)));
-      Z = __float2int_rd(__fadd_rn(static_cast<float>(BZ), __fmul_rn(rad, ct)));
+      X = __float2int_rd(__fadd_rn(static_cast<float>(BX), off.x));
+      Y = __float2int_rd(__fadd_rn(static_cast<float>(BY), off.y));
+      Z = __float2int_rd(__fadd_rn(static_cast<float>(BZ), off.z));
       // Candidates lie in the column and its spill; those of the staged region's cells 2 .. SYN_R - 3
       // in x and y (x1 <= x0 + SYN_B) and 2 .. nz - 3 in z (ZW <= gd * SYN_Q), so their
       // neighbourhoods lie inside the region.
@@ -405,7 +429,14 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, 8) k_bridson(const SynthTile* 
     }
     if (lane == 0) s_rmask[warp] = rest;
     __syncthreads();
-    if (warp == 0) {
+    if (warp != 0) {
+      // With registers to spare, the other warps draw for the next round meanwhile, one of them for
+      // the resolving warp too.
+      if (FEW) {
+        if (warp == 1) s_off[lane] = syn_draw(iter + 1, lane, lane, colkey, s_key);
+        off = syn_draw(iter + 1, tid, lane, colkey, s_key);
+      }
+    } else {
       // The round's steps in warp order, exactly as if they ran one after another: warp w keeps its
       // first candidate (lane order) that is free in the grid and at least r from the points
       // accepted for warps < w; with none left, its point retires.  The other warps wait meanwhile:
@@ -755,16 +786,17 @@ size_t bridson_smem(int gdmax);
 // Host wrappers (launch on `st`; all buffers preallocated so the sequence can be graph-captured).
 // cols[c] columns of class c; done holds one flag per column (zeroed here).
 void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], int gdmax, uint32_t* cells,
-                    uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, uint32_t wait_limit,
+                    uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, int sms, uint32_t wait_limit,
                     const uint32_t* probe) {
   const unsigned total = cols[0] + cols[1] + cols[2] + cols[3];
   if (total == 0) return;
   const int nz = gdmax + 4;
   const size_t smem = bridson_smem(gdmax);
   FG_CUDA(cudaMemsetAsync(done, 0, total * sizeof(uint32_t), st));
-  FG_CUDA(cudaFuncSetAttribute(k_bridson, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const auto kernel = total <= SYN_FEW * static_cast<unsigned>(sms) ? k_bridson<true> : k_bridson<false>;
+  FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   const uint4 cb = make_uint4(0u, cols[0], cols[0] + cols[1], cols[0] + cols[1] + cols[2]);
-  k_bridson<<<total, SYN_WARPS * 32, smem, st>>>(tiles, ntiles, cb, nz, cells, npts, done, err,
+  kernel<<<total, SYN_WARPS * 32, smem, st>>>(tiles, ntiles, cb, nz, cells, npts, done, err,
                                                   wait_limit ? wait_limit : (1u << 22), probe);
   FG_CUDA(cudaGetLastError());
 }

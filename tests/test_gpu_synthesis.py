@@ -39,3 +39,20 @@ def test_points_are_hard_core_and_dense(engine, cells, r_min):
     assert n <= target + 4 * np.sqrt(target) + 2
     if min(size) > 5 * r_min:
         assert abs(n - target) <= 0.02 * target + 4
+
+
+@pytest.mark.parametrize("stock,grain", [("t-max", 1.1), ("tri-x", 2.4)])
+def test_points_do_not_depend_on_the_columns_in_flight(engine, stock, grain):
+    """A tile's crystals are the same alone (few columns: the kernel that draws ahead) and beside others
+    (many columns)."""
+    params = [fg.tile_params(stock, 1 / grain, 190 + i, 170, 1.0, 0.0, 40 + i) for i in range(8)]
+    both = []
+    for ps in (params[:1], params):
+        b = fg.Batch(ps, engine, use_graph=False)
+        b.set_exposure([np.full((p.height_px, p.width_px), 0.5, np.float32) for p in ps])
+        b.run()
+        b.wait()
+        both.append(b.tile_crystals(0))
+        b.close()
+    for k in both[0]:
+        np.testing.assert_array_equal(both[0][k], both[1][k])
