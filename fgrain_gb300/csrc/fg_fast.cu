@@ -9,7 +9,7 @@
 //
 // Arithmetic is f32 in the shaders' operation order with every operation rounded on its own
 // (intrinsics, no contraction).  Where WGSL leaves a choice to the implementation the same choice
-// is made as in the CPU restatement: exp, log, sin and cos are evaluated in FP64 and rounded once;
+// is made as in the CPU restatement: exp, log, sin and cos are FP64 rounded once (fg_pair.cuh);
 // dot products sum (x + y) + z; the relaxation reads the positions from before its pass (the
 // shader updates them in place, in an order the API leaves undefined).
 //
@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "fg_internal.h"
+#include "fg_pair.cuh"
 
 namespace fg {
 
@@ -46,10 +47,13 @@ __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); 
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ float fexp_(float x) { return static_cast<float>(exp(static_cast<double>(x))); }
-__device__ __forceinline__ float flog_(float x) { return static_cast<float>(log(static_cast<double>(x))); }
-__device__ __forceinline__ float fsin_(float x) { return static_cast<float>(sin(static_cast<double>(x))); }
-__device__ __forceinline__ float fcos_(float x) { return static_cast<float>(cos(static_cast<double>(x))); }
+__device__ __forceinline__ float fexp_(float x) { return pair_expf(x); }
+__device__ __forceinline__ float flog_(float x) { return pair_logf(x); }
+__device__ __forceinline__ float fcos_(float x) {
+  float s, c;
+  pair_sincosf(x, s, c);
+  return c;
+}
 __device__ __forceinline__ float clampf_(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 __device__ __forceinline__ float dot3_(float ax, float ay, float az, float bx, float by, float bz) {
   return fa(fa(fm(ax, bx), fm(ay, by)), fm(az, bz));
@@ -110,13 +114,19 @@ __global__ void k_fast_generate(const FastTile* __restrict__ tiles, FastCell* __
       const float tilt = fm(rand_f32(rng), 0.20f);
       const float phi = fm(fm(rand_f32(rng), 2.0f), PI_F);
       const float half = fm(tilt, 0.5f);
-      c.rot = make_float4(fm(fsin_(half), fcos_(phi)), fm(fsin_(half), fsin_(phi)), 0.0f, fcos_(half));
+      float sh, ch, sp, cp;
+      pair_sincosf(half, sh, ch);
+      pair_sincosf(phi, sp, cp);
+      c.rot = make_float4(fm(sh, cp), fm(sh, sp), 0.0f, ch);
     } else {
       c.dims_exp = make_float4(radius, radius, radius, 0.0f);
       const float q1 = rand_f32(rng), q2 = rand_f32(rng), q3 = rand_f32(rng);
       const float a2 = fm(fm(2.0f, PI_F), q2), a3 = fm(fm(2.0f, PI_F), q3);
-      c.rot = make_float4(fm(__fsqrt_rn(fs(1.0f, q1)), fsin_(a2)), fm(__fsqrt_rn(fs(1.0f, q1)), fcos_(a2)),
-                          fm(__fsqrt_rn(q1), fsin_(a3)), fm(__fsqrt_rn(q1), fcos_(a3)));
+      float s2, c2, s3, c3;
+      pair_sincosf(a2, s2, c2);
+      pair_sincosf(a3, s3, c3);
+      c.rot = make_float4(fm(__fsqrt_rn(fs(1.0f, q1)), s2), fm(__fsqrt_rn(fs(1.0f, q1)), c2),
+                          fm(__fsqrt_rn(q1), s3), fm(__fsqrt_rn(q1), c3));
     }
     c.flags = make_uint4(1u, t.morph, 0u, 0u);
     cells[t.cell_base + i] = c;

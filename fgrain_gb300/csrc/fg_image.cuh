@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "fg_internal.h"
+#include "fg_pair.cuh"
 
 namespace fg {
 
@@ -11,15 +12,16 @@ __device__ __forceinline__ float hann_weight(uint32_t t, uint32_t g, uint32_t nt
                                             uint32_t pad) {
   const float pad2 = static_cast<float>(2 * pad);
   const float pi = 3.14159265358979323846f;
+  float s, c;
   if (t > 0 && g < o0 + pad) {
     const float u = __fdiv_rn(__fsub_rn(static_cast<float>(g), __fsub_rn(static_cast<float>(o0), static_cast<float>(pad))), pad2);
-    const float c = static_cast<float>(cos(static_cast<double>(__fmul_rn(pi, fminf(fmaxf(u, 0.0f), 1.0f)))));
+    pair_sincosf(__fmul_rn(pi, fminf(fmaxf(u, 0.0f), 1.0f)), s, c);
     return __fsub_rn(0.5f, __fmul_rn(0.5f, c));
   }
   if (t + 1 < nt && g >= o0 + step - pad) {
     const float u = __fdiv_rn(__fsub_rn(static_cast<float>(g), __fsub_rn(static_cast<float>(o0 + step), static_cast<float>(pad))),
                               pad2);
-    const float c = static_cast<float>(cos(static_cast<double>(__fmul_rn(pi, fminf(fmaxf(u, 0.0f), 1.0f)))));
+    pair_sincosf(__fmul_rn(pi, fminf(fmaxf(u, 0.0f), 1.0f)), s, c);
     return __fadd_rn(0.5f, __fmul_rn(0.5f, c));
   }
   return 1.0f;

@@ -1,0 +1,196 @@
+// Elementary functions rounded once from more than float precision, without the FP64 pipe (its rate on
+// sm_103a is far below the FP32 one): a value is evaluated as an unevaluated sum of two floats, to within
+// 2^-40.5 of its magnitude (measured against extended precision over the floats of the ranges below),
+// and rounded when every value within PAIR_ERR of it rounds to the same float; otherwise (about one
+// call in 10,000) FP64 decides.  The results are those of the FP64 function rounded to float.
+// Operations are the error-free transformations of Dekker (1971) and Knuth; the functions are their
+// Taylor series after a reduction of the argument by split constants (Cody and Waite).
+#pragma once
+#include <cmath>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace fg {
+
+#ifdef __CUDA_ARCH__
+#define PAIR_ADD(a, b) __fadd_rn(a, b)
+#define PAIR_SUB(a, b) __fsub_rn(a, b)
+#define PAIR_MUL(a, b) __fmul_rn(a, b)
+#define PAIR_FMA(a, b, c) __fmaf_rn(a, b, c)
+#else  // compiled without contraction on the host
+#define PAIR_ADD(a, b) ((a) + (b))
+#define PAIR_SUB(a, b) ((a) - (b))
+#define PAIR_MUL(a, b) ((a) * (b))
+#define PAIR_FMA(a, b, c) fmaf(a, b, c)
+#endif
+#define PAIR_FN __host__ __device__ __forceinline__
+
+struct Pair {
+  float h, l;  // |l| <= ulp(h) / 2
+};
+
+constexpr float PAIR_ERR = 3.637978807091713e-12f;  // 2^-38, relative
+
+// a + b for |a| >= |b| (or a = 0).
+PAIR_FN Pair pair_fast(float a, float b) {
+  const float s = PAIR_ADD(a, b);
+  return Pair{s, PAIR_SUB(b, PAIR_SUB(s, a))};
+}
+PAIR_FN Pair pair_sum(float a, float b) {
+  const float s = PAIR_ADD(a, b), t = PAIR_SUB(s, a);
+  return Pair{s, PAIR_ADD(PAIR_SUB(a, PAIR_SUB(s, t)), PAIR_SUB(b, t))};
+}
+PAIR_FN Pair pair_prod(float a, float b) {
+  const float p = PAIR_MUL(a, b);
+  return Pair{p, PAIR_FMA(a, b, -p)};
+}
+PAIR_FN Pair pair_add(Pair a, Pair b) {
+  const Pair s = pair_sum(a.h, b.h);
+  return pair_fast(s.h, PAIR_ADD(s.l, PAIR_ADD(a.l, b.l)));
+}
+// c + a for |c| >= |a|.
+PAIR_FN Pair pair_add(Pair c, float a) {
+  const Pair s = pair_fast(c.h, a);
+  return pair_fast(s.h, PAIR_ADD(s.l, c.l));
+}
+PAIR_FN Pair pair_mul(Pair a, Pair b) {
+  const Pair p = pair_prod(a.h, b.h);
+  return pair_fast(p.h, PAIR_FMA(a.h, b.l, PAIR_FMA(a.l, b.h, p.l)));
+}
+PAIR_FN Pair pair_mul(Pair a, float b) {
+  const Pair p = pair_prod(a.h, b);
+  return pair_fast(p.h, PAIR_FMA(a.l, b, p.l));
+}
+
+// Whether the value's rounding to float is settled; r receives it.
+PAIR_FN bool pair_round(Pair a, float& r) {
+  const float e = PAIR_MUL(fabsf(a.h), PAIR_ERR);
+  r = PAIR_ADD(a.h, PAIR_ADD(a.l, e));
+  return r == PAIR_ADD(a.h, PAIR_SUB(a.l, e));
+}
+
+// log of a positive normal float plus a low part: x = 2^k m, m in [sqrt(1/2), sqrt(2));
+// log m = 2 atanh(s), s = (m - 1) / (m + 1), |s| < .1716.
+PAIR_FN Pair pair_log(float x, float xl = 0.0f) {
+#ifdef __CUDA_ARCH__
+  const int b = __float_as_int(x);
+#else
+  union { float f; int i; } v{x};
+  const int b = v.i;
+#endif
+  const int k = (b - 0x3f3504f3) >> 23;  // 0x3f3504f3: sqrt(1/2)
+#ifdef __CUDA_ARCH__
+  const float m = __int_as_float(b - (k << 23)), up = __int_as_float((127 - k) << 23);
+#else
+  v.i = b - (k << 23);
+  const float m = v.f;
+  v.i = (127 - k) << 23;
+  const float up = v.f;
+#endif
+  const float f = PAIR_SUB(m, 1.0f), fl = PAIR_MUL(xl, up);  // f is exact
+  const Pair n = pair_fast(f, fl);
+  Pair d = pair_sum(2.0f, f);
+  d = pair_fast(d.h, PAIR_ADD(d.l, fl));
+  // s = n / d: a quotient and its remainder's.
+  const float inv = 1.0f / d.h;
+  const float q = PAIR_MUL(n.h, inv);
+  const float rem = PAIR_ADD(PAIR_FMA(-q, d.h, n.h), PAIR_FMA(-q, d.l, n.l));
+  const Pair s = pair_fast(q, PAIR_MUL(rem, inv));
+  const Pair z = pair_mul(s, s);
+  // 2 s (1 + z / 3 + z^2 / 5 + ...), z < .0295: the first two terms as pairs.
+  float p = 0.13333334f;  // 2 / 15
+  p = PAIR_FMA(p, z.h, 0.15384616f);
+  p = PAIR_FMA(p, z.h, 0.18181819f);
+  p = PAIR_FMA(p, z.h, 0.22222222f);
+  p = PAIR_FMA(p, z.h, 0.2857143f);
+  Pair t = pair_add(Pair{0.400000006f, -5.96046457e-09f}, PAIR_MUL(p, z.h));
+  t = pair_mul(t, z);
+  t = pair_add(Pair{0.666666687f, -1.98682155e-08f}, t);
+  t = pair_mul(pair_mul(t, z), s);
+  const Pair lm = pair_add(Pair{2.0f * s.h, 2.0f * s.l}, t);
+  // k log 2: the first part has 16 bits, its product is exact.
+  const float kf = static_cast<float>(k);
+  const Pair lk = pair_mul(Pair{1.42860677e-06f, 5.49792315e-14f}, kf);
+  return pair_add(pair_add(Pair{PAIR_MUL(kf, 0.693145751953125f), 0.0f}, lk), lm);
+}
+
+// exp for |x| <= 70 (the low part stays a normal float): x = k log 2 + r, |r| < .347, by the series of r / 8 and three squarings.
+PAIR_FN Pair pair_exp(float x) {
+  const float kf = rintf(PAIR_MUL(x, 1.4426950f));
+  const Pair c = pair_prod(-kf, 1.42860677e-06f);
+  Pair r = pair_sum(PAIR_FMA(-kf, 0.693145751953125f, x), c.h);
+  r = pair_fast(r.h, PAIR_ADD(r.l, PAIR_FMA(-kf, 5.49792315e-14f, c.l)));
+  r = Pair{PAIR_MUL(0.125f, r.h), PAIR_MUL(0.125f, r.l)};
+  // 1 + r + r^2 / 2 + r^3 / 6 + r^4 (1 / 24 + ...), |r| < .0434.
+  float p = 0.0013888889f;
+  p = PAIR_FMA(p, r.h, 0.008333334f);
+  p = PAIR_FMA(p, r.h, 0.041666668f);
+  Pair t = pair_add(Pair{0.166666672f, -4.96705388e-09f}, PAIR_MUL(p, r.h));
+  t = pair_add(Pair{0.5f, 0.0f}, pair_mul(t, r));
+  t = pair_add(Pair{1.0f, 0.0f}, pair_mul(t, r));
+  t = pair_add(Pair{1.0f, 0.0f}, pair_mul(t, r));
+  t = pair_mul(t, t);
+  t = pair_mul(t, t);
+  t = pair_mul(t, t);
+  const int k = static_cast<int>(kf);
+#ifdef __CUDA_ARCH__
+  const float up = __int_as_float((127 + k) << 23);
+#else
+  union { int i; float f; } v{(127 + k) << 23};
+  const float up = v.f;
+#endif
+  return Pair{PAIR_MUL(t.h, up), PAIR_MUL(t.l, up)};
+}
+
+// sin and cos for |x| <= 8: x = k pi / 2 + r, |r| <= pi / 4; the first part of pi / 2 has 20 bits, so
+// its product and the difference are exact.
+PAIR_FN void pair_sincos(float x, Pair& sn, Pair& cs) {
+  const float kf = rintf(PAIR_MUL(x, 0.63661975f));
+  const Pair c = pair_prod(-kf, 1.26759085e-06f);
+  Pair r = pair_sum(PAIR_FMA(-kf, 1.5707950592041016f, x), c.h);
+  r = pair_fast(r.h, PAIR_ADD(r.l, PAIR_FMA(-kf, -5.14531146e-14f, c.l)));
+  const Pair z = pair_mul(r, r);
+  // sin r = r + r z (S1 + z (S2 + z (S3 + ...))), cos r = 1 + z (-1/2 + z (C2 + z (C3 + ...))),
+  // z < .617: three coefficients each as pairs.
+  float p = 1.6059044e-10f;
+  p = PAIR_FMA(p, z.h, -2.5052108e-08f);
+  p = PAIR_FMA(p, z.h, 2.7557319e-06f);
+  Pair t = pair_add(Pair{-0.000198412701f, 2.72559687e-12f}, PAIR_MUL(p, z.h));
+  t = pair_add(Pair{0.00833333377f, -4.34617203e-10f}, pair_mul(t, z));
+  t = pair_add(Pair{-0.166666672f, 4.96705388e-09f}, pair_mul(t, z));
+  t = pair_mul(pair_mul(t, z), r);
+  const Pair s = pair_add(r, t);
+  p = -1.1470746e-11f;
+  p = PAIR_FMA(p, z.h, 2.0876757e-09f);
+  p = PAIR_FMA(p, z.h, -2.7557319e-07f);
+  p = PAIR_FMA(p, z.h, 2.4801588e-05f);
+  t = pair_add(Pair{-0.00138888892f, 3.36310944e-11f}, PAIR_MUL(p, z.h));
+  t = pair_add(Pair{0.0416666679f, -1.24176347e-09f}, pair_mul(t, z));
+  t = pair_add(Pair{-0.5f, 0.0f}, pair_mul(t, z));
+  const Pair q = pair_add(Pair{1.0f, 0.0f}, pair_mul(t, z));
+  const int k = static_cast<int>(kf) & 3;
+  const Pair a = k & 1 ? q : s, b = k & 1 ? s : q;
+  sn = k & 2 ? Pair{-a.h, -a.l} : a;
+  cs = (k + 1) & 2 ? Pair{-b.h, -b.l} : b;
+}
+
+// The FP64 functions rounded to float.
+PAIR_FN float pair_expf(float x) {
+  float r;
+  if (fabsf(x) <= 70.0f && pair_round(pair_exp(x), r)) return r;
+  return static_cast<float>(exp(static_cast<double>(x)));
+}
+PAIR_FN float pair_logf(float x) {
+  float r;
+  if (x >= 1.17549435e-38f && x <= 3.4028235e38f && pair_round(pair_log(x), r)) return r;
+  return static_cast<float>(log(static_cast<double>(x)));
+}
+PAIR_FN void pair_sincosf(float x, float& sn, float& cs) {
+  Pair s, c;
+  pair_sincos(x, s, c);
+  const bool in = fabsf(x) <= 8.0f;
+  if (!(in && pair_round(s, sn))) sn = static_cast<float>(sin(static_cast<double>(x)));
+  if (!(in && pair_round(c, cs))) cs = static_cast<float>(cos(static_cast<double>(x)));
+}
+
+}  // namespace fg

@@ -2,6 +2,7 @@
 #include <type_traits>
 
 #include "fg_internal.h"
+#include "fg_pair.cuh"
 #include "fg_scan.cuh"
 
 namespace fg {
@@ -740,16 +741,24 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* _
   }
 }
 
-// d = -log10(clamp(T, 1e-4, 1)) + 0.05 in FP64 (image_pipeline.rs:1007-1011), in place over the
-// pixels' mean transmittance.  A pass of its own so that every lane of a warp converts a pixel:
-// inside k_scan only one thread per pixel (of spp) would, and each FP64 instruction would occupy
-// GB300's narrow FP64 pipe for a whole warp.
+// d = -log10(clamp(T, 1e-4, 1)) + 0.05 as FP64 rounded to float (image_pipeline.rs:1007-1011), in
+// place over the pixels' mean transmittance; evaluated as a pair of floats, FP64 where that does not
+// settle the rounding (4.2 M px: 400 us in FP64 alone).
+// A pass of its own so that every lane of a warp converts a pixel: inside k_scan only one thread per
+// pixel (of spp) would.
 __global__ void k_density(float* __restrict__ d, unsigned long long n) {
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   for (unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; i < n;
        i += stride) {
-    const double tc = fmin(fmax(static_cast<double>(d[i]), 1e-4), 1.0);
-    d[i] = static_cast<float>(-log10(tc) + 0.05);
+    const float T = d[i];
+    float r;
+    const bool in = T > 1.0001e-4f && T <= 1.0f;
+    const Pair v = pair_add(pair_mul(pair_log(in ? T : 1.0f), Pair{-0.434294492f, 1.010305e-08f}), Pair{0.0500000007f, -7.45058071e-10f});
+    if (!(in && pair_round(v, r))) {
+      const double tc = fmin(fmax(static_cast<double>(T), 1e-4), 1.0);
+      r = tc == 1e-4 ? 4.05f : (tc == 1.0 ? 0.05f : static_cast<float>(-log10(tc) + 0.05));
+    }
+    d[i] = r;
   }
 }
 
