@@ -76,11 +76,14 @@ __global__ void __launch_bounds__(256, 4) k_transport(const TileDesc* __restrict
           if (move) cells_advance(g, ph.pos, ph.dir, inv_y, inv_z, v, err);
         } else if (test) {
           const uint32_t p = v.c;
-          const bool two = p + 1 < v.cend && nq + 1 < CELL_LIST;
-          const float4 a = __ldg(&g.pos[p]), b = __ldg(&g.pos[two ? p + 1 : p]);
-          if (cell_near(a, ph.pos, ph.dir, v.step)) s_rank[nq++][tid] = p;
-          if (two && cell_near(b, ph.pos, ph.dir, v.step)) s_rank[nq++][tid] = p + 1;
-          v.c = p + 1 + (two ? 1u : 0u);
+          const uint32_t m = min(min(v.cend - p, CELL_TEST), CELL_LIST - nq);
+          float4 a[CELL_TEST];
+#pragma unroll
+          for (uint32_t j = 0; j < CELL_TEST; ++j) a[j] = __ldg(&g.pos[j < m ? p + j : p]);
+#pragma unroll
+          for (uint32_t j = 0; j < CELL_TEST; ++j)
+            if (j < m && cell_near(a[j], ph.pos, ph.dir, v.step)) s_rank[nq++][tid] = p + j;
+          v.c = p + m;
         }
       }
     }

@@ -7,9 +7,10 @@
 
 namespace fg {
 
-constexpr int CELL_HITS = 12;     // hits of a segment absorbed per visit (the rest: visited again)
-constexpr int CELL_LIST = 16;     // hits and listed crystals of a lane
-constexpr int CELL_WAIT = 26;     // waiting lanes of a warp that resolve together
+constexpr int CELL_HITS = 12;      // hits of a segment absorbed per visit (the rest: visited again)
+constexpr int CELL_LIST = 16;      // hits and listed crystals of a lane
+constexpr uint32_t CELL_TEST = 4;  // crystals of a row that a lane tests in one step (2: 6 % slower, 6: the same)
+constexpr int CELL_WAIT = 28;      // waiting lanes of a warp that resolve together
 constexpr int WALK_LEAVES = 6;    // leaves a lane may hold while its warp still walks (speculative traversal)
 constexpr int WALK_RESTART = 24;  // idle lanes of a warp that end and start their bounces together
 constexpr int WALK_EMPTY = INT32_MIN;
