@@ -28,9 +28,9 @@ void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], 
                     uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, int sms, uint32_t wait_limit = 0,
                     const uint32_t* probe = nullptr);
 size_t bridson_smem(int gdmax);
-void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_cells, unsigned long long max_slots,
-                       uint32_t* cells, uint32_t* npts, uint32_t* flags, cudaStream_t st);
-void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_slots, const uint32_t* cells,
+void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_parts, uint32_t* cells,
+                       const uint32_t* npts, uint32_t* counts, cudaStream_t st);
+void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_parts, const uint32_t* cells,
                  const uint32_t* scan, float4* A, float4* Q, float4* D, uint64_t* keys, uint32_t* err,
                  cudaStream_t st);
 void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long long total,
@@ -78,7 +78,7 @@ __global__ void k_set_n(const SynthTile* syn, int ntiles, const uint32_t* slot_s
                         ScanTile* sc, uint32_t* ncrys, RTile* rt) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntiles) return;
-  const uint32_t n = slot_scan[syn[t].slot_base + (1ull << (2 * syn[t].slot_bits))] - slot_scan[syn[t].slot_base];
+  const uint32_t n = slot_scan[syn[t].slot_base + syn_parts(syn[t])] - slot_scan[syn[t].slot_base];
   const uint32_t nn = min(n, syn[t].ccap);
   bt[t].n = nn;
   bt[t].max_base = 0.0;
@@ -307,13 +307,13 @@ struct fg_batch {
   DBuf<TileDesc> d_td;
   DBuf<ScanTile> d_sc;
   DBuf<BTile> d_bt;
-  DBuf<uint32_t> cells, npts, flags, slot_scan, ncrys;  // flags: points per brick, slot_scan: their exclusive sum
+  DBuf<uint32_t> cells, npts, flags, slot_scan, ncrys;  // flags: points per part, slot_scan: their exclusive sum
   DBuf<uint32_t> coldone;  // one flag per synthesis column
   DBuf<uint32_t> probe;    // the failure drill's flag (zero, never set)
   uint32_t wait_limit = 0;
   bool wait_probe = false;
   bool key32 = true;       // every crystal is finite: the tree's centroids are the positions
-  unsigned long long maxcells = 0, maxslots = 0;  // the largest tile's cells and bricks
+  unsigned long long maxparts = 0;  // the largest tile's
   DBuf<float4> A, Q, D;
   CellBufs tcells;          // the crystals in cells, with their rank in the tree's walk order
   DBuf<uint64_t> keys;
@@ -333,7 +333,7 @@ struct fg_batch {
   DBuf<unsigned long long> dstats;  // [0] transport hits, [1] scan FP64 fallbacks, [2] scan hits, [3] clumps
   DBuf<unsigned char> cub_tmp;
   size_t cub_bytes = 0;
-  unsigned long long ncells = 0, nslots = 0, ncap = 0, nbins = 0, item_cap = 0, photons = 0, rays = 0;  // nslots: bricks
+  unsigned long long ncells = 0, nparts = 0, ncap = 0, nbins = 0, item_cap = 0, photons = 0, rays = 0;  // nparts: of slots
   unsigned long long exp_total = 0, out_total = 0;
   int gdmax = 0;
   unsigned cols[4] = {0, 0, 0, 0};
@@ -547,10 +547,10 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
   launch_bridson(B->d_syn.p, nt, B->cols, B->gdmax, B->cells.p, B->npts.p, B->coldone.p, e->d_err, st,
                  e->sm_count, B->wait_limit, B->wait_probe ? B->probe.p : nullptr);
   mark(B->ev[7], st, capturing);
-  FG_CUDA(cudaMemsetAsync(B->flags.p + B->nslots, 0, sizeof(uint32_t), st));
-  launch_synth_post(B->d_syn.p, nt, B->maxcells, B->maxslots, B->cells.p, B->npts.p, B->flags.p, st);
-  cub_scan(B, B->flags.p, B->slot_scan.p, B->nslots + 1, st);
-  launch_emit(B->d_syn.p, nt, B->maxslots, B->cells.p, B->slot_scan.p, B->A.p, B->Q.p, B->D.p, B->keys.p, e->d_err,
+  FG_CUDA(cudaMemsetAsync(B->flags.p + B->nparts, 0, sizeof(uint32_t), st));
+  launch_synth_post(B->d_syn.p, nt, B->maxparts, B->cells.p, B->npts.p, B->flags.p, st);
+  cub_scan(B, B->flags.p, B->slot_scan.p, B->nparts + 1, st);
+  launch_emit(B->d_syn.p, nt, B->maxparts, B->cells.p, B->slot_scan.p, B->A.p, B->Q.p, B->D.p, B->keys.p, e->d_err,
               st);
   k_set_n<<<grid_for(B->ntiles, 128), 128, 0, st>>>(B->d_syn.p, nt, B->slot_scan.p, B->d_bt.p, B->d_td.p, B->d_sc.p,
                                                     B->ncrys.p, B->rt.tiles.p);
@@ -734,9 +734,8 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       colc[c] += cxn * cyn;
     }
     cb += static_cast<unsigned long long>(s.gw) * s.gh * s.gd;
-    sb += 1ull << (2 * s.slot_bits);  // bricks
-    B->maxcells = std::max<unsigned long long>(B->maxcells, static_cast<unsigned long long>(s.gw) * s.gh * s.gd);
-    B->maxslots = std::max<unsigned long long>(B->maxslots, 1ull << (2 * s.slot_bits));
+    sb += syn_parts(s);
+    B->maxparts = std::max<unsigned long long>(B->maxparts, syn_parts(s));
     cap += s.ccap;
     B->td[i].photon_base = pb;
     pb += B->td[i].P;
@@ -759,7 +758,7 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   FG_REQUIRE(cap < 0x7fffffffull, "batch too large: more than 2^31 crystal slots");
   FG_REQUIRE(bridson_smem(B->gdmax) <= 220 * 1024, "emulsion too deep for the synthesis column");
   B->ncells = cb;
-  B->nslots = sb;
+  B->nparts = sb;
   B->ncap = cap;
   B->photons = pb;
   B->exp_total = eo;
@@ -897,9 +896,9 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   // Per crystal slot: records 48 (and 96 in the transport's cells), key 8, links and flags 36,
   // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
-  // 152 B (plus slack); transport cells 8 B; synthesis cells 4 B; bricks 8 B; photon order; images.
+  // 152 B (plus slack); transport cells 8 B; synthesis cells 4 B; parts 8 B; photon order; images.
   return static_cast<unsigned long long>(s.ccap) * 620ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
-         (8ull << (2 * s.slot_bits)) + static_cast<unsigned long long>(t.P) * 4ull +
+         8ull * syn_parts(s) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
 
@@ -948,20 +947,20 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
     DBuf<SynthTile> d_syn(1, st);
     FG_CUDA(cudaMemcpyAsync(d_syn.p, &s, sizeof(SynthTile), cudaMemcpyHostToDevice, st));
-    const unsigned long long nbr = 1ull << (2 * s.slot_bits);  // bricks
-    DBuf<uint32_t> cells(ncells, st), npts(1, st), flags(nbr + 1ull, st), scan(nbr + 1ull, st);
+    const unsigned long long np = syn_parts(s);
+    DBuf<uint32_t> cells(ncells, st), npts(1, st), flags(np + 1ull, st), scan(np + 1ull, st);
     DBuf<float4> A(s.ccap, st), Q(s.ccap, st), D(s.ccap, st);
     DBuf<uint64_t> keys(s.ccap, st);
     FG_CUDA(cudaMemsetAsync(cells.p, 0, ncells * sizeof(uint32_t), st));
     FG_CUDA(cudaMemsetAsync(npts.p, 0, sizeof(uint32_t), st));
     DBuf<uint32_t> coldone(std::max(cols[0] + cols[1] + cols[2] + cols[3], 1u), st);
     launch_bridson(d_syn.p, 1, cols, gdmax, cells.p, npts.p, coldone.p, e->d_err, st, e->sm_count);
-    FG_CUDA(cudaMemsetAsync(flags.p + nbr, 0, sizeof(uint32_t), st));
-    launch_synth_post(d_syn.p, 1, ncells, nbr, cells.p, npts.p, flags.p, st);
-    exclusive_scan_u32(flags.p, scan.p, nbr + 1ull, st);
-    launch_emit(d_syn.p, 1, nbr, cells.p, scan.p, A.p, Q.p, D.p, keys.p, e->d_err, st);
+    FG_CUDA(cudaMemsetAsync(flags.p + np, 0, sizeof(uint32_t), st));
+    launch_synth_post(d_syn.p, 1, np, cells.p, npts.p, flags.p, st);
+    exclusive_scan_u32(flags.p, scan.p, np + 1ull, st);
+    launch_emit(d_syn.p, 1, np, cells.p, scan.p, A.p, Q.p, D.p, keys.p, e->d_err, st);
     uint32_t n = 0;
-    FG_CUDA(cudaMemcpyAsync(&n, scan.p + nbr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    FG_CUDA(cudaMemcpyAsync(&n, scan.p + np, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     FG_CUDA(cudaStreamSynchronize(st));
     check_error_word(e);
     n = std::min(n, s.ccap);
@@ -1151,12 +1150,12 @@ fg_status fg_batch_wait(fg_batch* b, fg_batch_stats* stats) {
     s.transport_blocks = b->tr_blocks;
     s.scan_bin_px = b->bin_px;
     s.graph = b->exec ? 1u : 0u;
-    // Own kernels per run: Bridson (all colour classes in one launch; it also counts the points), thin +
-    // brick counts, emit, set_n, photon order x2, transport, maxdim + threshold + developed list + link +
+    // Own kernels per run: Bridson (all colour classes in one launch; it also counts the points), thinning
+    // with the part counts, emit, set_n, photon order x2, transport, maxdim + threshold + developed list + link +
     // roots + finalize, scan-tree inputs, scan prep, two bin passes, scan, density, the two passes over the
     // transport's cells, and the two tree builds (each level's launches included, also those that
     // find no work; CUB scans not counted).
-    s.kernel_launches = 1 + 2 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt, false);
+    s.kernel_launches = 1 + 1 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt, false);
     b->stats = s;
     if (stats) *stats = s;
   });

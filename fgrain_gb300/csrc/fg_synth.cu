@@ -578,48 +578,6 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
   }
 }
 
-// Independent deletion down to the Bridson-expected count: each point goes with probability p,
-// drawn from the Philox block of its cell.  blockIdx.y is the tile (the points per tile were
-// counted by k_bridson).  Each warp reads 32 cells at a time and queues the occupied ones; the
-// draws run once 32 are queued, with every lane busy.
-constexpr int THIN_T = 256;
-__global__ void __launch_bounds__(THIN_T) k_thin(const SynthTile* __restrict__ tiles, uint32_t* __restrict__ cells,
-                                                 const uint32_t* npts) {
-  const SynthTile& t = tiles[blockIdx.y];
-  const uint32_t n = npts[blockIdx.y];
-  if (n <= t.target) return;
-  const float p = 1.0f - static_cast<float>(t.target) / static_cast<float>(n);
-  const uint32_t nc = t.gw * t.gh * t.gd;
-  uint32_t* tc = cells + t.cell_base;
-  const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-  __shared__ uint32_t s_q[THIN_T / 32][64];
-  uint32_t* q = s_q[threadIdx.x >> 5];
-  uint32_t fill = 0;  // the same in every lane of the warp
-  auto thin = [&](uint32_t lin) {
-    if (uf(philox(lin, 0, 0, TAG_THIN, t.k0, t.k1).x) < p) tc[lin] = 0;
-  };
-  const uint32_t warps = gridDim.x * (THIN_T / 32);
-  for (uint32_t base = (blockIdx.x * THIN_T + threadIdx.x - lane); base < nc; base += warps * 32) {
-    const uint32_t lin = base + lane;
-    const bool occ = lin < nc && (tc[lin] & OCC);
-    const unsigned m = __ballot_sync(0xffffffffu, occ);
-    if (occ) q[fill + __popc(m & lt)] = lin;
-    fill += __popc(m);
-    __syncwarp();
-    if (fill >= 32) {
-      const uint32_t mine = q[lane];
-      const uint32_t rest = fill - 32;
-      const uint32_t moved = lane < rest ? q[32 + lane] : 0u;
-      __syncwarp();
-      if (lane < rest) q[lane] = moved;
-      fill = rest;
-      __syncwarp();
-      thin(mine);
-    }
-  }
-  if (lane < fill) thin(q[lane]);
-}
-
 // Cell of compaction slot sl: the brick (2D Morton over the high x, y bits) in the bits above
 // 3 * brick_bits, the cell inside it (3D Morton, x lowest) below.
 __device__ __forceinline__ void slot_cell(const SynthTile& t, uint32_t sl, uint32_t& x, uint32_t& y, uint32_t& z) {
@@ -630,33 +588,107 @@ __device__ __forceinline__ void slot_cell(const SynthTile& t, uint32_t sl, uint3
   z = morton3_compact(lo >> 2);
 }
 
-// Points per brick (the compaction unit): one block per brick counts the occupied cells of its
-// region, read row by row.  blockIdx.y is the tile.
-__global__ void k_brick_count(const SynthTile* __restrict__ tiles, const uint32_t* __restrict__ cells,
-                              uint32_t* counts) {
+// A part's cells as a warp reads them, word j of 16, one cell a lane.  A part of a brick of 8 cells or
+// more is a cube of 8 x 8 x 8, read in rows of 8 (a sector) and not in slot order; of a smaller brick,
+// 512 consecutive slots.
+struct PartCells {
+  bool cube, in;               // in: some cells lie inside the grid (its first slot, the lowest corner, does)
+  uint32_t lin, row4, layer;   // cube: the lane's cell of word 0 (linear index), steps of 4 rows, of a layer
+  uint32_t words;              // cube: bit j: the lane's cell of word j is inside the grid
+};
+__device__ __forceinline__ PartCells part_cells(const SynthTile& t, uint32_t p, uint32_t lane) {
+  PartCells c;
+  uint32_t x, y, z;
+  slot_cell(t, p * SYN_PART, x, y, z);
+  c.in = x < t.gw && y < t.gh && z < t.gd;
+  c.cube = t.brick_bits >= 3;
+  x += lane & 7u;
+  y += lane >> 3;
+  c.row4 = 4u * t.gw;
+  c.layer = t.gh * t.gw;
+  c.lin = z * c.layer + y * t.gw + x;
+  const uint32_t nz = min(t.gd - z, 8u);  // layers inside
+  c.words = x >= t.gw ? 0u
+                      : (y < t.gh ? 0x5555u : 0u) & ((1u << (2 * nz)) - 1u) |
+                            (y + 4u < t.gh ? 0xaaaau : 0u) & ((1u << (2 * nz)) - 1u);
+  return c;
+}
+// The linear index of the lane's cell of word j, NO_CELL outside the grid; its slot in the part.
+constexpr uint32_t NO_CELL = 0xffffffffu;
+__device__ __forceinline__ uint32_t part_cell(const SynthTile& t, const PartCells& c, uint32_t p, uint32_t j, uint32_t lane) {
+  if (c.cube) return (c.words >> j) & 1u ? c.lin + (j & 1u) * c.row4 + (j >> 1) * c.layer : NO_CELL;
+  uint32_t x, y, z;
+  const uint32_t sl = p * SYN_PART + j * 32 + lane;
+  slot_cell(t, sl, x, y, z);
+  return sl < t.slots && x < t.gw && y < t.gh && z < t.gd ? (z * t.gh + y) * t.gw + x : NO_CELL;
+}
+__device__ __forceinline__ uint32_t part_slot(const PartCells& c, uint32_t j, uint32_t lane) {
+  if (!c.cube) return j * 32 + lane;
+  const uint32_t x = lane & 7u, y = lane >> 3, z = j >> 1;
+  return (x & 1u) | (x & 2u) << 2 | (x & 4u) << 4 | (y & 1u) << 1 | (y & 2u) << 3 | (j & 1u) << 7 | (z & 1u) << 2 |
+         (z & 2u) << 4 | (z & 4u) << 6;
+}
+// Bit j: the lane's cell of word j holds a point (the loads are in flight together).
+__device__ __forceinline__ uint32_t part_points(const SynthTile& t, const PartCells& c, const uint32_t* tc, uint32_t p,
+                                                uint32_t lane) {
+  uint32_t occ = 0;
+  if (c.cube) {
+#pragma unroll
+    for (uint32_t j = 0; j < SYN_PART / 32; ++j)
+      occ |= ((c.words >> j) & 1u ? tc[c.lin + (j & 1u) * c.row4 + (j >> 1) * c.layer] >> 31 : 0u) << j;
+  } else {
+    for (uint32_t j = 0; j < SYN_PART / 32; ++j) {
+      const uint32_t lin = part_cell(t, c, p, j, lane);
+      occ |= (lin != NO_CELL ? tc[lin] >> 31 : 0u) << j;
+    }
+  }
+  return occ;
+}
+
+// Thinning to the Bridson-expected count (a point goes with the probability of the excess, n points as
+// counted by k_bridson), and the points left per part, a warp to a part.  The draws run over the
+// part's points, with the lanes busy.  blockIdx.y is the tile.
+//
+// Bound by the latency of its loads (DRAM 15 %).  A pass for thinning and one for the counts, a block to
+// a brick of up to 32^3 cells, took 320 + 420 us on a 1600 x 1600 px t-max image, this one 438; for the
+// four bricks of a 64 x 64 px tri-x tile 3.5 + 24 us, now 7.4.
+constexpr int PART_T = 256;
+__global__ void __launch_bounds__(PART_T) k_thin_count(const SynthTile* __restrict__ tiles, uint32_t* __restrict__ cells,
+                                                       const uint32_t* __restrict__ npts, uint32_t* __restrict__ counts) {
   const SynthTile& t = tiles[blockIdx.y];
-  const uint32_t L = t.brick_bits, E = 1u << L;
-  const uint32_t nbricks = 1u << (2 * t.slot_bits);
-  const uint32_t* tc = cells + t.cell_base;
-  __shared__ uint32_t s_sum[32];
-  for (uint32_t b = blockIdx.x; b < nbricks; b += gridDim.x) {
-    const uint32_t xb = morton2_compact(b) << L, yb = morton2_compact(b >> 1) << L;
-    const uint32_t ex = xb < t.gw ? min(E, t.gw - xb) : 0u, ey = yb < t.gh ? min(E, t.gh - yb) : 0u;
-    const uint32_t ez = min(E, t.gd), n = ex * ey * ez;
-    uint32_t c = 0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const uint32_t x = xb + i % ex, y = yb + (i / ex) % ey, z = i / (ex * ey);
-      c += (tc[(static_cast<size_t>(z) * t.gh + y) * t.gw + x] & OCC) ? 1u : 0u;
+  const uint32_t nparts = syn_parts(t), lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  const uint32_t n = npts[blockIdx.y];
+  const bool thin = n > t.target;
+  const float excess = 1.0f - static_cast<float>(t.target) / static_cast<float>(n);
+  uint32_t* tc = cells + t.cell_base;
+  __shared__ uint32_t s_q[PART_T / 32][SYN_PART];  // the part's points
+  uint32_t* q = s_q[threadIdx.x >> 5];
+  for (uint32_t p = blockIdx.x * (PART_T / 32) + (threadIdx.x >> 5); p < nparts; p += gridDim.x * (PART_T / 32)) {
+    const PartCells c = part_cells(t, p, lane);
+    uint32_t left = 0;
+    if (c.in) {
+      const uint32_t occ = part_points(t, c, tc, p, lane);
+      left = __popc(occ);
+      if (thin) {
+        uint32_t fill = 0;
+        for (uint32_t j = 0; j < SYN_PART / 32; ++j) {
+          const unsigned m = __ballot_sync(0xffffffffu, (occ >> j) & 1u);
+          if ((occ >> j) & 1u) q[fill + __popc(m & lt)] = part_cell(t, c, p, j, lane);
+          fill += __popc(m);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < fill; i += 32) {
+          const uint32_t lin = q[i];
+          if (uf(philox(lin, 0, 0, TAG_THIN, t.k0, t.k1).x) < excess) {
+            tc[lin] = 0;
+            --left;
+          }
+        }
+        __syncwarp();
+      }
+      left = __reduce_add_sync(0xffffffffu, left);
     }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t tot = 0;
-      for (uint32_t w = 0; w < (blockDim.x + 31) / 32; ++w) tot += s_sum[w];
-      counts[t.slot_base + b] = tot;
-    }
-    __syncthreads();
+    if (lane == 0) counts[t.slot_base + p] = left;
   }
 }
 
@@ -708,73 +740,74 @@ __device__ __forceinline__ void emit_crystal(const SynthTile& t, const uint32_t*
   keys[o] = sl;
 }
 
-// The crystals of each brick in slot order (slot_cell): the brick's slots are walked in chunks of
-// the block, a block-wide prefix sum of the occupied ones numbers them after the points of the
-// earlier bricks (scan: exclusive sum of k_brick_count).  About one cell in nine holds a point,
-// so the numbered crystals are queued in shared memory and made once the queue holds a block's
-// worth, with every lane busy.  blockIdx.y is the tile.
-constexpr int EMIT_T = 256;
-__global__ void __launch_bounds__(EMIT_T) k_emit(const SynthTile* __restrict__ tiles,
+// The crystals of each part in slot order (slot_cell), numbered after the points of the earlier parts
+// (scan: exclusive sum of k_thin_count).  A warp to a part, without the block's barriers: a part's words
+// are loaded together, and as about one cell in nine holds a point, the warp queues the occupied ones
+// and makes 32 crystals at a time, with every lane busy; the queue outlives the part.
+// blockIdx.y is the tile.
+//
+// Bound by the latency of its loads.  A block to a brick, with its barriers, took 85 us for the four
+// bricks of a 64 x 64 px tri-x tile (now 9.8), 475 us for a 2048 x 2048 px image (now 213) and 1,100 us for
+// 1600 x 1600 px of t-max (now 683).
+__global__ void __launch_bounds__(PART_T) k_emit(const SynthTile* __restrict__ tiles,
                                                  const uint32_t* __restrict__ cells,
                                                  const uint32_t* __restrict__ scan, float4* A, float4* Q,
                                                  float4* D, uint64_t* keys, uint32_t* err) {
   const SynthTile& t = tiles[blockIdx.y];
-  const uint32_t L = t.brick_bits;
-  const uint32_t nbricks = 1u << (2 * t.slot_bits), per = 1u << (3 * L);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr uint32_t NW = EMIT_T / 32;
-  __shared__ uint32_t s_w[NW + 1];
-  __shared__ uint32_t s_k[2 * EMIT_T], s_sl[2 * EMIT_T];  // queued crystals: number and slot
-  uint32_t fill = 0;                                      // queue length (the same in every thread)
-  auto drain = [&]() {
-    for (uint32_t i = threadIdx.x; i < fill; i += EMIT_T) {
-      const uint32_t sl = s_sl[i], k = s_k[i];
-      if (k >= t.ccap) continue;  // past the tile's capacity (flagged when queued)
-      uint32_t x, y, z;
-      slot_cell(t, sl, x, y, z);
-      emit_crystal(t, cells, sl, x, y, z, k, A, Q, D, keys);
+  const uint32_t nparts = syn_parts(t);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const uint32_t* tc = cells + t.cell_base;
+  const uint32_t kbase = scan[t.slot_base];
+  __shared__ uint2 s_q[PART_T / 32][64];             // queued crystals: number and slot
+  __shared__ uint32_t s_m[PART_T / 32][SYN_PART / 32];  // the part's points in slot order
+  uint32_t* pts = s_m[warp];
+  uint2* q = s_q[warp];
+  uint32_t fill = 0;  // the same in every lane
+  auto emit = [&](uint2 c) {
+    if (c.x >= t.ccap) {  // past the tile's capacity
+      atomicOr(err, ERR_LIST_OVERFLOW);
+      return;
     }
-    fill = 0;
-    __syncthreads();
+    uint32_t x, y, z;
+    slot_cell(t, c.y, x, y, z);
+    emit_crystal(t, cells, c.y, x, y, z, c.x, A, Q, D, keys);
   };
-  for (uint32_t b = blockIdx.x; b < nbricks; b += gridDim.x) {
-    const unsigned long long bi = t.slot_base + b;
-    if (scan[bi + 1] == scan[bi]) continue;  // block-uniform
-    uint32_t k0 = scan[bi] - scan[t.slot_base];
-    const uint32_t xb = morton2_compact(b) << L, yb = morton2_compact(b >> 1) << L;
-    for (uint32_t c0 = 0; c0 < per; c0 += EMIT_T) {
-      const uint32_t lo = c0 + threadIdx.x;
-      const uint32_t x = xb | morton3_compact(lo), y = yb | morton3_compact(lo >> 1), z = morton3_compact(lo >> 2);
-      const bool occ = lo < per && x < t.gw && y < t.gh && z < t.gd &&
-                       (cells[t.cell_base + (static_cast<size_t>(z) * t.gh + y) * t.gw + x] & OCC);
-      const unsigned m = __ballot_sync(0xffffffffu, occ);
-      if (lane == 0) s_w[warp] = __popc(m);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (uint32_t w = 0; w < NW; ++w) {
-          const uint32_t v = s_w[w];
-          s_w[w] = acc;
-          acc += v;
-        }
-        s_w[NW] = acc;
+  for (uint32_t p = blockIdx.x * (PART_T / 32) + warp; p < nparts; p += gridDim.x * (PART_T / 32)) {
+    const uint32_t k0 = scan[t.slot_base + p];
+    if (scan[t.slot_base + p + 1] == k0) continue;
+    uint32_t k = k0 - kbase;
+    const PartCells c = part_cells(t, p, lane);
+    const uint32_t occ = part_points(t, c, tc, p, lane);
+    if (lane < SYN_PART / 32) pts[lane] = 0;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t j = 0; j < SYN_PART / 32; ++j)
+      if ((occ >> j) & 1u) {
+        const uint32_t sl = part_slot(c, j, lane);
+        atomicOr(pts + (sl >> 5), 1u << (sl & 31u));
       }
-      __syncthreads();
-      if (occ) {
-        const uint32_t r = s_w[warp] + __popc(m & ((1u << lane) - 1u));
-        const uint32_t k = k0 + r;
-        if (k >= t.ccap) atomicOr(err, ERR_LIST_OVERFLOW);
-        s_k[fill + r] = k;
-        s_sl[fill + r] = (b << (3 * L)) | lo;
+    __syncwarp();
+    for (uint32_t j = 0; j < SYN_PART / 32; ++j) {
+      const unsigned m = pts[j];
+      const bool o = (m >> lane) & 1u;
+      const uint32_t r = __popc(m & lt);
+      if (o) q[fill + r] = make_uint2(k + r, p * SYN_PART + j * 32 + lane);
+      k += __popc(m);
+      fill += __popc(m);
+      __syncwarp();
+      if (fill >= 32) {
+        const uint2 mine = q[lane];
+        const uint32_t rest = fill - 32;
+        const uint2 moved = lane < rest ? q[32 + lane] : make_uint2(0u, 0u);
+        __syncwarp();
+        if (lane < rest) q[lane] = moved;
+        fill = rest;
+        __syncwarp();
+        emit(mine);
       }
-      const uint32_t got = s_w[NW];
-      k0 += got;
-      fill += got;
-      __syncthreads();
-      if (fill >= EMIT_T) drain();
     }
   }
-  drain();
+  if (lane < fill) emit(q[lane]);
 }
 
 }  // namespace fg
@@ -806,25 +839,24 @@ size_t bridson_smem(int gdmax) {
          static_cast<size_t>(SYN_B) * SYN_B * gdmax * sizeof(uint16_t);
 }
 
-// Per-tile grids (blockIdx.y is the tile): max_cells and max_bricks are the largest tile's.
-void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_cells, unsigned long long max_bricks,
-                       uint32_t* cells, uint32_t* npts, uint32_t* counts, cudaStream_t st) {
+static unsigned part_blocks(unsigned long long max_parts) {
+  return static_cast<unsigned>(std::min<unsigned long long>((max_parts + PART_T / 32 - 1) / (PART_T / 32), 4096));
+}
+// Per-tile grids (blockIdx.y is the tile): max_parts: the largest tile's.
+void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_parts, uint32_t* cells,
+                       const uint32_t* npts, uint32_t* counts, cudaStream_t st) {
   if (ntiles == 0) return;
   FG_REQUIRE(ntiles <= 65535, "too many tiles for one launch");
-  const unsigned bc = static_cast<unsigned>(std::min<unsigned long long>(std::max(grid_for(max_cells, 256), 1u), 1024));
-  const unsigned bb = static_cast<unsigned>(std::min<unsigned long long>(std::max(max_bricks, 1ull), 4096));
-  k_thin<<<dim3(bc, ntiles), THIN_T, 0, st>>>(tiles, cells, npts);
-  k_brick_count<<<dim3(bb, ntiles), 256, 0, st>>>(tiles, cells, counts);
+  k_thin_count<<<dim3(part_blocks(max_parts), ntiles), PART_T, 0, st>>>(tiles, cells, npts, counts);
   FG_CUDA(cudaGetLastError());
 }
 
-void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_bricks, const uint32_t* cells,
+void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_parts, const uint32_t* cells,
                  const uint32_t* scan, float4* A, float4* Q, float4* D, uint64_t* keys, uint32_t* err,
                  cudaStream_t st) {
   if (ntiles == 0) return;
   FG_REQUIRE(ntiles <= 65535, "too many tiles for one launch");
-  const unsigned bb = static_cast<unsigned>(std::min<unsigned long long>(std::max(max_bricks, 1ull), 4096));
-  k_emit<<<dim3(bb, ntiles), EMIT_T, 0, st>>>(tiles, cells, scan, A, Q, D, keys, err);
+  k_emit<<<dim3(part_blocks(max_parts), ntiles), PART_T, 0, st>>>(tiles, cells, scan, A, Q, D, keys, err);
   FG_CUDA(cudaGetLastError());
 }
 

@@ -47,7 +47,7 @@ __host__ __device__ inline double bridson_density(double W, double H, double D, 
 
 struct __align__(16) SynthTile {
   unsigned long long cell_base;  // first cell of this tile in the batch grid
-  unsigned long long slot_base;  // first brick of this tile in the batch's brick counts
+  unsigned long long slot_base;  // first part of this tile in the batch's part counts
   unsigned long long cbase;      // first crystal slot
   uint32_t gw, gh, gd;           // cell grid
   uint32_t nbx, nby;             // columns per axis
@@ -70,5 +70,10 @@ struct __align__(16) SynthTile {
   float aspect;                  // tabular aspect ratio
   int morph;
 };
+
+// The compaction counts and emits crystals by parts of 512 consecutive slots (8 x 8 x 8 cells of a brick
+// of that size or more), a warp to a part.
+constexpr uint32_t SYN_PART = 512;
+__host__ __device__ inline uint32_t syn_parts(const SynthTile& t) { return (t.slots + SYN_PART - 1) / SYN_PART; }
 
 }  // namespace fg

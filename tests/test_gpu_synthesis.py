@@ -56,3 +56,33 @@ def test_points_do_not_depend_on_the_columns_in_flight(engine, stock, grain):
         b.close()
     for k in both[0]:
         np.testing.assert_array_equal(both[0][k], both[1][k])
+
+
+# Depths of 1 .. 33 cells: bricks of 1 to 64 cells an edge, whose slots the compaction takes 512 at a time.
+@pytest.mark.parametrize("cells", [(70.0, 45.3, 1.0), (41.0, 77.2, 1.9), (50.0, 33.3, 3.5), (9.0, 70.0, 7.6),
+                                   (61.0, 40.0, 14.0), (35.5, 66.0, 19.0), (40.0, 30.0, 33.0)])
+def test_crystals_come_in_slot_order(engine, cells):
+    cfg = fg.EmulsionConfig(tuple(c * CELL for c in cells), 1.0, 0.4, 0.2)
+    # The density model's count against the capacity of a film: the thinnest exceeds it and is refused.
+    vol = np.prod([c * CELL for c in cells])
+    target = (0.57793168 + 0.11306788 * sum(2 / (c * CELL) for c in cells)) * vol
+    if target > 0.8 * vol + 64 + 4 * np.sqrt(0.01 * target):
+        with pytest.raises(fg.GpuError, match="overflow"):
+            fg.VirtualEmulsionLayer.synthesize(cfg, 9, engine)
+        return
+    em = fg.VirtualEmulsionLayer.synthesize(cfg, 9, engine)
+    pos = em.crystals()["pos"].astype(np.float64)
+    em.close()
+    # Points are whole 1/1024ths of a cell, rounded to float.
+    c = np.rint(pos * 1024 / CELL).astype(np.int64) >> 10
+    grid = [int(np.ceil(x)) for x in cells]
+    assert len(c) > 20 and (c < grid).all()
+    depth_bits = max(grid[2] - 1, 0).bit_length()
+
+    def spread(v, step):
+        return sum(((v >> b) & 1) << (step * b) for b in range(12))
+
+    lo, hi = c & ((1 << depth_bits) - 1), c >> depth_bits
+    slot = ((spread(hi[:, 0], 2) | spread(hi[:, 1], 2) << 1) << (3 * depth_bits)
+            | spread(lo[:, 0], 3) | spread(lo[:, 1], 3) << 1 | spread(lo[:, 2], 3) << 2)
+    assert (np.diff(slot) > 0).all()
