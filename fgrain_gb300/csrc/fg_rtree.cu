@@ -83,12 +83,45 @@ __device__ __forceinline__ float unord32(uint32_t u) {
 __device__ __forceinline__ unsigned long long umin64(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
 __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
+// The split of a node whose centroids span lo .. hi (subdivide, bvh.rs:200-243): the axis of the largest
+// extent, -1 for a leaf (degenerate centroids), and the midpoint.
+__device__ __forceinline__ int split64(const double lo[3], const double hi[3], double& mid) {
+  const double ex = __dsub_rn(hi[0], lo[0]), ey = __dsub_rn(hi[1], lo[1]), ez = __dsub_rn(hi[2], lo[2]);
+  const int axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
+  const double ext = axis == 0 ? ex : (axis == 1 ? ey : ez);
+  const double a = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]), b = axis == 0 ? hi[0] : (axis == 1 ? hi[1] : hi[2]);
+  mid = __dmul_rn(0.5, __dadd_rn(a, b));
+  return ext <= 1e-7 ? -1 : axis;
+}
+
 // Centroid keys of either width: made so that -0 orders as +0, as the FP64 comparisons see them.
-// key >= threshold(mid) iff the centroid >= mid.
+// split: as split64, with the midpoint as a key: key >= thr iff the centroid >= the midpoint.
 struct Key32 {
   using T = uint32_t;
-  __device__ static double value(T k) { return static_cast<double>(unord32(k)); }
-  __device__ static T threshold(double mid) { return ord32(__double2float_ru(mid) + 0.0f); }
+  static constexpr bool WIDE = false;
+  // As split64, in float arithmetic (FP64 instructions are slow on sm_103a, and a level waits for this
+  // chain).  32-bit keys are those of synthesized crystals, whose coordinates are 0 or at least 1/1024 of
+  // one of at most 16,000 cells: 48 bits hold any difference or sum of two, so the FP64 ones are exact.
+  // Here they are exact float pairs, compared word by word.
+  __device__ static int split(const T lo[3], const T hi[3], T& thr) {
+    float e[3], el[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const float a = unord32(hi[f]), b = unord32(lo[f]);
+      e[f] = __fsub_rn(a, b);
+      const float t = __fsub_rn(e[f], a);
+      el[f] = __fsub_rn(__fsub_rn(a, __fsub_rn(e[f], t)), __fadd_rn(b, t));
+    }
+    auto ge = [&](int f, int g) { return e[f] > e[g] || (e[f] == e[g] && el[f] >= el[g]); };
+    const int axis = ge(0, 1) && ge(0, 2) ? 0 : (ge(1, 2) ? 1 : 2);
+    const float ext = axis == 0 ? e[0] : (axis == 1 ? e[1] : e[2]);
+    const float exl = axis == 0 ? el[0] : (axis == 1 ? el[1] : el[2]);
+    const float a = unord32(axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]));
+    const float b = unord32(axis == 0 ? hi[0] : (axis == 1 ? hi[1] : hi[2]));
+    thr = ord32(__fmul_rn(0.5f, __fadd_ru(a, b)) + 0.0f);
+    if (ext > 1.1e-7f) return axis;
+    return __dadd_rn(static_cast<double>(ext), static_cast<double>(exl)) <= 1e-7 ? -1 : axis;
+  }
   __device__ static T warp_min(T k) { return __reduce_min_sync(0xffffffffu, k); }
   __device__ static T warp_max(T k) { return __reduce_max_sync(0xffffffffu, k); }
   __device__ static void make(const RTile& t, uint32_t s, T k[3]) {
@@ -100,8 +133,19 @@ struct Key32 {
 };
 struct Key64 {
   using T = unsigned long long;
-  __device__ static double value(T k) { return unord64(k); }
-  __device__ static T threshold(double mid) { return ord64(mid); }
+  static constexpr bool WIDE = true;
+  __device__ static int split(const T lo[3], const T hi[3], T& thr) {
+    double clo[3], chi[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      clo[f] = unord64(lo[f]);
+      chi[f] = unord64(hi[f]);
+    }
+    double mid;
+    const int axis = split64(clo, chi, mid);
+    thr = ord64(mid);
+    return axis;
+  }
   // As two 32-bit reductions: the high words, then the low words of the lanes holding that high word.
   __device__ static T warp_min(T k) {
     const uint32_t hi = static_cast<uint32_t>(k >> 32), h = __reduce_min_sync(0xffffffffu, hi);
@@ -409,22 +453,20 @@ __global__ void __launch_bounds__(RT_BLOCK, 4) k_rt_levels(RtArgs A, int levels)
       const uint32_t node = A.wl[c][i];
       const int t = static_cast<int>(A.ntile[node]);
       const unsigned long long* a = A.acc + 6ull * node;
-      double clo[3], chi[3];
+      T clo[3], chi[3], thr;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        clo[k] = K::value(static_cast<T>(__ldcg(a + k)));
-        chi[k] = K::value(static_cast<T>(__ldcg(a + 3 + k)));
+        clo[k] = static_cast<T>(__ldcg(a + k));
+        chi[k] = static_cast<T>(__ldcg(a + 3 + k));
       }
-      const double ex = __dsub_rn(chi[0], clo[0]), ey = __dsub_rn(chi[1], clo[1]), ez = __dsub_rn(chi[2], clo[2]);
-      const int axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
-      const double ext = axis == 0 ? ex : (axis == 1 ? ey : ez);
+      const int axis = K::split(clo, chi, thr);
       uint32_t l = 0;
-      if (ext <= 1e-7 || !alloc_pair(A, t, l)) {
+      if (axis < 0 || !alloc_pair(A, t, l)) {
         A.nsplit[node] = -1;  // leaf (degenerate centroids, or no node capacity left)
         continue;
       }
       A.nsplit[node] = axis;
-      A.nthr[node] = K::threshold(__dmul_rn(0.5, __dadd_rn(clo[axis], chi[axis])));
+      A.nthr[node] = thr;
       const uint32_t id = static_cast<uint32_t>(A.tiles[t].nbase + l);
       A.nchild[node] = make_int2(static_cast<int>(id), static_cast<int>(id + 1));
       A.parent[id] = node;
@@ -638,12 +680,11 @@ __global__ void __launch_bounds__(RT_BLOCK, 4) k_rt_levels(RtArgs A, int levels)
 // the same node in between).  On return the first lane of each run holds the run's minima
 // (k[0..2]) and maxima (k[3..5]); the return value says whether this lane is a run's first.
 // Lanes without a node pass a seg value no other lane has.  All 32 lanes call it.
-template <class K>
-__device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, typename K::T k[6]) {
+__device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, uint32_t k[6]) {
   const int lane = threadIdx.x & 31;
   if (__all_sync(0xffffffffu, __shfl_sync(0xffffffffu, seg, 0) == seg)) {  // one node across the warp
 #pragma unroll
-    for (int i = 0; i < 6; ++i) k[i] = i < 3 ? K::warp_min(k[i]) : K::warp_max(k[i]);
+    for (int i = 0; i < 6; ++i) k[i] = i < 3 ? __reduce_min_sync(0xffffffffu, k[i]) : __reduce_max_sync(0xffffffffu, k[i]);
     return lane == 0;
   }
 #pragma unroll
@@ -652,7 +693,7 @@ __device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, typename K::T k[6]) 
     const bool take = lane + o < 32 && ns == seg;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      const typename K::T y = __shfl_down_sync(0xffffffffu, k[i], o);
+      const uint32_t y = __shfl_down_sync(0xffffffffu, k[i], o);
       if (take) k[i] = i < 3 ? min(k[i], y) : max(k[i], y);
     }
   }
@@ -662,8 +703,8 @@ __device__ __forceinline__ bool rt_seg_reduce(uint32_t seg, typename K::T k[6]) 
 
 // The block queue: one block builds the whole subtree of a node of at most RT_CTA_MAX elements
 // with its elements in shared memory.  Each level runs the passes of the global levels over all
-// of the level's nodes of more than RT_LEAF_MAX elements at once (segment-wise reduce, decide,
-// flags and prefix sum, ranks, place); a child of at most RT_LEAF_MAX elements is a leaf
+// of the level's nodes of more than RT_LEAF_MAX elements at once (segment-wise reduce, decide, flags
+// with their prefix sum and P / Q, children, place); a child of at most RT_LEAF_MAX elements is a leaf
 // (bvh.rs:200-204), whose fields one thread writes at the start of the next level.
 constexpr int RT_CTA_T = 256;                                // threads per block
 constexpr int RT_CTA_PER = RT_CTA_MAX / RT_CTA_T;            // positions per thread
@@ -674,37 +715,46 @@ constexpr uint8_t RT_CTA_FREE = 0xff;                        // position of a fi
 static_assert(RT_CTA_LV < RT_CTA_FREE, "level slots must fit a byte");
 static_assert(RT_CTA_MAX <= 2048, "positions are packed in 11 bits");
 
+// A node of the level as split: x: offset | count << 16; y: bigs before it | smalls in it << 16; z: left
+// child's size | end of the left stream << 16; w: next-level slots of the children (RT_CTA_FREE for a
+// small leaf) | << 8, | 1 << 16 when it splits.
 template <class K>
 struct RtCtaSmem {
   typename K::T key[3][RT_CTA_MAX];  // the job's centroid keys, at their load position (home)
-  // Per level: the nodes' centroid accumulators (reduce to decide), then the flags' prefix sum and
-  // the ranks (flags to place); the two uses do not overlap.
+  // Per level: the nodes' centroid boxes (reduce to decide), by words of 32 positions; then the flags' prefix sum, P, Q
+  // and the nodes as split (flags to place); the two uses do not overlap.
   union {
-    typename K::T acc[RT_CTA_LV][6];        // per level node: minima, maxima
     struct {
-      uint16_t bb[RT_CTA_MAX + 1];          // exclusive prefix sum of the flags
-      uint16_t P[RT_CTA_MAX], Q[RT_CTA_MAX];
+      typename K::T acc[RT_CTA_LV][6];      // minima, maxima of a node (64-bit keys: from its start to the end of that word)
+      typename K::T head[RT_CTA_MAX / 32][6];  // 64-bit keys: of the node's elements at the start of a word
+    } c;
+    struct {
+      uint4 node[RT_CTA_LV];                // what placing reads of a node (as above)
+      alignas(8) uint16_t bb[RT_CTA_MAX + 4];  // flag << 15 | exclusive prefix sum of the flags
+      uint16_t P[RT_CTA_MAX], Q[RT_CTA_MAX];  // positions of the bigs and of the others, by number
     } r;
   } u;
   typename K::T thr[RT_CTA_LV];           // split threshold
   uint32_t idx[RT_CTA_MAX];               // element slot
-  uint16_t home[RT_CTA_MAX];              // element's load position (its keys)
+  alignas(8) uint16_t home[RT_CTA_MAX];   // element's load position (its keys)
   uint32_t id[2][RT_CTA_LV];              // this level's nodes and the next's
-  uint32_t child[RT_CTA_LV];              // first child id of a splitting node
   uint32_t sl[RT_CTA_SL];                 // small leaves: position | count << 11 | depth << 14
   uint32_t slid[RT_CTA_SL];
   uint32_t scan[RT_CTA_T / 32];
   uint16_t off[2][RT_CTA_LV], cnt[2][RT_CTA_LV];
-  uint16_t sp[RT_CTA_LV];                 // left child size
-  uint8_t nd[RT_CTA_MAX];                 // level slot of the position's node, RT_CTA_FREE when done
-  uint8_t flag[RT_CTA_MAX];
+  alignas(4) uint8_t nd[RT_CTA_MAX];      // level slot of the position's node, RT_CTA_FREE when done
   uint8_t dep[2][RT_CTA_LV];
-  uint8_t cslot[RT_CTA_LV][2];            // next-level slot of each child, RT_CTA_FREE for a small leaf
   int8_t axis[RT_CTA_LV];
   int nl, nsl, nnext, nslnew;
   uint32_t maxdep;
 };
 
+// What bounds it: latency.  A level is seven barriers with short chains of shared-memory reads between
+// them, 7,200 cycles (32-bit keys; 10,100 with 64-bit ones) for 1,024 elements.  With the ranks in a
+// pass of their own, a global atomic and FP64 decisions in the chain, and 64-bit minima accumulated in
+// shared memory, the blocks of a 64 x 64 px tri-x tile took 50 us (64-bit keys 58), now 38 (45); the
+// 18.9 M elements of a 1600 x 1600 px t-max image 2.40 ms, now 2.05.
+//
 // Four blocks per SM (64 registers; the block's shared memory is about 53 KB with 64-bit keys): 9 %
 // faster than two.
 template <class K>
@@ -720,6 +770,7 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
     const int n = static_cast<int>(min(A.ncount[root], static_cast<uint32_t>(RT_CTA_MAX)));
     const uint32_t t = A.ntile[root];
     const unsigned long long nb = A.tiles[t].nbase;
+    const uint32_t ncap = A.tiles[t].ncap;
     const uint32_t dep0 = min(A.ndepth[root], 255u);
     for (int x = tid; x < RT_CTA_MAX; x += RT_CTA_T) {
       if (x < n) {
@@ -764,82 +815,113 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
         A.nsplit[id] = -1;
         atomicMax(&S.maxdep, dp);
       }
-      for (int i = tid; i < nl * 6; i += RT_CTA_T) S.u.acc[i / 6][i % 6] = (i % 6) < 3 ? ~static_cast<T>(0) : static_cast<T>(0);
-      __syncthreads();
       if (nl == 0) break;
+      if (!K::WIDE) {
+        for (int i = tid; i < nl * 6; i += RT_CTA_T) S.u.c.acc[i / 6][i % 6] = (i % 6) < 3 ? ~static_cast<T>(0) : static_cast<T>(0);
+        __syncthreads();
+      }
       if (tid == 0) {
         S.nnext = 0;
         S.nslnew = 0;
       }
-      // Reduce: position x = k * RT_CTA_T + tid, so a warp holds 32 consecutive positions.
-#pragma unroll 1
+      // Reduce: position x = k * RT_CTA_T + tid, so a warp holds 32 consecutive positions, those of at
+      // most eight nodes (of more than four elements each).  32-bit keys: the nodes' runs reduced side by
+      // side, their heads joined in shared memory.  64-bit keys, whose minimum in shared memory is a
+      // loop: a reduction over the warp for each node; its box in the word goes to the word when the
+      // node may start before it, else to the node, so nothing is accumulated in place.  (The other way
+      // round: 25 k cycles a block against 20 with 32-bit keys, 37 against 22 with 64-bit ones.)
+#pragma unroll 2
       for (int k = 0; k < RT_CTA_PER; ++k) {
         const int x = k * RT_CTA_T + tid;
         const uint32_t node = S.nd[x];
         const bool act = node != RT_CTA_FREE;
-        if (!__any_sync(0xffffffffu, act)) continue;
-        T kk[6];
+        unsigned todo = __ballot_sync(0xffffffffu, act);
+        if (!todo) continue;
+        T kk[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const T v = S.key[i][act ? S.home[x] : 0];
-          kk[i] = act ? v : ~static_cast<T>(0);
-          kk[3 + i] = act ? v : static_cast<T>(0);
-        }
-        const bool head = rt_seg_reduce<K>(act ? node : (0x100u | static_cast<uint32_t>(lane)), kk);
-        if (act && head) {
+        for (int i = 0; i < 3; ++i) kk[i] = S.key[i][act ? S.home[x] : 0];
+        if constexpr (!K::WIDE) {
+          T box[6];
 #pragma unroll
-          for (int i = 0; i < 3; ++i) atomicMin(&S.u.acc[node][i], kk[i]);
+          for (int i = 0; i < 3; ++i) {
+            box[i] = act ? kk[i] : ~static_cast<T>(0);
+            box[3 + i] = act ? kk[i] : static_cast<T>(0);
+          }
+          if (rt_seg_reduce(act ? node : (0x100u | static_cast<uint32_t>(lane)), box) && act) {
 #pragma unroll
-          for (int i = 3; i < 6; ++i) atomicMax(&S.u.acc[node][i], kk[i]);
+            for (int i = 0; i < 3; ++i) {
+              atomicMin(&S.u.c.acc[node][i], box[i]);
+              atomicMax(&S.u.c.acc[node][3 + i], box[3 + i]);
+            }
+          }
+        } else {
+          while (todo) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t nd = __shfl_sync(0xffffffffu, node, src);
+            const bool in = node == nd;
+            todo &= ~__ballot_sync(0xffffffffu, in);
+            T lo[3], hi[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              lo[i] = K::warp_min(in ? kk[i] : ~static_cast<T>(0));
+              hi[i] = K::warp_max(in ? kk[i] : static_cast<T>(0));
+            }
+            if (lane == src) {
+              T* out = src == 0 ? S.u.c.head[k * (RT_CTA_T / 32) + w] : S.u.c.acc[nd];
+#pragma unroll
+              for (int i = 0; i < 3; ++i) {
+                out[i] = lo[i];
+                out[3 + i] = hi[i];
+              }
+            }
+          }
         }
       }
       __syncthreads();
-      // Decide (subdivide, bvh.rs:200-270), one thread per node of the level.
-      for (int i = tid; i < nl; i += RT_CTA_T) {
-        const uint32_t id = S.id[cur][i];
-        const int cn = S.cnt[cur][i];
-        double clo[3], chi[3];
+      // Decide (subdivide, bvh.rs:200-270), one thread per node of the level.  The ids of its children
+      // are asked for here and used after the flags: the counter is a microsecond away.
+      static_assert(RT_CTA_LV <= RT_CTA_T, "a thread to a node");
+      int axis = -1;
+      uint32_t l = 0;
+      if (tid < nl) {
+        T clo[3], chi[3], thr;
+        const int o0 = S.off[cur][tid], cn = S.cnt[cur][tid];
+        const bool own = !K::WIDE || (o0 & 31) != 0;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-          clo[m] = K::value(S.u.acc[i][m]);
-          chi[m] = K::value(S.u.acc[i][3 + m]);
+          clo[m] = own ? S.u.c.acc[tid][m] : ~static_cast<T>(0);
+          chi[m] = own ? S.u.c.acc[tid][3 + m] : static_cast<T>(0);
         }
-        A.nstart[id] = s + S.off[cur][i];
-        A.ncount[id] = static_cast<uint32_t>(cn);
-        A.ntile[id] = t;
-        A.ndepth[id] = S.dep[cur][i];
-        atomicMax(&S.maxdep, static_cast<uint32_t>(S.dep[cur][i]));
-        const double ex = __dsub_rn(chi[0], clo[0]), ey = __dsub_rn(chi[1], clo[1]), ez = __dsub_rn(chi[2], clo[2]);
-        const int axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
-        const double ext = axis == 0 ? ex : (axis == 1 ? ey : ez);
-        uint32_t l = 0;
-        if (cn <= RT_LEAF_MAX || ext <= 1e-7 || !alloc_pair(A, static_cast<int>(t), l)) {
-          S.axis[i] = -1;  // leaf (degenerate centroids, or no node capacity left)
-          A.nsplit[id] = -1;
-        } else {
-          const double ca = axis == 0 ? clo[0] : (axis == 1 ? clo[1] : clo[2]);
-          const double cb = axis == 0 ? chi[0] : (axis == 1 ? chi[1] : chi[2]);
-          const double mid = __dmul_rn(0.5, __dadd_rn(ca, cb));
-          S.axis[i] = static_cast<int8_t>(axis);
-          S.thr[i] = K::threshold(mid);
-          S.child[i] = static_cast<uint32_t>(nb + l);
-          A.nsplit[id] = axis;
-          A.nchild[id] = make_int2(static_cast<int>(nb + l), static_cast<int>(nb + l + 1));
-          A.parent[nb + l] = id;
-          A.parent[nb + l + 1] = id;
+        for (int word = (o0 + 31) >> 5; K::WIDE && word <= (o0 + cn - 1) >> 5; ++word)
+#pragma unroll
+          for (int m = 0; m < 3; ++m) {
+            clo[m] = min(clo[m], S.u.c.head[word][m]);
+            chi[m] = max(chi[m], S.u.c.head[word][3 + m]);
+          }
+        axis = cn > RT_LEAF_MAX ? K::split(clo, chi, thr) : -1;
+        if (axis >= 0) {
+          l = atomicAdd(&A.tiles[t].nodes, 2u);
+          S.thr[tid] = thr;
         }
+        S.axis[tid] = static_cast<int8_t>(axis);
       }
       __syncthreads();
-      // Flags and their exclusive prefix sum: thread tid owns positions RT_CTA_PER * tid + k.
+      // Flags, their exclusive prefix sum, and the positions of the bigs and of the others by number:
+      // thread tid owns positions RT_CTA_PER * tid + k.
       {
+        static_assert(RT_CTA_PER == 4, "four positions to a thread");
+        const uint32_t nd4 = *reinterpret_cast<const uint32_t*>(S.nd + RT_CTA_PER * tid);
+        const uint2 home4 = *reinterpret_cast<const uint2*>(S.home + RT_CTA_PER * tid);
         uint32_t f[RT_CTA_PER], sum = 0;
 #pragma unroll
         for (int k = 0; k < RT_CTA_PER; ++k) {
-          const int x = RT_CTA_PER * tid + k;
-          const uint32_t node = S.nd[x];
+          const uint32_t node = (nd4 >> (8 * k)) & 0xffu;
+          const uint32_t home = ((k < 2 ? home4.x : home4.y) >> (16 * (k & 1))) & 0xffffu;
           f[k] = 0;
-          if (node != RT_CTA_FREE && S.axis[node] >= 0)
-            f[k] = S.key[S.axis[node]][S.home[x]] < S.thr[node] ? 0u : 1u;
+          if (node != RT_CTA_FREE) {
+            const int ax = S.axis[node];
+            if (ax >= 0) f[k] = S.key[ax][home] < S.thr[node] ? 0u : 1u;
+          }
           sum += f[k];
         }
         uint32_t incl = sum;
@@ -852,56 +934,67 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
         __syncthreads();
         uint32_t acc = incl - sum;
         for (int i = 0; i < w; ++i) acc += S.scan[i];
+        uint32_t b[RT_CTA_PER];
 #pragma unroll
         for (int k = 0; k < RT_CTA_PER; ++k) {
-          const int x = RT_CTA_PER * tid + k;
-          S.flag[x] = static_cast<uint8_t>(f[k]);
-          S.u.r.bb[x] = static_cast<uint16_t>(acc);
+          const uint32_t x = RT_CTA_PER * tid + k;
+          b[k] = f[k] << 15 | acc;
+          if (f[k]) S.u.r.P[acc] = static_cast<uint16_t>(x); else S.u.r.Q[x - acc] = static_cast<uint16_t>(x);
           acc += f[k];
         }
+        *reinterpret_cast<uint2*>(S.u.r.bb + RT_CTA_PER * tid) = make_uint2(b[0] | b[1] << 16, b[2] | b[3] << 16);
         if (tid == RT_CTA_T - 1) S.u.r.bb[RT_CTA_MAX] = static_cast<uint16_t>(acc);
       }
       __syncthreads();
-      // Ranks P / Q; the children of every splitting node go to the next level (more than four
-      // elements) or become small leaves.
-      for (int x = tid; x < RT_CTA_MAX; x += RT_CTA_T) {
-        const uint32_t node = S.nd[x];
-        if (node == RT_CTA_FREE || S.axis[node] < 0) continue;
-        const int o0 = S.off[cur][node], cn = S.cnt[cur][node];
-        const int r = x - o0;
-        const int bs = S.u.r.bb[o0];
-        const int Bb = S.u.r.bb[x] - bs, Bt = S.u.r.bb[o0 + cn] - bs, St = cn - Bt;
-        if (S.flag[x]) {
-          S.u.r.P[o0 + Bb] = static_cast<uint16_t>(r);
-        } else {
-          S.u.r.Q[o0 + (St - (r - Bb)) - 1] = static_cast<uint16_t>(r);
+      // The nodes, and the children of those that split: to the next level (more than four elements) or
+      // small leaves.
+      if (tid < nl) {
+        const uint32_t id = S.id[cur][tid], dep = S.dep[cur][tid];
+        const int o0 = S.off[cur][tid], cn = S.cnt[cur][tid];
+        A.nstart[id] = s + static_cast<uint32_t>(o0);
+        A.ncount[id] = static_cast<uint32_t>(cn);
+        A.ntile[id] = t;
+        A.ndepth[id] = dep;
+        atomicMax(&S.maxdep, dep);
+        if (axis >= 0 && l + 2 > ncap) {  // no node capacity left
+          atomicOr(A.err, ERR_LIST_OVERFLOW);
+          axis = -1;
         }
-      }
-      for (int i = tid; i < nl; i += RT_CTA_T) {
-        if (S.axis[i] < 0) continue;
-        const int o0 = S.off[cur][i], cn = S.cnt[cur][i];
-        const int St = cn - (S.u.r.bb[o0 + cn] - S.u.r.bb[o0]);
-        const int Sp = (St == 0 || St == cn) ? cn / 2 : St;  // bvh.rs:260-265
-        S.sp[i] = static_cast<uint16_t>(Sp);
-        const uint32_t cd = min(static_cast<uint32_t>(S.dep[cur][i]) + 1u, 255u);  // saturates past the depth check
+        A.nsplit[id] = axis;
+        uint4 N = make_uint4(static_cast<uint32_t>(o0) | static_cast<uint32_t>(cn) << 16, 0u, 0u, 0u);
+        if (axis >= 0) {
+          const int bs = S.u.r.bb[o0] & 0x7fff, Bt = (S.u.r.bb[o0 + cn] & 0x7fff) - bs, St = cn - Bt;
+          const int li = St + (St < cn ? S.u.r.bb[o0 + St] >> 15 : 0);
+          const int Sp = (St == 0 || St == cn) ? cn / 2 : St;  // bvh.rs:260-265
+          const uint32_t kid = static_cast<uint32_t>(nb + l);
+          A.nchild[id] = make_int2(static_cast<int>(kid), static_cast<int>(kid + 1));
+          A.parent[kid] = id;
+          A.parent[kid + 1] = id;
+          const uint32_t cd = min(dep + 1u, 255u);  // saturates past the depth check
+          uint32_t slots = 0;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const uint32_t cid = S.child[i] + static_cast<uint32_t>(c);
-          const int coff = o0 + (c ? Sp : 0), csz = c ? cn - Sp : Sp;
-          if (csz > RT_LEAF_MAX) {
-            const int slot = atomicAdd(&S.nnext, 1);
-            S.id[cur ^ 1][slot] = cid;
-            S.off[cur ^ 1][slot] = static_cast<uint16_t>(coff);
-            S.cnt[cur ^ 1][slot] = static_cast<uint16_t>(csz);
-            S.dep[cur ^ 1][slot] = static_cast<uint8_t>(cd);
-            S.cslot[i][c] = static_cast<uint8_t>(slot);
-          } else {
-            const int qi = atomicAdd(&S.nslnew, 1);
-            S.sl[qi] = static_cast<uint32_t>(coff) | static_cast<uint32_t>(csz) << 11 | cd << 14;
-            S.slid[qi] = cid;
-            S.cslot[i][c] = RT_CTA_FREE;
+          for (int c = 0; c < 2; ++c) {
+            const uint32_t cid = kid + static_cast<uint32_t>(c);
+            const int coff = o0 + (c ? Sp : 0), csz = c ? cn - Sp : Sp;
+            if (csz > RT_LEAF_MAX) {
+              const int slot = atomicAdd(&S.nnext, 1);
+              S.id[cur ^ 1][slot] = cid;
+              S.off[cur ^ 1][slot] = static_cast<uint16_t>(coff);
+              S.cnt[cur ^ 1][slot] = static_cast<uint16_t>(csz);
+              S.dep[cur ^ 1][slot] = static_cast<uint8_t>(cd);
+              slots |= static_cast<uint32_t>(slot) << (8 * c);
+            } else {
+              const int qi = atomicAdd(&S.nslnew, 1);
+              S.sl[qi] = static_cast<uint32_t>(coff) | static_cast<uint32_t>(csz) << 11 | cd << 14;
+              S.slid[qi] = cid;
+              slots |= static_cast<uint32_t>(RT_CTA_FREE) << (8 * c);
+            }
           }
+          N.y = static_cast<uint32_t>(bs) | static_cast<uint32_t>(St) << 16;
+          N.z = static_cast<uint32_t>(Sp) | static_cast<uint32_t>(li) << 16;
+          N.w = slots | 1u << 16;
         }
+        S.u.r.node[tid] = N;
       }
       __syncthreads();
       // Place: every element of a splitting node moves to its place after the swap partition.
@@ -911,31 +1004,26 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
       uint8_t vn[RT_CTA_PER];
 #pragma unroll
       for (int k = 0; k < RT_CTA_PER; ++k) {
+        // Without branches: the four positions' chains of reads run side by side.
         const int x = k * RT_CTA_T + tid;
         const uint32_t node = S.nd[x];
-        dst[k] = -1;
-        vn[k] = RT_CTA_FREE;
-        if (node == RT_CTA_FREE) continue;
+        const bool act = node != RT_CTA_FREE;
         vp[k] = S.home[x];
         vi[k] = S.idx[x];
-        if (S.axis[node] < 0) {  // a leaf of this level: its order is final
-          dst[k] = x;
-          continue;
-        }
-        const int o0 = S.off[cur][node], cn = S.cnt[cur][node];
-        const int r = x - o0;
-        const int bs = S.u.r.bb[o0];
-        const int Bb = S.u.r.bb[x] - bs, Bt = S.u.r.bb[o0 + cn] - bs, St = cn - Bt;
-        const int li = St + (St < cn ? S.flag[o0 + St] : 0);
-        const bool big = S.flag[x] != 0;
-        int d;
-        if (r < li) {
-          d = big ? ((Bb == 0 ? cn : S.u.r.Q[o0 + Bb - 1]) - 1) : r;
-        } else {
-          d = big ? r - 1 : S.u.r.P[o0 + (St - (r - Bb)) - 1];
-        }
-        dst[k] = o0 + d;
-        vn[k] = S.cslot[node][d < S.sp[node] ? 0 : 1];
+        const uint4 N = S.u.r.node[act ? node : 0u];
+        const uint32_t b = S.u.r.bb[x];
+        const bool move = act && (N.w >> 16) != 0;  // else a leaf of this level (its order is final), or done
+        const int o0 = static_cast<int>(N.x & 0xffffu), cn = static_cast<int>(N.x >> 16);
+        const int bs = static_cast<int>(N.y & 0xffffu), St = static_cast<int>(N.y >> 16);
+        const int Sp = static_cast<int>(N.z & 0xffffu), li = static_cast<int>(N.z >> 16);
+        const int r = x - o0, Bb = static_cast<int>(b & 0x7fffu) - bs;
+        const bool big = (b >> 15) != 0, look = move && (r < li) == big && !(big && Bb == 0);
+        const int at = big ? o0 - bs + (St - Bb) : bs + (St - (r - Bb)) - 1;
+        const int got = (big ? S.u.r.Q : S.u.r.P)[look ? at : 0];
+        // Block position: P's; one before Q's, or before the node's end for the first big; one less; the same.
+        const int d = look ? (big ? got - 1 : got) : (big && move ? (r < li ? o0 + cn : x) - 1 : x);
+        dst[k] = act ? d : -1;
+        vn[k] = static_cast<uint8_t>(!move ? RT_CTA_FREE : (d - o0 < Sp ? N.w : N.w >> 8));
       }
       __syncthreads();
 #pragma unroll

@@ -76,3 +76,26 @@ def test_synthesized_sets(engine, stock, w, h):
     c = em.crystals()
     check(em, orc.Crystals(c["pos"], c["dims"], c["quat"], c["sensitivity"], c["morphology"]))
     em.close()
+
+
+# One block's subtree with 64-bit keys: nodes that start, end and straddle the words of 32 positions.
+@pytest.mark.parametrize("kind", ["even", "clustered", "one axis", "pairs"])
+@pytest.mark.parametrize("n", [1, 4, 5, 31, 32, 33, 64, 65, 200, 1023, 1024])
+def test_uploaded_sets_of_one_block(engine, kind, n):
+    rng = np.random.default_rng(100 + n)
+    if kind == "even":
+        pos = rng.random((n, 3)) * [60.0, 50.0, 12.0]
+    elif kind == "clustered":
+        pos = np.exp(rng.normal(size=(n, 3)))
+    elif kind == "one axis":
+        pos = np.stack([np.full(n, 1.0), rng.random(n) * 50.0, np.full(n, 3.0)], 1)
+    else:
+        pos = np.repeat(rng.random((n // 2 + 1, 3)) * 30.0, 2, axis=0)[:n]
+    dims = rng.uniform(0.1, 0.6, (n, 3))
+    quat = rng.normal(size=(n, 4))
+    quat /= np.linalg.norm(quat, axis=1, keepdims=True)
+    sens = np.ones(n)
+    em = fg.VirtualEmulsionLayer.from_crystals(fg.EmulsionConfig((100.0, 60.0, 20.0), 1.0), pos, dims, quat, sens,
+                                               engine=engine)
+    check(em, orc.Crystals(pos, dims, quat, sens, np.zeros(n, np.int32)))
+    em.close()
