@@ -252,11 +252,12 @@ def profile_traffic(name):
 
 def rooflines(stats, workload_key):
     """The transport and Bridson kernels against the measured HBM bandwidth (algorithmic bytes:
-    transport 4 B exposure per photon + 8 B count read-modify-write per hit + 116 B per crystal
-    read once; Bridson 4 B read + 4 B written per synthesis cell)."""
+    transport 4 B exposure per photon + 8 B count read-modify-write per hit + 100 B per crystal
+    read once (records 48, leaf box and rank 32, slot and sensitivity by rank 8, cells 8, count 4);
+    Bridson 4 B read + 4 B written per synthesis cell)."""
     peak, kind = measured_peak()
     P, H, N = stats["photons"], stats["hits"], stats["crystals"]
-    t_alg = 4.0 * P + 8.0 * H + 116.0 * N
+    t_alg = 4.0 * P + 8.0 * H + 100.0 * N
     t_ach = t_alg / (stats["transport_ms"] / 1e3) / 1e9 if stats["transport_ms"] > 0 else 0.0
     b_alg = 8.0 * stats["cells"]
     b_ach = b_alg / (stats["bridson_ms"] / 1e3) / 1e9 if stats["bridson_ms"] > 0 else 0.0
@@ -581,7 +582,7 @@ def run_fast(args):
                                    "jittered grid, per-crystal Poisson counts, column scan), host to host",
                        "tiles": len(grid), "output_px": C2_OUT * C2_OUT, "parallelism": f"replicas x{world}"},
             "e2e": {"value": value, "unit": "Mpx/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": h2d},
-            "gpu_launches": 5 * args.steps, "clocks": ck.summary()}))
+            "gpu_launches": 6 * args.steps, "clocks": ck.summary()}))
 
 
 # ------------------------------------------------------------------------------------------------
