@@ -167,11 +167,11 @@ fg_status fg_emulsion_preset(const char* name, double width, double height, fg_e
 /* ---- emulsions ---- */
 /* VirtualEmulsionLayer::synthesize (src/emulsion.rs:155-220) on the device: Poisson-disk
  * positions (src/poisson.rs:14-132, column-parallel Bridson thinned to the reference sampler's
- * density) and crystal attributes, then the LBVH.  Crystal ids follow the Morton order of the
- * synthesis grid. */
+ * density) and crystal attributes, then the reference's tree and the crystals in cells.  Crystal ids
+ * follow the Morton order of the synthesis grid. */
 fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint64_t seed, fg_emulsion** out);
 /* Upload a crystal set (for parity runs on exactly the oracle's crystals).  The device keeps the
- * FP64 values for exact predicates and builds the Morton-ordered LBVH. */
+ * FP64 values for exact predicates and builds the reference's tree, and cells where they suit. */
 fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_crystals_host* c,
                              size_t n, fg_emulsion** out);
 fg_status fg_emulsion_destroy(fg_engine* e, fg_emulsion* em);
