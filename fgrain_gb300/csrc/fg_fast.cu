@@ -401,10 +401,11 @@ __device__ __forceinline__ FastHit fast_load(const FastCell* c) {
 // LANES 1: a thread lists what its pixel can meet and tests each crystal against four of its rays.
 // LANES 4: a ray to a lane, for wide pixels, whose rays look at different cells, and for few pixels.
 // Measured on 1024 x 1024 px of tri-x (1.9 ms before, testing every crystal of the 25 columns and
-// finding the direction in its frame for each ray): .52 ms.
+// finding the direction in its frame for each ray): .52 ms, .47 with
+// eight CTAs per SM (64 registers; ten: .58).
 constexpr int FSCAN_T = 128, FSCAN_LIST = 64;
 template <int LANES>
-__global__ void __launch_bounds__(FSCAN_T) k_fast_scan(const FastTile* __restrict__ tiles,
+__global__ void __launch_bounds__(FSCAN_T, 8) k_fast_scan(const FastTile* __restrict__ tiles,
                                                        const FastCell* __restrict__ cells,
                                                        const float4* __restrict__ near,
                                                        const uint32_t* __restrict__ count, float* __restrict__ d_neg) {

@@ -678,7 +678,10 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan(const ScanTile* __rest
 // does and writes the pixels' transmittance; pass 2 stages the bin's crystals again (unless all of
 // them are still there) and adds w[p] / spp * T_ray * chord_s for every hit to a per-crystal FP64 sum
 // in shared memory, flushed with one global atomic per staged crystal.
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_adjoint(const ScanTile* __restrict__ tiles,
+//
+// Bound by issue, as k_scan.  Four CTAs per SM (64 registers) as there: a gradient step takes 4.39 ms with the two
+// that 126 registers leave, 4.16 with three, 4.04 with four (spills included).
+__global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan_adjoint(const ScanTile* __restrict__ tiles,
                                                                const float* __restrict__ wpx,
                                                                double* __restrict__ g, float* __restrict__ Tpx,
                                                                unsigned long long* stats) {
