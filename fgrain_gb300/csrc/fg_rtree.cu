@@ -61,6 +61,9 @@ int levels_for(uint32_t emax) {
 constexpr int RT_WARPS = RT_BLOCK / 32;
 constexpr int RT_WPW_LARGE = 8, RT_WPW_SMALL = 2;
 constexpr unsigned long long RT_LARGE = 600ull * 1000ull;  // elements from which chunks are long
+// Blocks per SM that a build's registers leave (32-bit keys: trees of a 1400 x 1400 px t-max image in
+// 6.77 ms with four, 6.33 with five, 6.51 with six; 64-bit keys: a gradient step in 4.07, 4.30, 4.36).
+constexpr int rt_blocks(bool wide) { return wide ? 4 : 5; }
 constexpr unsigned rt_chunk(int wpw) { return 32u * RT_WARPS * static_cast<unsigned>(wpw); }
 constexpr unsigned RT_CNT_BAR = 4;               // RtArgs::cnt: the grid barrier's arrivals
 constexpr unsigned RT_CNT_TILES = 16;            // first of ntiles + 1 words: chunks before each tile
@@ -355,10 +358,10 @@ __device__ __forceinline__ int rt_chunk_tile(const uint32_t* start, int ntiles, 
 //
 // Bound by latency more than by the streams (Key32: about 56 B per element and level, a third of the
 // copy bandwidth): each word's node, element and keys are read while the word before is placed.
-// Against eight launches per level with 64-bit keys, 18.9 M elements in 25 tiles: 11.5 -> 4.9 ms; the
+// Against eight launches per level with 64-bit keys, 18.9 M elements in 25 tiles: 11.5 -> 4.3 ms; the
 // whole build of one tile's 3,556: 0.19 -> 0.10 ms, of 309 k: 0.60 -> 0.35 ms.
 template <class K, int WPW>
-__global__ void __launch_bounds__(RT_BLOCK, 4) k_rt_levels(RtArgs A, int levels) {
+__global__ void __launch_bounds__(RT_BLOCK, rt_blocks(K::WIDE)) k_rt_levels(RtArgs A, int levels) {
   using T = typename K::T;
   constexpr unsigned RT_CHUNK = rt_chunk(WPW), RT_WORDS = RT_CHUNK / 32;
   __shared__ int s_tile;
@@ -1464,8 +1467,9 @@ void build_topology(const RTreeBufs& B, const RtArgs& A, cudaStream_t st) {
   int dev = 0, sms = 0;
   FG_CUDA(cudaGetDevice(&dev));
   FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // The launch bounds let four blocks share an SM, so the whole grid runs at once.
-  const unsigned GL = static_cast<unsigned>(std::max<unsigned long long>(std::min<unsigned long long>(B.nblk, 4ull * sms), 1));
+  // The launch bounds let that many blocks share an SM, so the whole grid runs at once.
+  const unsigned long long room = 1ull * rt_blocks(K::WIDE) * sms;
+  const unsigned GL = static_cast<unsigned>(std::max<unsigned long long>(std::min<unsigned long long>(B.nblk, room), 1));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(GL);
   cfg.blockDim = dim3(RT_BLOCK);
