@@ -62,6 +62,14 @@ PAIR_FN Pair pair_mul(Pair a, float b) {
   return pair_fast(p.h, PAIR_FMA(a.l, b, p.l));
 }
 
+// A quotient and its remainder's.
+PAIR_FN Pair pair_div(Pair n, Pair d) {
+  const float inv = 1.0f / d.h;
+  const float q = PAIR_MUL(n.h, inv);
+  const float rem = PAIR_ADD(PAIR_FMA(-q, d.h, n.h), PAIR_FMA(-q, d.l, n.l));
+  return pair_fast(q, PAIR_MUL(rem, inv));
+}
+
 // Whether the value's rounding to float is settled; r receives it.
 PAIR_FN bool pair_round(Pair a, float& r) {
   const float e = PAIR_MUL(fabsf(a.h), PAIR_ERR);
@@ -91,11 +99,7 @@ PAIR_FN Pair pair_log(float x, float xl = 0.0f) {
   const Pair n = pair_fast(f, fl);
   Pair d = pair_sum(2.0f, f);
   d = pair_fast(d.h, PAIR_ADD(d.l, fl));
-  // s = n / d: a quotient and its remainder's.
-  const float inv = 1.0f / d.h;
-  const float q = PAIR_MUL(n.h, inv);
-  const float rem = PAIR_ADD(PAIR_FMA(-q, d.h, n.h), PAIR_FMA(-q, d.l, n.l));
-  const Pair s = pair_fast(q, PAIR_MUL(rem, inv));
+  const Pair s = pair_div(n, d);
   const Pair z = pair_mul(s, s);
   // 2 s (1 + z / 3 + z^2 / 5 + ...), z < .0295: the first two terms as pairs.
   float p = 0.13333334f;  // 2 / 15
@@ -172,6 +176,14 @@ PAIR_FN void pair_sincos(float x, Pair& sn, Pair& cs) {
   const Pair a = k & 1 ? q : s, b = k & 1 ? s : q;
   sn = k & 2 ? Pair{-a.h, -a.l} : a;
   cs = (k + 1) & 2 ? Pair{-b.h, -b.l} : b;
+}
+
+// n / d of FP64 values, given also as pairs (to 2^-48), rounded to float.
+PAIR_FN float pair_quotf(double n, double d, Pair np, Pair dp) {
+  float r;
+  const float lo = 8.7e-19f, hi = 1.1e18f;  // 2^-60, 2^60: the low parts stay normal floats
+  if (fabsf(np.h) > lo && fabsf(np.h) < hi && fabsf(dp.h) > lo && fabsf(dp.h) < hi && pair_round(pair_div(np, dp), r)) return r;
+  return static_cast<float>(n / d);
 }
 
 // The FP64 functions rounded to float.

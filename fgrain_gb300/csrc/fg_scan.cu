@@ -59,20 +59,23 @@ __device__ __forceinline__ void two_prod(float a, float b, float& p, float& e) {
   p = a * b;
   e = fmaf(a, b, -p);
 }
+// hi = v rounded to float, lo = v - hi (exact) rounded to float.  In integer arithmetic: hi takes the
+// upper 24 bits of v's 53, lo is the signed rest of at most 2^28 (the FP64 pipe, with the conversions it
+// also does, bounds the staging terms).  Zero and magnitudes outside 2^-60 .. 2^120 take it still.
 __device__ __forceinline__ void split64(double v, float& hi, float& lo) {
-  hi = static_cast<float>(v);
-  lo = static_cast<float>(v - static_cast<double>(hi));
-}
-// A float widened to double by moving its bits (integer pipes); zero and subnormals (T below
-// 2^-126, rare) take the conversion instruction.
-__device__ __forceinline__ double f2d_exact(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const uint32_t e = (b >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return static_cast<double>(f);
-  const unsigned long long d = (static_cast<unsigned long long>(b & 0x80000000u) << 32) |
-                               (static_cast<unsigned long long>(e + (1023u - 127u)) << 52) |
-                               (static_cast<unsigned long long>(b & 0x7fffffu) << 29);
-  return __longlong_as_double(static_cast<long long>(d));
+  const uint32_t h = static_cast<uint32_t>(__double2hiint(v)), l = static_cast<uint32_t>(__double2loint(v));
+  const uint32_t e = (h >> 20) & 0x7ffu;
+  if (e - 963u > 180u) {
+    hi = static_cast<float>(v);
+    lo = static_cast<float>(v - static_cast<double>(hi));
+    return;
+  }
+  const uint32_t q = ((h & 0xfffffu) << 3) | (l >> 29), r = l & 0x1fffffffu;  // q: 23 bits below the leading one
+  const bool up = r > 0x10000000u || (r == 0x10000000u && (q & 1u));           // to nearest, ties to even
+  const int d = static_cast<int>(r) - (up ? 0x20000000 : 0);
+  hi = __uint_as_float((h & 0x80000000u) | (((e - 896u) << 23) + q + (up ? 1u : 0u)));
+  // d in units of 2^(e - 1075); a rest of zero is +0 whatever the sign.
+  lo = __fmul_rn(__int2float_rn(static_cast<int>(h) < 0 ? -d : d), __uint_as_float((e - 948u) << 23));
 }
 
 // (ah + al) - (bh + bl) as a float pair, to about 2^-48 of the operands.
@@ -162,7 +165,9 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
     const float Dmax = static_cast<float>(fmax(fmax(D[0], D[1]), D[2]));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const float inv = static_cast<float>(1.0 / (-R2[i]));
+      Pair r2;
+      split64(-R2[i], r2.h, r2.l);
+      const float inv = pair_quotf(1.0, -R2[i], Pair{1.0f, 0.0f}, r2);
       float r0, r0l, r1, r1l, d, dl;
       split64(R0[i], r0, r0l);
       split64(R1[i], r1, r1l);
@@ -195,10 +200,14 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const double ei = -R2[i] / D[i];
-      P.g[i] = make_float4(static_cast<float>(R0[i] / D[i]), static_cast<float>(R1[i] / D[i]), static_cast<float>(ei), 0.0f);
+      Pair r0, r1, d;
+      split64(R0[i], r0.h, r0.l);
+      split64(R1[i], r1.h, r1.l);
+      split64(D[i], d.h, d.l);
+      P.g[i] = make_float4(pair_quotf(R0[i], D[i], r0, d), pair_quotf(R1[i], D[i], r1, d), static_cast<float>(ei), 0.0f);
       P.g[3 + i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       A += ei * ei;
-      const float Df = static_cast<float>(D[i]), u = static_cast<float>(R0[i]) * Df, v = static_cast<float>(R1[i]) * Df;
+      const float u = r0.h * d.h, v = r1.h * d.h;
       hx += u * u;
       hy += v * v;
     }

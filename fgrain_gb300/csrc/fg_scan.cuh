@@ -95,6 +95,18 @@ __device__ __forceinline__ void scan_origin64(const ScanTile& t, uint32_t px, ui
   oy = __dmul_rn(__dadd_rn(static_cast<double>(py), suby), t.ph);
 }
 
+// A float widened to double by moving its bits (integer pipes); zero and subnormals (T below
+// 2^-126, rare) take the conversion instruction.
+__device__ __forceinline__ double f2d_exact(float f) {
+  const uint32_t b = __float_as_uint(f);
+  const uint32_t e = (b >> 23) & 0xffu;
+  if (e == 0u || e == 0xffu) return static_cast<double>(f);
+  const unsigned long long d = (static_cast<unsigned long long>(b & 0x80000000u) << 32) |
+                               (static_cast<unsigned long long>(e + (1023u - 127u)) << 52) |
+                               (static_cast<unsigned long long>(b & 0x7fffffu) << 29);
+  return __longlong_as_double(static_cast<long long>(d));
+}
+
 __device__ __forceinline__ Crystal64 load64_parts(const ScanTile& t, uint32_t s) {
   Crystal64 k;
   const float4 d = t.d[s];
@@ -106,9 +118,9 @@ __device__ __forceinline__ Crystal64 load64_parts(const ScanTile& t, uint32_t s)
     for (int j = 0; j < 4; ++j) k.q[j] = t.quat64[4 * s + j];
   } else {
     const float4 a = t.a[s], q = t.q[s];
-    k.pos = d3(a.x, a.y, a.z);
-    k.dims = d3(d.x, d.y, d.z);
-    k.q[0] = q.x; k.q[1] = q.y; k.q[2] = q.z; k.q[3] = q.w;
+    k.pos = d3(f2d_exact(a.x), f2d_exact(a.y), f2d_exact(a.z));
+    k.dims = d3(f2d_exact(d.x), f2d_exact(d.y), f2d_exact(d.z));
+    k.q[0] = f2d_exact(q.x); k.q[1] = f2d_exact(q.y); k.q[2] = f2d_exact(q.z); k.q[3] = f2d_exact(q.w);
   }
   k.sens = 1.0;
   return k;
