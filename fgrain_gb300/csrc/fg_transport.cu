@@ -26,7 +26,8 @@ namespace fg {
 // absorption, ends and beginnings of bounces) runs with many lanes.  Which lane traces a photon,
 // and when, never changes its result: its draws are named by (photon, bounce, slot, tag), and its
 // hits are absorbed in rank order.
-__global__ void __launch_bounds__(256, 4) k_transport(const TileDesc* __restrict__ tiles, int ntiles,
+template <int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_transport(const TileDesc* __restrict__ tiles, int ntiles,
                                                      unsigned long long total, const uint32_t* __restrict__ order,
                                                      unsigned long long* next, uint32_t* err,
                                                      unsigned long long* stats, int lanes) {
@@ -491,12 +492,17 @@ void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long
   // Few photons are spread over all the warps that run at once, a few lanes of each: the lanes of a
   // warp take turns (they are at different rows, tests and bounces), so a warp with one photon is done
   // in a fraction of the time of one with 32 (one 64 x 64 px tri-x tile, 4,267 photons: 243 -> 137 us).
+  // Up to two photons a lane the time is that of the longest ones: three blocks of 256 per SM leave the
+  // registers that four spill (exposing 101,400 photons 502 -> 464 us; 279 k: the same; 3.8 M: transport 3.16
+  // ms with four, 3.31 with three).
   unsigned long long lanes = 32;
+  bool few = false;
   if (!walk) {
     int dev = 0, sms = 0;
     FG_CUDA(cudaGetDevice(&dev));
     FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const unsigned long long room = 32ull * sms;  // warps of the launch bounds
+    few = total <= 2ull * 32 * 32 * sms;
+    const unsigned long long room = (few ? 24ull : 32ull) * sms;  // warps of the launch bounds
     lanes = std::min<unsigned long long>((total + room - 1) / room, 32);
   }
   const unsigned long long warps = (total + lanes - 1) / lanes;
@@ -505,8 +511,8 @@ void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long
   if (walk) {
     k_transport_walk<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err, stats);
   } else {
-    k_transport<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err, stats,
-                                            static_cast<int>(lanes));
+    (few ? k_transport<3> : k_transport<4>)<<<blocks, threads, 0, st>>>(tiles_dev, ntiles, total, order, counter, err,
+                                                                        stats, static_cast<int>(lanes));
   }
   FG_CUDA(cudaGetLastError());
 }

@@ -93,3 +93,22 @@ def test_clumps_match_the_oracle(engine, name):
     np.testing.assert_array_equal(ex, np.where(cr.developed, cr.expansion, 0.0))
     assert rep.total_clumps == ref["total_clumps"]
     em.close()
+
+
+@pytest.mark.parametrize("stock,grain,side", [("t-max", 1.1, 120), ("tri-x", 2.4, 150)])
+def test_counts_do_not_depend_on_the_photons_in_flight(engine, stock, grain, side):
+    """A tile's latent photons are the same alone (a few photons a lane) and beside others (many)."""
+    params = [fg.tile_params(stock, 1 / grain, side, side + i, 1.0, 0.0, 70 + i) for i in range(16)]
+    rng = np.random.default_rng(6)
+    tiles = [rng.random((p.height_px, p.width_px)).astype(np.float32) for p in params]
+    both, photons = [], []
+    for k in (1, 16):
+        b = fg.Batch(params[:k], engine, use_graph=False)
+        b.set_exposure(tiles[:k])
+        b.run()
+        photons.append(b.wait()["photons"])
+        both.append(b.tile_crystals(0)["counts"])
+        b.close()
+    assert photons[1] > 10 * photons[0]
+    np.testing.assert_array_equal(both[0], both[1])
+    assert both[0].sum() > 1000
