@@ -179,7 +179,8 @@ __global__ void k_finalize(uint32_t n, const uint8_t* developed, const int* pare
   clump_by_id[id] = static_cast<int64_t>(rank_by_id[minid[r]]);
 }
 
-__global__ void k_maxdim(CrystalsView cv, uint32_t n, unsigned long long* out) {
+constexpr unsigned MAXDIM_T = 256;
+__global__ void __launch_bounds__(MAXDIM_T) k_maxdim(CrystalsView cv, uint32_t n, unsigned long long* out) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   double m = 0.0;
   if (s < n) {
@@ -190,8 +191,21 @@ __global__ void k_maxdim(CrystalsView cv, uint32_t n, unsigned long long* out) {
       m = (double)fmaxf(fmaxf(d.x, d.y), d.z);
     }
   }
-  // Non-negative doubles order like their bit patterns.
-  atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(m)));
+  // Non-negative doubles order like their bit patterns.  One atomic a block: one a crystal, all on one
+  // word, took 31 us for 44,000 of them.
+  auto warp_max = [](unsigned long long v) {
+    const uint32_t hi = static_cast<uint32_t>(v >> 32), h = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t l = __reduce_max_sync(0xffffffffu, hi == h ? static_cast<uint32_t>(v) : 0u);
+    return (static_cast<unsigned long long>(h) << 32) | l;
+  };
+  __shared__ unsigned long long s_max[MAXDIM_T / 32];
+  const unsigned long long w = warp_max(static_cast<unsigned long long>(__double_as_longlong(m)));
+  if ((threadIdx.x & 31u) == 0) s_max[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const unsigned long long b = warp_max(threadIdx.x < MAXDIM_T / 32 ? s_max[threadIdx.x] : 0ull);
+    if (threadIdx.x == 0) atomicMax(out, b);
+  }
 }
 
 void develop(fg_engine* e, fg_emulsion* em, const fg_dev_cfg& cfg, fg_dev_report* rep) {
@@ -214,7 +228,7 @@ void develop(fg_engine* e, fg_emulsion* em, const fg_dev_cfg& cfg, fg_dev_report
   FG_CUDA(cudaMemsetAsync(mb.p, 0, sizeof(unsigned long long), st));
   const unsigned G = grid_for(n, 256);
   const uint32_t* s2id = em->h_s2id.empty() ? nullptr : em->sorted_to_id.p;
-  k_maxdim<<<G, 256, 0, st>>>(em->view(), n, mb.p);
+  k_maxdim<<<G, MAXDIM_T, 0, st>>>(em->view(), n, mb.p);
   k_threshold<<<G, 256, 0, st>>>(em->counts.p, n, cfg.threshold_photons, cfg.filament_expansion,
                                  em->developed.p, em->exp64.p, parent.p, dc.p);
   unsigned long long mbits = 0;
