@@ -25,6 +25,7 @@ namespace {
 
 struct Taps {
   double k[3], dk[3];
+  double kk[3][3];  // products of two taps
 };
 
 Taps otf_taps(double s) {
@@ -37,6 +38,8 @@ Taps otf_taps(double s) {
   const double dg = g / (s * s * s);
   t.dk[0] = t.dk[2] = dg / (n * n);
   t.dk[1] = -2.0 * dg / (n * n);
+  for (int j = 0; j < 3; ++j)
+    for (int q = 0; q < 3; ++q) t.kk[j][q] = t.k[j] * t.k[q];
   return t;
 }
 
@@ -61,14 +64,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_otf_grads(const float* __restri
       double hv = 0.0, dh = 0.0;
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
-        const double v = row[xs[q]];
+        const double v = f2d_exact(row[xs[q]]);
         hv += tp.k[q] * v;
         dh += tp.dk[q] * v;
       }
       o += tp.k[j] * hv;
       d += tp.dk[j] * hv + tp.k[j] * dh;
     }
-    const double g = G[i];
+    const double g = f2d_exact(G[i]);
     s0 += g * o;
     s1 += g * d;
   }
@@ -89,21 +92,29 @@ __global__ void __launch_bounds__(RED_THREADS) k_otf_grads(const float* __restri
   }
 }
 
-// The partials' sums in index order (one chain of additions each, so the result does not depend on the
-// launch): the block stages them in shared memory, thread 0 adds one sum and thread 1 the other.
-// (One thread reading them from global memory took 107 us for 1,024.)
+// The partials' sums, in an order that depends on their number only (strided, then a tree).  As two chains
+// of 878 additions it took 44 us.
 __global__ void __launch_bounds__(RED_THREADS) k_sum_partials(const double* __restrict__ partial, int n, double* out) {
-  __shared__ double sh[2 * RED_THREADS];
-  double a = 0.0;
-  for (int base = 0; base < n; base += RED_THREADS) {
-    const int m = min(RED_THREADS, n - base);
-    for (int i = threadIdx.x; i < 2 * m; i += RED_THREADS) sh[i] = partial[2 * base + i];
-    __syncthreads();
-    if (threadIdx.x < 2)
-      for (int i = 0; i < m; ++i) a += sh[2 * i + threadIdx.x];
+  __shared__ double r0[RED_THREADS], r1[RED_THREADS];
+  double a = 0.0, b = 0.0;
+  for (int i = threadIdx.x; i < n; i += RED_THREADS) {
+    a += partial[2 * i];
+    b += partial[2 * i + 1];
+  }
+  r0[threadIdx.x] = a;
+  r1[threadIdx.x] = b;
+  __syncthreads();
+  for (int o = RED_THREADS / 2; o > 0; o >>= 1) {
+    if (static_cast<int>(threadIdx.x) < o) {
+      r0[threadIdx.x] += r0[threadIdx.x + o];
+      r1[threadIdx.x] += r1[threadIdx.x + o];
+    }
     __syncthreads();
   }
-  if (threadIdx.x < 2) out[threadIdx.x] = a;
+  if (threadIdx.x == 0) {
+    out[0] = r0[0];
+    out[1] = r1[0];
+  }
 }
 
 // Weight of output position o on input position i for one clamp-to-edge 3-tap pass.
@@ -123,6 +134,17 @@ __global__ void k_otf_adjoint(const float* __restrict__ G, uint32_t w, uint32_t 
   if (i >= static_cast<size_t>(w) * h) return;
   const uint32_t x = static_cast<uint32_t>(i % w), y = static_cast<uint32_t>(i / w);
   double acc = 0.0;
+  if (x > 0 && y > 0 && x + 1 < w && y + 1 < h && tp.k[0] != 0.0 && tp.k[1] != 0.0 && tp.k[2] != 0.0) {
+    // Away from the edges each tap has one weight, and the products are the launch's (FP64 instructions bound
+    // the kernel: 45 us for 449,000 px with the weights formed for each tap, 28 so).
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+      for (int dx = -1; dx <= 1; ++dx)
+        acc += tp.kk[1 - dy][1 - dx] * f2d_exact(G[(static_cast<size_t>(y) + dy) * w + x + dx]);
+    wpx[i] = static_cast<float>(-e * acc);
+    return;
+  }
   for (int dy = -1; dy <= 1; ++dy) {
     const int oy = static_cast<int>(y) + dy;
     if (oy < 0 || oy >= static_cast<int>(h)) continue;

@@ -277,6 +277,18 @@ __device__ __forceinline__ bool fcanonical_hit(float4 a, float4 q, float4 d, flo
   return fintersect(a, q, d, e, o, dir, t0, t1);
 }
 
+// A float widened to double by moving its bits (integer pipes); zero, subnormals (rare) and
+// infinities take the conversion instruction.
+__device__ __forceinline__ double f2d_exact(float f) {
+  const uint32_t b = __float_as_uint(f);
+  const uint32_t e = (b >> 23) & 0xffu;
+  if (e == 0u || e == 0xffu) return static_cast<double>(f);
+  const unsigned long long d = (static_cast<unsigned long long>(b & 0x80000000u) << 32) |
+                               (static_cast<unsigned long long>(e + (1023u - 127u)) << 52) |
+                               (static_cast<unsigned long long>(b & 0x7fffffu) << 29);
+  return __longlong_as_double(static_cast<long long>(d));
+}
+
 // 2D Morton interleave of 16-bit coordinates.
 __host__ __device__ inline uint32_t morton2_spread(uint32_t v) {
   v &= 0xffffu;

@@ -95,18 +95,6 @@ __device__ __forceinline__ void scan_origin64(const ScanTile& t, uint32_t px, ui
   oy = __dmul_rn(__dadd_rn(static_cast<double>(py), suby), t.ph);
 }
 
-// A float widened to double by moving its bits (integer pipes); zero and subnormals (T below
-// 2^-126, rare) take the conversion instruction.
-__device__ __forceinline__ double f2d_exact(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const uint32_t e = (b >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return static_cast<double>(f);
-  const unsigned long long d = (static_cast<unsigned long long>(b & 0x80000000u) << 32) |
-                               (static_cast<unsigned long long>(e + (1023u - 127u)) << 52) |
-                               (static_cast<unsigned long long>(b & 0x7fffffu) << 29);
-  return __longlong_as_double(static_cast<long long>(d));
-}
-
 __device__ __forceinline__ Crystal64 load64_parts(const ScanTile& t, uint32_t s) {
   Crystal64 k;
   const float4 d = t.d[s];
