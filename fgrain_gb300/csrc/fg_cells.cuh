@@ -52,8 +52,11 @@ inline void cells_reach(CellGrid& g, double m, bool cubes) {
 // 3.49 / 4.10 / 2.90; 0.3, 0.75, 1.5: 3.60 / 4.30 / 2.96; layers of the full depth: 5.4 / 25 / 5.4.
 constexpr double CELL_X = 0.20, CELL_Y = 1.0, CELL_Z = 2.5;
 
-// Cells of a box of w x h x d um holding about n crystals, at most 8 n + 64 of them.  False when the
-// box has no volume.
+// Cells of a box of w x h x d um holding about n crystals, at most 8 n + 64 of them.  The cells of an axis
+// are numbered in float arithmetic and those of the box in 32 bits, so an axis has at most 2^24 (their
+// numbers are exact: rounded up, the last one would name a cell past the row) and the box fewer than
+// 2^32.  False when the box has no volume.
+constexpr double CELLS_AXIS_MAX = 16777216.0, CELLS_BOX_MAX = 4294967295.0;
 inline bool cells_layout(double w, double h, double d, double n, CellGrid& g) {
   if (!(w > 0 && h > 0 && d > 0 && n > 0) || !std::isfinite(w * h * d)) return false;
   double a = std::cbrt(w * h * d / n);
@@ -62,7 +65,9 @@ inline bool cells_layout(double w, double h, double d, double n, CellGrid& g) {
     cx = std::fmax(std::floor(w / (CELL_X * a)), 1.0);
     cy = std::fmax(std::floor(h / (CELL_Y * a)), 1.0);
     cz = std::fmax(std::floor(d / (CELL_Z * a) + 0.5), 1.0);
-    if (cx * cy * cz <= 8.0 * n + 64.0) break;
+    if (cx * cy * cz <= std::fmin(8.0 * n + 64.0, CELLS_BOX_MAX) &&
+        std::fmax(std::fmax(cx, cy), cz) <= CELLS_AXIS_MAX)
+      break;
   }
   auto axis = [](CellAxis& x, double len, double cells) {
     x.n = static_cast<uint32_t>(cells);
