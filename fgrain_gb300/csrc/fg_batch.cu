@@ -28,7 +28,6 @@ namespace fg {
 void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], int gdmax, uint32_t* cells,
                     uint32_t* npts, uint32_t* done, uint32_t* err, cudaStream_t st, int sms, uint32_t wait_limit = 0,
                     const uint32_t* probe = nullptr);
-size_t bridson_smem(int gdmax);
 void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_parts, uint32_t* cells,
                        const uint32_t* npts, uint32_t* counts, cudaStream_t st);
 void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_parts, const uint32_t* cells,

@@ -188,9 +188,8 @@ __device__ __forceinline__ float3 syn_draw(int iter, int slot, int lane, uint32_
 }
 
 // An entry of the active list: the cell's region coordinates (SYN_R < 16; a region that fits in
-// shared memory has fewer than 256 layers).
-static_assert(SYN_R <= 16 && 256 * SYN_R * (SYN_R + 1) * 4 + 252 * SYN_B * SYN_B * 2 > 220 * 1024,
-              "4 + 4 + 8 bits hold a position");
+// shared memory has at most 256 layers).
+static_assert(SYN_R <= 16 && bridson_smem(253) > 220 * 1024, "4 + 4 + 8 bits hold a position");
 __device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
   return static_cast<uint16_t>(rx | ry << 4 | rz << 8);
 }
@@ -205,8 +204,10 @@ __device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
 // 2048 x 2048 px tri-x one.
 //
 // Launch bounds of 8 CTAs per SM (32 registers): more columns in flight hide the round's barriers.
-// A column with its one-cell spill and the halo stages 14 x 14 cells per layer, so eight CTAs fit
-// in the SM's 228 KB of shared memory for depths up to 23 cells.
+// A column with its one-cell spill and the halo stages 14 x 14 cells per layer, and its list of active
+// points has an entry for each that can fit (26 a layer; with one for each of the 64 cells seven CTAs
+// ran at 23 cells, tri-x-1600's depth), so eight CTAs fit in the SM's 228 KB of shared memory for
+// depths up to 24 cells.
 //
 // FEW: with few columns in flight the latency of a round counts instead (5,600 cycles, of which 1,950
 // are the resolution by one warp).  4 CTAs per SM leave 64 registers, and the seven warps that wait
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
   extern __shared__ uint32_t syn_sm[];
   uint32_t* grid = syn_sm;                                   // SYN_R^2 * nz cell words
   uint32_t* rows = grid + SYN_R * SYN_R * nz;                // SYN_R * nz occupancy rows (syn_mark)
-  uint16_t* active = reinterpret_cast<uint16_t*>(rows + SYN_R * nz);  // SYN_B^2 * (nz - 4)
+  uint16_t* active = reinterpret_cast<uint16_t*>(rows + SYN_R * nz);  // syn_active_cap(nz - 4)
   __shared__ int s_nact, s_wsum[SYN_WARPS];
   __shared__ int s_ncom;  // points this column commits (each fills one empty cell of its tile)
   __shared__ int4 s_pick[SYN_WARPS / 4];   // the steps' picks
@@ -242,6 +243,10 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
   __shared__ int4 s_near[27];
   __shared__ uint4 s_key[5];              // Philox round keys
   __shared__ float3 s_off[FEW ? 32 : 1];  // the next round's draws of the resolving warp
+  static_assert(FEW || 8 * (bridson_smem(24) + sizeof(s_nact) + sizeof(s_wsum) + sizeof(s_ncom) + sizeof(s_pick) +
+                            sizeof(s_win) + sizeof(s_rmask) + sizeof(s_cxy) + sizeof(s_cz) + sizeof(s_near) +
+                            sizeof(s_key) + sizeof(s_off) + 1024) <= 228 * 1024,
+                "eight CTAs of 24 cells (and 1 KB each) in an SM's shared memory");
 
   // Column of this CTA: colour class, tile, then the j-th column of this class in that tile.
   const uint32_t cb[4] = {class_base.x, class_base.y, class_base.z, class_base.w};
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
   const uint32_t colkey = by * t.nbx + bx;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ncell = SYN_R * SYN_R * nz;
-  const int acap = SYN_B * SYN_B * (nz - 4);  // active list capacity: one entry per column cell
+  const int acap = syn_active_cap(nz - 4);  // active list capacity
   uint32_t* tc = cells + t.cell_base;
 
   // Wait for the neighbouring columns of lower classes.
@@ -344,10 +349,16 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
     __syncthreads();
     int off = s_nact;
     for (int w = 0; w < warp; ++w) off += s_wsum[w];
-    if (o) active[off + __popc(m & ((1u << lane) - 1u))] = syn_pos(lx + SYN_HALO, ly + SYN_HALO, lz + 2);
+    const int at = off + __popc(m & ((1u << lane) - 1u));
+    // (Past the capacity only after a wait that gave up: the neighbours' points may then be too close.)
+    if (o && index_ok(at < acap, err, SITE_SYN_ACTIVE, at, blockIdx.x))
+      active[at] = syn_pos(lx + SYN_HALO, ly + SYN_HALO, lz + 2);
     __syncthreads();
-    if (tid == 0)
-      for (int w = 0; w < SYN_WARPS; ++w) s_nact += s_wsum[w];
+    if (tid == 0) {
+      int n = s_nact;
+      for (int w = 0; w < SYN_WARPS; ++w) n += s_wsum[w];
+      s_nact = min(n, acap);
+    }
     __syncthreads();
   }
   // An empty column starts from one random point (poisson.rs:46-57), up to 30 tries.
@@ -810,12 +821,6 @@ __global__ void __launch_bounds__(PART_T) k_emit(const SynthTile* __restrict__ t
   if (lane < fill) emit(q[lane]);
 }
 
-}  // namespace fg
-
-namespace fg {
-
-size_t bridson_smem(int gdmax);
-
 // Host wrappers (launch on `st`; all buffers preallocated so the sequence can be graph-captured).
 // cols[c] columns of class c; done holds one flag per column (zeroed here).
 void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], int gdmax, uint32_t* cells,
@@ -832,11 +837,6 @@ void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], 
   kernel<<<total, SYN_WARPS * 32, smem, st>>>(tiles, ntiles, cb, nz, cells, npts, done, err,
                                                   wait_limit ? wait_limit : (1u << 22), probe);
   FG_CUDA(cudaGetLastError());
-}
-
-size_t bridson_smem(int gdmax) {
-  return static_cast<size_t>(SYN_R) * (SYN_R + 1) * (gdmax + 4) * sizeof(uint32_t) +
-         static_cast<size_t>(SYN_B) * SYN_B * gdmax * sizeof(uint16_t);
 }
 
 static unsigned part_blocks(unsigned long long max_parts) {

@@ -41,6 +41,18 @@ constexpr int32_t SYN_R2 = 3 * SYN_Q * SYN_Q;  // r^2 with r = sqrt(3) cells
 constexpr int32_t SYN_R2X = SYN_R2 + 128;
 constexpr uint32_t OCC = 0x80000000u;
 
+// Points that a column of SYN_B x SYN_B x gd cells can hold, all at least r = sqrt(3) cells apart: the
+// balls of radius r / 2 around them do not overlap and lie in the column's box grown by r / 2 on every
+// side, and no packing of equal balls fills more than pi / sqrt(18) of space (Hales 2005; copies of
+// the box side by side make the packing a periodic one).  That is 25.78 gd + 44.65.
+__host__ __device__ constexpr int syn_active_cap(int gd) { return 26 * gd + 45; }
+// Dynamic shared memory of k_bridson for columns of gd cells: the staged cells and their occupancy rows
+// (with two empty layers at either end), and the active list.
+constexpr size_t bridson_smem(int gd) {
+  return static_cast<size_t>(SYN_R) * (SYN_R + 1) * (gd + 4) * sizeof(uint32_t) +
+         static_cast<size_t>(syn_active_cap(gd)) * sizeof(uint16_t);
+}
+
 __host__ __device__ inline double bridson_density(double W, double H, double D, double r) {
   return (0.57793168 + 0.11306788 * r * (2.0 / W + 2.0 / H + 2.0 / D)) / (r * r * r);
 }
