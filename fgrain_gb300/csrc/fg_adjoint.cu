@@ -218,6 +218,7 @@ fg_status fg_scan_backward(fg_engine* e, const fg_emulsion* em, const fg_scan_cf
   return guard(e, [&] {
     FG_REQUIRE(em && cfg && dL_dsignal, "null argument");
     FG_REQUIRE(std::isfinite(exposure), "exposure multiplier must be finite");
+    (void)scan_grid(*cfg);  // before anything is launched over its pixels
     cudaStream_t st = e->stream;
     begin_call(e);
     const Taps tp = otf_taps(otf_sigma);

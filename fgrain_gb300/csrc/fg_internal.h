@@ -344,6 +344,8 @@ void begin_call(fg_engine* e);
 void end_call(fg_engine* e);
 float elapsed(cudaEvent_t a, cudaEvent_t b);
 
+// Strata per axis of a scan's pixels; refuses a size or a number of samples that cannot be scanned.
+uint32_t scan_grid(const fg_scan_cfg& cfg);
 void scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed,
           const float* sigma_sorted, const ScanOut& out);
 // g_sorted[s] += sum over the rays of each pixel p of wpx[p] / spp * T_ray * chord_s (device

@@ -806,14 +806,18 @@ struct ScanPlan {
   unsigned nbins = 0, threads = 0;
 };
 
+uint32_t scan_grid(const fg_scan_cfg& cfg) {
+  const uint32_t spp_req = std::max<uint32_t>(cfg.samples_per_pixel, 1);
+  const uint32_t g = static_cast<uint32_t>(std::lround(std::sqrt(static_cast<double>(spp_req))));
+  FG_REQUIRE(std::max<uint32_t>(g * g, 1) <= SCAN_THREADS, "samples_per_pixel too large (at most 256 strata)");
+  FG_REQUIRE(cfg.width_px > 0 && cfg.height_px > 0, "scan size must be positive");
+  return g;
+}
+
 static void plan_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg& cfg, uint64_t seed,
                       const float* sigma_sorted, const ScanOut& out, ScanPlan& P) {
   cudaStream_t st = e->stream;
-  const uint32_t spp_req = std::max<uint32_t>(cfg.samples_per_pixel, 1);
-  const uint32_t g = static_cast<uint32_t>(std::lround(std::sqrt(static_cast<double>(spp_req))));
-  const uint32_t a = std::max<uint32_t>(g * g, 1);
-  FG_REQUIRE(a <= SCAN_THREADS, "samples_per_pixel too large (at most 256 strata)");
-  FG_REQUIRE(cfg.width_px > 0 && cfg.height_px > 0, "scan size must be positive");
+  const uint32_t g = scan_grid(cfg), a = std::max<uint32_t>(g * g, 1);
   build_emulsion_tree(e, em, true, P.tree, P.tree_list, false);
   ScanTile& t = P.t;
   t = ScanTile{};
