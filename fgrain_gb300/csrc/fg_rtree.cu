@@ -1044,8 +1044,8 @@ __global__ void __launch_bounds__(RT_CTA_T, 4) k_rt_cta(RtArgs A) {
       __syncthreads();
     }
     for (int x = tid; x < n; x += RT_CTA_T) A.ridx[s + x] = S.idx[x];
+    __syncthreads();  // the last level's leaves have joined S.maxdep; the next job may write the rest
     if (tid == 0) atomicMax(&A.tiles[t].depth, S.maxdep);
-    __syncthreads();
   }
 }
 
