@@ -31,8 +31,7 @@ void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], 
 void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long max_parts, uint32_t* cells,
                        const uint32_t* npts, uint32_t* counts, cudaStream_t st);
 void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_parts, const uint32_t* cells,
-                 const uint32_t* scan, float4* A, float4* Q, float4* D, uint64_t* keys, uint32_t* err,
-                 cudaStream_t st);
+                 const uint32_t* scan, float4* A, float4* Q, float4* D, uint32_t* err, cudaStream_t st);
 void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long long total,
                             const uint32_t* order, unsigned long long* counter, uint32_t* err,
                             unsigned long long* stats, unsigned blocks, unsigned threads, cudaStream_t st,
@@ -316,7 +315,6 @@ struct fg_batch {
   unsigned long long maxparts = 0;  // the largest tile's
   DBuf<float4> A, Q, D;
   CellBufs tcells;          // the crystals in cells, with their rank in the tree's walk order
-  DBuf<uint64_t> keys;
   RTreeBufs rt;             // the reference tree of every tile: over its crystals, then its developed ones
   DBuf<RTile> rt_scan;      // the tree tiles of the scan's build (developed crystals, their expansion)
   DBuf<int> parent;
@@ -550,8 +548,7 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
   FG_CUDA(cudaMemsetAsync(B->flags.p + B->nparts, 0, sizeof(uint32_t), st));
   launch_synth_post(B->d_syn.p, nt, B->maxparts, B->cells.p, B->npts.p, B->flags.p, st);
   cub_scan(B, B->flags.p, B->slot_scan.p, B->nparts + 1, st);
-  launch_emit(B->d_syn.p, nt, B->maxparts, B->cells.p, B->slot_scan.p, B->A.p, B->Q.p, B->D.p, B->keys.p, e->d_err,
-              st);
+  launch_emit(B->d_syn.p, nt, B->maxparts, B->cells.p, B->slot_scan.p, B->A.p, B->Q.p, B->D.p, e->d_err, st);
   k_set_n<<<grid_for(B->ntiles, 128), 128, 0, st>>>(B->d_syn.p, nt, B->slot_scan.p, B->d_bt.p, B->d_td.p, B->d_sc.p,
                                                     B->ncrys.p, B->rt.tiles.p);
   FG_CUDA(cudaGetLastError());
@@ -790,7 +787,6 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   B->A.alloc(std::max<unsigned long long>(cap, 1), st);
   B->Q.alloc(std::max<unsigned long long>(cap, 1), st);
   B->D.alloc(std::max<unsigned long long>(cap, 1), st);
-  B->keys.alloc(std::max<unsigned long long>(cap, 1), st);
   B->parent.alloc(std::max<unsigned long long>(cap, 1), st);
   B->counts.alloc(std::max<unsigned long long>(cap, 1), st);
   B->size.alloc(std::max<unsigned long long>(cap, 1), st);
@@ -893,11 +889,11 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   uint32_t bits = 0;
   while ((1u << bits) < static_cast<uint32_t>(std::ceil(side))) ++bits;
   const unsigned long long px = static_cast<unsigned long long>(p.width_px) * p.height_px;
-  // Per crystal slot: records 48 (and 96 in the transport's cells), key 8, links and flags 36,
+  // Per crystal slot: records 48 (and 96 in the transport's cells), links and flags 36,
   // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
   // 152 B (plus slack); transport cells 8 B; synthesis cells 4 B; parts 8 B; photon order; images.
-  return static_cast<unsigned long long>(s.ccap) * 620ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
+  return static_cast<unsigned long long>(s.ccap) * 612ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          8ull * syn_parts(s) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
@@ -907,9 +903,9 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
 extern "C" {
 
 // VirtualEmulsionLayer::synthesize (emulsion.rs:155-220) on the device: the tile synthesis of this
-// file over the whole emulsion as one tile, then the LBVH.  Crystal ids are the Morton slot order
-// of the synthesis (the reference numbers crystals in its sampler's output order, which the random
-// streams do not pin either).
+// file over the whole emulsion as one tile, then the reference's tree and the
+// cells.  Crystal ids are the Morton slot order of the synthesis (the reference numbers crystals in its
+// sampler's output order, which the random streams do not pin either).
 fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint64_t seed, fg_emulsion** out) {
   if (!out) return FG_ERR_INVALID_ARG;
   *out = nullptr;
@@ -950,7 +946,6 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     const unsigned long long np = syn_parts(s);
     DBuf<uint32_t> cells(ncells, st), npts(1, st), flags(np + 1ull, st), scan(np + 1ull, st);
     DBuf<float4> A(s.ccap, st), Q(s.ccap, st), D(s.ccap, st);
-    DBuf<uint64_t> keys(s.ccap, st);
     FG_CUDA(cudaMemsetAsync(cells.p, 0, ncells * sizeof(uint32_t), st));
     FG_CUDA(cudaMemsetAsync(npts.p, 0, sizeof(uint32_t), st));
     DBuf<uint32_t> coldone(std::max(cols[0] + cols[1] + cols[2] + cols[3], 1u), st);
@@ -958,7 +953,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     FG_CUDA(cudaMemsetAsync(flags.p + np, 0, sizeof(uint32_t), st));
     launch_synth_post(d_syn.p, 1, np, cells.p, npts.p, flags.p, st);
     exclusive_scan_u32(flags.p, scan.p, np + 1ull, st);
-    launch_emit(d_syn.p, 1, np, cells.p, scan.p, A.p, Q.p, D.p, keys.p, e->d_err, st);
+    launch_emit(d_syn.p, 1, np, cells.p, scan.p, A.p, Q.p, D.p, e->d_err, st);
     uint32_t n = 0;
     FG_CUDA(cudaMemcpyAsync(&n, scan.p + np, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     FG_CUDA(cudaStreamSynchronize(st));

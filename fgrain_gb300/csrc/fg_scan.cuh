@@ -26,7 +26,7 @@ constexpr int SCAN_CH = 128;        // crystals staged per pass
 constexpr int SCAN_THREADS = 256;   // rays per CTA (bin_px^2 * strata)
 
 // Bin-independent part of a developed crystal's staging, derived once per crystal in FP64 and
-// rounded (k_scan_prep): each bin that lists the crystal only adds its centre relative to the
+// rounded (k_scan_prep_list): each bin that lists the crystal only adds its centre relative to the
 // bin's corner.  160 bytes, read with vector loads.
 struct __align__(16) ScanPrep {
   // Centre x, y (um) as the scan sees it, and the x and y extent of the crystal's leaf box in the

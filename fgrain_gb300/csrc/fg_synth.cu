@@ -703,11 +703,10 @@ __global__ void __launch_bounds__(PART_T) k_thin_count(const SynthTile* __restri
   }
 }
 
-// Crystal k of a tile at compaction slot sl (cell x, y, z): position from the fixed-point cell
+// Crystal k of a tile, the one of cell (x, y, z): position from the fixed-point cell
 // word, attributes from the tile's Philox stream keyed by the cell (emulsion.rs:162-200).
-__device__ __forceinline__ void emit_crystal(const SynthTile& t, const uint32_t* __restrict__ cells, uint32_t sl,
-                                             uint32_t x, uint32_t y, uint32_t z, uint32_t k, float4* A, float4* Q,
-                                             float4* D, uint64_t* keys) {
+__device__ __forceinline__ void emit_crystal(const SynthTile& t, const uint32_t* __restrict__ cells, uint32_t x,
+                                             uint32_t y, uint32_t z, uint32_t k, float4* A, float4* Q, float4* D) {
   const uint32_t lin = (z * t.gh + y) * t.gw + x;
   const uint32_t w = cells[t.cell_base + lin];
   const float px = static_cast<float>(static_cast<int>(x) * SYN_Q + static_cast<int>(w & 1023u)) * (t.cell / SYN_Q);
@@ -748,7 +747,6 @@ __device__ __forceinline__ void emit_crystal(const SynthTile& t, const uint32_t*
   A[o] = make_float4(px, py, pz, sens);
   Q[o] = q;
   D[o] = d;
-  keys[o] = sl;
 }
 
 // The crystals of each part in slot order (slot_cell), numbered after the points of the earlier parts
@@ -763,7 +761,7 @@ __device__ __forceinline__ void emit_crystal(const SynthTile& t, const uint32_t*
 __global__ void __launch_bounds__(PART_T) k_emit(const SynthTile* __restrict__ tiles,
                                                  const uint32_t* __restrict__ cells,
                                                  const uint32_t* __restrict__ scan, float4* A, float4* Q,
-                                                 float4* D, uint64_t* keys, uint32_t* err) {
+                                                 float4* D, uint32_t* err) {
   const SynthTile& t = tiles[blockIdx.y];
   const uint32_t nparts = syn_parts(t);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
@@ -781,7 +779,7 @@ __global__ void __launch_bounds__(PART_T) k_emit(const SynthTile* __restrict__ t
     }
     uint32_t x, y, z;
     slot_cell(t, c.y, x, y, z);
-    emit_crystal(t, cells, c.y, x, y, z, c.x, A, Q, D, keys);
+    emit_crystal(t, cells, x, y, z, c.x, A, Q, D);
   };
   for (uint32_t p = blockIdx.x * (PART_T / 32) + warp; p < nparts; p += gridDim.x * (PART_T / 32)) {
     const uint32_t k0 = scan[t.slot_base + p];
@@ -852,11 +850,10 @@ void launch_synth_post(const SynthTile* tiles, int ntiles, unsigned long long ma
 }
 
 void launch_emit(const SynthTile* tiles, int ntiles, unsigned long long max_parts, const uint32_t* cells,
-                 const uint32_t* scan, float4* A, float4* Q, float4* D, uint64_t* keys, uint32_t* err,
-                 cudaStream_t st) {
+                 const uint32_t* scan, float4* A, float4* Q, float4* D, uint32_t* err, cudaStream_t st) {
   if (ntiles == 0) return;
   FG_REQUIRE(ntiles <= 65535, "too many tiles for one launch");
-  k_emit<<<dim3(part_blocks(max_parts), ntiles), PART_T, 0, st>>>(tiles, cells, scan, A, Q, D, keys, err);
+  k_emit<<<dim3(part_blocks(max_parts), ntiles), PART_T, 0, st>>>(tiles, cells, scan, A, Q, D, err);
   FG_CUDA(cudaGetLastError());
 }
 
