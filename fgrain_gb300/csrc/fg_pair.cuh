@@ -8,6 +8,7 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace fg {
@@ -28,6 +29,34 @@ namespace fg {
 struct Pair {
   float h, l;  // |l| <= ulp(h) / 2
 };
+
+PAIR_FN uint32_t pair_bits(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t b;
+  std::memcpy(&b, &f, sizeof(b));
+  return b;
+#endif
+}
+PAIR_FN float pair_float(uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(b);
+#else
+  float f;
+  std::memcpy(&f, &b, sizeof(f));
+  return f;
+#endif
+}
+PAIR_FN uint64_t pair_bits64(double v) {
+#ifdef __CUDA_ARCH__
+  return static_cast<uint64_t>(__double_as_longlong(v));
+#else
+  uint64_t b;
+  std::memcpy(&b, &v, sizeof(b));
+  return b;
+#endif
+}
 
 constexpr float PAIR_ERR = 3.637978807091713e-12f;  // 2^-38, relative
 
@@ -78,23 +107,13 @@ PAIR_FN bool pair_round(Pair a, float& r) {
 }
 
 // log of a positive normal float plus a low part: x = 2^k m, m in [sqrt(1/2), sqrt(2));
-// log m = 2 atanh(s), s = (m - 1) / (m + 1), |s| < .1716.
+// log m = 2 atanh(s), s = (m - 1) / (m + 1), |s| < .1716.  (From 2^127.5 on, k is 128 and the low part's
+// scale overflows: the result is a NaN, which pair_round does not settle.)
 PAIR_FN Pair pair_log(float x, float xl = 0.0f) {
-#ifdef __CUDA_ARCH__
-  const int b = __float_as_int(x);
-#else
-  union { float f; int i; } v{x};
-  const int b = v.i;
-#endif
+  const int b = static_cast<int>(pair_bits(x));
   const int k = (b - 0x3f3504f3) >> 23;  // 0x3f3504f3: sqrt(1/2)
-#ifdef __CUDA_ARCH__
-  const float m = __int_as_float(b - (k << 23)), up = __int_as_float((127 - k) << 23);
-#else
-  v.i = b - (k << 23);
-  const float m = v.f;
-  v.i = (127 - k) << 23;
-  const float up = v.f;
-#endif
+  const float m = pair_float(static_cast<uint32_t>(b - (k << 23)));
+  const float up = pair_float(static_cast<uint32_t>(127 - k) << 23);
   const float f = PAIR_SUB(m, 1.0f), fl = PAIR_MUL(xl, up);  // f is exact
   const Pair n = pair_fast(f, fl);
   Pair d = pair_sum(2.0f, f);
@@ -136,13 +155,7 @@ PAIR_FN Pair pair_exp(float x) {
   t = pair_mul(t, t);
   t = pair_mul(t, t);
   t = pair_mul(t, t);
-  const int k = static_cast<int>(kf);
-#ifdef __CUDA_ARCH__
-  const float up = __int_as_float((127 + k) << 23);
-#else
-  union { int i; float f; } v{(127 + k) << 23};
-  const float up = v.f;
-#endif
+  const float up = pair_float(static_cast<uint32_t>(127 + static_cast<int>(kf)) << 23);
   return Pair{PAIR_MUL(t.h, up), PAIR_MUL(t.l, up)};
 }
 
@@ -178,10 +191,32 @@ PAIR_FN void pair_sincos(float x, Pair& sn, Pair& cs) {
   cs = (k + 1) & 2 ? Pair{-b.h, -b.l} : b;
 }
 
+// hi = v rounded to float, lo = v - hi (exact) rounded to float.  In integer arithmetic: hi takes the
+// upper 24 bits of v's 53, lo is the signed rest of at most 2^28.  Zero and magnitudes outside 2^-60 ..
+// 2^120 are converted.
+PAIR_FN void split64(double v, float& hi, float& lo) {
+  const uint64_t b = pair_bits64(v);
+  const uint32_t h = static_cast<uint32_t>(b >> 32), l = static_cast<uint32_t>(b);
+  const uint32_t e = (h >> 20) & 0x7ffu;
+  if (e - 963u > 180u) {
+    hi = static_cast<float>(v);
+    lo = static_cast<float>(v - static_cast<double>(hi));
+    return;
+  }
+  const uint32_t q = ((h & 0xfffffu) << 3) | (l >> 29), r = l & 0x1fffffffu;  // q: 23 bits below the leading one
+  const bool up = r > 0x10000000u || (r == 0x10000000u && (q & 1u));           // to nearest, ties to even
+  const int d = static_cast<int>(r) - (up ? 0x20000000 : 0);
+  hi = pair_float((h & 0x80000000u) | (((e - 896u) << 23) + q + (up ? 1u : 0u)));
+  // d in units of 2^(e - 1075); a rest of zero is +0 whatever the sign.
+  lo = PAIR_MUL(static_cast<float>(static_cast<int>(h) < 0 ? -d : d), pair_float((e - 948u) << 23));
+}
+
 // n / d of FP64 values, given also as pairs (to 2^-48), rounded to float.
 PAIR_FN float pair_quotf(double n, double d, Pair np, Pair dp) {
   float r;
-  const float lo = 8.7e-19f, hi = 1.1e18f;  // 2^-60, 2^60: the low parts stay normal floats
+  // About 2^-50, 2^50: quotients from 2^-100 on, whose low parts a float's smallest step (2^-149) holds to
+  // 2^-49 of the quotient.  (With 2^-60 and 2^60, quotients below 2^-115 could round the wrong way.)
+  const float lo = 8.9e-16f, hi = 1.1e15f;
   if (fabsf(np.h) > lo && fabsf(np.h) < hi && fabsf(dp.h) > lo && fabsf(dp.h) < hi && pair_round(pair_div(np, dp), r)) return r;
   return static_cast<float>(n / d);
 }
@@ -203,6 +238,17 @@ PAIR_FN void pair_sincosf(float x, float& sn, float& cs) {
   const bool in = fabsf(x) <= 8.0f;
   if (!(in && pair_round(s, sn))) sn = static_cast<float>(sin(static_cast<double>(x)));
   if (!(in && pair_round(c, cs))) cs = static_cast<float>(cos(static_cast<double>(x)));
+}
+
+// The density -log10(clamp(T, 1e-4, 1)) + 0.05 of a transmittance.
+PAIR_FN float pair_densityf(float T) {
+  float r;
+  const bool in = T > 1.0001e-4f && T <= 1.0f;
+  const Pair v = pair_add(pair_mul(pair_log(in ? T : 1.0f), Pair{-0.434294492f, 1.010305e-08f}),
+                          Pair{0.0500000007f, -7.45058071e-10f});
+  if (in && pair_round(v, r)) return r;
+  const double tc = fmin(fmax(static_cast<double>(T), 1e-4), 1.0);
+  return tc == 1e-4 ? 4.05f : (tc == 1.0 ? 0.05f : static_cast<float>(-log10(tc) + 0.05));
 }
 
 }  // namespace fg

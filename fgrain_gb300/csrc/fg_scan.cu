@@ -59,24 +59,6 @@ __device__ __forceinline__ void two_prod(float a, float b, float& p, float& e) {
   p = a * b;
   e = fmaf(a, b, -p);
 }
-// hi = v rounded to float, lo = v - hi (exact) rounded to float.  In integer arithmetic: hi takes the
-// upper 24 bits of v's 53, lo is the signed rest of at most 2^28 (the FP64 pipe, with the conversions it
-// also does, bounds the staging terms).  Zero and magnitudes outside 2^-60 .. 2^120 take it still.
-__device__ __forceinline__ void split64(double v, float& hi, float& lo) {
-  const uint32_t h = static_cast<uint32_t>(__double2hiint(v)), l = static_cast<uint32_t>(__double2loint(v));
-  const uint32_t e = (h >> 20) & 0x7ffu;
-  if (e - 963u > 180u) {
-    hi = static_cast<float>(v);
-    lo = static_cast<float>(v - static_cast<double>(hi));
-    return;
-  }
-  const uint32_t q = ((h & 0xfffffu) << 3) | (l >> 29), r = l & 0x1fffffffu;  // q: 23 bits below the leading one
-  const bool up = r > 0x10000000u || (r == 0x10000000u && (q & 1u));           // to nearest, ties to even
-  const int d = static_cast<int>(r) - (up ? 0x20000000 : 0);
-  hi = __uint_as_float((h & 0x80000000u) | (((e - 896u) << 23) + q + (up ? 1u : 0u)));
-  // d in units of 2^(e - 1075); a rest of zero is +0 whatever the sign.
-  lo = __fmul_rn(__int2float_rn(static_cast<int>(h) < 0 ? -d : d), __uint_as_float((e - 948u) << 23));
-}
 
 // (ah + al) - (bh + bl) as a float pair, to about 2^-48 of the operands.
 __device__ __forceinline__ void pair_sub(float ah, float al, float bh, float bl, float& h, float& l) {
@@ -761,17 +743,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 4) k_scan_adjoint(const ScanTile
 __global__ void k_density(float* __restrict__ d, unsigned long long n) {
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   for (unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; i < n;
-       i += stride) {
-    const float T = d[i];
-    float r;
-    const bool in = T > 1.0001e-4f && T <= 1.0f;
-    const Pair v = pair_add(pair_mul(pair_log(in ? T : 1.0f), Pair{-0.434294492f, 1.010305e-08f}), Pair{0.0500000007f, -7.45058071e-10f});
-    if (!(in && pair_round(v, r))) {
-      const double tc = fmin(fmax(static_cast<double>(T), 1e-4), 1.0);
-      r = tc == 1e-4 ? 4.05f : (tc == 1.0 ? 0.05f : static_cast<float>(-log10(tc) + 0.05));
-    }
-    d[i] = r;
-  }
+       i += stride)
+    d[i] = pair_densityf(d[i]);
 }
 
 void launch_density(float* d, unsigned long long n, cudaStream_t st) {
