@@ -53,10 +53,10 @@ inline void cells_reach(CellGrid& g, double m, bool cubes) {
 constexpr double CELL_X = 0.20, CELL_Y = 1.0, CELL_Z = 2.5;
 
 // Cells of a box of w x h x d um holding about n crystals, at most 8 n + 64 of them.  The cells of an axis
-// are numbered in float arithmetic and those of the box in 32 bits, so an axis has at most 2^24 (their
-// numbers are exact: rounded up, the last one would name a cell past the row) and the box fewer than
-// 2^32.  False when the box has no volume.
-constexpr double CELLS_AXIS_MAX = 16777216.0, CELLS_BOX_MAX = 4294967295.0;
+// are numbered in float arithmetic and those of the box in 32 bits, which the prefix sum over an emulsion's
+// cells counts with a sign, so an axis has at most 2^24 (their numbers are exact: rounded up, the last one
+// would name a cell past the row) and the box fewer than 2^31.  False when the box has no volume.
+constexpr double CELLS_AXIS_MAX = 16777216.0, CELLS_BOX_MAX = 2147483000.0;
 inline bool cells_layout(double w, double h, double d, double n, CellGrid& g) {
   if (!(w > 0 && h > 0 && d > 0 && n > 0) || !std::isfinite(w * h * d)) return false;
   double a = std::cbrt(w * h * d / n);

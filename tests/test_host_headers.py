@@ -28,8 +28,8 @@ def run(tmp_path_factory):
 
 def test_every_coordinate_names_a_cell_of_its_axis(run):
     """cells_layout over boxes from a cube to a thread a million times as long as wide: the last cell's
-    number is exact in float (a coordinate is clamped to it), the box's cells are numbered in 32 bits,
-    and there are at most 8 n + 64 of them."""
+    number is exact in float (a coordinate is clamped to it), the box's cells and one more are counted in
+    31 bits, and there are at most 8 n + 64 of them."""
     r = run("cells", r"""
 #include <cstdio>
 #include "fg_cells.cuh"
@@ -46,7 +46,7 @@ int main() {
           const double cells = 1.0 * g.x.n * g.y.n * g.z.n;
           for (const fg::CellAxis* a : {&g.x, &g.y, &g.z})
             if (a->n < 1 || static_cast<double>(a->last) != a->n - 1.0) ++bad;
-          if (cells > 8.0 * n + 64.0 || cells >= 4294967296.0) ++bad;
+          if (cells > 8.0 * n + 64.0 || cells + 1.0 >= 2147483648.0) ++bad;
         }
   std::printf("{\"bad\": %d, \"boxes\": %d}\n", bad, boxes);
 }
