@@ -527,9 +527,8 @@ void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long
 constexpr double CELLS_MAX_REACH = 1.0;   // mean spacings
 constexpr uint32_t CELLS_MAX_COUNT = 16;  // crystals in one cell (half a crystal on average)
 
-void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
+static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   cudaStream_t st = e->stream;
-  em->grid = CellGrid{};
   const uint32_t n = em->n;
   CellGrid g{};
   if (!n || !cells_layout(em->cfg.width, em->cfg.height, em->cfg.depth, n, g)) return;
@@ -558,9 +557,23 @@ void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
     em->cells = CellBufs{};
     return;
   }
-  em->grid = g;
   em->grid_dev.alloc(1, st);
+  em->grid = g;
   FG_CUDA(cudaMemcpyAsync(em->grid_dev.p, &em->grid, sizeof(CellGrid), cudaMemcpyHostToDevice, st));
+}
+
+// The cells take about 110 bytes a crystal over the tree's; where those cannot be had the set keeps the walk.
+void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
+  em->grid = CellGrid{};
+  try {
+    make_emulsion_cells(e, em);
+  } catch (const Error& x) {
+    if (x.st != FG_ERR_OOM) throw;
+    (void)cudaGetLastError();
+    em->cells = CellBufs{};
+    em->grid_dev.release();
+    em->grid = CellGrid{};
+  }
 }
 
 void expose(fg_engine* e, fg_emulsion* em, const float* tile_dev, uint32_t tw, uint32_t th,

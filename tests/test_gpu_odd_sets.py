@@ -1,0 +1,78 @@
+"""Sets and settings at the limits of what the calls accept: emulsions for whose cells there is no memory
+left."""
+import numpy as np
+import pytest
+
+import fgrain_gb300 as fg
+from fgrain_gb300 import _abi
+
+pytestmark = pytest.mark.gpu
+
+SIZE = (30.0, 28.0, 12.0)
+
+
+def lattice(radius=0.5, morph=0):
+    """A jittered lattice of about 4,300 crystals: positions, half-sizes, quaternions and the film's
+    configuration."""
+    rng = np.random.default_rng(3)
+    k = [int(v / 1.3) for v in SIZE]
+    g = np.stack(np.meshgrid(*[np.arange(q) for q in k], indexing="ij"), -1).reshape(-1, 3)
+    pos = (g + 0.5 + rng.uniform(-0.12, 0.12, g.shape)) * (np.array(SIZE) / k)
+    quat = rng.normal(size=(len(pos), 4))
+    quat /= np.linalg.norm(quat, axis=1, keepdims=True)
+    cfg = fg.EmulsionConfig(SIZE, 1.0, 0.5, 0.2, fg.Morphology(morph), 1.0, fg.GelatinOptics(), 1.0)
+    return cfg, pos, np.full((len(pos), 3), radius), quat
+
+
+def smallest_budget(make):
+    """The least device budget (to 4 KB) under which make() gives an emulsion, and that emulsion: it has
+    no cells, since what they need comes on top of everything else."""
+    lib = _abi.load()
+    lo, hi = 0, 1 << 28
+    try:
+        while hi - lo > 4096:
+            mid = (lo + hi) // 2
+            lib.fg_set_device_budget(mid)
+            try:
+                make().close()
+                hi = mid
+            except fg.GpuError as x:
+                assert x.status == _abi.FG_ERR_OOM
+                lo = mid
+        lib.fg_set_device_budget(hi)
+        return hi, make()
+    finally:
+        lib.fg_set_device_budget(0)
+
+
+def counts(em):
+    tile = np.random.default_rng(4).random((32, 32)).astype(np.float32)
+    em.set_latent_counts(np.zeros(len(em), np.uint32))
+    fg.expose_emulsion(em, tile, fg.ExposureConfig(20.0, 0.12, 1.3, 48), 7)
+    return em.latent_counts()
+
+
+# Bytes a crystal without cells: records (also in FP64, and as they came, when uploaded), state and the
+# tree with its walk records; cells take about 110 more.
+@pytest.mark.parametrize("kind,bytes_per_crystal", [("uploaded", 600), ("synthesized", 470)])
+def test_an_emulsion_without_room_for_cells_keeps_the_walk(engine, kind, bytes_per_crystal):
+    cfg, pos, dims, quat = lattice()
+
+    def make():
+        if kind == "uploaded":
+            return fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(len(pos)), engine=engine)
+        return fg.VirtualEmulsionLayer.synthesize(fg.EmulsionConfig.preset("tri-x", 40.0, 40.0), 3, engine)
+
+    budget, tight = smallest_budget(make)
+    roomy = make()
+    assert budget <= bytes_per_crystal * len(roomy) + (1 << 16)
+    a, b = counts(tight), counts(roomy)
+    assert b.sum() > 1000
+    np.testing.assert_array_equal(a, b)
+    dcfg = fg.DevelopmentConfig(4, 1.2, 1.25, 0.85)
+    fg.develop_emulsion(tight, dcfg)
+    fg.develop_emulsion(roomy, dcfg)
+    for x, y in zip(tight.development(), roomy.development()):
+        np.testing.assert_array_equal(x, y)
+    tight.close()
+    roomy.close()
