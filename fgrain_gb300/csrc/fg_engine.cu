@@ -219,7 +219,11 @@ fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_
     em->stream = st;
     em->has64 = true;
     for (size_t i = 0; i < 3 * n; ++i) em->extent = std::max(em->extent, std::fabs(c->pos[i]));
-    for (size_t i = 0; i < 3 * n; ++i) em->max_half_dim = std::max(em->max_half_dim, c->dims[i]);
+    bool sized = true;  // no half-size is negative or NaN
+    for (size_t i = 0; i < 3 * n; ++i) {
+      em->max_half_dim = std::max(em->max_half_dim, c->dims[i]);
+      sized = sized && c->dims[i] >= 0.0;
+    }
     em->any_cubic = c->morphology ? std::any_of(c->morphology, c->morphology + n, [](int32_t m) { return m == FG_CUBIC; })
                                   : cfg->morphology == FG_CUBIC;
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
@@ -246,7 +250,9 @@ fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_
       FG_CUDA(cudaStreamSynchronize(st));
       DBuf<uint32_t> none;
       build_emulsion_tree(e, em.get(), false, em->rt, none);
-      build_emulsion_cells(e, em.get());
+      // The cells' reach is that of the largest half-size, which a negative one has no part in though the
+      // geometry (which squares or pairs it) has its magnitude: such sets stay on the walk.
+      if (sized) build_emulsion_cells(e, em.get());
     } else {
       alloc_state(em.get(), st);
     }

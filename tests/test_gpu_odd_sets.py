@@ -1,5 +1,5 @@
 """Sets and settings at the limits of what the calls accept: emulsions for whose cells there is no memory
-left."""
+left, and crystals with negative half-sizes."""
 import numpy as np
 import pytest
 
@@ -76,3 +76,30 @@ def test_an_emulsion_without_room_for_cells_keeps_the_walk(engine, kind, bytes_p
         np.testing.assert_array_equal(x, y)
     tight.close()
     roomy.close()
+
+
+@pytest.mark.parametrize("signs", [(-1, -1, -1), (-1, 1, 1)])
+@pytest.mark.parametrize("morph", [0, 2])
+@pytest.mark.parametrize("every", [1, 5])
+def test_negative_half_sizes_keep_the_walk(engine, signs, morph, every):
+    """A negative half-size has no part in the set's largest one, by which the cells search; counts and
+    development are those of the walk, which the set takes for certain without room for cells."""
+    cfg, pos, dims, quat = lattice(morph=morph)
+    dims[::every] *= np.array(signs) * (1.0, 1.2, 0.9)
+
+    def make():
+        return fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(len(pos)), engine=engine)
+
+    _, walk = smallest_budget(make)
+    em = make()
+    a = counts(walk)
+    assert a.sum() > 100
+    np.testing.assert_array_equal(counts(em), a)
+    for prox in (1.25, 0.7):
+        dcfg = fg.DevelopmentConfig(2, 1.2, prox, 0.85)
+        fg.develop_emulsion(walk, dcfg)
+        fg.develop_emulsion(em, dcfg)
+        for x, y in zip(em.development(), walk.development()):
+            np.testing.assert_array_equal(x, y)
+    walk.close()
+    em.close()
