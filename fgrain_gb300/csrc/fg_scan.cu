@@ -157,8 +157,8 @@ __device__ __forceinline__ void prep_crystal(const ScanTile& t, uint32_t s, Scan
       P.g[i] = make_float4(r0, r1, inv, d);
       P.g[3 + i] = make_float4(r0l, r1l, dl, 0.0f);
       invmax = fmaxf(invmax, fabsf(inv));
-      hx += fabsf(r0) * d;
-      hy += fabsf(r1) * d;
+      hx += fabsf(r0 * d);  // a negative half-size acts by its magnitude
+      hy += fabsf(r1 * d);
     }
     if (!(invmax < 1e30f)) {
       P.kind = K_FP64;

@@ -1,10 +1,12 @@
 """Sets and settings at the limits of what the calls accept: emulsions for whose cells there is no memory
-left, and crystals with negative half-sizes."""
+left, and crystals with negative half-sizes (whose geometry is that of their magnitudes:
+crystal.rs:140-217 pairs or squares them)."""
 import numpy as np
 import pytest
 
 import fgrain_gb300 as fg
 from fgrain_gb300 import _abi
+from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -103,3 +105,22 @@ def test_negative_half_sizes_keep_the_walk(engine, signs, morph, every):
             np.testing.assert_array_equal(x, y)
     walk.close()
     em.close()
+
+
+@pytest.mark.parametrize("signs", [(-1, 1, 1), (1, -1, 1), (1, 1, -1)])
+def test_cubes_with_a_negative_half_size_scan_as_in_the_oracle(engine, signs):
+    cfg, pos, dims, quat = lattice()
+    dims = dims * (1.0, 1.2, 0.8) * np.array(signs)
+    n = len(pos)
+    developed = (np.random.default_rng(1).random(n) < 0.3).astype(np.uint8)
+    expansion = np.full(n, 1.2)
+    em = fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(n), engine=engine)
+    em.set_development(developed, expansion)
+    cr = orc.Crystals(pos, dims, quat, np.ones(n), np.zeros(n, np.int32))
+    cr.developed[:], cr.expansion[:] = developed, expansion
+    scfg = fg.ScanConfig(40, 36, 4, 0, 0.3)
+    hits = np.asarray(fg.scan_ray_hits(em, scfg, 5)).ravel()
+    em.close()
+    ref = orc.scan(cr, cfg, scfg, 5, want_hits=True)["ray_hits"]
+    assert ref.sum() > 10_000
+    np.testing.assert_array_equal(hits, ref)
