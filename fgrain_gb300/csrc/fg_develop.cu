@@ -106,7 +106,8 @@ __global__ void k_link(CrystalsView cv, const CellGrid* __restrict__ grid, const
     }
     if (touch_hit) uf_unite(parent, static_cast<int>(s), static_cast<int>(j), err);
   };
-  if (grid) {
+  // (A negative search distance, which only the tree's boxes give a meaning, goes to the tree.)
+  if (grid && !(R < 0.0f)) {
     const float R2 = R * R;
     cells_around(*grid, make_float3(a.x, a.y, a.z), R, place[s], err, [&](uint32_t p, float d2) {
       if (d2 <= R2) test(cell_slot(*grid, p));

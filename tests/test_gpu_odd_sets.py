@@ -124,3 +124,26 @@ def test_cubes_with_a_negative_half_size_scan_as_in_the_oracle(engine, signs):
     ref = orc.scan(cr, cfg, scfg, 5, want_hits=True)["ray_hits"]
     assert ref.sum() > 10_000
     np.testing.assert_array_equal(hits, ref)
+
+
+@pytest.mark.parametrize("prox,expansion", [(-0.3, 1.2), (0.3, -1.2), (-0.3, -1.2), (0.0, 1.2)])
+def test_a_negative_touch_distance_develops_as_by_the_walk(engine, prox, expansion):
+    """The reference's query box is then inside out and meets the leaves that hold it (bvh.rs:350-402)."""
+    cfg, pos, dims, quat = lattice()
+    pos[1::2] = pos[::2][:len(pos[1::2])] + [0.25, 0.1, -0.1]  # pairs that touch
+
+    def make():
+        return fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(len(pos)), engine=engine)
+
+    _, walk = smallest_budget(make)
+    em = make()
+    dcfg = fg.DevelopmentConfig(2, expansion, prox, 0.85)
+    n = np.random.default_rng(5).integers(0, 5, len(pos)).astype(np.uint32)
+    got = []
+    for x in (em, walk):
+        x.set_latent_counts(n)
+        fg.develop_emulsion(x, dcfg)
+        got.append(x.development())
+        x.close()
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
