@@ -205,9 +205,10 @@ __device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
 //
 // Launch bounds of 8 CTAs per SM (32 registers): more columns in flight hide the round's barriers.
 // A column with its one-cell spill and the halo stages 14 x 14 cells per layer, and its list of active
-// points has an entry for each that can fit (26 a layer; with one for each of the 64 cells seven CTAs
-// ran at 23 cells, tri-x-1600's depth), so eight CTAs fit in the SM's 228 KB of shared memory for
-// depths up to 24 cells.
+// points has an entry for each that can fit (26 a layer), so eight CTAs fit in the SM's 228 KB of shared
+// memory for depths up to 24 cells.  With an entry for each of the 64 cells of a layer seven ran at 23
+// cells, tri-x-1600's depth (1600 x 1600 px of tri-x pushed two stops: 3.87 ms, now 3.69; 22 cells are
+// the same), two instead of three at 77 (36.8, now 30.0).
 //
 // FEW: with few columns in flight the latency of a round counts instead (5,600 cycles, of which 1,950
 // are the resolution by one warp).  4 CTAs per SM leave 64 registers, and the seven warps that wait
@@ -350,17 +351,15 @@ __global__ void __launch_bounds__(SYN_WARPS * 32, FEW ? 4 : 8) k_bridson(const S
     int off = s_nact;
     for (int w = 0; w < warp; ++w) off += s_wsum[w];
     const int at = off + __popc(m & ((1u << lane) - 1u));
-    // (Past the capacity only after a wait that gave up: the neighbours' points may then be too close.)
-    if (o && index_ok(at < acap, err, SITE_SYN_ACTIVE, at, blockIdx.x))
-      active[at] = syn_pos(lx + SYN_HALO, ly + SYN_HALO, lz + 2);
+    if (o) active[min(at, acap - 1)] = syn_pos(lx + SYN_HALO, ly + SYN_HALO, lz + 2);
     __syncthreads();
-    if (tid == 0) {
-      int n = s_nact;
-      for (int w = 0; w < SYN_WARPS; ++w) n += s_wsum[w];
-      s_nact = min(n, acap);
-    }
+    if (tid == 0)
+      for (int w = 0; w < SYN_WARPS; ++w) s_nact += s_wsum[w];
     __syncthreads();
   }
+  // (Past the capacity only after a wait that gave up, which has set the error: the neighbours' points may
+  // then be too close.)
+  if (tid == 0) s_nact = min(s_nact, acap);
   // An empty column starts from one random point (poisson.rs:46-57), up to 30 tries.
   if (tid == 0 && s_nact == 0 && bw > 0 && bh > 0) {
     for (int k = 0; k < SYN_K; ++k) {
