@@ -47,11 +47,12 @@ constexpr unsigned RT_BLOCK = 256;
 
 // Most global split levels for trees of up to emax elements: halving down to the per-block size,
 // plus a wide margin for uneven splits (the kernel ends with the last level that has work).
+constexpr int RT_LEVELS = 44;
 int levels_for(uint32_t emax) {
   if (emax <= static_cast<uint32_t>(RT_CTA_MAX)) return 0;
   int lv = 0;
   while ((static_cast<unsigned long long>(RT_CTA_MAX) << lv) < emax) ++lv;
-  return std::min(lv + 8, 44);
+  return std::min(lv + 8, RT_LEVELS);
 }
 
 // Work goes by chunks of consecutive positions (a tile's chunks start at its first): wpw words of 32
@@ -1563,6 +1564,8 @@ void build_emulsion_tree(fg_engine* e, const fg_emulsion* em, bool developed_onl
   t.n = developed_only ? m : n;
   std::vector<RTile> v{t};
   rtree_alloc(B, v, true, st, 1.0, n, !developed_only, walks);
+  // The developed crystals of a set that was accepted can be more uneven than the set.
+  if (developed_only) B.levels = std::max(B.levels, m > static_cast<uint32_t>(RT_CTA_MAX) ? RT_LEVELS : 0);
   // FP32 crystals without expansion: the centroids are the positions themselves.
   rtree_build(B, e->d_err, st, walks, !em->has64 && !developed_only && std::isfinite(em->max_half_dim));
   B.count = t.n;
