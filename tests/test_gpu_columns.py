@@ -1,5 +1,6 @@
 """The sampler's columns where their shared memory sets how many run at once: at the deepest films that
-eight columns of an SM take, one cell deeper, and at the deepest accepted (100 cells)."""
+eight columns of an SM take, one cell deeper, and at the deepest accepted (100 cells); and the points of a
+tile by the kernel for few columns and by the one for many."""
 import numpy as np
 import pytest
 
@@ -24,3 +25,28 @@ def test_points_are_hard_core_and_dense(engine, depth):
     vol = np.prod(size)
     target = (0.57793168 + 0.11306788 * sum(2 / s for s in size)) * vol
     assert abs(len(pos) - target) <= 0.02 * target + 4
+
+
+@pytest.mark.parametrize("stock,grain,tiles", [("t-max", 1.1, 8), ("tri-x", 2.4, 32), ("hp5", 2.0, 24)])
+def test_points_are_the_same_by_either_kernel(engine, stock, grain, tiles):
+    """A tile alone has few columns (at most 20 an SM: the kernel that draws ahead), beside the others many."""
+    import torch
+
+    params = [fg.tile_params(stock, 1 / grain, 190 + i, 170, 1.0, 0.0, 40 + i) for i in range(tiles)]
+
+    def columns(ps):
+        return sum(int(np.ceil(np.ceil(p.film_w / (p.r_min * CELL)) / 8)) * int(np.ceil(np.ceil(p.film_h / (p.r_min * CELL)) / 8))
+                   for p in ps)
+
+    line = 20 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert columns(params[:1]) <= line < columns(params)
+    both = []
+    for ps in (params[:1], params):
+        b = fg.Batch(ps, engine, use_graph=False)
+        b.set_exposure([np.full((p.height_px, p.width_px), 0.5, np.float32) for p in ps])
+        b.run()
+        b.wait()
+        both.append(b.tile_crystals(0))
+        b.close()
+    for k in both[0]:
+        np.testing.assert_array_equal(both[0][k], both[1][k])
