@@ -57,11 +57,14 @@ int levels_for(uint32_t emax) {
 
 // Work goes by chunks of consecutive positions (a tile's chunks start at its first): wpw words of 32
 // positions for each of a block's eight warps.  A warp's words follow one another, so small builds
-// take short chunks: enough blocks, and less latency in a row (309 k elements:
-// 330 us with eight words, 242 with two; 705 k with 64-bit keys: 454 and 542).
+// take short chunks: enough blocks, and less latency in a row.  The line is drawn by capacity (about 1.33 times a
+// synthesized tile's crystals).  Trees and cells of one t-max tile with two words and with eight, in ms: 260 k
+// crystals .346 and .364, 301 k .362 and .364, 342 k (455 k of capacity) .391 and .377, 382 k .418 and .384,
+// 502 k .521 and .445, 1.0 M .847 and .630; scan stages with all of them developed (64-bit keys): .681 and
+// .726, .730 and .755, .809 and .801, .844 and .810, .996 and .961, 1.715 and 1.465.  Tri-x is within 2 % of these.
 constexpr int RT_WARPS = RT_BLOCK / 32;
 constexpr int RT_WPW_LARGE = 8, RT_WPW_SMALL = 2;
-constexpr unsigned long long RT_LARGE = 600ull * 1000ull;  // elements from which chunks are long
+constexpr unsigned long long RT_LARGE = 450ull * 1000ull;  // elements from which chunks are long
 // Blocks per SM that a build's registers leave (32-bit keys: trees of a 1400 x 1400 px t-max image in
 // 6.77 ms with four, 6.33 with five, 6.51 with six; 64-bit keys: a gradient step in 4.07, 4.30, 4.36).
 constexpr int rt_blocks(bool wide) { return wide ? 4 : 5; }
