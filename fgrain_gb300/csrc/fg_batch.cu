@@ -99,6 +99,23 @@ __global__ void k_scan_tree_tiles(const BTile* bt, int ntiles, const uint32_t* d
   rt[t].n = last - first;
 }
 
+// The walk's crystal records in each tree's element order (TileDesc): rec holds all tiles' positions, then
+// their quaternions, then their half-sizes.
+__global__ void k_element_records_b(const BTile* __restrict__ bt, int ntiles, unsigned long long ncap,
+                                    const uint32_t* __restrict__ ridx, const float4* __restrict__ A,
+                                    const float4* __restrict__ Q, const float4* __restrict__ D, float4* rec,
+                                    uint32_t* err) {
+  const unsigned long long g = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
+  if (g >= ncap) return;
+  const BTile& t = bt[btile_of(bt, ntiles, g)];
+  if (g - t.cbase >= t.n) return;
+  const uint32_t s = ridx[g];
+  if (!index_ok(s < t.n, err, SITE_LEAF, s, t.n)) return;
+  rec[g] = A[t.cbase + s];
+  rec[ncap + g] = Q[t.cbase + s];
+  rec[2 * ncap + g] = D[t.cbase + s];
+}
+
 // ---- development (development.rs:59-188), batched; see fg_develop.cu for the reasoning ----
 
 // Largest max_dim of each tile's crystals (the reach of the development's proximity search):
@@ -313,7 +330,10 @@ struct fg_batch {
   bool wait_probe = false;
   bool key32 = true;       // every crystal is finite: the tree's centroids are the positions
   unsigned long long maxparts = 0;  // the largest tile's
+  std::vector<uint32_t> walk_base;  // first walk record of each tile
   DBuf<float4> A, Q, D;
+  bool walk = false;        // transport by the tree walk
+  DBuf<float4> rec;         // A, Q, D in the tree's element order, for the walk (TileDesc)
   CellBufs tcells;          // the crystals in cells, with their rank in the tree's walk order
   RTreeBufs rt;             // the reference tree of every tile: over its crystals, then its developed ones
   DBuf<RTile> rt_scan;      // the tree tiles of the scan's build (developed crystals, their expansion)
@@ -360,6 +380,23 @@ static double synth_max_half_dim(const fg_tile_params& p) {
   const double r = 0.48 * p.r_min, ar = p.tabular_aspect_ratio;
   if (p.morphology != FG_TABULAR) return r;
   return std::max(r, ar >= 0.0 ? std::max(r / ar, 0.05) : 0.05);
+}
+
+// Mean projected area of the synthesis's crystals (cells_area) at the root mean square of their radii (a
+// log-normal's, clamped).
+static double synth_mean_area(const fg_tile_params& p) {
+  const double sg = p.size_variance, m = p.mean_crystal_radius * std::exp(sg * sg);
+  const double rmax = 0.48 * p.r_min, r = m <= rmax ? m : rmax;
+  const double ht = p.morphology == FG_TABULAR ? std::max(r / p.tabular_aspect_ratio, 0.05) : r;
+  return cells_area(r, r, ht, p.morphology == FG_CUBIC);
+}
+
+// Whether the walk suits a tile's segments better than the cells; by the bulk density, so that the tiles of
+// one film agree.
+static bool tile_walks(const fg_tile_params& p, const TileDesc& t) {
+  const double n = 0.578 / (p.r_min * p.r_min * p.r_min);
+  return !(cells_hits(n * synth_mean_area(p), t.mu_t, p.film_d) <= CELLS_MAX_HITS &&
+           t.cells.reach * std::cbrt(n) <= CELLS_MAX_REACH_ALL);
 }
 
 static void derive_tile(const fg_tile_params& p, SynthTile& s, TileDesc& t, ScanTile& c, BTile& b) {
@@ -494,6 +531,14 @@ static void upload_descriptors(fg_batch* B, cudaStream_t st) {
     t.cbase = cb;
     t.nbase = nb;
     B->tcells.attach(t.cells, cb);
+    if (B->walk) {
+      t.a = B->rec.p + cb;
+      t.q = t.a + B->ncap;
+      t.d = t.q + B->ncap;
+      t.rnode = B->rt.rnode.p + B->walk_base[i];
+      t.rleaf = B->rt.rleaf.p + nb;
+      t.ridx = B->rt.ridx.p + cb;
+    }
     t.s2id = nullptr;
     t.counts = B->counts.p + cb;
     t.tile = B->exposure.p + B->exp_off[i];
@@ -557,18 +602,23 @@ static void stage_synth(fg_batch* B, cudaStream_t st, bool capturing = false) {
 // The reference tree of every tile over its crystals (in slot order), for its leaf boxes and walk
 // order, and the crystals in cells.
 static void stage_bvh(fg_batch* B, cudaStream_t st) {
-  rtree_build(B->rt, B->e->d_err, st, false, B->key32);
+  rtree_build(B->rt, B->e->d_err, st, B->walk, B->key32);
   const int nt = static_cast<int>(B->ntiles);
   FG_CUDA(cudaMemsetAsync(B->tcells.cnt.p, 0, (B->tcells.ncells + 1) * sizeof(uint32_t), st));
   launch_cells_count(B->d_td.p, nt, B->ncap, B->A.p, B->tcells.cnt.p, B->tcells.place.p, st);
   cub_scan(B, B->tcells.cnt.p, B->tcells.off.p, B->tcells.ncells + 1, st);
   launch_cells_fill(B->d_td.p, nt, B->ncap, B->A.p, B->Q.p, B->D.p, B->rt, B->tcells, B->e->d_err, st);
+  if (B->walk) {
+    k_element_records_b<<<grid_for(B->ncap, 256), 256, 0, st>>>(B->d_bt.p, nt, B->ncap, B->rt.ridx.p, B->A.p, B->Q.p,
+                                                                B->D.p, B->rec.p, B->e->d_err);
+    FG_CUDA(cudaGetLastError());
+  }
 }
 
 static void stage_transport(fg_batch* B, cudaStream_t st) {
   FG_CUDA(cudaMemsetAsync(B->counts.p, 0, B->ncap * sizeof(uint32_t), st));
   launch_transport_shape(B->d_td.p, static_cast<int>(B->ntiles), B->photons, B->porder.p, B->counter.p,
-                         B->e->d_err, B->dstats.p, B->tr_blocks, B->tr_threads, st, false);
+                         B->e->d_err, B->dstats.p, B->tr_blocks, B->tr_threads, st, B->walk);
 }
 
 // Orders photon ids by emission cell (independent of the crystals: runs with synthesis).
@@ -721,6 +771,7 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   unsigned colc[4] = {0, 0, 0, 0};
   for (uint32_t i = 0; i < n; ++i) {
     derive_tile(B->params[i], B->syn[i], B->td[i], B->sc[i], B->bt[i]);
+    B->walk = B->walk || tile_walks(B->params[i], B->td[i]);
     SynthTile& s = B->syn[i];
     s.cell_base = cb;
     s.slot_base = sb;
@@ -806,11 +857,14 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
       // The synthesis's radius clamp (emulsion.rs:162-170) for cubes; the other shapes lie in their boxes.
       t.reach = rt_reach(B->params[i].morphology == FG_CUBIC ? 0.48 * B->params[i].r_min : 0.0);
     }
-    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC, 0, true, false);
+    rtree_alloc(B->rt, rt, true, st, RT_NODE_FRAC, 0, true, B->walk);
+    if (B->walk) B->rec.alloc(std::max<unsigned long long>(3 * cap, 1), st);
     for (uint32_t i = 0; i < n; ++i) {
       FG_REQUIRE(rt[i].ebase == B->syn[i].cbase, "tree layout differs from the crystal slots");
       B->bt[i].nbase = rt[i].nbase;
       B->td[i].nnodes = rt[i].ncap;
+      B->td[i].nrec = rt[i].rcap;
+      B->walk_base.push_back(rt[i].rbase);
       B->td[i].reach = rt[i].reach;
       rs[i] = rt[i];
       rs[i].exp64 = B->exp64.p + B->syn[i].cbase;
@@ -892,8 +946,8 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   // Per crystal slot: records 48 (and 96 in the transport's cells), links and flags 36,
   // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
-  // 152 B (plus slack); transport cells 8 B; synthesis cells 4 B; parts 8 B; photon order; images.
-  return static_cast<unsigned long long>(s.ccap) * 612ull + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
+  // 152 B (plus slack); for the walk records 48 and 0.8 nodes of 80 B more; transport cells 8 B; synthesis cells 4 B; parts 8 B; photon order; images.
+  return static_cast<unsigned long long>(s.ccap) * (tile_walks(p, t) ? 612ull + 112ull : 612ull) + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          8ull * syn_parts(s) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
@@ -966,6 +1020,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
     em->has64 = false;
     em->extent = std::max(std::max(cfg->width, cfg->height), cfg->depth);
     em->max_half_dim = synth_max_half_dim(p);
+    em->mean_area = synth_mean_area(p);
     em->any_cubic = cfg->morphology == FG_CUBIC;
     em->a = std::move(A);
     em->q = std::move(Q);
@@ -1150,7 +1205,8 @@ fg_status fg_batch_wait(fg_batch* b, fg_batch_stats* stats) {
     // roots + finalize, scan-tree inputs, scan prep, two bin passes, scan, density, the two passes over the
     // transport's cells, and the two tree builds (each level's launches included, also those that
     // find no work; CUB scans not counted).
-    s.kernel_launches = 1 + 1 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + 2 * rtree_kernel_launches(b->rt, false);
+    s.kernel_launches = 1 + 1 + 1 + 1 + 2 + 1 + 6 + 1 + 1 + 2 + 1 + 1 + 2 + (b->walk ? 1 : 0) + rtree_kernel_launches(b->rt, b->walk) +
+                       rtree_kernel_launches(b->rt, false);
     b->stats = s;
     if (stats) *stats = s;
   });

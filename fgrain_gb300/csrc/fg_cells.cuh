@@ -45,6 +45,42 @@ inline void cells_reach(CellGrid& g, double m, bool cubes) {
   g.reach = static_cast<float>(m * (cubes ? 1.7320508075688773 : 1.0) * 1.002) + g.slack;
 }
 
+// Cells suit a crystal set whose crystals reach no further than the mean spacing and that fills the
+// box evenly: then a segment tests a handful of crystals per layer of cells.  One giant crystal
+// drags every segment's rows out to its reach, a set bunched in a corner puts many crystals into one
+// cell, and a centre outside the box has no cell; such sets keep the tree walk, whose cost follows
+// the boxes.  Measured with one giant among the crystals of a 140 um film (ms, cells / walk): none
+// (reach 0.4 spacings for t-max's, 0.7 for tri-x's) 0.49 / 0.92 and 0.47 / 0.72; reach 1 spacing
+// 0.92 / 0.93 and 0.63 / 0.82; 1.5 spacings 1.45 / 0.90 and 0.97 / 0.91.
+constexpr double CELLS_MAX_REACH = 1.0;      // mean spacings, of an emulsion's largest crystal
+constexpr uint32_t CELLS_MAX_COUNT = 16;     // crystals in one cell (half a crystal on average)
+// A synthesized tile's reach is that of nearly all its crystals; 200-256 px of t-max crystals thicker than wide
+// (ms, cells / walk): 2.0 spacings 2.79 / 3.40, 2.7 spacings 5.90 / 5.43, 4.0 spacings 13.3 / 10.0.
+constexpr double CELLS_MAX_REACH_ALL = 2.5;
+// A segment of many hits is visited again for every twelve, so its cost grows with the square of its hits
+// (cells_hits: H), the walk's with the hits.  Transport of 200 x 200 px films, 10 to 60 um deep, mean free path
+// 20 um to none (cells / walk): tri-x H 9 .57, 13 .71 - .86, 18 .82 - .98, 20 .99, 23 1.03 - 1.15, 27 1.14 - 1.32,
+// 40 1.76; hp5 H 19 .69, 23 .88; t-max H 8 .58.
+constexpr double CELLS_MAX_HITS = 20.0;
+// In evenly spaced sets it also grows with the crystals' reach.  60 x 60 um, reach in spacings and where cells
+// and walk are even: .42 H 18 - 20, .6 H 16, .72 H 14, .9 H 11 - 14, .99 H 9 (H 16: 1.2 - 1.6; H 78: 4 - 6).
+constexpr double CELLS_MAX_HITS_REACH = 10.0;  // hits times spacings of reach, emulsions
+
+// Hits that a segment expects to absorb, weighted by hits (E[h^2] / E[h]): per_um of them per um of a free
+// path of mean 1 / mu_t that ends at the film's depth at the latest.
+inline double cells_hits(double per_um, double mu_t, double depth) {
+  const double x = mu_t * depth;
+  if (!(x > 1e-3)) return per_um * depth;
+  const double e = std::exp(-x);
+  return per_um * 2.0 * (1.0 - e * (1.0 + x)) / (mu_t * (1.0 - e));
+}
+
+// Mean projected area (um^2) of a crystal of half-sizes a, b, c: a quarter of a box's surface (Cauchy); for the
+// ellipsoid shapes pi times the mean product of two.
+inline double cells_area(double a, double b, double c, bool cube) {
+  return (a * b + b * c + c * a) * (cube ? 2.0 : 1.0471975511965976);
+}
+
 // Cell edges in units of the mean crystal spacing a = (volume / crystals)^(1/3).  Rows run along x,
 // so x cells are short (a row's span is cut close to the segment at no cost); rows are wide and
 // layers high enough that a row holds a few crystals near the segment.  Transport of 800 x 800 px

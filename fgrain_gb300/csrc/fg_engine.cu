@@ -224,6 +224,10 @@ fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_
       em->max_half_dim = std::max(em->max_half_dim, c->dims[i]);
       sized = sized && c->dims[i] >= 0.0;
     }
+    for (size_t i = 0; i < n; ++i) {
+      const double* d = c->dims + 3 * i;
+      em->mean_area += cells_area(d[0], d[1], d[2], (c->morphology ? c->morphology[i] : cfg->morphology) == FG_CUBIC) / n;
+    }
     em->any_cubic = c->morphology ? std::any_of(c->morphology, c->morphology + n, [](int32_t m) { return m == FG_CUBIC; })
                                   : cfg->morphology == FG_CUBIC;
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));

@@ -187,7 +187,7 @@ struct fg_emulsion {
   // radius queries).
   fg::RTreeBufs rt;
   // The crystals in cells for the transport and the touch queries; grid.x.n is 0 for sets that stay
-  // on the tree walk (cells_suit).
+  // on the tree walk (build_emulsion_cells).
   fg::CellBufs cells;
   fg::CellGrid grid{};
   fg::DBuf<fg::CellGrid> grid_dev;  // grid, in device memory (device code reads its axes as vectors)
@@ -200,6 +200,7 @@ struct fg_emulsion {
   bool has64 = false;
   double extent = 0.0;             // largest coordinate magnitude (sets the box padding)
   double max_half_dim = 0.0;       // largest crystal half-dimension (sets the walks' reach)
+  double mean_area = 0.0;          // mean projected area of a crystal, um^2 (cells_area)
   bool any_cubic = true;           // some crystal is a cube (only a cube reaches out of its box)
   std::vector<uint32_t> h_s2id;    // host copy of sorted_to_id (empty: identity)
 

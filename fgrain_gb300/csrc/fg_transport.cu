@@ -517,24 +517,17 @@ void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long
   FG_CUDA(cudaGetLastError());
 }
 
-// Cells suit a crystal set whose crystals reach no further than the mean spacing and that fills the
-// box evenly: then a segment tests a handful of crystals per layer of cells.  One giant crystal
-// drags every segment's rows out to its reach, a set bunched in a corner puts many crystals into one
-// cell, and a centre outside the box has no cell; such sets keep the tree walk, whose cost follows
-// the boxes.  Measured with one giant among the crystals of a 140 um film (ms, cells / walk): none
-// (reach 0.4 spacings for t-max's, 0.7 for tri-x's) 0.49 / 0.92 and 0.47 / 0.72; reach 1 spacing
-// 0.92 / 0.93 and 0.63 / 0.82; 1.5 spacings 1.45 / 0.90 and 0.97 / 0.91.
-constexpr double CELLS_MAX_REACH = 1.0;   // mean spacings
-constexpr uint32_t CELLS_MAX_COUNT = 16;  // crystals in one cell (half a crystal on average)
-
 static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   cudaStream_t st = e->stream;
   const uint32_t n = em->n;
   CellGrid g{};
   if (!n || !cells_layout(em->cfg.width, em->cfg.height, em->cfg.depth, n, g)) return;
   cells_reach(g, em->max_half_dim, em->any_cubic);
-  const double spacing = std::cbrt(em->cfg.width * em->cfg.height * em->cfg.depth / n);
-  if (!(g.reach <= CELLS_MAX_REACH * spacing)) return;
+  const double vol = em->cfg.width * em->cfg.height * em->cfg.depth;
+  const fg_optics& o = em->cfg.optics;
+  const double reach = g.reach / std::cbrt(vol / n);
+  const double hits = cells_hits(n / vol * em->mean_area, o.absorption_coeff + o.scattering_coeff, em->cfg.depth);
+  if (!(reach <= CELLS_MAX_REACH && hits <= CELLS_MAX_HITS && hits * reach <= CELLS_MAX_HITS_REACH)) return;
   em->cells.alloc(n, cells_of(g), st);
   em->cells.attach(g, 0);
   TileDesc t{};
