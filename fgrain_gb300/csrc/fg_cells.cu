@@ -42,6 +42,34 @@ __global__ void k_cells_count(const TileDesc* __restrict__ tiles, int ntiles, un
   if (unfit && (k == limit || !in)) *unfit = 1u;
 }
 
+// The density about a crystal over the mean one, times crystals: the sum of n_b^2 / v_b over blocks of about 80
+// crystals (4 mean spacings in x and y, 5 in z), n_b the block's crystals and v_b its cells.
+constexpr uint32_t UNEVEN_X = 20, UNEVEN_Y = 4, UNEVEN_Z = 2;
+__global__ void k_cells_uneven(CellAxis x, CellAxis y, CellAxis z, const uint32_t* __restrict__ off, double* out) {
+  const uint32_t bx = (x.n + UNEVEN_X - 1) / UNEVEN_X, by = (y.n + UNEVEN_Y - 1) / UNEVEN_Y;
+  const unsigned long long blocks = 1ull * bx * by * ((z.n + UNEVEN_Z - 1) / UNEVEN_Z);
+  double sum = 0.0;
+  for (unsigned long long b = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; b < blocks;
+       b += 1ull * gridDim.x * blockDim.x) {
+    const uint32_t x0 = static_cast<uint32_t>(b % bx) * UNEVEN_X, y0 = static_cast<uint32_t>(b / bx % by) * UNEVEN_Y;
+    const uint32_t z0 = static_cast<uint32_t>(b / bx / by) * UNEVEN_Z;
+    const uint32_t x1 = min(x0 + UNEVEN_X, x.n), y1 = min(y0 + UNEVEN_Y, y.n), z1 = min(z0 + UNEVEN_Z, z.n);
+    uint32_t n = 0;
+    for (uint32_t j = y0; j < y1; ++j)
+      for (uint32_t k = z0; k < z1; ++k) {
+        const uint32_t* row = off + (j * z.n + k) * x.n;
+        n += row[x1] - row[x0];
+      }
+    sum += static_cast<double>(n) * n / ((x1 - x0) * (y1 - y0) * (z1 - z0));
+  }
+  if (sum != 0.0) atomicAdd(out, sum);
+}
+
+void launch_cells_uneven(const CellGrid& g, double* out, cudaStream_t st) {
+  k_cells_uneven<<<256, 128, 0, st>>>(g.x, g.y, g.z, g.off, out);
+  FG_CUDA(cudaGetLastError());
+}
+
 __global__ void k_cells_fill(const TileDesc* __restrict__ tiles, int ntiles, unsigned long long ncap,
                              const float4* __restrict__ A, const float4* __restrict__ Q, const float4* __restrict__ D,
                              const uint32_t* __restrict__ off, uint32_t* __restrict__ place,

@@ -62,9 +62,11 @@ constexpr double CELLS_MAX_REACH_ALL = 2.5;
 // 20 um to none (cells / walk): tri-x H 9 .57, 13 .71 - .86, 18 .82 - .98, 20 .99, 23 1.03 - 1.15, 27 1.14 - 1.32,
 // 40 1.76; hp5 H 19 .69, 23 .88; t-max H 8 .58.
 constexpr double CELLS_MAX_HITS = 20.0;
-// In evenly spaced sets it also grows with the crystals' reach.  60 x 60 um, reach in spacings and where cells
-// and walk are even: .42 H 18 - 20, .6 H 16, .72 H 14, .9 H 11 - 14, .99 H 9 (H 16: 1.2 - 1.6; H 78: 4 - 6).
-constexpr double CELLS_MAX_HITS_REACH = 10.0;  // hits times spacings of reach, emulsions
+// In uploaded sets it also grows with the crystals' reach.  Lattices, reach in spacings and where cells
+// and walk are even: .42 H 18 - 20, .6 H 16, .72 H 14, .9 H 11 - 14, .99 H 9 (H 16: 1.2 - 1.6; H 78: 4 - 6).  Uneven
+// sets, by the density about a crystal (H, reach in its spacings, cells / walk): 6.5 .45 .57 - .63; 9.9 .52 .67 - .87;
+// 12 .56 .74 - .96; 11 .72 1.04 - 1.27; 14 .77 1.02 - 1.35; 16 .61 1.2 - 1.5; 18 .85 1.8 - 2.3.
+constexpr double CELLS_MAX_HITS_REACH = 7.5;  // hits times spacings of reach, emulsions
 
 // Hits that a segment expects to absorb, weighted by hits (E[h^2] / E[h]): per_um of them per um of a free
 // path of mean 1 / mu_t that ends at the film's depth at the latest.

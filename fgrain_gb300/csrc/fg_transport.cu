@@ -523,11 +523,14 @@ static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   CellGrid g{};
   if (!n || !cells_layout(em->cfg.width, em->cfg.height, em->cfg.depth, n, g)) return;
   cells_reach(g, em->max_half_dim, em->any_cubic);
-  const double vol = em->cfg.width * em->cfg.height * em->cfg.depth;
+  const double vol = em->cfg.width * em->cfg.height * em->cfg.depth, density = n / vol;
   const fg_optics& o = em->cfg.optics;
-  const double reach = g.reach / std::cbrt(vol / n);
-  const double hits = cells_hits(n / vol * em->mean_area, o.absorption_coeff + o.scattering_coeff, em->cfg.depth);
-  if (!(reach <= CELLS_MAX_REACH && hits <= CELLS_MAX_HITS && hits * reach <= CELLS_MAX_HITS_REACH)) return;
+  const double hits = cells_hits(em->mean_area, o.absorption_coeff + o.scattering_coeff, em->cfg.depth);
+  auto suits = [&](double per_um3) {
+    const double reach = g.reach * std::cbrt(per_um3), h = hits * per_um3;
+    return h <= CELLS_MAX_HITS && h * reach <= CELLS_MAX_HITS_REACH;
+  };
+  if (!(g.reach * std::cbrt(density) <= CELLS_MAX_REACH && suits(density))) return;
   em->cells.alloc(n, cells_of(g), st);
   em->cells.attach(g, 0);
   TileDesc t{};
@@ -536,17 +539,24 @@ static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   t.nnodes = static_cast<uint32_t>(em->rt.N);
   DBuf<TileDesc> td(1, st);
   DBuf<uint32_t> unfit(1, st);
+  DBuf<double> uneven(1, st);
   FG_CUDA(cudaMemcpyAsync(td.p, &t, sizeof(TileDesc), cudaMemcpyHostToDevice, st));
   FG_CUDA(cudaMemsetAsync(unfit.p, 0, sizeof(uint32_t), st));
+  FG_CUDA(cudaMemsetAsync(uneven.p, 0, sizeof(double), st));
   FG_CUDA(cudaMemsetAsync(em->cells.cnt.p, 0, (em->cells.ncells + 1) * sizeof(uint32_t), st));
   launch_cells_count(td.p, 1, n, em->a.p, em->cells.cnt.p, em->cells.place.p, st, CELLS_MAX_COUNT, unfit.p);
   exclusive_scan_u32(em->cells.cnt.p, em->cells.off.p, em->cells.ncells + 1, st);
+  launch_cells_uneven(g, uneven.p, st);
   launch_cells_fill(td.p, 1, n, em->a.p, em->q.p, em->d.p, em->rt, em->cells, e->d_err, st);
   uint32_t c = 0;
+  double dense = 0.0;
   FG_CUDA(cudaMemcpyAsync(&c, unfit.p, sizeof(c), cudaMemcpyDeviceToHost, st));
+  FG_CUDA(cudaMemcpyAsync(&dense, uneven.p, sizeof(dense), cudaMemcpyDeviceToHost, st));
   FG_CUDA(cudaStreamSynchronize(st));
   em->cells.cnt.release();
-  if (c) {
+  // Again with the density about a crystal.
+  dense *= static_cast<double>(em->cells.ncells) / n / vol;
+  if (c || !suits(std::fmax(dense, density))) {
     em->cells = CellBufs{};
     return;
   }

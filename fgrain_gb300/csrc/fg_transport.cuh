@@ -394,6 +394,7 @@ struct RTreeBufs;
 struct CellBufs;
 void launch_cells_count(const TileDesc* tiles, int ntiles, unsigned long long ncap, const float4* A, uint32_t* cnt,
                         uint32_t* place, cudaStream_t st, uint32_t limit = 0, uint32_t* unfit = nullptr);
+void launch_cells_uneven(const CellGrid& g, double* out, cudaStream_t st);
 void launch_cells_fill(const TileDesc* tiles, int ntiles, unsigned long long ncap, const float4* A, const float4* Q,
                        const float4* D, const RTreeBufs& tree, const CellBufs& c, uint32_t* err, cudaStream_t st);
 

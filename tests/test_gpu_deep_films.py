@@ -1,6 +1,6 @@
 """Films so deep, or crystals so large, that a segment absorbs many hits: transport by the tree walk, in
-batches and emulsions, against the oracle's exposure of the same crystals (transport.rs:48-188), and beside
-tiles of ordinary depth.
+batches and emulsions, against the oracle's exposure of the same crystals (transport.rs:48-188), beside
+tiles of ordinary depth, and where the crystals lie unevenly.
 
 Tolerance: FP32 decides few hits and draws differently from the oracle: 99 % of the crystals have its count
 exactly, as the batch's pipeline test asks, and the photons in all agree to 1e-3."""
@@ -93,3 +93,26 @@ def test_emulsions_of_many_hits_expose_as_batches(engine):
     fg.expose_emulsion(em, exposures([p])[0], ecfg, 6)
     np.testing.assert_array_equal(em.latent_counts(), c["counts"])
     em.close()
+
+
+@pytest.mark.parametrize("share,area", [(0.0, 1.0), (0.5, 0.2), (0.5, 0.1), (0.8, 0.15)])
+def test_uneven_sets_match_the_oracle(engine, share, area):
+    """A share of the crystals in a corner of the film: cells while the corner is not too dense, then the walk."""
+    rng = np.random.default_rng(3)
+    size, n = np.array([30.0, 28.0, 12.0]), 5000
+    pos = rng.random((n, 3)) * size
+    pos[:int(n * share), :2] *= np.sqrt(area)
+    quat = rng.normal(size=(n, 4))
+    quat /= np.linalg.norm(quat, axis=1, keepdims=True)
+    dims = np.full((n, 3), 0.4)
+    cfg = fg.EmulsionConfig(tuple(size), 1.0, 0.5, 0.2, fg.Morphology(0), 1.0, fg.GelatinOptics(), 1.0)
+    tile = rng.uniform(0.2, 1.0, (24, 26)).astype(np.float32)
+    ecfg = fg.ExposureConfig(20.0, 0.12, 1.3, 48)
+    cr = orc.Crystals(pos, dims, quat, np.ones(n), np.zeros(n, np.int32))
+    orc.expose(cr, cfg, tile, ecfg, 7)
+    em = fg.VirtualEmulsionLayer.from_crystals(cfg, pos, dims, quat, np.ones(n), engine=engine)
+    fg.expose_emulsion(em, tile, ecfg, 7)
+    got, ref = em.latent_counts().astype(np.int64), cr.latent.astype(np.int64)
+    em.close()
+    assert ref.sum() > 1000 and (got == ref).mean() > 0.99
+    assert abs(got.sum() - ref.sum()) <= 1e-3 * ref.sum()
