@@ -502,7 +502,9 @@ void launch_transport_shape(const TileDesc* tiles_dev, int ntiles, unsigned long
     FG_CUDA(cudaGetDevice(&dev));
     FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     few = total <= 2ull * 32 * 32 * sms;
-    const unsigned long long room = (few ? 24ull : 32ull) * sms;  // warps of the launch bounds
+    // Warps of the launch bounds, or of the launch shape where that has fewer: each of those takes more lanes.
+    const unsigned long long room = std::max<unsigned long long>(
+        std::min<unsigned long long>((few ? 24ull : 32ull) * sms, 1ull * blocks * threads / 32), 1);
     lanes = std::min<unsigned long long>((total + room - 1) / room, 32);
   }
   const unsigned long long warps = (total + lanes - 1) / lanes;
