@@ -194,9 +194,10 @@ fg_status fg_scan_signal(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg*
     const Taps tp = otf_taps(otf_sigma);
     const size_t np = static_cast<size_t>(cfg->width_px) * cfg->height_px;
     DBuf<float> sig, T(std::max<size_t>(np, 1), st), H(std::max<size_t>(np, 1), st), S(std::max<size_t>(np, 1), st);
+    IdCopy<float> by_id;
     if (sigma_per_crystal) {
       sig.alloc(std::max<uint32_t>(em->n, 1), st);
-      by_id_to_device(em, sigma_per_crystal, sig.p, st);
+      by_id.to_slots(em, sigma_per_crystal, sig.p, st);
     }
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
     scan_T(e, em, *cfg, seed, sigma_per_crystal ? sig.p : nullptr, T.p);
@@ -225,9 +226,10 @@ fg_status fg_scan_backward(fg_engine* e, const fg_emulsion* em, const fg_scan_cf
     const uint32_t w = cfg->width_px, h = cfg->height_px;
     const size_t np = static_cast<size_t>(w) * h;
     DBuf<float> sig, T(std::max<size_t>(np, 1), st), Gd(std::max<size_t>(np, 1), st), W(std::max<size_t>(np, 1), st);
+    IdCopy<float> by_id;
     if (sigma_per_crystal) {
       sig.alloc(std::max<uint32_t>(em->n, 1), st);
-      by_id_to_device(em, sigma_per_crystal, sig.p, st);
+      by_id.to_slots(em, sigma_per_crystal, sig.p, st);
     }
     if (np) FG_CUDA(cudaMemcpyAsync(Gd.p, dL_dsignal, np * sizeof(float), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
@@ -260,8 +262,10 @@ fg_status fg_scan_backward(fg_engine* e, const fg_emulsion* em, const fg_scan_cf
     double hs[2] = {0.0, 0.0};
     FG_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
     FG_CUDA(cudaEventRecord(e->timer.ev[1], st));
-    if (crystals) device_to_by_id(em, gf.p, dL_dsigma, st);
+    IdCopy<float> gc;
+    if (crystals) gc.from_slots(em, gf.p, dL_dsigma, st);
     FG_CUDA(cudaStreamSynchronize(st));
+    gc.finish(em, dL_dsigma);
     if (dL_dexposure) *dL_dexposure = hs[0];
     if (dL_dotf_sigma) *dL_dotf_sigma = exposure * hs[1];
     e->timings.scan_ms = elapsed(e->timer.ev[0], e->timer.ev[1]);

@@ -54,6 +54,7 @@ inline void cells_reach(CellGrid& g, double m, bool cubes) {
 // 0.92 / 0.93 and 0.63 / 0.82; 1.5 spacings 1.45 / 0.90 and 0.97 / 0.91.
 constexpr double CELLS_MAX_REACH = 1.0;      // mean spacings, of an emulsion's largest crystal
 constexpr uint32_t CELLS_MAX_COUNT = 16;     // crystals in one cell (half a crystal on average)
+constexpr uint32_t CELLS_UNEVEN_MIN = 512;   // crystals from which the set's unevenness is looked at
 // A synthesized tile's reach is that of nearly all its crystals; 200-256 px of t-max crystals thicker than wide
 // (ms, cells / walk): 2.0 spacings 2.79 / 3.40, 2.7 spacings 5.90 / 5.43, 4.0 spacings 13.3 / 10.0.
 constexpr double CELLS_MAX_REACH_ALL = 2.5;

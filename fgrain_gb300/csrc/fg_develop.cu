@@ -237,7 +237,7 @@ void develop(fg_engine* e, fg_emulsion* em, const fg_dev_cfg& cfg, fg_dev_report
   FG_CUDA(cudaStreamSynchronize(st));
   double max_base;
   std::memcpy(&max_base, &mbits, sizeof(double));
-  k_link<<<G, 256, 0, st>>>(em->view(), em->grid_dev.p, em->cells.place.p, em->rt.rnode.p, static_cast<uint32_t>(em->rt.R), em->rt.rleaf.p,
+  k_link<<<G, 256, 0, st>>>(em->view(), em->fit.p ? &em->fit.p->tile.cells : nullptr, em->cells.place.p, em->rt.rnode.p, static_cast<uint32_t>(em->rt.R), em->rt.rleaf.p,
                             static_cast<uint32_t>(em->rt.N), em->rt.ridx.p, n, em->developed.p, cfg.filament_expansion,
                             cfg.clumping_proximity_factor, max_base, parent.p, dc.p, e->d_err);
   k_roots<<<G, 256, 0, st>>>(n, em->developed.p, parent.p, s2id, size.p, minid.p, e->d_err);

@@ -218,16 +218,20 @@ fg_status fg_emulsion_upload(fg_engine* e, const fg_emulsion_cfg* cfg, const fg_
     em->n = static_cast<uint32_t>(n);
     em->stream = st;
     em->has64 = true;
-    for (size_t i = 0; i < 3 * n; ++i) em->extent = std::max(em->extent, std::fabs(c->pos[i]));
     bool sized = true;  // no half-size is negative or NaN
-    for (size_t i = 0; i < 3 * n; ++i) {
-      em->max_half_dim = std::max(em->max_half_dim, c->dims[i]);
-      sized = sized && c->dims[i] >= 0.0;
-    }
+    double ext[3] = {0.0, 0.0, 0.0}, half[3] = {0.0, 0.0, 0.0}, area[2] = {0.0, 0.0};
     for (size_t i = 0; i < n; ++i) {
-      const double* d = c->dims + 3 * i;
-      em->mean_area += cells_area(d[0], d[1], d[2], (c->morphology ? c->morphology[i] : cfg->morphology) == FG_CUBIC) / n;
+      const double *p = c->pos + 3 * i, *d = c->dims + 3 * i;
+      for (int k = 0; k < 3; ++k) {
+        ext[k] = std::max(ext[k], std::fabs(p[k]));
+        half[k] = std::max(half[k], d[k]);
+        sized &= d[k] >= 0.0;
+      }
+      area[(c->morphology ? c->morphology[i] : cfg->morphology) == FG_CUBIC] += cells_area(d[0], d[1], d[2], false);
     }
+    em->extent = std::max(std::max(ext[0], ext[1]), ext[2]);
+    em->max_half_dim = std::max(std::max(half[0], half[1]), half[2]);
+    em->mean_area = n ? (area[0] + area[1] * cells_area(1.0, 0.0, 1.0, true) / cells_area(1.0, 0.0, 1.0, false)) / n : 0.0;
     em->any_cubic = c->morphology ? std::any_of(c->morphology, c->morphology + n, [](int32_t m) { return m == FG_CUBIC; })
                                   : cfg->morphology == FG_CUBIC;
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
@@ -325,15 +329,18 @@ fg_status fg_emulsion_download(fg_engine* e, const fg_emulsion* em, fg_crystals_
 fg_status fg_emulsion_get_counts(fg_engine* e, const fg_emulsion* em, uint32_t* counts) {
   return guard(e, [&] {
     FG_REQUIRE(em && counts, "null argument");
-    device_to_by_id(em, em->counts.p, counts, e->stream);
+    IdCopy<uint32_t> c;
+    c.from_slots(em, em->counts.p, counts, e->stream);
     FG_CUDA(cudaStreamSynchronize(e->stream));
+    c.finish(em, counts);
   });
 }
 
 fg_status fg_emulsion_set_counts(fg_engine* e, fg_emulsion* em, const uint32_t* counts) {
   return guard(e, [&] {
     FG_REQUIRE(em && counts, "null argument");
-    by_id_to_device(em, counts, em->counts.p, e->stream);
+    IdCopy<uint32_t> c;
+    c.to_slots(em, counts, em->counts.p, e->stream);
     FG_CUDA(cudaStreamSynchronize(e->stream));
   });
 }
@@ -343,10 +350,14 @@ fg_status fg_emulsion_get_development(fg_engine* e, const fg_emulsion* em, uint8
   return guard(e, [&] {
     FG_REQUIRE(em, "null emulsion");
     const uint32_t n = em->n;
-    if (developed) device_to_by_id(em, em->developed.p, developed, e->stream);
-    if (expansion) device_to_by_id(em, em->exp64.p, expansion, e->stream);
+    IdCopy<uint8_t> dv;
+    IdCopy<double> ex;
+    if (developed) dv.from_slots(em, em->developed.p, developed, e->stream);
+    if (expansion) ex.from_slots(em, em->exp64.p, expansion, e->stream);
     if (clump && n) FG_CUDA(cudaMemcpyAsync(clump, em->clump.p, n * sizeof(int64_t), cudaMemcpyDeviceToHost, e->stream));
     FG_CUDA(cudaStreamSynchronize(e->stream));
+    dv.finish(em, developed);
+    ex.finish(em, expansion);
   });
 }
 
@@ -360,9 +371,11 @@ fg_status fg_emulsion_set_development(fg_engine* e, fg_emulsion* em, const uint8
   return guard(e, [&] {
     FG_REQUIRE(em && developed && expansion, "null argument");
     const uint32_t n = em->n;
+    IdCopy<uint8_t> dv;
+    IdCopy<double> ex;
     if (n) {
-      by_id_to_device(em, developed, em->developed.p, e->stream);
-      by_id_to_device(em, expansion, em->exp64.p, e->stream);
+      dv.to_slots(em, developed, em->developed.p, e->stream);
+      ex.to_slots(em, expansion, em->exp64.p, e->stream);
       k_to_float<<<grid_for(n, 256), 256, 0, e->stream>>>(em->exp64.p, n, em->exp32.p);
       FG_CUDA(cudaGetLastError());
       FG_CUDA(cudaMemsetAsync(em->clump.p, 0xff, n * sizeof(int64_t), e->stream));
@@ -420,6 +433,7 @@ static void run_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg* cfg
   const uint32_t g = static_cast<uint32_t>(std::lround(std::sqrt(static_cast<double>(spp))));
   const size_t a = std::max<uint32_t>(g * g, 1);
   DBuf<float> d_out, d_sig;
+  IdCopy<float> by_id;
   DBuf<uint8_t> d_img;
   DBuf<uint16_t> d_hits;
   ScanOut so;
@@ -428,7 +442,7 @@ static void run_scan(fg_engine* e, const fg_emulsion* em, const fg_scan_cfg* cfg
   if (ray_hits) { d_hits.alloc(npx * a, st); so.ray_hits = d_hits.p; }
   if (sigma) {
     d_sig.alloc(std::max<uint32_t>(em->n, 1), st);
-    by_id_to_device(em, sigma, d_sig.p, st);
+    by_id.to_slots(em, sigma, d_sig.p, st);
   }
   FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
   scan(e, em, *cfg, seed, sigma ? d_sig.p : nullptr, so);

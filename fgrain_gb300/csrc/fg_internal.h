@@ -13,6 +13,7 @@
 #include "fg_cells.cuh"
 #include "fg_device.cuh"
 #include "fg_rtree.cuh"
+#include "fg_transport.cuh"
 
 namespace fg {
 
@@ -149,6 +150,13 @@ struct RTreeBufs {
   DBuf<uint32_t> rank;            // optional: place of each element slot in the reference walk's order
 };
 
+// An emulsion's cells as they are built: the descriptor, and what is found of the set.
+struct CellFit {
+  TileDesc tile;
+  double uneven;   // launch_cells_uneven
+  uint32_t unfit;  // k_cells_count
+};
+
 // fg_cells.cu: the crystals of a batch's tiles (or one emulsion) in cells (CellGrid).
 struct CellBufs {
   unsigned long long ncells = 0;
@@ -190,7 +198,7 @@ struct fg_emulsion {
   // on the tree walk (build_emulsion_cells).
   fg::CellBufs cells;
   fg::CellGrid grid{};
-  fg::DBuf<fg::CellGrid> grid_dev;  // grid, in device memory (device code reads its axes as vectors)
+  fg::DBuf<fg::CellFit> fit;        // its descriptor in device memory (device code reads the axes as vectors)
   // Mutable per-crystal state (Morton order).
   fg::DBuf<uint32_t> counts;
   fg::DBuf<uint8_t> developed;
@@ -271,8 +279,10 @@ struct ScanOut {
   uint16_t* ray_hits = nullptr;
 };
 // Host arrays in crystal-id order to and from device arrays in slot order.  The permutation runs on
-// the device (a random gather of millions of values costs the host milliseconds); where its scratch
-// cannot be allocated it runs on the host.
+// the device (a random gather of millions of values costs the host milliseconds; latent counts of 338 k
+// crystals read in 50 us, 206 on the host); for few crystals, where its launch and scratch cost more (64: 20 us
+// and 14, 9,000: 21 and 20), and where that scratch cannot be allocated, it runs on the host.
+constexpr uint32_t PERMUTE_MIN = 8192;
 template <class T>
 __global__ void k_permute(const T* __restrict__ in, const uint32_t* __restrict__ idx, uint32_t n, T* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -280,6 +290,7 @@ __global__ void k_permute(const T* __restrict__ in, const uint32_t* __restrict__
 }
 template <class T>
 bool permute_scratch(DBuf<T>& b, size_t n, cudaStream_t st) {
+  if (n < PERMUTE_MIN) return false;
   try {
     b.alloc(n, st);
   } catch (const Error& x) {
@@ -289,43 +300,49 @@ bool permute_scratch(DBuf<T>& b, size_t n, cudaStream_t st) {
   }
   return true;
 }
+// One such array on its way; it holds host memory of the copy, so it outlives the caller's synchronisation.
 template <class T>
-void by_id_to_device(const fg_emulsion* em, const T* by_id, T* slots, cudaStream_t st) {
-  const uint32_t n = em->n;
-  if (!n) return;
-  DBuf<T> tmp;
-  if (em->h_s2id.empty()) {
-    FG_CUDA(cudaMemcpyAsync(slots, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
-  } else if (permute_scratch(tmp, n, st)) {
-    FG_CUDA(cudaMemcpyAsync(tmp.p, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
-    k_permute<<<(n + 255) / 256, 256, 0, st>>>(tmp.p, em->sorted_to_id.p, n, slots);
-    FG_CUDA(cudaGetLastError());
-  } else {
-    std::vector<T> v(n);
-    for (uint32_t s = 0; s < n; ++s) v[s] = by_id[em->h_s2id[s]];
-    FG_CUDA(cudaMemcpyAsync(slots, v.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaStreamSynchronize(st));
+class IdCopy {
+  std::vector<T> host_;
+
+ public:
+  // Enqueues by_id (crystal-id order) to slots (slot order).
+  void to_slots(const fg_emulsion* em, const T* by_id, T* slots, cudaStream_t st) {
+    const uint32_t n = em->n;
+    if (!n) return;
+    DBuf<T> tmp;
+    if (em->h_s2id.empty()) {
+      FG_CUDA(cudaMemcpyAsync(slots, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
+    } else if (permute_scratch(tmp, n, st)) {
+      FG_CUDA(cudaMemcpyAsync(tmp.p, by_id, n * sizeof(T), cudaMemcpyHostToDevice, st));
+      k_permute<<<(n + 255) / 256, 256, 0, st>>>(tmp.p, em->sorted_to_id.p, n, slots);
+      FG_CUDA(cudaGetLastError());
+    } else {
+      host_.resize(n);
+      for (uint32_t s = 0; s < n; ++s) host_[s] = by_id[em->h_s2id[s]];
+      FG_CUDA(cudaMemcpyAsync(slots, host_.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
+    }
   }
-}
-// Enqueues the copy; the caller synchronises before it reads by_id.
-template <class T>
-void device_to_by_id(const fg_emulsion* em, const T* slots, T* by_id, cudaStream_t st) {
-  const uint32_t n = em->n;
-  if (!n) return;
-  DBuf<T> tmp;
-  if (em->h_s2id.empty()) {
-    FG_CUDA(cudaMemcpyAsync(by_id, slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
-  } else if (permute_scratch(tmp, n, st)) {
-    k_permute<<<(n + 255) / 256, 256, 0, st>>>(slots, em->id_to_sorted.p, n, tmp.p);
-    FG_CUDA(cudaGetLastError());
-    FG_CUDA(cudaMemcpyAsync(by_id, tmp.p, n * sizeof(T), cudaMemcpyDeviceToHost, st));
-  } else {
-    std::vector<T> v(n);
-    FG_CUDA(cudaMemcpyAsync(v.data(), slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
-    FG_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t s = 0; s < n; ++s) by_id[em->h_s2id[s]] = v[s];
+  // Enqueues slots to by_id; finish, after the stream was synchronised, puts the last of it in place.
+  void from_slots(const fg_emulsion* em, const T* slots, T* by_id, cudaStream_t st) {
+    const uint32_t n = em->n;
+    if (!n) return;
+    DBuf<T> tmp;
+    if (em->h_s2id.empty()) {
+      FG_CUDA(cudaMemcpyAsync(by_id, slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+    } else if (permute_scratch(tmp, n, st)) {
+      k_permute<<<(n + 255) / 256, 256, 0, st>>>(slots, em->id_to_sorted.p, n, tmp.p);
+      FG_CUDA(cudaGetLastError());
+      FG_CUDA(cudaMemcpyAsync(by_id, tmp.p, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+    } else {
+      host_.resize(n);
+      FG_CUDA(cudaMemcpyAsync(host_.data(), slots, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+    }
   }
-}
+  void finish(const fg_emulsion* em, T* by_id) const {
+    for (uint32_t s = 0; s < host_.size(); ++s) by_id[em->h_s2id[s]] = host_[s];
+  }
+};
 
 // fg_image.cu: the separable 3-tap clamp-to-edge filter (two passes through tmp), in the
 // reference's FP32 operation order, the second pass scaled by `scale`.

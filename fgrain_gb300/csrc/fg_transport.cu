@@ -535,36 +535,30 @@ static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   if (!(g.reach * std::cbrt(density) <= CELLS_MAX_REACH && suits(density))) return;
   em->cells.alloc(n, cells_of(g), st);
   em->cells.attach(g, 0);
-  TileDesc t{};
-  t.cells = g;
-  t.n = n;
-  t.nnodes = static_cast<uint32_t>(em->rt.N);
-  DBuf<TileDesc> td(1, st);
-  DBuf<uint32_t> unfit(1, st);
-  DBuf<double> uneven(1, st);
-  FG_CUDA(cudaMemcpyAsync(td.p, &t, sizeof(TileDesc), cudaMemcpyHostToDevice, st));
-  FG_CUDA(cudaMemsetAsync(unfit.p, 0, sizeof(uint32_t), st));
-  FG_CUDA(cudaMemsetAsync(uneven.p, 0, sizeof(double), st));
+  // Descriptor and findings in one buffer: a copy there, a copy back.
+  em->fit.alloc(1, st);
+  CellFit f{};
+  f.tile.cells = g;
+  f.tile.n = n;
+  f.tile.nnodes = static_cast<uint32_t>(em->rt.N);
+  FG_CUDA(cudaMemcpyAsync(em->fit.p, &f, sizeof(f), cudaMemcpyHostToDevice, st));
+  const TileDesc* td = &em->fit.p->tile;
   FG_CUDA(cudaMemsetAsync(em->cells.cnt.p, 0, (em->cells.ncells + 1) * sizeof(uint32_t), st));
-  launch_cells_count(td.p, 1, n, em->a.p, em->cells.cnt.p, em->cells.place.p, st, CELLS_MAX_COUNT, unfit.p);
+  launch_cells_count(td, 1, n, em->a.p, em->cells.cnt.p, em->cells.place.p, st, CELLS_MAX_COUNT, &em->fit.p->unfit);
   exclusive_scan_u32(em->cells.cnt.p, em->cells.off.p, em->cells.ncells + 1, st);
-  launch_cells_uneven(g, uneven.p, st);
-  launch_cells_fill(td.p, 1, n, em->a.p, em->q.p, em->d.p, em->rt, em->cells, e->d_err, st);
-  uint32_t c = 0;
-  double dense = 0.0;
-  FG_CUDA(cudaMemcpyAsync(&c, unfit.p, sizeof(c), cudaMemcpyDeviceToHost, st));
-  FG_CUDA(cudaMemcpyAsync(&dense, uneven.p, sizeof(dense), cudaMemcpyDeviceToHost, st));
+  if (n >= CELLS_UNEVEN_MIN) launch_cells_uneven(g, &em->fit.p->uneven, st);
+  launch_cells_fill(td, 1, n, em->a.p, em->q.p, em->d.p, em->rt, em->cells, e->d_err, st);
+  FG_CUDA(cudaMemcpyAsync(&f, em->fit.p, sizeof(f), cudaMemcpyDeviceToHost, st));
   FG_CUDA(cudaStreamSynchronize(st));
   em->cells.cnt.release();
   // Again with the density about a crystal.
-  dense *= static_cast<double>(em->cells.ncells) / n / vol;
-  if (c || !suits(std::fmax(dense, density))) {
+  const double dense = f.uneven * static_cast<double>(em->cells.ncells) / n / vol;
+  if (f.unfit || !suits(std::fmax(dense, density))) {
     em->cells = CellBufs{};
+    em->fit.release();
     return;
   }
-  em->grid_dev.alloc(1, st);
   em->grid = g;
-  FG_CUDA(cudaMemcpyAsync(em->grid_dev.p, &em->grid, sizeof(CellGrid), cudaMemcpyHostToDevice, st));
 }
 
 // The cells take about 110 bytes a crystal over the tree's; where those cannot be had the set keeps the walk.
@@ -576,7 +570,7 @@ void build_emulsion_cells(fg_engine* e, fg_emulsion* em) {
     if (x.st != FG_ERR_OOM) throw;
     (void)cudaGetLastError();
     em->cells = CellBufs{};
-    em->grid_dev.release();
+    em->fit.release();
     em->grid = CellGrid{};
   }
 }
