@@ -804,7 +804,7 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   }
   for (int c = 0; c < 4; ++c) B->cols[c] = colc[c];
   FG_REQUIRE(cap < 0x7fffffffull, "batch too large: more than 2^31 crystal slots");
-  FG_REQUIRE(bridson_smem(B->gdmax) <= 220 * 1024, "emulsion too deep for the synthesis column");
+  FG_REQUIRE(bridson_smem(B->gdmax) <= BRIDSON_SMEM_MAX, "emulsion too deep for the synthesis column");
   B->ncells = cb;
   B->nparts = sb;
   B->ncap = cap;
@@ -993,7 +993,7 @@ fg_status fg_emulsion_synthesize(fg_engine* e, const fg_emulsion_cfg* cfg, uint6
       cols[c] = ((s.nbx + 1 - (c & 1)) / 2) * ((s.nby + 1 - (c >> 1)) / 2);
     }
     const int gdmax = static_cast<int>(s.gd);
-    FG_REQUIRE(bridson_smem(gdmax) <= 220 * 1024, "emulsion too deep for the synthesis column");
+    FG_REQUIRE(bridson_smem(gdmax) <= BRIDSON_SMEM_MAX, "emulsion too deep for the synthesis column");
     FG_CUDA(cudaEventRecord(e->timer.ev[0], st));
     DBuf<SynthTile> d_syn(1, st);
     FG_CUDA(cudaMemcpyAsync(d_syn.p, &s, sizeof(SynthTile), cudaMemcpyHostToDevice, st));

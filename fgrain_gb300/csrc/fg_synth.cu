@@ -189,7 +189,7 @@ __device__ __forceinline__ float3 syn_draw(int iter, int slot, int lane, uint32_
 
 // An entry of the active list: the cell's region coordinates (SYN_R < 16; a region that fits in
 // shared memory has at most 256 layers).
-static_assert(SYN_R <= 16 && bridson_smem(253) > 220 * 1024, "4 + 4 + 8 bits hold a position");
+static_assert(SYN_R <= 16 && bridson_smem(253) > BRIDSON_SMEM_MAX, "4 + 4 + 8 bits hold a position");
 __device__ __forceinline__ uint16_t syn_pos(int rx, int ry, int rz) {
   return static_cast<uint16_t>(rx | ry << 4 | rz << 8);
 }
@@ -829,7 +829,9 @@ void launch_bridson(const SynthTile* tiles, int ntiles, const unsigned cols[4], 
   const size_t smem = bridson_smem(gdmax);
   FG_CUDA(cudaMemsetAsync(done, 0, total * sizeof(uint32_t), st));
   const auto kernel = total <= SYN_FEW * static_cast<unsigned>(sms) ? k_bridson<true> : k_bridson<false>;
-  FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  // The most that any launch asks for, whatever this one does: the attribute is the process's, and another
+  // thread's launch may come between.
+  FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(BRIDSON_SMEM_MAX)));
   const uint4 cb = make_uint4(0u, cols[0], cols[0] + cols[1], cols[0] + cols[1] + cols[2]);
   kernel<<<total, SYN_WARPS * 32, smem, st>>>(tiles, ntiles, cb, nz, cells, npts, done, err,
                                                   wait_limit ? wait_limit : (1u << 22), probe);

@@ -52,6 +52,7 @@ constexpr size_t bridson_smem(int gd) {
   return static_cast<size_t>(SYN_R) * (SYN_R + 1) * (gd + 4) * sizeof(uint32_t) +
          static_cast<size_t>(syn_active_cap(gd)) * sizeof(uint16_t);
 }
+constexpr size_t BRIDSON_SMEM_MAX = 220 * 1024;
 
 __host__ __device__ inline double bridson_density(double W, double H, double D, double r) {
   return (0.57793168 + 0.11306788 * r * (2.0 / W + 2.0 / H + 2.0 / D)) / (r * r * r);
