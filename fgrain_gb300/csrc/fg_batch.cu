@@ -1,8 +1,8 @@
 // Batched tile pipeline: many exposure tiles (uneven sizes, stocks, push, seeds) rendered to
 // negative density in one sequence of launches:
 //   synthesis (column Bridson, 4 colour classes) -> thinning -> compaction in brick order -> the
-//   reference tree (fg_rtree.cuh), its leaf boxes and ranks -> the crystals in cells (fg_cells.cuh) ->
-//   persistent transport over all tiles' photons -> development -> the reference tree over the
+//   reference tree (fg_rtree.cuh), its leaf boxes and ranks -> the crystals in cells (fg_cells.cuh; and
+//   walk records where a tile's segments meet too many crystals) -> persistent transport over all tiles' photons -> development -> the reference tree over the
 //   developed crystals -> bins -> binned scan.
 // Every kernel covers all tiles at once (per-tile descriptors in HBM, tile found by binary search
 // on a prefix of work items), every buffer is allocated when the plan is made, and nothing waits

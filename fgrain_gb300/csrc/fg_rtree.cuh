@@ -16,8 +16,9 @@
 // order (right subtree first, leaf crystals in index order), which sets how the packet energy is
 // shared between the crystals along a segment.
 //
-// Walk records, for the sets whose crystals cells do not suit and for recorded segments (production
-// transport takes only the leaf boxes and the ranks from the tree: fg_cells.cuh).  Node ids are tile-local; the root is id 1, children come in pairs (l, l + 1) =
+// Walk records, for the sets whose crystals cells do not suit (otherwise production transport takes only
+// the leaf boxes and the ranks from the tree: fg_cells.cuh; recorded segments walk the nodes themselves, in
+// FP64).  Node ids are tile-local; the root is id 1, children come in pairs (l, l + 1) =
 // (left, right).  The walks run over four-wide records: the record of an internal node at odd depth
 // (the root's is record 0, any other's is record l / 2 of its children's pair l) holds that node's
 // grandchildren, a leaf child taking one slot itself, in the order the reference's walk visits
