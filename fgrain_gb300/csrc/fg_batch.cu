@@ -1,9 +1,9 @@
 // Batched tile pipeline: many exposure tiles (uneven sizes, stocks, push, seeds) rendered to
 // negative density in one sequence of launches:
 //   synthesis (column Bridson, 4 colour classes) -> thinning -> compaction in brick order -> the
-//   reference tree (fg_rtree.cuh), its leaf boxes and ranks -> the crystals in cells (fg_cells.cuh; and
-//   walk records where a tile's segments meet too many crystals) -> persistent transport over all tiles' photons -> development -> the reference tree over the
-//   developed crystals -> bins -> binned scan.
+//   reference tree (fg_rtree.cuh), its leaf boxes and ranks -> the crystals in cells (fg_cells.cuh; the
+//   walk's records too where a tile's segments meet too many crystals) -> persistent transport over all
+//   tiles' photons -> development -> the reference tree over the developed crystals -> bins -> binned scan.
 // Every kernel covers all tiles at once (per-tile descriptors in HBM, tile found by binary search
 // on a prefix of work items), every buffer is allocated when the plan is made, and nothing waits
 // on the host, so the sequence is captured once into a CUDA graph and replayed.  An autotuner
@@ -946,8 +946,10 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   // Per crystal slot: records 48 (and 96 in the transport's cells), links and flags 36,
   // expansion 8, scan prep 160, bin entries 32, tree elements 92 (order, node of, two copies of
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
-  // 152 B (plus slack); for the walk records 48 and 0.8 nodes of 80 B more; transport cells 8 B; synthesis cells 4 B; parts 8 B; photon order; images.
-  return static_cast<unsigned long long>(s.ccap) * (tile_walks(p, t) ? 612ull + 112ull : 612ull) + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
+  // 152 B (plus slack); for the walk records 48 and 0.8 nodes of 80 B more; transport cells 8 B;
+  // synthesis cells 4 B; parts 8 B; photon order; images.
+  const unsigned long long slot = 612ull + (tile_walks(p, t) ? 112ull : 0ull);
+  return s.ccap * slot + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          8ull * syn_parts(s) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;
 }
