@@ -391,11 +391,10 @@ static double synth_mean_area(const fg_tile_params& p) {
   return cells_area(r, r, ht, p.morphology == FG_CUBIC);
 }
 
-// Whether the walk suits a tile's segments better than the cells; by the bulk density, so that the tiles of
-// one film agree.
-static bool tile_walks(const fg_tile_params& p, const TileDesc& t) {
+// Whether the walk suits a tile's segments, of `length` um at most, better than the cells.
+static bool tile_walks(const fg_tile_params& p, const TileDesc& t, double length) {
   const double n = 0.578 / (p.r_min * p.r_min * p.r_min);
-  return !(cells_hits(n * synth_mean_area(p), t.mu_t, p.film_d) <= CELLS_MAX_HITS &&
+  return !(cells_hits(n * synth_mean_area(p), t.mu_t, length) <= CELLS_MAX_HITS &&
            t.cells.reach * std::cbrt(n) <= CELLS_MAX_REACH_ALL);
 }
 
@@ -771,7 +770,8 @@ static void plan(fg_batch* B, const fg_batch_options* opt) {
   unsigned colc[4] = {0, 0, 0, 0};
   for (uint32_t i = 0; i < n; ++i) {
     derive_tile(B->params[i], B->syn[i], B->td[i], B->sc[i], B->bt[i]);
-    B->walk = B->walk || tile_walks(B->params[i], B->td[i]);
+    const fg_tile_params& p = B->params[i];
+    B->walk = B->walk || tile_walks(p, B->td[i], std::min(p.film_d, std::min(p.film_w, p.film_h)));
     SynthTile& s = B->syn[i];
     s.cell_base = cb;
     s.slot_base = sb;
@@ -948,7 +948,8 @@ unsigned long long tile_footprint(const fg_tile_params& p, unsigned long long* s
   // three 8-byte keys, flags, prefix sums, ranks, final order, leaf and rank of) and 0.8 nodes of
   // 152 B (plus slack); for the walk records 48 and 0.8 nodes of 80 B more; transport cells 8 B;
   // synthesis cells 4 B; parts 8 B; photon order; images.
-  const unsigned long long slot = 612ull + (tile_walks(p, t) ? 112ull : 0ull);
+  // (By the depth alone: a narrow tile walks beside wide ones.)
+  const unsigned long long slot = 612ull + (tile_walks(p, t, p.film_d) ? 112ull : 0ull);
   return s.ccap * slot + cells_of(t.cells) * 8ull + static_cast<unsigned long long>(s.gw) * s.gh * s.gd * 4ull +
          8ull * syn_parts(s) + static_cast<unsigned long long>(t.P) * 4ull +
          (1ull << (2 * bits)) * 12ull + px * 8ull + 4096ull;

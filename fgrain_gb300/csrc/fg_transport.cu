@@ -527,10 +527,12 @@ static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   cells_reach(g, em->max_half_dim, em->any_cubic);
   const double vol = em->cfg.width * em->cfg.height * em->cfg.depth, density = n / vol;
   const fg_optics& o = em->cfg.optics;
-  const double hits = cells_hits(em->mean_area, o.absorption_coeff + o.scattering_coeff, em->cfg.depth);
+  const double length = std::fmin(em->cfg.depth, std::fmin(em->cfg.width, em->cfg.height));
+  const double hits = cells_hits(em->mean_area, o.absorption_coeff + o.scattering_coeff, length);
   auto suits = [&](double per_um3) {
     const double reach = g.reach * std::cbrt(per_um3), h = hits * per_um3;
-    return h <= CELLS_MAX_HITS && h * reach <= CELLS_MAX_HITS_REACH;
+    // A synthesized set is a tile's: evenly dense, its reach that of nearly all its crystals.
+    return h <= CELLS_MAX_HITS && (!em->has64 || h * reach <= CELLS_MAX_HITS_REACH);
   };
   if (!(g.reach * std::cbrt(density) <= CELLS_MAX_REACH && suits(density))) return;
   em->cells.alloc(n, cells_of(g), st);
@@ -546,7 +548,7 @@ static void make_emulsion_cells(fg_engine* e, fg_emulsion* em) {
   FG_CUDA(cudaMemsetAsync(em->cells.cnt.p, 0, (em->cells.ncells + 1) * sizeof(uint32_t), st));
   launch_cells_count(td, 1, n, em->a.p, em->cells.cnt.p, em->cells.place.p, st, CELLS_MAX_COUNT, &em->fit.p->unfit);
   exclusive_scan_u32(em->cells.cnt.p, em->cells.off.p, em->cells.ncells + 1, st);
-  if (n >= CELLS_UNEVEN_MIN) launch_cells_uneven(g, &em->fit.p->uneven, st);
+  if (em->has64 && n >= CELLS_UNEVEN_MIN) launch_cells_uneven(g, &em->fit.p->uneven, st);
   launch_cells_fill(td, 1, n, em->a.p, em->q.p, em->d.p, em->rt, em->cells, e->d_err, st);
   FG_CUDA(cudaMemcpyAsync(&f, em->fit.p, sizeof(f), cudaMemcpyDeviceToHost, st));
   FG_CUDA(cudaStreamSynchronize(st));

@@ -40,13 +40,14 @@ def run(engine, params, use_graph=False):
     return out
 
 
-# Scattering 0 and 45 um: about 30 hits a segment.  Aspect 0.1: crystals ten times as long as wide.
-CASES = [("tri-x", 45.0, None, 0.0), ("tri-x", 60.0, None, None), ("t-max", None, 0.1, None)]
+# Scattering 0 and 45 um: about 30 hits a segment, in tiles of 54 x 50 um (a narrower one's photons leave by its
+# sides).  Aspect 0.1: crystals ten times as long as wide.
+CASES = [("tri-x", 45.0, None, 0.0), ("tri-x", 60.0, None, 0.02), ("t-max", None, 0.1, None)]
 
 
 @pytest.mark.parametrize("stock,depth,aspect,scatter", CASES)
 def test_batch_counts_match_the_oracle(engine, stock, depth, aspect, scatter):
-    p = tile(stock, 60, 52, 5, depth, aspect, scatter)
+    p = tile(stock, 130, 120, 5, depth, aspect, scatter)
     crystals, density = run(engine, [p])
     c = crystals[0]
     cr = orc.Crystals(c["pos"], c["dims"], c["quat"], c["sensitivity"], c["morphology"])
@@ -68,7 +69,7 @@ def test_batch_counts_match_the_oracle(engine, stock, depth, aspect, scatter):
 def test_a_deep_tile_changes_no_other(engine, stock, depth, aspect, scatter):
     """One deep tile takes its whole batch to the walk; an ordinary tile's crystals, counts and density are those
     it has alone, through the cells; plain launches and the captured graph agree."""
-    small, deep = tile("tri-x", 64, 48, 9), tile(stock, 60, 52, 5, depth, aspect, scatter)
+    small, deep = tile("tri-x", 64, 48, 9), tile(stock, 130, 120, 5, depth, aspect, scatter)
     (c0,), (d0,) = run(engine, [small])
     for graph in (False, True):
         crystals, density = run(engine, [small, deep], graph)
@@ -79,7 +80,7 @@ def test_a_deep_tile_changes_no_other(engine, stock, depth, aspect, scatter):
 
 def test_emulsions_of_many_hits_expose_as_batches(engine):
     """An uploaded set of the crystals of a deep tile gets the tile's counts."""
-    p = tile("tri-x", 60, 52, 5, 45.0, None, 0.0)
+    p = tile("tri-x", 130, 120, 5, 45.0, None, 0.0)
     c = run(engine, [p])[0][0]
     cfg = fg.EmulsionConfig((p.film_w, p.film_h, p.film_d), p.r_min, p.mean_crystal_radius, p.size_variance,
                             fg.Morphology(p.morphology), p.tabular_aspect_ratio,
