@@ -62,9 +62,11 @@ int levels_for(uint32_t emax) {
 // crystals .346 and .364, 301 k .362 and .364, 342 k (455 k of capacity) .391 and .377, 382 k .418 and .384,
 // 502 k .521 and .445, 1.0 M .847 and .630; scan stages with all of them developed (64-bit keys): .681 and
 // .726, .730 and .755, .809 and .801, .844 and .810, .996 and .961, 1.715 and 1.465.  Tri-x is within 2 % of these.
+// Several tiles have fewer levels of the same elements, and the two are even a little later: 4 to 36 tiles of
+// 360 k crystals in all .23 - .30 and .25 - .33, 415 k (550 k of capacity) .36 and .34, 500 k .38 and .35.
 constexpr int RT_WARPS = RT_BLOCK / 32;
 constexpr int RT_WPW_LARGE = 8, RT_WPW_SMALL = 2;
-constexpr unsigned long long RT_LARGE = 450ull * 1000ull;  // elements from which chunks are long
+constexpr unsigned long long RT_LARGE = 520ull * 1000ull;  // elements from which chunks are long
 // Blocks per SM that a build's registers leave (32-bit keys: trees of a 1400 x 1400 px t-max image in
 // 6.77 ms with four, 6.33 with five, 6.51 with six; 64-bit keys: a gradient step in 4.07, 4.30, 4.36).
 constexpr int rt_blocks(bool wide) { return wide ? 4 : 5; }

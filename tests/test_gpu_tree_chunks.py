@@ -69,7 +69,7 @@ def test_a_leaf_of_many_equal_centroids(engine, equal):
     em.close()
 
 
-@pytest.mark.parametrize("n", [449_999, 450_000, 640_000])
+@pytest.mark.parametrize("n", [519_999, 520_000, 640_000])
 def test_uploaded_sets_about_the_longer_chunks(engine, n):
     rng = np.random.default_rng(n)
     pos = rng.random((n, 3)) * [300.0, 260.0, 12.0]
@@ -80,10 +80,10 @@ def test_uploaded_sets_about_the_longer_chunks(engine, n):
     em.close()
 
 
-@pytest.mark.parametrize("w,h", [(240.0, 270.0), (300.0, 340.0)])
+@pytest.mark.parametrize("w,h", [(240.0, 310.0), (300.0, 340.0)])
 def test_synthesized_sets_about_the_longer_chunks(engine, w, h):
     em = fg.VirtualEmulsionLayer.synthesize(fg.EmulsionConfig.preset("t-max", w, h), 9, engine)
-    assert (len(em) > 450_000) == (w * h > 90_000.0)
+    assert (len(em) > 520_000) == (w * h > 90_000.0)
     c = em.crystals()
     check(em, orc.Crystals(c["pos"], c["dims"], c["quat"], c["sensitivity"], c["morphology"]))
     em.close()
